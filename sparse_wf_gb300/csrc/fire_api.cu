@@ -15,6 +15,7 @@
 
 #include "fire_gemm.cuh"
 #include "fire_kernels.cuh"
+#include "fire_sliced.cuh"
 
 using namespace fire;
 
@@ -160,18 +161,62 @@ void tc_offsets(const fire_problem* p, size_t float_bytes, size_t* off) {
   off[TC_COUNT] = o;
 }
 
-// Byte offset of the FP64 prepared weights (the refinement pass's) in an FP32 / mixed prepared buffer: after the
-// float slots and, in the mixed path, the BF16 tensor-core weights.
-size_t prep64_offset(const fire_problem* p) {
-  int64_t off[PR_COUNT + 1];
-  prep_offsets(p, off);
-  size_t end = (size_t)off[PR_COUNT] * 4;
-  if (p->precision == FIRE_PREC_MIXED) {
-    size_t to[TC_COUNT + 1];
-    tc_offsets(p, end, to);
-    end = to[TC_COUNT];
+// Weights of the sliced contractions (fire_sliced.cuh), cut when the parameters are prepared: of the value rows in the
+// FP32 and mixed paths (SL_PAIR), of every layer in FP64 (SL_F64).
+enum SlSlot {
+  SLW_GLU, SLW_DENSE, SLW_OUT, SLW_UPD1, SLW_UPD2, SLW_ORB_UP, SLW_ORB_DN, SLW_V, SLW_JMLP1, SLW_JMLP2, SLW_ENV_UP,
+  SLW_ENV_DN, SLW_READ1, SLW_READ2, SLW_COUNT
+};
+struct SlSrc {
+  int slot, K, N, batch;
+};
+SlSrc sl_src(int k, const fire_problem* p) {
+  const int DN = NDET * p->n_el, K8 = NENV_ORB * p->n_nuc;
+  switch (k) {
+    case SLW_GLU: return {FIRE_P_EI_GLU_W, F, 2 * F, 1};
+    case SLW_DENSE: return {FIRE_P_EI_DENSE_W, F, F, 1};
+    case SLW_OUT: return {FIRE_P_EI_OUT_W, F, 5 * F, 1};
+    case SLW_UPD1: return {PR_UPD1_W_S0, F, F, 1};
+    case SLW_UPD2: return {FIRE_P_UPD2_W, F, F, 1};
+    case SLW_ORB_UP: return {PR_ORB_UP_W_S1, F, DN, 1};
+    case SLW_ORB_DN: return {PR_ORB_DN_W_S1, F, DN, 1};
+    case SLW_V: return {PR_V_W_S1, F, F, 1};
+    case SLW_JMLP1: return {PR_JMLP1_W_S1, F, F, 1};
+    case SLW_JMLP2: return {FIRE_P_JMLP2_W, F, F, 1};
+    case SLW_ENV_UP: return {PR_ENV_UP_PI, K8, p->n_el, NDET};
+    case SLW_ENV_DN: return {PR_ENV_DN_PI, K8, p->n_el, NDET};
+    case SLW_READ1: return {FIRE_P_ATT_OUT1_W, 2 * F, F, 1};
+    default: return {FIRE_P_ATT_OUT2_W, F, F, 1};
   }
-  return (end + 255) / 256 * 256;
+}
+// byte offsets of the sliced weights behind the `float_bytes` of the slots of T (and, in the mixed path, the tensor-core
+// weights); off[SLW_COUNT] = end.  The attention readout is sliced in FP64 only.
+template <typename T>
+void sl_offsets(const fire_problem* p, size_t* off) {
+  int64_t po[PR_COUNT + 1];
+  prep_offsets(p, po);
+  size_t o = (size_t)po[PR_COUNT] * sizeof(T);
+  if (sizeof(T) == 4 && p->precision == FIRE_PREC_MIXED) {
+    size_t to[TC_COUNT + 1];
+    tc_offsets(p, o, to);
+    o = to[TC_COUNT];
+  }
+  for (int k = 0; k < SLW_COUNT; ++k) {
+    o = (o + 255) / 256 * 256;
+    off[k] = o;
+    const SlSrc q = sl_src(k, p);
+    if (sizeof(T) == 8) o += q.batch * sl_w_bytes<SL_F64>(q.K, q.N);
+    else if (k < SLW_READ1) o += q.batch * sl_w_bytes<SL_PAIR>(q.K, q.N);
+  }
+  off[SLW_COUNT] = (o + 255) / 256 * 256;
+}
+
+// Byte offset of the FP64 prepared weights (the refinement pass's) in an FP32 / mixed prepared buffer: after the
+// float slots, in the mixed path the tensor-core weights, and the sliced weights.
+size_t prep64_offset(const fire_problem* p) {
+  size_t so[SLW_COUNT + 1];
+  sl_offsets<float>(p, so);
+  return so[SLW_COUNT];
 }
 
 bool valid(const fire_problem* p) {
@@ -191,8 +236,26 @@ struct Plan {
   size_t JAx, JAj, JAl, Xo2, Jo2, Lo2, JMx, JMl, JMj, rn, lpn, plr, tile_mask, aD1, aD2, ajsq;
   // double
   size_t ld, sd, dlap, cond, gjw, enn;
+  size_t sl;  // slices of a contraction's rows: shares gjw (never in use at the same time)
   size_t total;
 };
+
+// Scratch of the largest sliced contraction of a chunk (fire_sliced.cuh).
+template <int KIND>
+size_t sl_plan_bytes(const fire_problem* p, size_t W, bool fl) {
+  const long n = p->n_el, nu = p->n_up, nd = n - nu;
+  const int K8 = NENV_ORB * p->n_nuc;
+  const bool all = KIND == SL_F64 && fl;  // FP64: the derivative rows too
+  const long nv = all ? 5 : 1, jr = 3L * (long)W * (n + p->cap_pairs);
+  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+  size_t b = up(sl_scratch_bytes<KIND>((long)W * n * nv, F));
+  b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * nu, F)) + up(sl_scratch_bytes<KIND>((long)W * nd, F)));
+  b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * nu * nv, K8, NDET)) +
+                      up(sl_scratch_bytes<KIND>((long)W * nd * nv, K8, NDET)));
+  if (KIND == SL_F64) b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * (fl ? 3 * n : 1), 2 * F)));
+  if (all) b = std::max(b, up(sl_scratch_bytes<KIND>(jr, F)));
+  return b;
+}
 
 Plan make_plan(const fire_problem* p, int Wc, bool fl) {
   Plan P;
@@ -285,7 +348,11 @@ Plan make_plan(const fire_problem* p, int Wc, bool fl) {
     take(P.JMl, W * 2, es);
     take(P.JMj, W * 3 * n * 2, es);
   }
-  take(P.gjw, 2 * W * NDET * n * n, 8);  // two working copies per matrix for the Gauss-Jordan / LU kernel
+  // two working copies per matrix for the Gauss-Jordan / LU kernel; the sliced contractions before and after it cut
+  // their rows into the same bytes
+  const size_t slb = es == 8 ? sl_plan_bytes<SL_F64>(p, W, fl) : sl_plan_bytes<SL_PAIR>(p, W, fl);
+  take(P.gjw, std::max(2 * W * NDET * n * n * 8, slb), 1);
+  P.sl = P.gjw;
   take(P.enn, 1, 8);
   take(P.tile_mask, (fl ? 3 * Pc : G) / 128 + 2, 4);
   take(P.rn, G * 3, es);
@@ -472,6 +539,16 @@ fire_status prepare_impl(cudaStream_t s, const fire_problem* p, const float* blo
   g_nlaunch++;
   k_scalars<T><<<1, 32, 0, s>>>(blob + boff[FIRE_P_CUTOFF_PARAM], blob + boff[FIRE_P_LOG_BIAS], p->cutoff,
                                 out + off[PR_SCALARS]);
+  size_t so[SLW_COUNT + 1];
+  sl_offsets<T>(p, so);
+  unsigned char* base = reinterpret_cast<unsigned char*>(prepared);
+  for (int k = 0; k < SLW_COUNT; ++k) {
+    const SlSrc q = sl_src(k, p);
+    if (sizeof(T) == 4 && k >= SLW_READ1) continue;
+    g_nlaunch++;
+    if constexpr (sizeof(T) == 4) sl_prepare_f32(out + off[q.slot], q.K, q.N, q.batch, base + so[k], s);
+    else sl_prepare_f64(out + off[q.slot], q.K, q.N, q.batch, base + so[k], s);
+  }
   return launch_status(__func__);
 }
 
@@ -508,9 +585,8 @@ struct Ctx {
   // energy, log|psi| and the low-rank state); the Metropolis blocks' proposals, which only compare log|psi| values,
   // take the plain contraction
   bool comp = true;
-  // the refinement pass's FP64 value path: its envelope value rows by the double-FP32 compensated contraction
-  bool env_df = false;
   TcWeights tcw[TC_COUNT];
+  const unsigned char* slw[SLW_COUNT];  // sliced weights
   template <typename U>
   U* buf(size_t off) const {
     return reinterpret_cast<U*>(ws + off);
@@ -554,8 +630,49 @@ GemmP<T> gp0() {
   return g;
 }
 
+// The sliced contraction of one weight (sl_id) with one set of rows.
+template <typename T>
+SlCall<T> sl_call(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
+  SlCall<T> q;
+  std::memset(&q, 0, sizeof(q));
+  q.nseg = 1;
+  q.batch = 1;
+  q.p[0] = g;
+  q.w[0] = c.slw[sl_id];
+  return q;
+}
+// ... of both spins' rows (one per electron), each with its own weight; mode and strides are the caller's.
+template <typename T>
+SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, int sl_up, int sl_dn, int rows_per_el) {
+  SlCall<T> q = sl_call(c, g, sl_up);
+  const int nu = c.p->n_up, nd = c.p->n_el - nu;
+  q.nseg = 2;
+  q.p[1] = g;
+  q.w[1] = c.slw[sl_dn];
+  q.p[0].M = c.Wc * nu * rows_per_el;
+  q.p[1].M = c.Wc * nd * rows_per_el;
+  q.p[0].n_el = q.p[1].n_el = c.p->n_el;
+  q.ns[0] = nu;
+  q.ns[1] = nd;
+  q.soff[1] = nu;
+  q.spin[1] = 1;
+  return q;
+}
+template <typename T>
+cudaError_t sl_gemm(const Ctx<T>& c, int mode, const SlCall<T>& q) {
+  Prof pr(sizeof(T) == 4 ? "gemm_comp" : "gemm", c.s);
+  g_nlaunch += 2;
+  unsigned char* scratch = c.template buf<unsigned char>(c.P.sl);
+  if constexpr (sizeof(T) == 4) return sl_gemm_f32(mode, q, scratch, c.status, c.s);
+  else return sl_gemm_f64(mode, q, scratch, c.status, c.s);
+}
+
+// tc_id: tensor-core weight of the mixed path's derivative rows; sl_id: sliced weight of the FP64 path
 template <typename T, int MODE>
-cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1) {
+cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
+  if constexpr (sizeof(T) == 8) {
+    if (sl_id >= 0) return sl_gemm(c, MODE, sl_call(c, g, sl_id));
+  }
   // profile stages: "gemm_tc" the tensor-core contractions, "gemm" the CUDA-core ones
   const bool tc = sizeof(T) == 4 && c.mixed && tc_id >= 0;
   Prof pr(tc ? "gemm_tc" : "gemm", c.s);
@@ -569,23 +686,15 @@ cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1) {
   return launch_gemm<T, MODE>(g, c.s);
 }
 
-// compensated value contraction (FP32 and mixed paths): low parts into C_lo / read from env_lo, row stride ld_lo
-template <int MODE>
-cudaError_t gemm_comp(const Ctx<float>& c, const GemmP<float>& g, float* C_lo, const float* env_lo, long ld_lo) {
-  Prof pr("gemm_comp", c.s);
-  g_nlaunch++;
-  return launch_gemm_comp<MODE>(g, C_lo, env_lo, ld_lo, c.s);
-}
-
-// Value-plane contraction of a dense layer (EPI_PLAIN or EPI_SILU_X): compensated in the FP32 and mixed paths.
+// Value-plane contraction of a dense layer (EPI_PLAIN or EPI_SILU_X): hi + lo accuracy in the FP32 and mixed paths.
 template <typename T, int MODE>
-cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g) {
+cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
   if constexpr (sizeof(T) == 4) {
     static_assert(MODE == EPI_PLAIN || MODE == EPI_SILU_X, "value_gemm: plain or SiLU layers");
-    if (!c.comp) return gemm<T, MODE>(c, g);
-    return gemm_comp<MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU>(c, g, nullptr, nullptr, 0);
-  } else {
+    if (c.comp) return sl_gemm(c, MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU, sl_call(c, g, sl_id));
     return gemm<T, MODE>(c, g);
+  } else {
+    return gemm<T, MODE>(c, g, -1, sl_id);
   }
 }
 
@@ -615,18 +724,18 @@ cudaError_t stage_neighbors(Ctx<T>& c, bool fl) {
 // the tensor cores take the derivative rows (the value rows they also compute are not stored) and the
 // CUDA cores the value rows, read with a stride of NV rows: the value plane stays FP32.
 template <typename T>
-cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id) {
-  if (NV == 1) return value_gemm<T, EPI_PLAIN>(c, g);
+cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id, int sl_id) {
+  if (NV == 1) return value_gemm<T, EPI_PLAIN>(c, g, sl_id);
   GemmP<T> gv = g;  // the value rows (every NV-th row), compensated in the FP32 and mixed paths
   gv.lda = g.lda * NV;
   gv.ldc = g.ldc * NV;
   gv.M = g.M / NV;
   gv.bias_period = g.bias ? 1 : 0;
   if (!c.mixed) {
-    // FP32 (and FP64): all rows by the CUDA-core contraction; in FP32 the value rows once more, compensated
-    cudaError_t e = gemm<T, EPI_PLAIN>(c, g);
+    // FP32: all rows by the CUDA-core contraction, the value rows once more at hi + lo accuracy; FP64: all rows sliced
+    cudaError_t e = gemm<T, EPI_PLAIN>(c, g, -1, sl_id);
     if (e != cudaSuccess || sizeof(T) == 8) return e;
-    return value_gemm<T, EPI_PLAIN>(c, gv);
+    return value_gemm<T, EPI_PLAIN>(c, gv, sl_id);
   }
   GemmP<T> gt = g;
   gt.bias = nullptr;
@@ -634,7 +743,7 @@ cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id) {
   gt.row_skip = NV;
   cudaError_t e = gemm<T, EPI_PLAIN>(c, gt, tc_id);
   if (e != cudaSuccess) return e;
-  return value_gemm<T, EPI_PLAIN>(c, gv);
+  return value_gemm<T, EPI_PLAIN>(c, gv, sl_id);
 }
 
 template <typename T, int NT>
@@ -653,21 +762,21 @@ cudaError_t stage_embedding(Ctx<T>& c) {
   GemmP<T> g = gp0<T>();
   g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_GLU_W]; g.ldb = 2 * F; g.C = Z1; g.ldc = 2 * F;
   g.M = G * NV; g.N = 2 * F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_GLU);
+  ei_gemm<T>(c, g, NV, TC_EI_GLU, SLW_GLU);
   g_nlaunch++;
   k_glu<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, E5a, G);
   g = gp0<T>();
   g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_DENSE_W]; g.ldb = F; g.C = Z1; g.ldc = F;
   g.bias = c.W.w[FIRE_P_EI_DENSE_B]; g.bias_period = NV;
   g.M = G * NV; g.N = F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_DENSE);
+  ei_gemm<T>(c, g, NV, TC_EI_DENSE, SLW_DENSE);
   g_nlaunch++;
   k_silu5<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, G);
   g = gp0<T>();
   g.A = Z1; g.lda = F; g.B = c.W.w[FIRE_P_EI_OUT_W]; g.ldb = 5 * F; g.C = E5o; g.ldc = 5 * F;
   g.bias = c.W.w[FIRE_P_EI_OUT_B]; g.bias_period = NV;
   g.M = G * NV; g.N = 5 * F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_OUT);
+  ei_gemm<T>(c, g, NV, TC_EI_OUT, SLW_OUT);
   Prof pr("edge_contract", c.s);
   k_edge_contract<T, NT><<<G, 256, 0, c.s>>>(c.r, c.nb, c.L, c.W, E5o, c.template buf<T>(c.P.HX),
                                              NT ? c.template buf<T>(c.P.HL) : nullptr,
@@ -683,7 +792,7 @@ struct Planes {
 template <typename T>
 cudaError_t silu_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
                        int rowsX, int rowsJcap, const int* rowsJdev, const int* node_map, int node_div, size_t zx,
-                       size_t jsq, int tc_id = -1) {
+                       size_t jsq, int tc_id, int sl_id) {
   GemmP<T> g = gp0<T>();
   g.A = c.template buf<T>(in.X); g.lda = K; g.B = Wt; g.ldb = N; g.bias = b; g.C = c.template buf<T>(out.X);
   g.ldc = N; g.M = rowsX; g.N = N; g.K = K; g.ld_aux = N;
@@ -691,36 +800,36 @@ cudaError_t silu_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, c
     g.aux0 = c.template buf<T>(zx);
     g.aux2 = c.template buf<T>(c.P.Zx2);
   }
-  value_gemm<T, EPI_SILU_X>(c, g);
+  value_gemm<T, EPI_SILU_X>(c, g, sl_id);
   if (!fl) return cudaPeekAtLastError();
   cudaMemsetAsync(c.template buf<T>(jsq), 0, sizeof(T) * (size_t)rowsX * N, c.s);
   g = gp0<T>();
   g.A = c.template buf<T>(in.J); g.lda = K; g.B = Wt; g.ldb = N; g.C = c.template buf<T>(out.J); g.ldc = N;
   g.M = rowsJcap; g.M_dev = rowsJdev; g.M_scale = 3; g.N = N; g.K = K; g.node_map = node_map;
   g.node_div = node_div; g.aux1 = c.template buf<T>(zx); g.aux2 = c.template buf<T>(jsq); g.ld_aux = N;
-  gemm<T, EPI_SILU_J>(c, g, tc_id);
+  gemm<T, EPI_SILU_J>(c, g, tc_id, sl_id);
   g = gp0<T>();
   g.A = c.template buf<T>(in.L); g.lda = K; g.B = Wt; g.ldb = N; g.C = c.template buf<T>(out.L); g.ldc = N;
   g.M = rowsX; g.N = N; g.K = K; g.aux1 = c.template buf<T>(zx); g.aux0 = c.template buf<T>(c.P.Zx2);
   g.aux3 = c.template buf<T>(jsq); g.ld_aux = N;
-  gemm<T, EPI_SILU_L>(c, g, tc_id);
+  gemm<T, EPI_SILU_L>(c, g, tc_id, sl_id);
   return cudaPeekAtLastError();
 }
 
 // Linear(F -> N) without activation on a node (bias on X only)
 template <typename T>
 cudaError_t linear_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
-                         int rowsX, int rowsJcap, const int* rowsJdev, int tc_id = -1) {
+                         int rowsX, int rowsJcap, const int* rowsJdev, int tc_id, int sl_id) {
   GemmP<T> g = gp0<T>();
   g.A = c.template buf<T>(in.X); g.lda = K; g.B = Wt; g.ldb = N; g.bias = b; g.bias_period = 1;
   g.C = c.template buf<T>(out.X); g.ldc = N; g.M = rowsX; g.N = N; g.K = K;
-  value_gemm<T, EPI_PLAIN>(c, g);
+  value_gemm<T, EPI_PLAIN>(c, g, sl_id);
   if (!fl) return cudaPeekAtLastError();
   g.A = c.template buf<T>(in.J); g.bias = nullptr; g.C = c.template buf<T>(out.J); g.M = rowsJcap;
   g.M_dev = rowsJdev; g.M_scale = rowsJdev ? 3 : 1;
-  gemm<T, EPI_PLAIN>(c, g, tc_id);
+  gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id);
   g.A = c.template buf<T>(in.L); g.C = c.template buf<T>(out.L); g.M = rowsX; g.M_dev = nullptr; g.M_scale = 1;
-  gemm<T, EPI_PLAIN>(c, g, tc_id);
+  gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id);
   return cudaPeekAtLastError();
 }
 
@@ -767,46 +876,57 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
           const cudaError_t e = env_tc(ep, c.tcw[slot].tiles + (size_t)d * tc_tiles_bytes((size_t)K8, (size_t)n) / 2,
                                        c.status, c.s, tc_val);
           if (e != cudaSuccess) return e;
-          if (tc_val) continue;
+        } else if (nvc > 1 || !c.comp) {
+          // the CUDA-core contraction: the Metropolis blocks' value rows, the FP32 forward Laplacian's derivative rows
+          // (whose value rows the sliced contraction below computes again)
+          GemmP<T> g = gp0<T>();
+          g.A = coef + d * rows * K8; g.lda = K8;
+          g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (long)d * K8 * n; g.ldb = n;
+          g.C = env + (long)d * n; g.ldc = (long)DN * (NV / nvc); g.M = (int)rows; g.N = n; g.K = (int)K8;
+          g.n_el = n; g.env_ns = ns; g.env_soff = s == 0 ? 0 : nu; g.env_nv = nvc;
+          gemm<T, EPI_ENV>(c, g);
         }
-      }
-      GemmP<T> g = gp0<T>();
-      g.A = coef + d * rows * K8; g.lda = K8;
-      g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (long)d * K8 * n; g.ldb = n;
-      g.C = env + (long)d * n; g.ldc = (long)DN * (NV / nvc); g.M = (int)rows; g.N = n; g.K = (int)K8;
-      g.n_el = n; g.env_ns = ns; g.env_soff = s == 0 ? 0 : nu; g.env_nv = nvc;
-      if constexpr (sizeof(T) == 8) {
-        if (c.env_df && nvc == 1) {
-          Prof pg("gemm", c.s);
-          g_nlaunch++;
-          const cudaError_t e = launch_gemm_env_df(g, c.s);
-          if (e != cudaSuccess) return e;
-          continue;
-        }
-      }
-      if (sizeof(T) == 8 || !c.comp) {
-        gemm<T, EPI_ENV>(c, g);
-      } else if constexpr (sizeof(T) == 4) {
-        // the value rows by the compensated contraction (hi into the carrier, lo into env_lo); with derivative
-        // rows in the same coefficient block (FP32 forward Laplacian) the plain contraction takes those first
-        if (nvc > 1) gemm<T, EPI_ENV>(c, g);
-        GemmP<float> gv = g;
-        gv.lda = (long)nvc * K8; gv.M = c.Wc * ns; gv.ldc = (long)NV * DN; gv.env_nv = 1;
-        gemm_comp<COMP_ENV>(c, gv, c.template buf<float>(c.P.env_lo) + (long)d * n, nullptr, DN);
       }
     }
+  }
+  // value rows of the FP32 and mixed paths (hi into the carrier, lo into env_lo), all rows in FP64: one sliced
+  // contraction over both spins and the determinants
+  if (sizeof(T) == 8 || c.comp) {
+    const bool value_only = sizeof(T) == 4;
+    const int nvc = (sizeof(T) == 4 && c.mixed && NENV_ORB * N <= ENV_TC_KMAX) ? 1 : NV;  // coefficient rows per electron
+    const int nvr = value_only ? 1 : NV;                                                  // rows taken per electron
+    const long K8 = (long)N * NENV_ORB;
+    GemmP<T> g = gp0<T>();
+    g.lda = K8 * (nvc / nvr); g.C = env; g.ldc = (long)DN * (NV / nvr); g.N = n; g.K = (int)K8; g.n_el = n;
+    g.env_nv = nvr;
+    SlCall<T> q = sl_spin_call(c, g, SLW_ENV_UP, SLW_ENV_DN, nvr);
+    q.batch = NDET;
+    q.p[0].A = c.template buf<T>(c.P.coef_up);
+    q.p[1].A = c.template buf<T>(c.P.coef_dn);
+    q.a_bs[0] = (long)c.Wc * nu * nvc * K8;
+    q.a_bs[1] = (long)c.Wc * (n - nu) * nvc * K8;
+    q.c_bs = q.lo_bs = n;
+    if constexpr (sizeof(T) == 4) q.C_lo = c.template buf<float>(c.P.env_lo);
+    q.ld_lo = DN;
+    const cudaError_t e = sl_gemm(c, sizeof(T) == 4 ? (int)COMP_ENV : (int)EPI_ENV, q);
+    if (e != cudaSuccess) return e;
   }
   GemmP<T> g = gp0<T>();
   g.A = c.template buf<T>(c.P.B2X); g.lda = F; g.B = c.W.w[PR_ORB_UP_W_S1]; g.B2 = c.W.w[PR_ORB_DN_W_S1];
   g.ldb = DN; g.bias = c.W.w[FIRE_P_ORB_UP_B]; g.bias2 = c.W.w[FIRE_P_ORB_DN_B];
   g.C = c.template buf<T>(c.P.Apl); g.ldc = DN; g.M = G; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.aux0 = c.template buf<T>(c.P.rawx); g.aux1 = env; g.ld_aux = DN; g.env_nv = NV;
-  if constexpr (sizeof(T) == 4) {
-    if (c.comp)
-      gemm_comp<COMP_ORB>(c, g, c.template buf<float>(c.P.Apl_lo), c.template buf<float>(c.P.env_lo), DN);
-    else
-      gemm<T, EPI_ORB_X>(c, g);
-  } else {
+  if (sizeof(T) == 8 || c.comp) {
+    SlCall<T> q = sl_spin_call(c, g, SLW_ORB_UP, SLW_ORB_DN, 1);
+    q.map_a = 1;
+    if constexpr (sizeof(T) == 4) {
+      q.C_lo = c.template buf<float>(c.P.Apl_lo);
+      q.env_lo = c.template buf<float>(c.P.env_lo);
+    }
+    q.ld_lo = DN;
+    const cudaError_t e = sl_gemm(c, sizeof(T) == 4 ? (int)COMP_ORB : (int)EPI_ORB_X, q);
+    if (e != cudaSuccess) return e;
+  } else if constexpr (sizeof(T) == 4) {
     gemm<T, EPI_ORB_X>(c, g);
   }
   if (!fl) return cudaPeekAtLastError();
@@ -816,7 +936,22 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   g.M_dev = c.L.pos_off + c.Wc; g.M_scale = 3; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.node_map = c.L.pos_ctr; g.node_div = 3; g.dep_map = c.L.pos_dep; g.aux1 = env;
   g.aux2 = c.template buf<T>(c.P.rjs); g.aux3 = c.template buf<T>(c.P.rawx); g.ld_aux = DN; g.env_nv = 5;
-  gemm<T, EPI_ORB_J>(c, g, TC_ORB_UP);
+  if constexpr (sizeof(T) == 8) {  // rows sorted by center: both spins' weights over the same slices
+    SlCall<T> q = sl_call(c, g, SLW_ORB_UP);
+    q.nseg = 2;
+    q.p[1] = g;
+    q.w[1] = c.slw[SLW_ORB_DN];
+    q.spin[1] = 1;
+    q.share_a = 1;
+    int* mask = c.template buf<int>(c.P.tile_mask);
+    g_nlaunch++;
+    sl_tile_mask(g, mask, c.s);
+    q.tile_mask = mask;
+    const cudaError_t e = sl_gemm(c, EPI_ORB_J, q);
+    if (e != cudaSuccess) return e;
+  } else {
+    gemm<T, EPI_ORB_J>(c, g, TC_ORB_UP);
+  }
   g = gp0<T>();
   g.A = c.template buf<T>(c.P.B2L); g.lda = F; g.B = c.W.w[PR_ORB_UP_W_S1]; g.B2 = c.W.w[PR_ORB_DN_W_S1];
   g.ldb = DN; g.C = c.template buf<T>(c.P.lapA); g.ldc = DN; g.M = G; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
@@ -838,7 +973,13 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
       return cudaPeekAtLastError();
     }
   }
-  gemm<T, EPI_ORB_L>(c, g, TC_ORB_UP);
+  if constexpr (sizeof(T) == 8) {
+    SlCall<T> q = sl_spin_call(c, g, SLW_ORB_UP, SLW_ORB_DN, 1);
+    q.map_a = 1;
+    return sl_gemm(c, EPI_ORB_L, q);
+  } else {
+    gemm<T, EPI_ORB_L>(c, g, TC_ORB_UP);
+  }
   return cudaPeekAtLastError();
 }
 
@@ -901,7 +1042,7 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
         FLM ? c.template buf<T>(c.P.aJ) : nullptr, FLM ? c.template buf<T>(c.P.aL) : nullptr, c.status, nullptr,
         nullptr);
   }
-  linear_layer<T>(c, FLM, B2, B1, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, G, Jcap, Jdev, TC_V);
+  linear_layer<T>(c, FLM, B2, B1, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, G, Jcap, Jdev, TC_V, SLW_V);
   cudaMemsetAsync(c.template buf<T>(c.P.Ax), 0, sizeof(T) * Wc * 2 * 272, c.s);
   if (FLM) cudaMemsetAsync(c.template buf<T>(c.P.Al), 0, sizeof(T) * Wc * 2 * 272, c.s);
   g_nlaunch++;
@@ -919,7 +1060,7 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
   {
     GemmP<T> g = gp0<T>();
     // layer 1/2 with dense Jacobian rows: node of a J row = row / (3n)
-    auto dense_silu = [&](Planes in, Planes out, const T* Wt, const T* b, int K) {
+    auto dense_silu = [&](Planes in, Planes out, const T* Wt, const T* b, int K, int sl_id) {
       GemmP<T> q = gp0<T>();
       q.A = c.template buf<T>(in.X); q.lda = K; q.B = Wt; q.ldb = F; q.bias = b; q.C = c.template buf<T>(out.X);
       q.ldc = F; q.M = Wc; q.N = F; q.K = K; q.ld_aux = F;
@@ -927,22 +1068,22 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
         q.aux0 = c.template buf<T>(c.P.Zr);
         q.aux2 = c.template buf<T>(c.P.Zr2);
       }
-      gemm<T, EPI_SILU_X>(c, q);
+      gemm<T, EPI_SILU_X>(c, q, -1, sl_id);
       if (!FLM) return;
       cudaMemsetAsync(c.template buf<T>(c.P.jsqr), 0, sizeof(T) * Wc * F, c.s);
       q = gp0<T>();
       q.A = c.template buf<T>(in.J); q.lda = K; q.B = Wt; q.ldb = F; q.C = c.template buf<T>(out.J); q.ldc = F;
       q.M = Wc * 3 * n; q.N = F; q.K = K; q.node_div = 3 * n; q.aux1 = c.template buf<T>(c.P.Zr);
       q.aux2 = c.template buf<T>(c.P.jsqr); q.ld_aux = F;
-      gemm<T, EPI_SILU_J>(c, q);
+      gemm<T, EPI_SILU_J>(c, q, -1, sl_id);
       q = gp0<T>();
       q.A = c.template buf<T>(in.L); q.lda = K; q.B = Wt; q.ldb = F; q.C = c.template buf<T>(out.L); q.ldc = F;
       q.M = Wc; q.N = F; q.K = K; q.aux1 = c.template buf<T>(c.P.Zr); q.aux0 = c.template buf<T>(c.P.Zr2);
       q.aux3 = c.template buf<T>(c.P.jsqr); q.ld_aux = F;
-      gemm<T, EPI_SILU_L>(c, q);
+      gemm<T, EPI_SILU_L>(c, q, -1, sl_id);
     };
-    dense_silu(RI, R1, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F);
-    dense_silu(R1, R2, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F);
+    dense_silu(RI, R1, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F, SLW_READ1);
+    dense_silu(R1, R2, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F, SLW_READ2);
     g.A = c.template buf<T>(R2.X); g.lda = F; g.B = c.W.w[FIRE_P_ATT_OUT3_W]; g.ldb = 2; g.bias = c.W.w[FIRE_P_ATT_OUT3_B];
     g.bias_period = 1; g.C = c.template buf<T>(c.P.JAx); g.ldc = 2; g.M = Wc; g.N = 2; g.K = F;
     gemm<T, EPI_PLAIN>(c, g);
@@ -955,9 +1096,9 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
   }
   // MLP Jastrow: SparseMLP [256, 256, 2] (silu on every layer), * mlp_scale + [0, log_bias], sum over nodes
   silu_layer<T>(c, FLM, B2, B1, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
-                c.P.Zx, c.P.jsq, TC_JMLP1);
+                c.P.Zx, c.P.jsq, TC_JMLP1, SLW_JMLP1);
   silu_layer<T>(c, FLM, B1, H, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
-                c.P.Zx, c.P.jsq, TC_JMLP2);
+                c.P.Zx, c.P.jsq, TC_JMLP2, SLW_JMLP2);
   g_nlaunch++;
   k_narrow<T, 2, 0, FLM><<<G, 256, 0, c.s>>>(
       c.template buf<T>(H.X), FLM ? c.template buf<T>(H.J) : nullptr, FLM ? c.template buf<T>(H.L) : nullptr, c.nb,
@@ -982,9 +1123,9 @@ cudaError_t stage_update(Ctx<T>& c) {
   const Planes H{c.P.HX, c.P.HJ, c.P.HL}, B1{c.P.B1X, c.P.B1J, c.P.B1L}, B2{c.P.B2X, c.P.B2J, c.P.B2L};
   Prof pr("update_mlp", c.s);
   silu_layer<T>(c, FLM, H, B1, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
-                c.P.jsq, TC_UPD1);
+                c.P.jsq, TC_UPD1, SLW_UPD1);
   silu_layer<T>(c, FLM, B1, B2, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
-                c.P.jsq, TC_UPD2);
+                c.P.jsq, TC_UPD2, SLW_UPD2);
   return cudaPeekAtLastError();
 }
 
@@ -1115,6 +1256,13 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
 }
 
 template <typename T>
+void set_sliced(Ctx<T>& c, const fire_problem* p, const void* prepared) {
+  size_t so[SLW_COUNT + 1];
+  sl_offsets<T>(p, so);
+  for (int k = 0; k < SLW_COUNT; ++k) c.slw[k] = reinterpret_cast<const unsigned char*>(prepared) + so[k];
+}
+
+template <typename T>
 Ctx<T> make_ctx(const fire_problem* p, cudaStream_t s, const float* R, const float* Z, const void* prepared,
                 int32_t* status, void* ws, int Wmax, bool fl) {
   Ctx<T> c;
@@ -1129,6 +1277,7 @@ Ctx<T> make_ctx(const fire_problem* p, cudaStream_t s, const float* R, const flo
   c.ws = reinterpret_cast<unsigned char*>(ws);
   c.P = make_plan(p, Wmax, fl);
   c.mixed = p->precision == FIRE_PREC_MIXED;
+  set_sliced(c, p, prepared);
   if (c.mixed) {
     int64_t off[PR_COUNT + 1];
     prep_offsets(p, off);
@@ -1204,7 +1353,6 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
                                        ws + L.c64, KC, false);
     c64.w0 = 0;
     c64.Wc = KC;
-    c64.env_df = true;
     c64.r = r64;
     setup_ctx(c64, false);
     stage_neighbors(c64, false);
@@ -1212,6 +1360,7 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     stage_update<double, 0>(c64);
     stage_orbitals<double, 0>(c64);
     Ctx<T> c = make_ctx<T>(&pr_, s, R, Z, prepared, status, ws, KC, true);
+    set_sliced(c, p, prepared);  // where the batch's own precision has them
     c.w0 = 0;
     c.Wc = KC;
     c.r = r_ref;
@@ -1473,7 +1622,8 @@ cudaError_t chunk_state(Ctx<T>& c, const LrPlan& Q, void* logpsi, void* sign, in
   }
   stage_jastrow<T, 0>(c);
   const Planes B2{c.P.B2X, 0, 0}, VL{Q.vals, 0, 0};
-  linear_layer<T>(c, false, B2, VL, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, c.Wc * c.p->n_el, 0, nullptr);
+  linear_layer<T>(c, false, B2, VL, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, c.Wc * c.p->n_el, 0, nullptr,
+                  -1, SLW_V);
   AssembleOut o;
   std::memset(&o, 0, sizeof(o));
   o.logpsi = logpsi;
@@ -1541,9 +1691,9 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
                                                 c.template buf<T>(Q.HS));
   const Planes HS{Q.HS, 0, 0}, B1S{Q.B1S, 0, 0}, hS{Q.hS, 0, 0};
   silu_layer<T>(c, false, HS, B1S, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
-                0);
+                0, -1, SLW_UPD1);
   silu_layer<T>(c, false, B1S, hS, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
-                0);
+                0, -1, SLW_UPD2);
   // raw orbital rows of the changed centers (both spins' contractions, then each row's own)
   for (int sp = 0; sp < 2; ++sp) {
     GemmP<T> g = gp0<T>();
@@ -1608,11 +1758,11 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
                                                       c.template buf<T>(Q.aS), nullptr, nullptr, c.status, nullptr,
                                                       nullptr);
     const Planes vS{Q.vS, 0, 0};
-    linear_layer<T>(c, false, hS, vS, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, rows, 0, nullptr);
+    linear_layer<T>(c, false, hS, vS, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, rows, 0, nullptr, -1, SLW_V);
     silu_layer<T>(c, false, hS, HS, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, rows, 0, nullptr, nullptr, 1,
-                  0, 0);
+                  0, 0, -1, SLW_JMLP1);
     silu_layer<T>(c, false, HS, B1S, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, rows, 0, nullptr, nullptr,
-                  1, 0, 0);
+                  1, 0, 0, -1, SLW_JMLP2);
     g_nlaunch++;
     k_narrow<T, 2, 0, false><<<rows, 256, 0, s>>>(c.template buf<T>(Q.B1S), nullptr, nullptr, c.nb, c.L,
                                                   c.W.w[FIRE_P_JMLP3_W], c.W.w[FIRE_P_JMLP3_B],
@@ -1832,10 +1982,10 @@ fire_status fire_param_layout(const fire_problem* prob, int64_t* offsets) {
 
 fire_status fire_prepared_size(const fire_problem* prob, size_t* bytes) {
   if (!valid(prob) || !bytes) return FIRE_ERR_INVALID;
-  int64_t off[PR_COUNT + 1];
-  prep_offsets(prob, off);
-  *bytes = (size_t)off[PR_COUNT] * elem_size(prob);
-  if (prob->precision != FIRE_PREC_FP64) *bytes = prep64_offset(prob) + (size_t)off[PR_COUNT] * 8;
+  const fire_problem p64 = refine_problem64(prob, 1);
+  size_t so[SLW_COUNT + 1];
+  sl_offsets<double>(&p64, so);
+  *bytes = so[SLW_COUNT] + (prob->precision != FIRE_PREC_FP64 ? prep64_offset(prob) : 0);
   return FIRE_OK;
 }
 
