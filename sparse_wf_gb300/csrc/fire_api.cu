@@ -161,8 +161,8 @@ void tc_offsets(const fire_problem* p, size_t float_bytes, size_t* off) {
   off[TC_COUNT] = o;
 }
 
-// Weights of the sliced contractions (fire_sliced.cuh), cut when the parameters are prepared: of the value rows in the
-// FP32 and mixed paths (SL_PAIR), of every layer in FP64 (SL_F64).
+// Weights of the sliced contractions (fire_sliced.cuh), cut when the parameters are prepared: for the value path of the FP32
+// and mixed builds (SL_PAIR, without the attention readout's), for every layer in FP64 (SL_F64).
 enum SlSlot {
   SLW_GLU, SLW_DENSE, SLW_OUT, SLW_UPD1, SLW_UPD2, SLW_ORB_UP, SLW_ORB_DN, SLW_V, SLW_JMLP1, SLW_JMLP2, SLW_ENV_UP,
   SLW_ENV_DN, SLW_READ1, SLW_READ2, SLW_COUNT
@@ -189,8 +189,8 @@ SlSrc sl_src(int k, const fire_problem* p) {
     default: return {FIRE_P_ATT_OUT2_W, F, F, 1};
   }
 }
-// byte offsets of the sliced weights behind the `float_bytes` of the slots of T (and, in the mixed path, the tensor-core
-// weights); off[SLW_COUNT] = end.  The attention readout is sliced in FP64 only.
+// Byte offsets of the sliced weights behind the slots of T (and, in the mixed path, the tensor-core weights);
+// off[SLW_COUNT] = end.
 template <typename T>
 void sl_offsets(const fire_problem* p, size_t* off) {
   int64_t po[PR_COUNT + 1];
@@ -201,14 +201,14 @@ void sl_offsets(const fire_problem* p, size_t* off) {
     tc_offsets(p, o, to);
     o = to[TC_COUNT];
   }
-  for (int k = 0; k < SLW_COUNT; ++k) {
+  for (int k = 0; k <= SLW_COUNT; ++k) {
     o = (o + 255) / 256 * 256;
     off[k] = o;
+    if (k == SLW_COUNT) break;
     const SlSrc q = sl_src(k, p);
     if (sizeof(T) == 8) o += q.batch * sl_w_bytes<SL_F64>(q.K, q.N);
     else if (k < SLW_READ1) o += q.batch * sl_w_bytes<SL_PAIR>(q.K, q.N);
   }
-  off[SLW_COUNT] = (o + 255) / 256 * 256;
 }
 
 // Byte offset of the FP64 prepared weights (the refinement pass's) in an FP32 / mixed prepared buffer: after the
@@ -243,17 +243,14 @@ struct Plan {
 // Scratch of the largest sliced contraction of a chunk (fire_sliced.cuh).
 template <int KIND>
 size_t sl_plan_bytes(const fire_problem* p, size_t W, bool fl) {
-  const long n = p->n_el, nu = p->n_up, nd = n - nu;
+  const long n = p->n_el, nu = p->n_up, ms = std::max<long>(nu, n - nu), w = (long)W;
   const int K8 = NENV_ORB * p->n_nuc;
-  const bool all = KIND == SL_F64 && fl;  // FP64: the derivative rows too
-  const long nv = all ? 5 : 1, jr = 3L * (long)W * (n + p->cap_pairs);
-  auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-  size_t b = up(sl_scratch_bytes<KIND>((long)W * n * nv, F));
-  b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * nu, F)) + up(sl_scratch_bytes<KIND>((long)W * nd, F)));
-  b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * nu * nv, K8, NDET)) +
-                      up(sl_scratch_bytes<KIND>((long)W * nd * nv, K8, NDET)));
-  if (KIND == SL_F64) b = std::max(b, up(sl_scratch_bytes<KIND>((long)W * (fl ? 3 * n : 1), 2 * F)));
-  if (all) b = std::max(b, up(sl_scratch_bytes<KIND>(jr, F)));
+  const long nv = fl ? 5 : 1;
+  size_t b = sl_scratch_bytes<KIND>(w * n * nv, F);
+  b = std::max(b, sl_scratch_bytes<KIND>(w * ms, F, 2));
+  b = std::max(b, sl_scratch_bytes<KIND>(w * ms * nv, K8, 2 * NDET));
+  if (KIND == SL_F64) b = std::max(b, sl_scratch_bytes<KIND>(w * (fl ? 3 * n : 1), 2 * F));
+  if (fl) b = std::max(b, sl_scratch_bytes<KIND>(3 * w * (n + p->cap_pairs), F));
   return b;
 }
 
@@ -348,9 +345,9 @@ Plan make_plan(const fire_problem* p, int Wc, bool fl) {
     take(P.JMl, W * 2, es);
     take(P.JMj, W * 3 * n * 2, es);
   }
-  // two working copies per matrix for the Gauss-Jordan / LU kernel; the sliced contractions before and after it cut
-  // their rows into the same bytes
-  const size_t slb = es == 8 ? sl_plan_bytes<SL_F64>(p, W, fl) : sl_plan_bytes<SL_PAIR>(p, W, fl);
+  // two working copies per matrix for the Gauss-Jordan / LU kernel; the sliced contractions before and after it (all of
+  // FP64, the value path in FP32) cut their rows into the same bytes
+  const size_t slb = es == 8 ? sl_plan_bytes<SL_F64>(p, W, fl) : sl_plan_bytes<SL_PAIR>(p, W, false);
   take(P.gjw, std::max(2 * W * NDET * n * n * 8, slb), 1);
   P.sl = P.gjw;
   take(P.enn, 1, 8);
@@ -541,13 +538,13 @@ fire_status prepare_impl(cudaStream_t s, const fire_problem* p, const float* blo
                                 out + off[PR_SCALARS]);
   size_t so[SLW_COUNT + 1];
   sl_offsets<T>(p, so);
-  unsigned char* base = reinterpret_cast<unsigned char*>(prepared);
   for (int k = 0; k < SLW_COUNT; ++k) {
     const SlSrc q = sl_src(k, p);
     if (sizeof(T) == 4 && k >= SLW_READ1) continue;
+    unsigned char* dst = reinterpret_cast<unsigned char*>(prepared) + so[k];
     g_nlaunch++;
-    if constexpr (sizeof(T) == 4) sl_prepare_f32(out + off[q.slot], q.K, q.N, q.batch, base + so[k], s);
-    else sl_prepare_f64(out + off[q.slot], q.K, q.N, q.batch, base + so[k], s);
+    if constexpr (sizeof(T) == 4) sl_prepare_pair(out + off[q.slot], q.K, q.N, q.batch, dst, s);
+    else sl_prepare_f64(out + off[q.slot], q.K, q.N, q.batch, dst, s);
   }
   return launch_status(__func__);
 }
@@ -585,6 +582,13 @@ struct Ctx {
   // energy, log|psi| and the low-rank state); the Metropolis blocks' proposals, which only compare log|psi| values,
   // take the plain contraction
   bool comp = true;
+  // the value path of its own (log|psi|, the embedding, the pseudopotential's state): those value planes by the sliced
+  // tensor-core contraction, else by k_gemm_comp.  The two agree to ~10^-14, yet now and then a hidden value rounds to the
+  // other neighbouring float.  log|psi| hardly sees that (10^-8); a local energy near a node, where the terms cancel to 10^-4
+  // and less, moved by up to 10^-4 of itself.  A local energy keeps the sums it always had.
+  bool pair = false;
+  // the refinement pass's FP64 value path: its envelope rows by k_gemm_env_df
+  bool env_df = false;
   TcWeights tcw[TC_COUNT];
   const unsigned char* slw[SLW_COUNT];  // sliced weights
   template <typename U>
@@ -630,25 +634,26 @@ GemmP<T> gp0() {
   return g;
 }
 
-// The sliced contraction of one weight (sl_id) with one set of rows.
+// The sliced contraction of one weight with one set of rows.
 template <typename T>
-SlCall<T> sl_call(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
+SlCall<T> sl_call(const GemmP<T>& g, const unsigned char* w) {
   SlCall<T> q;
   std::memset(&q, 0, sizeof(q));
   q.nseg = 1;
   q.batch = 1;
   q.p[0] = g;
-  q.w[0] = c.slw[sl_id];
+  q.w[0] = w;
   return q;
 }
-// ... of both spins' rows (one per electron), each with its own weight; mode and strides are the caller's.
+// ... of both spins' rows (rows_per_el per electron, the walkers' electrons of a spin in a row), each with its own weight.
 template <typename T>
-SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, int sl_up, int sl_dn, int rows_per_el) {
-  SlCall<T> q = sl_call(c, g, sl_up);
+SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, const unsigned char* w_up, const unsigned char* w_dn,
+                       int rows_per_el) {
+  SlCall<T> q = sl_call(g, w_up);
   const int nu = c.p->n_up, nd = c.p->n_el - nu;
   q.nseg = 2;
   q.p[1] = g;
-  q.w[1] = c.slw[sl_dn];
+  q.w[1] = w_dn;
   q.p[0].M = c.Wc * nu * rows_per_el;
   q.p[1].M = c.Wc * nd * rows_per_el;
   q.p[0].n_el = q.p[1].n_el = c.p->n_el;
@@ -658,22 +663,26 @@ SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, int sl_up, int sl_dn,
   q.spin[1] = 1;
   return q;
 }
+// SL_F64: mode is an EpiMode; SL_PAIR (hi + lo value rows): a CompMode
 template <typename T>
 cudaError_t sl_gemm(const Ctx<T>& c, int mode, const SlCall<T>& q) {
   Prof pr(sizeof(T) == 4 ? "gemm_comp" : "gemm", c.s);
-  g_nlaunch += 2;
   unsigned char* scratch = c.template buf<unsigned char>(c.P.sl);
-  if constexpr (sizeof(T) == 4) return sl_gemm_f32(mode, q, scratch, c.status, c.s);
-  else return sl_gemm_f64(mode, q, scratch, c.status, c.s);
+  int k;
+  if constexpr (sizeof(T) == 4) k = sl_gemm_pair(mode, q, scratch, c.status, c.s);
+  else k = sl_gemm_f64(mode, q, scratch, c.status, c.s);
+  g_nlaunch += k < 0 ? 0 : k;
+  return k < 0 ? cudaErrorInvalidValue : cudaPeekAtLastError();
 }
 
-// tc_id: tensor-core weight of the mixed path's derivative rows; sl_id: sliced weight of the FP64 path
+// tc_id: tensor-core weight of the mixed path's derivative rows; sl_id: sliced weight in FP64; neither: the CUDA-core
+// contraction
 template <typename T, int MODE>
 cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
   if constexpr (sizeof(T) == 8) {
-    if (sl_id >= 0) return sl_gemm(c, MODE, sl_call(c, g, sl_id));
+    if (sl_id >= 0) return sl_gemm(c, MODE, sl_call(g, c.slw[sl_id]));
   }
-  // profile stages: "gemm_tc" the tensor-core contractions, "gemm" the CUDA-core ones
+  // profile stages: "gemm_tc" the mixed path's tensor-core contractions, "gemm" the others
   const bool tc = sizeof(T) == 4 && c.mixed && tc_id >= 0;
   Prof pr(tc ? "gemm_tc" : "gemm", c.s);
   g_nlaunch++;
@@ -686,12 +695,21 @@ cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
   return launch_gemm<T, MODE>(g, c.s);
 }
 
+// hi + lo value rows by the CUDA cores: low parts into C_lo / read from env_lo, row stride ld_lo
+template <int MODE>
+cudaError_t gemm_comp(const Ctx<float>& c, const GemmP<float>& g, float* C_lo, const float* env_lo, long ld_lo) {
+  Prof pr("gemm_comp", c.s);
+  g_nlaunch++;
+  return launch_gemm_comp<MODE>(g, C_lo, env_lo, ld_lo, c.s);
+}
+
 // Value-plane contraction of a dense layer (EPI_PLAIN or EPI_SILU_X): hi + lo accuracy in the FP32 and mixed paths.
 template <typename T, int MODE>
 cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
   if constexpr (sizeof(T) == 4) {
     static_assert(MODE == EPI_PLAIN || MODE == EPI_SILU_X, "value_gemm: plain or SiLU layers");
-    if (c.comp) return sl_gemm(c, MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU, sl_call(c, g, sl_id));
+    if (c.comp && c.pair) return sl_gemm(c, MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU, sl_call(g, c.slw[sl_id]));
+    if (c.comp) return gemm_comp<MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU>(c, g, nullptr, nullptr, 0);
     return gemm<T, MODE>(c, g);
   } else {
     return gemm<T, MODE>(c, g, -1, sl_id);
@@ -732,7 +750,7 @@ cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id, int sl_id) 
   gv.M = g.M / NV;
   gv.bias_period = g.bias ? 1 : 0;
   if (!c.mixed) {
-    // FP32: all rows by the CUDA-core contraction, the value rows once more at hi + lo accuracy; FP64: all rows sliced
+    // FP32: all rows, then the value rows once more at hi + lo accuracy
     cudaError_t e = gemm<T, EPI_PLAIN>(c, g, -1, sl_id);
     if (e != cudaSuccess || sizeof(T) == 8) return e;
     return value_gemm<T, EPI_PLAIN>(c, gv, sl_id);
@@ -861,7 +879,6 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
       else
         k_env_coef<T, NV><<<nblk(tot), 256, 0, c.s>>>(c.r, c.R, sp, n, ns, s == 0 ? 0 : nu, N, c.Wc, coef);
     }
-    const long rows = (long)c.Wc * ns * nvc;
     for (int d = 0; d < NDET; ++d) {
       if constexpr (sizeof(T) == 4) {
         if (tc_env || tc_val) {
@@ -876,39 +893,65 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
           const cudaError_t e = env_tc(ep, c.tcw[slot].tiles + (size_t)d * tc_tiles_bytes((size_t)K8, (size_t)n) / 2,
                                        c.status, c.s, tc_val);
           if (e != cudaSuccess) return e;
-        } else if (nvc > 1 || !c.comp) {
-          // the CUDA-core contraction: the Metropolis blocks' value rows, the FP32 forward Laplacian's derivative rows
-          // (whose value rows the sliced contraction below computes again)
-          GemmP<T> g = gp0<T>();
-          g.A = coef + d * rows * K8; g.lda = K8;
-          g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (long)d * K8 * n; g.ldb = n;
-          g.C = env + (long)d * n; g.ldc = (long)DN * (NV / nvc); g.M = (int)rows; g.N = n; g.K = (int)K8;
-          g.n_el = n; g.env_ns = ns; g.env_soff = s == 0 ? 0 : nu; g.env_nv = nvc;
-          gemm<T, EPI_ENV>(c, g);
         }
       }
     }
   }
-  // value rows of the FP32 and mixed paths (hi into the carrier, lo into env_lo), all rows in FP64: one sliced
-  // contraction over both spins and the determinants
-  if (sizeof(T) == 8 || c.comp) {
-    const bool value_only = sizeof(T) == 4;
-    const int nvc = (sizeof(T) == 4 && c.mixed && NENV_ORB * N <= ENV_TC_KMAX) ? 1 : NV;  // coefficient rows per electron
-    const int nvr = value_only ? 1 : NV;                                                  // rows taken per electron
+  // The rest of the envelope rows: in FP64 all of them (the refinement pass's by k_gemm_env_df), in FP32 the derivative rows
+  // (with their value rows) and the Metropolis blocks' value rows by the plain contraction, then the value rows hi + lo (hi
+  // into the carrier, lo into env_lo).  The sliced contractions take both spins and all determinants in one launch.
+  {
+    const bool tc_ok = sizeof(T) == 4 && c.mixed && NENV_ORB * N <= ENV_TC_KMAX;
+    const int nvc = tc_ok ? 1 : NV;  // coefficient rows per electron
     const long K8 = (long)N * NENV_ORB;
-    GemmP<T> g = gp0<T>();
-    g.lda = K8 * (nvc / nvr); g.C = env; g.ldc = (long)DN * (NV / nvr); g.N = n; g.K = (int)K8; g.n_el = n;
-    g.env_nv = nvr;
-    SlCall<T> q = sl_spin_call(c, g, SLW_ENV_UP, SLW_ENV_DN, nvr);
-    q.batch = NDET;
-    q.p[0].A = c.template buf<T>(c.P.coef_up);
-    q.p[1].A = c.template buf<T>(c.P.coef_dn);
-    q.a_bs[0] = (long)c.Wc * nu * nvc * K8;
-    q.a_bs[1] = (long)c.Wc * (n - nu) * nvc * K8;
-    q.c_bs = q.lo_bs = n;
-    if constexpr (sizeof(T) == 4) q.C_lo = c.template buf<float>(c.P.env_lo);
-    q.ld_lo = DN;
-    const cudaError_t e = sl_gemm(c, sizeof(T) == 4 ? (int)COMP_ENV : (int)EPI_ENV, q);
+    auto both = [&](int nvr) {  // nvr: rows taken per electron
+      GemmP<T> g = gp0<T>();
+      g.lda = K8 * (nvc / nvr); g.C = env; g.ldc = (long)DN * (NV / nvr); g.N = n; g.K = (int)K8; g.n_el = n;
+      g.env_nv = nvr;
+      SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ENV_UP], c.slw[SLW_ENV_DN], nvr);
+      q.batch = NDET;
+      q.p[0].A = c.template buf<T>(c.P.coef_up);
+      q.p[1].A = c.template buf<T>(c.P.coef_dn);
+      q.a_bs[0] = (long)c.Wc * nu * nvc * K8;
+      q.a_bs[1] = (long)c.Wc * (n - nu) * nvc * K8;
+      q.c_bs = q.lo_bs = n;
+      q.ld_lo = DN;
+      return q;
+    };
+    // go(contraction of one spin's rows for one determinant, determinant) over all of them
+    auto each = [&](const SlCall<T>& q, auto go) -> cudaError_t {
+      for (int s = 0; s < 2; ++s)
+        for (int d = 0; d < NDET && q.p[s].M > 0; ++d) {
+          GemmP<T> g = q.p[s];
+          g.A += d * q.a_bs[s];
+          g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (long)d * K8 * n; g.ldb = n;
+          g.C += d * q.c_bs;
+          g.env_ns = q.ns[s]; g.env_soff = q.soff[s];
+          const cudaError_t e = go(g, d);
+          if (e != cudaSuccess) return e;
+        }
+      return cudaSuccess;
+    };
+    cudaError_t e = cudaSuccess;
+    if constexpr (sizeof(T) == 8) {
+      if (!c.env_df) {
+        e = sl_gemm(c, EPI_ENV, both(NV));
+      } else {
+        e = each(both(NV), [&](const GemmP<T>& g, int) {
+          Prof pg("gemm", c.s);
+          g_nlaunch++;
+          return launch_gemm_env_df(g, c.s);
+        });
+      }
+    } else {
+      if (nvc > 1 || (!c.comp && !tc_ok)) e = each(both(nvc), [&](const GemmP<T>& g, int) { return gemm<T, EPI_ENV>(c, g); });
+      if (e == cudaSuccess && c.comp) {
+        SlCall<T> q = both(1);
+        q.C_lo = c.template buf<float>(c.P.env_lo);
+        if (c.pair) e = sl_gemm(c, COMP_ENV, q);
+        else e = each(q, [&](const GemmP<T>& g, int d) { return gemm_comp<COMP_ENV>(c, g, q.C_lo + (long)d * n, nullptr, DN); });
+      }
+    }
     if (e != cudaSuccess) return e;
   }
   GemmP<T> g = gp0<T>();
@@ -916,8 +959,8 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   g.ldb = DN; g.bias = c.W.w[FIRE_P_ORB_UP_B]; g.bias2 = c.W.w[FIRE_P_ORB_DN_B];
   g.C = c.template buf<T>(c.P.Apl); g.ldc = DN; g.M = G; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.aux0 = c.template buf<T>(c.P.rawx); g.aux1 = env; g.ld_aux = DN; g.env_nv = NV;
-  if (sizeof(T) == 8 || c.comp) {
-    SlCall<T> q = sl_spin_call(c, g, SLW_ORB_UP, SLW_ORB_DN, 1);
+  if (sizeof(T) == 8 || c.pair) {
+    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN], 1);
     q.map_a = 1;
     if constexpr (sizeof(T) == 4) {
       q.C_lo = c.template buf<float>(c.P.Apl_lo);
@@ -927,7 +970,10 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     const cudaError_t e = sl_gemm(c, sizeof(T) == 4 ? (int)COMP_ORB : (int)EPI_ORB_X, q);
     if (e != cudaSuccess) return e;
   } else if constexpr (sizeof(T) == 4) {
-    gemm<T, EPI_ORB_X>(c, g);
+    if (c.comp)
+      gemm_comp<COMP_ORB>(c, g, c.template buf<float>(c.P.Apl_lo), c.template buf<float>(c.P.env_lo), DN);
+    else
+      gemm<T, EPI_ORB_X>(c, g);
   }
   if (!fl) return cudaPeekAtLastError();
   g = gp0<T>();
@@ -936,8 +982,8 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   g.M_dev = c.L.pos_off + c.Wc; g.M_scale = 3; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.node_map = c.L.pos_ctr; g.node_div = 3; g.dep_map = c.L.pos_dep; g.aux1 = env;
   g.aux2 = c.template buf<T>(c.P.rjs); g.aux3 = c.template buf<T>(c.P.rawx); g.ld_aux = DN; g.env_nv = 5;
-  if constexpr (sizeof(T) == 8) {  // rows sorted by center: both spins' weights over the same slices
-    SlCall<T> q = sl_call(c, g, SLW_ORB_UP);
+  if constexpr (sizeof(T) == 8) {  // rows sorted by center: both spins' weights over the same slices, tiles without a spin skipped
+    SlCall<T> q = sl_call(g, c.slw[SLW_ORB_UP]);
     q.nseg = 2;
     q.p[1] = g;
     q.w[1] = c.slw[SLW_ORB_DN];
@@ -974,7 +1020,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     }
   }
   if constexpr (sizeof(T) == 8) {
-    SlCall<T> q = sl_spin_call(c, g, SLW_ORB_UP, SLW_ORB_DN, 1);
+    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN], 1);
     q.map_a = 1;
     return sl_gemm(c, EPI_ORB_L, q);
   } else {
@@ -1353,6 +1399,7 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
                                        ws + L.c64, KC, false);
     c64.w0 = 0;
     c64.Wc = KC;
+    c64.env_df = true;
     c64.r = r64;
     setup_ctx(c64, false);
     stage_neighbors(c64, false);
@@ -1360,7 +1407,6 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     stage_update<double, 0>(c64);
     stage_orbitals<double, 0>(c64);
     Ctx<T> c = make_ctx<T>(&pr_, s, R, Z, prepared, status, ws, KC, true);
-    set_sliced(c, p, prepared);  // where the batch's own precision has them
     c.w0 = 0;
     c.Wc = KC;
     c.r = r_ref;
@@ -1415,6 +1461,7 @@ fire_status run_logpsi(const fire_problem* p, cudaStream_t s, const float* R, co
   const int Wc = choose_chunk(p, wsb, false);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
   Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false);
+  c.pair = true;
   const T* rr = reinterpret_cast<const T*>(r);
   for (int w0 = 0; w0 < p->n_walkers; w0 += Wc) {
     c.w0 = w0;
@@ -1431,6 +1478,7 @@ fire_status run_embedding(const fire_problem* p, cudaStream_t s, const float* R,
   const int Wc = choose_chunk(p, wsb, false);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
   Ctx<T> c = make_ctx<T>(p, s, R, nullptr, prepared, status, ws, Wc, false);
+  c.pair = true;
   const T* rr = reinterpret_cast<const T*>(r);
   for (int w0 = 0; w0 < p->n_walkers; w0 += Wc) {
     c.w0 = w0;
@@ -1878,6 +1926,7 @@ fire_status run_ecp(const fire_problem* p, cudaStream_t s, const float* R, const
   const int Wc = choose_chunk_lr(p, wsb, KS);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
   Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false);
+  c.pair = true;
   const LrPlan Q = make_lr_plan(p, Wc, KS);
   const EcpQuad qt = ecp_quadratures();
   T* rr = const_cast<T*>(reinterpret_cast<const T*>(r));  // read only: nothing is committed

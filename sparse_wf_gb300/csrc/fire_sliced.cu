@@ -42,8 +42,8 @@ struct Mag<double> {
 __device__ __forceinline__ float rint_small(float x) {  // |x| < 2^22
   return __fsub_rn(__fadd_rn(x, 12582912.f), 12582912.f);
 }
-__device__ __forceinline__ void slices2(float a, float b, int code, uint32_t (&w)[SlFmt<SL_PAIR>::NS]) {
-  constexpr int NS = SlFmt<SL_PAIR>::NS;
+template <int NS>
+__device__ __forceinline__ void slices2(float a, float b, int code, uint32_t (&w)[NS]) {
   const float inv = (code == SL_ZERO || code == SL_NAN) ? 0.f : __int_as_float((127 + 6 - code) << 23);
   float x = a * inv, y = b * inv;
 #pragma unroll
@@ -68,8 +68,8 @@ __device__ __forceinline__ long long fixed56(double a, int code) {
   else q = d > 56 ? 0 : (long long)((m + (1ull << (d - 1))) >> d);
   return bits < 0 ? -q : q;
 }
-__device__ __forceinline__ void slices2(double a, double b, int code, uint32_t (&w)[SlFmt<SL_F64>::NS]) {
-  constexpr int NS = SlFmt<SL_F64>::NS;
+template <int NS>
+__device__ __forceinline__ void slices2(double a, double b, int code, uint32_t (&w)[NS]) {
   long long qa = fixed56(a, code), qb = fixed56(b, code);
   const __half2 off = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));  // 1536
 #pragma unroll
@@ -120,6 +120,7 @@ struct SliceArgs {
   int M[2];
   const int* M_dev;
   int M_scale;
+  int row0, row1;  // this pass's rows of every segment
   int K, nkb, n_el;
   int ns[2], soff[2];  // ns > 0: row q is row (q / ns) n_el + soff + q % ns of A
   long a_bs[2];
@@ -141,9 +142,10 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
   const int g = blockIdx.z, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int rows = a.M[g];
   if (a.M_dev) rows = min(rows, a.M_scale * *a.M_dev);
-  const int q = blockIdx.x * 32 + lane;
-  if (blockIdx.x * 32 >= (rows + 127) / 128 * 128) return;
-  const bool ok = q < rows;
+  rows = min(rows, a.row1) - a.row0;  // of this pass
+  const int ql = blockIdx.x * 32 + lane, q = a.row0 + ql;
+  if ((int)blockIdx.x * 32 >= (rows + 127) / 128 * 128) return;
+  const bool ok = ql < rows;
   const long src = a.ns[g] > 0 ? (long)(q / a.ns[g]) * a.n_el + a.soff[g] + q % a.ns[g] : (long)q;
   const T* p = a.A[g] + b * a.a_bs[g] + (ok ? src : 0) * a.lda[g];
   const bool vec = (a.lda[g] * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.A[g] + b * a.a_bs[g]) & 15) == 0;
@@ -174,9 +176,9 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
 #pragma unroll
   for (int w = 0; w < SLR_WARPS; ++w) mx = max(mx, part[w][lane]);
   const int code = sl_code(mx);
-  if (warp == 0) a.code[g][b * a.code_bs[g] + q] = code;
+  if (warp == 0) a.code[g][b * a.code_bs[g] + ql] = code;
   // [128-row tile][16-deep step][slice][k-group][128 rows][16 bytes]
-  unsigned char* out = a.out[g] + b * a.out_bs[g] + (size_t)(q >> 7) * a.nkb * NS * 4096 + (q & 127) * 16;
+  unsigned char* out = a.out[g] + b * a.out_bs[g] + (size_t)(ql >> 7) * a.nkb * NS * 4096 + (ql & 127) * 16;
   auto put = [&](const T (&x)[8], int kg) {
     store_slices<KIND>(x, code, out + (size_t)(kg >> 1) * NS * 4096 + (kg & 1) * 2048, 4096);
   };
@@ -255,6 +257,7 @@ struct SlArgs {
   const unsigned char* Bt[2];
   size_t Bt_bs, b_code;
   SlTile tl;
+  int row0, row1;  // this pass's rows of every segment
   int ns[2], soff[2], spin[2];
   const int* tile_mask;
   long c_bs, lo_bs;
@@ -269,21 +272,6 @@ struct SlBar {
   uint32_t tmem;
   int abort;
 };
-
-// One elected lane of a converged warp issues.
-__device__ __forceinline__ void sl_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n elect.sync _|q, 0xffffffff;\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void sl_commit(uint32_t mbar) {
-  asm volatile(
-      "{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n"
-      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(mbar)
-      : "memory");
-}
 
 // Three 16-column pieces of this warp's 32 lanes, in flight together.
 __device__ __forceinline__ void tmem_ld16x3(uint32_t a0, uint32_t a1, uint32_t a2, float (&v)[3][16]) {
@@ -472,6 +460,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     if (g < a.nseg) {
       rows[g] = a.p[g].M;
       if (a.p[g].M_dev) rows[g] = min(rows[g], a.p[g].M_scale * *a.p[g].M_dev);
+      rows[g] = max(0, min(rows[g], a.row1) - a.row0);
       mt[g] = (rows[g] + 127) / 128;
     }
   const int t0 = a.batch * mt[0] * nt, total = t0 + a.batch * mt[1] * nt;
@@ -485,7 +474,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     const int r = t / nt;
     m = r % mt[g];
     b = r / mt[g];
-    return !a.tile_mask || ((a.tile_mask[m] >> a.spin[g]) & 1);
+    return !a.tile_mask || ((a.tile_mask[a.row0 / 128 + m] >> a.spin[g]) & 1);
   };
 
   if (tid == 0) {
@@ -555,11 +544,11 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
         for (int i = 0; i < NS; ++i)
 #pragma unroll
           for (int j = 0; j < NS - i; ++j)  // level i + j; i == 0 is the level's first product of the step
-            sl_mma(tmem + (uint32_t)((i + j) * Fm::NMAX), da + (uint64_t)(i * 256), db + (uint64_t)(j * 2 * Fm::NMAX), idesc,
-                   (start && i == 0) ? 0u : 1u);
-        sl_commit(smem_u32(&bars->empty[q]));
+            tc_mma_elect(tmem + (uint32_t)((i + j) * Fm::NMAX), da + (uint64_t)(i * 256), db + (uint64_t)(j * 2 * Fm::NMAX),
+                         idesc, (start && i == 0) ? 0u : 1u);
+        tc_commit_elect(smem_u32(&bars->empty[q]));
         if (kb % SL_KCH == SL_KCH - 1 || kb == nkb - 1) {
-          sl_commit(smem_u32(&bars->tfull));
+          tc_commit_elect(smem_u32(&bars->tfull));
           ++uc;
         }
       }
@@ -574,9 +563,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
       int g, b, m, n;
       if (!decode(t, g, b, m, n)) continue;
       const GemmP<T>& p = a.p[g];
-      const int M = rows[g], N = p.N, m0 = m * 128 + quad * 32, n0 = n * nc;
+      const int M = a.row0 + rows[g], N = p.N, l0 = m * 128 + quad * 32, m0 = a.row0 + l0, n0 = n * nc;
       const int* bc = reinterpret_cast<const int*>(a.Bt[g] + (size_t)b * a.Bt_bs + a.b_code);
-      const int rc = a.ac[g][b * a.ac_bs[g] + m0 + lane];
+      const int rc = a.ac[g][b * a.ac_bs[g] + l0 + lane];
       SlAcc<KIND> acc;
       for (int k0 = 0; k0 < nkb; k0 += SL_KCH) {
         live = __all_sync(0xffffffffu, tc_wait(&bars->tfull, (uint32_t)(uc & 1), abort));
@@ -727,10 +716,10 @@ int device_sms() {
 }
 
 template <int KIND, int MODE>
-cudaError_t sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
+int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
   using T = typename SlFmt<KIND>::T;
   const GemmP<T>& p0 = c.p[0];
-  if (c.nseg < 1 || c.nseg > 2 || c.batch < 1 || p0.K < 1 || p0.N < 1) return cudaErrorInvalidValue;
+  if (c.nseg < 1 || c.nseg > 2 || c.batch < 1 || p0.K < 1 || p0.N < 1) return -1;
   SlArgs<T> a;
   SliceArgs<T> r;
   std::memset(&a, 0, sizeof(a));
@@ -751,30 +740,25 @@ cudaError_t sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* s
   r.K = p0.K;
   r.nkb = a.tl.nkb;
   r.n_el = p0.n_el;
-  long tiles = 0, mmax = 0;
-  size_t o = 0;
+  const int sliced = c.share_a ? 1 : c.nseg, blocks = sliced * c.batch;
+  long mmax = 0;
+  for (int g = 0; g < c.nseg; ++g) mmax = std::max<long>(mmax, c.p[g].M);
+  if (mmax == 0) return 0;
+  const long pass = sl_pass_rows(mmax, blocks);
+  const size_t a_bytes = sl_a_bytes<KIND>(pass, p0.K), block = (a_bytes + (size_t)pass * 4 + 255) / 256 * 256;
   for (int g = 0; g < c.nseg; ++g) {
     const GemmP<T>& p = c.p[g];
-    if (p.K != p0.K || p.N != p0.N) return cudaErrorInvalidValue;
+    if (p.K != p0.K || p.N != p0.N) return -1;
+    const int q = c.share_a ? 0 : g;  // whose slices
     a.p[g] = p;
     a.Bt[g] = c.w[g];
     a.ns[g] = c.ns[g];
     a.soff[g] = c.soff[g];
     a.spin[g] = c.spin[g];
-    tiles += (long)c.batch * ((p.M + 127) / 128) * a.tl.nt;
-    if (g == 1 && c.share_a) {
-      a.At[1] = a.At[0];
-      a.ac[1] = a.ac[0];
-      a.At_bs[1] = a.At_bs[0];
-      a.ac_bs[1] = a.ac_bs[0];
-      continue;
-    }
-    mmax = std::max<long>(mmax, p.M);
-    a.At_bs[g] = sl_a_bytes<KIND>(p.M, p.K);
-    a.ac_bs[g] = sl_rows(p.M);
-    a.At[g] = scratch + o;
-    a.ac[g] = reinterpret_cast<const int*>(scratch + o + (size_t)c.batch * a.At_bs[g]);
-    o += (sl_scratch_bytes<KIND>(p.M, p.K, c.batch) + 255) / 256 * 256;
+    a.At[g] = scratch + (size_t)q * c.batch * block;
+    a.At_bs[g] = block;
+    a.ac[g] = reinterpret_cast<const int*>(a.At[g] + a_bytes);
+    a.ac_bs[g] = (long)(block / 4);
     r.A[g] = p.A;
     r.lda[g] = p.lda;
     r.a_bs[g] = c.a_bs[g];
@@ -782,19 +766,29 @@ cudaError_t sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* s
     r.ns[g] = c.map_a ? c.ns[g] : 0;
     r.soff[g] = c.soff[g];
     r.out[g] = const_cast<unsigned char*>(a.At[g]);
-    r.out_bs[g] = a.At_bs[g];
+    r.out_bs[g] = block;
     r.code[g] = const_cast<int*>(a.ac[g]);
     r.code_bs[g] = a.ac_bs[g];
   }
-  if (tiles == 0) return cudaSuccess;
   constexpr int smem = SlSmem<KIND>::TOTAL;
-  const cudaError_t e = cudaFuncSetAttribute(k_gemm_sl<KIND, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  const dim3 gr((unsigned)(sl_rows(mmax) / 32), (unsigned)c.batch, (unsigned)(c.share_a ? 1 : c.nseg));
-  k_slice_rows<KIND, T><<<gr, 32 * SLR_WARPS, 0, s>>>(r);
-  const unsigned grid = (unsigned)std::min<long>(tiles, device_sms());
-  k_gemm_sl<KIND, MODE><<<grid, SL_THREADS, smem, s>>>(a, status);
-  return cudaPeekAtLastError();
+  if (cudaFuncSetAttribute(k_gemm_sl<KIND, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
+  const int sms = device_sms();
+  int launched = 0;
+  for (long r0 = 0; r0 < mmax; r0 += pass) {
+    a.row0 = r.row0 = (int)r0;
+    a.row1 = r.row1 = (int)std::min<long>(r0 + pass, mmax);
+    long tiles = 0, rows = 0;
+    for (int g = 0; g < c.nseg; ++g) {
+      const long m = std::max<long>(0, std::min<long>(c.p[g].M, a.row1) - r0);
+      tiles += (long)c.batch * ((m + 127) / 128) * a.tl.nt;
+      rows = std::max(rows, m);
+    }
+    const dim3 gr((unsigned)(sl_rows(rows) / 32), (unsigned)c.batch, (unsigned)sliced);
+    k_slice_rows<KIND, T><<<gr, 32 * SLR_WARPS, 0, s>>>(r);
+    k_gemm_sl<KIND, MODE><<<(unsigned)std::min<long>(tiles, sms), SL_THREADS, smem, s>>>(a, status);
+    launched += 2;
+  }
+  return cudaPeekAtLastError() == cudaSuccess ? launched : -1;
 }
 
 template <int KIND>
@@ -803,15 +797,6 @@ cudaError_t sl_prepare(const typename SlFmt<KIND>::T* W, int K, int N, int batch
   const dim3 grid((unsigned)((t.nt * t.nc + 31) / 32), (unsigned)batch);
   k_slice_w<KIND><<<grid, 256, 0, s>>>(W, K, N, t, out, sl_w_code_offset<KIND>(K, N), sl_w_bytes<KIND>(K, N));
   return cudaPeekAtLastError();
-}
-
-}  // namespace
-
-cudaError_t sl_prepare_f32(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
-  return sl_prepare<SL_PAIR>(W, K, N, batch, out, s);
-}
-cudaError_t sl_prepare_f64(const double* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
-  return sl_prepare<SL_F64>(W, K, N, batch, out, s);
 }
 
 __global__ void k_sl_tile_mask(GemmP<double> p, int* mask) {
@@ -826,21 +811,31 @@ __global__ void k_sl_tile_mask(GemmP<double> p, int* mask) {
   dn = __syncthreads_or(dn);
   if (threadIdx.x == 0) mask[blockIdx.x] = up | (dn << 1);
 }
+
+}  // namespace
+
+cudaError_t sl_prepare_pair(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
+  return sl_prepare<SL_PAIR>(W, K, N, batch, out, s);
+}
+cudaError_t sl_prepare_f64(const double* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
+  return sl_prepare<SL_F64>(W, K, N, batch, out, s);
+}
+
 void sl_tile_mask(const GemmP<double>& p, int* mask, cudaStream_t s) {
   if (p.M > 0) k_sl_tile_mask<<<(unsigned)((p.M + 127) / 128), 128, 0, s>>>(p, mask);
 }
 
-cudaError_t sl_gemm_f32(int mode, const SlCall<float>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
+int sl_gemm_pair(int mode, const SlCall<float>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
   switch (mode) {
     case COMP_PLAIN: return sl_launch<SL_PAIR, COMP_PLAIN>(c, scratch, status, s);
     case COMP_SILU: return sl_launch<SL_PAIR, COMP_SILU>(c, scratch, status, s);
     case COMP_ENV: return sl_launch<SL_PAIR, COMP_ENV>(c, scratch, status, s);
     case COMP_ORB: return sl_launch<SL_PAIR, COMP_ORB>(c, scratch, status, s);
-    default: return cudaErrorInvalidValue;
+    default: return -1;
   }
 }
 
-cudaError_t sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
+int sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
   switch (mode) {
     case EPI_PLAIN: return sl_launch<SL_F64, EPI_PLAIN>(c, scratch, status, s);
     case EPI_SILU_X: return sl_launch<SL_F64, EPI_SILU_X>(c, scratch, status, s);
@@ -850,7 +845,7 @@ cudaError_t sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratc
     case EPI_ORB_J: return sl_launch<SL_F64, EPI_ORB_J>(c, scratch, status, s);
     case EPI_ORB_L: return sl_launch<SL_F64, EPI_ORB_L>(c, scratch, status, s);
     case EPI_ENV: return sl_launch<SL_F64, EPI_ENV>(c, scratch, status, s);
-    default: return cudaErrorInvalidValue;
+    default: return -1;
   }
 }
 

@@ -10,7 +10,7 @@
 // together.  Two formats:
 //   SL_PAIR  FP32 operands, 6 slices (8 + 5 x 9 bits), 21 MMAs per product; the result is a hi + lo float pair.  The slices
 //            hold 53 bits below the row's largest value.  Five slices of 9 bits (15 MMAs) left errors up to 10 times those
-//            of the compensated dot product on the CUDA cores that this replaced.
+//            of the compensated dot product on the CUDA cores (k_gemm_comp).
 //   SL_F64   FP64 operands, 8 slices of 8 bits, 36 MMAs per product; the levels are put together in integer arithmetic and
 //            rounded once.  64 bits below the largest value: 11 more than an FP64 number has, for rows whose values spread
 //            over many powers of two (envelope coefficients; 7 slices left errors up to twice FP64's own there).
@@ -20,14 +20,18 @@
 // of the result times 2^-24.
 //
 // The CUDA-core FP64 contraction ran at the FP64 pipe's rate (about 1.2 TFLOP/s on GB300, 1/64 of FP32): one 128 x 128 x 256
-// tile took 1.05 ms.  Here it takes ~12 us.
+// tile took 1.05 ms.  Here it takes ~25 us.
 //
 // Work split.  k_slice_rows cuts the rows of A once per contraction into the order the MMA reads (every column tile of
 // the output reads it again, from L2), the weights are cut when the parameters are prepared.  k_gemm_sl is persistent,
 // one CTA per SM: a loader thread streams 16-deep steps of all slices of A and W through a ring with bulk copies, one
 // thread issues the MMAs, eight warps drain tensor memory.  The accumulators of one 128-row tile fill tensor memory, so
-// the next tile's MMAs wait for the drain, but not for the element-wise epilogue and its stores.
+// the next tile's MMAs wait for the drain, but not for the element-wise epilogue and its stores.  Both kernels run over
+// blocks of rows that give every SM a whole number of tiles and whose slices (~60 MB at K = 256) stay in L2: the slices of
+// a larger launch would go through HBM twice, and need scratch in proportion.
 #pragma once
+#include <algorithm>
+
 #include "fire_gemm.cuh"
 #include "fire_internal.cuh"
 
@@ -78,10 +82,18 @@ template <int KIND>
 inline size_t sl_a_bytes(long M, int K) {  // slices of M rows (whole 128-row tiles)
   return (size_t)sl_rows(M) * ((K + 15) / 16) * 32 * SlFmt<KIND>::NS;
 }
-// scratch of a contraction's A: the slices, then one exponent per row, for `batch` blocks of M rows
+// Row tiles of one pass over all segments and batch blocks: one per SM, as many whole tiles as that leaves to each of the
+// `blocks` segments and batch blocks.
+constexpr int SL_SMS = 152;
+inline long sl_pass_rows(long M, int blocks) {
+  return std::min<long>(sl_rows(M), 128 * std::max<long>(1, SL_SMS / blocks));
+}
+// scratch of a contraction's A: the slices of a pass, then one exponent per row, for every segment and batch block (M: the
+// larger segment's rows)
 template <int KIND>
-inline size_t sl_scratch_bytes(long M, int K, int batch = 1) {
-  return (size_t)batch * (sl_a_bytes<KIND>(M, K) + (size_t)sl_rows(M) * 4);
+inline size_t sl_scratch_bytes(long M, int K, int blocks = 1) {
+  const long r = sl_pass_rows(M, blocks);
+  return (size_t)blocks * ((sl_a_bytes<KIND>(r, K) + (size_t)r * 4 + 255) / 256 * 256);
 }
 
 // One contraction, or two that differ in their rows and weights (the spins).  Segment g multiplies its own rows
@@ -103,12 +115,13 @@ struct SlCall {
   const float* env_lo;
   long ld_lo;
 };
-cudaError_t sl_prepare_f32(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s);
+cudaError_t sl_prepare_pair(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s);
 cudaError_t sl_prepare_f64(const double* W, int K, int N, int batch, unsigned char* out, cudaStream_t s);
 // spins present in every 128-row tile (bit 0 up, bit 1 down) of a contraction's rows
 void sl_tile_mask(const GemmP<double>& p, int* mask, cudaStream_t s);
-// mode: CompMode for float, EpiMode for double.  scratch: sl_scratch_bytes per segment (each 256-byte aligned).
-cudaError_t sl_gemm_f32(int mode, const SlCall<float>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
-cudaError_t sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
+// mode: CompMode for hi + lo pairs, EpiMode for FP64.  scratch: sl_scratch_bytes over the call's segments (one if
+// they share A) and batch blocks, 256-byte aligned.  Returns the number of kernels launched, or -1 on an error.
+int sl_gemm_pair(int mode, const SlCall<float>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
+int sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
 
 }  // namespace fire
