@@ -406,6 +406,13 @@ size_t eloc_ws_bytes(const fire_problem* p, int Wc, size_t* list_off) {
   return KF > 0 ? t + ((size_t)(2 * KF + 1) * 4 + 255) / 256 * 256 : t;
 }
 
+// A pass of c walkers reduced to whole rounds of the elimination where that fills the GPU with two CTAs per SM (512 threads,
+// gjg_threads): 153 walkers of 322 electrons are 612 matrices, three rounds of 304 where 152 walkers take two.
+int whole_rounds(const fire_problem* p, int c) {
+  constexpr int ROUND = 2 * SL_SMS / NDET;  // walkers of a round
+  return gjg_threads(p->n_el) == 512 && c > ROUND ? c - c % ROUND : c;
+}
+
 int choose_chunk(const fire_problem* p, size_t ws_bytes, bool fl) {
   int B = p->n_walkers;
   auto need = [&](int c) { return fl ? eloc_ws_bytes(p, c, nullptr) : make_plan(p, c, fl).total; };
@@ -414,6 +421,7 @@ int choose_chunk(const fire_problem* p, size_t ws_bytes, bool fl) {
     // a fixed pass is reduced to what the CUDA-core contraction of the Jacobian planes can launch: 65535 row tiles
     // of 128 in the grid's y dimension
     if (fl) c = (int)std::min<long>(c, std::max<long>(1, 65535L * 128 / (3L * (p->n_el + p->cap_pairs))));
+    if (fl) c = whole_rounds(p, c);
     return need(c) <= ws_bytes ? c : 0;
   }
   // the rows of a pass's largest contraction (the Jacobian planes; the electron rows of the value path) stay within
@@ -425,7 +433,7 @@ int choose_chunk(const fire_problem* p, size_t ws_bytes, bool fl) {
     const int mid = (lo + hi + 1) / 2;
     if (need(mid) <= ws_bytes) lo = mid; else hi = mid - 1;
   }
-  return lo;
+  return fl && lo < p->n_walkers ? whole_rounds(p, lo) : lo;
 }
 
 // ------------------------------------------------------------------------------ prepare kernels
@@ -1043,7 +1051,7 @@ cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, 
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   g_nlaunch++;
-  kern<<<c.Wc * NDET, GJG_THREADS_DECL, smem, c.s>>>(A, A_lo, n, c.template buf<S>(c.P.gjw),
+  kern<<<c.Wc * NDET, gjg_threads(n), smem, c.s>>>(A, A_lo, n, c.template buf<S>(c.P.gjw),
                                                       c.template buf<double>(c.P.ld), c.template buf<double>(c.P.sd),
                                                       cond, Ainv, c.status);
   return cudaPeekAtLastError();

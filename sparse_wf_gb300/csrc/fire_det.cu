@@ -16,6 +16,7 @@
 //               -sum_xyz sum_{i,k} B[(i,m)][k] B[(k,m)][i]; the first Laplacian term tr(lap A A^-1) is
 //               accumulated row by row.
 #include "fire_df64.cuh"
+#include "fire_f32x2.cuh"
 #include "fire_internal.cuh"
 
 namespace fire {
@@ -53,23 +54,66 @@ __global__ void k_env_coef(const T* __restrict__ r, const float* __restrict__ R,
   }
 }
 
-// two adjacent elements with one 16-byte (double, df64) or 8-byte (float) shared-memory load; p is aligned to
-// twice the element size
-__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b) {
-  const float2 v = *reinterpret_cast<const float2*>(p);
-  a = v.x;
-  b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b) {
-  const double2 v = *reinterpret_cast<const double2*>(p);
-  a = v.x;
-  b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const df64* p, df64& a, df64& b) {
-  const float4 v = *reinterpret_cast<const float4*>(p);
-  a = df64(v.x, v.y);
-  b = df64(v.z, v.w);
-}
+// Two adjacent columns' SubDot sums against one row's factors; Y holds the columns' factors of one term, read with one
+// 16-byte load (8 bytes for float) from an aligned pair.
+template <typename S>
+struct PairDot {
+  struct Y {
+    S y0, y1;
+    __device__ __forceinline__ explicit Y(const S* p) : y0(p[0]), y1(p[1]) {}
+  };
+  SubDot<S> d0, d1;
+  __device__ __forceinline__ void add(S w, const Y& y) {
+    d0.add(w, y.y0);
+    d1.add(w, y.y1);
+  }
+  __device__ __forceinline__ S finish0(S a) const { return d0.finish(a); }
+  __device__ __forceinline__ S finish1(S a) const { return d1.finish(a); }
+};
+// double-FP32: SubDot<df64>'s operations on packed pairs, in the same order and with the same roundings.  The packed
+// instructions have no operand negation, so the sums run with the opposite sign (ns = -s; rounding to nearest is symmetric)
+// and differences are a - b = fma(b, -1, a).  Columns staged as (hi0, hi1, lo0, lo1).
+template <>
+struct PairDot<df64> {
+  struct Y {
+    f32x2 hi, lo;
+    __device__ __forceinline__ explicit Y(const df64* p) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+      hi = v.x;
+      lo = v.y;
+    }
+  };
+  f32x2 ns, c;
+  __device__ __forceinline__ PairDot() : ns(0x8000000080000000ull), c(0ull) {}
+  __device__ __forceinline__ void add(df64 w, const Y& y) {
+    const f32x2 m1 = pack2(-1.f, -1.f), wh = pack2(w.hi, w.hi), wl = pack2(w.lo, w.lo), nwh = pack2(-w.hi, -w.hi);
+    const f32x2 np = mul2(nwh, y.hi);      // -p
+    const f32x2 e = fma2(wh, y.hi, np);    // the product's exact low part
+    c = fma2(wh, y.lo, c);
+    c = fma2(wl, y.hi, c);
+    const f32x2 ns1 = add2(ns, np);        // -(s + p)
+    const f32x2 nbb = fma2(ns, m1, ns1);
+    const f32x2 nq = add2(fma2(fma2(nbb, m1, ns1), m1, ns), fma2(nbb, m1, np));  // -(TwoSum error)
+    c = add2(c, fma2(nq, m1, e));
+    ns = ns1;
+  }
+  __device__ __forceinline__ df64 finish(df64 a, float nsx, float cx) const {
+    const df64 r = df_two_sum(a.hi, nsx);
+    return df_two_sum(r.hi, __fadd_rn(r.lo, __fsub_rn(a.lo, cx)));
+  }
+  __device__ __forceinline__ df64 finish0(df64 a) const {
+    float n0, n1, c0, c1;
+    unpack2(ns, n0, n1);
+    unpack2(c, c0, c1);
+    return finish(a, n0, c0);
+  }
+  __device__ __forceinline__ df64 finish1(df64 a) const {
+    float n0, n1, c0, c1;
+    unpack2(ns, n0, n1);
+    unpack2(c, c0, c1);
+    return finish(a, n1, c1);
+  }
+};
 
 __device__ __forceinline__ uint32_t smem_u32_det(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -90,6 +134,10 @@ constexpr int GJG_BW = 16, GJG_THREADS = 512;
 //     of GJG_BW columns and updated with that rank-b product.
 // A: element (i, o) of matrix (w, d) at A[((w * n + i) * NDET + d) * n + o]  (the orbital plane [G][D * n]);
 // A_lo (double-FP32 elimination only, may be null): the low parts of the same elements.
+// The block has 32 to 512 threads (launch_gjg): n steps with three barriers each leave a small matrix waiting, so small
+// matrices take small blocks and more of them share an SM.  The double-FP32 update packs two columns (SubDot2: 12 packed
+// operations for two products; it is bound by their issue rate).  LU of 1024 matrices of 82: 1.53 ms with 512 threads each,
+// the logarithm of every pivot inside its step and scalar arithmetic.
 // Outputs: logdet[w * NDET + d], sign[...] (double); if INV the inverse, transposed and aligned for
 // k_detlap: Ainv[((w * NDET + d) * n + i) * ainv_ld(n) + sh + o] = (A^-1)[o][i] with sh = (d n) mod 4 and zeros
 // in the other entries of the row, written after undoing the column permutation; if INV and cond is not null,
@@ -146,14 +194,19 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
     for (int q = 0; q < nwarp; ++q) a2 += redd[q];
   double ld = 0.0;
   int neg = 0, sing = 0;
+  // the pivots, one per thread and round of steps (n <= 2 blockDim): their logarithms are taken together at the end
+  double pv_keep[2] = {1.0, 1.0};
   const int npan = (n + BW - 1) / BW;
   const int cj = tid % BW, rg = tid / BW, rn = blockDim.x / BW;  // chunk update: column, row group
+  // panel update: row, and its share of the columns when the block has several threads per row
+  const int nr32 = (n + 31) & ~31, ncg = max(1, (int)blockDim.x / nr32), cg = tid / nr32, prow = tid % nr32;
   for (int P = 0; P < npan; ++P) {
     const int k0 = P * BW, bw = min(BW, n - k0);
     const S* src = Mb[P & 1];
     S* dst = Mb[(P + 1) & 1];
     if (cj < bw)
       for (int i = rg; i < n; i += rn) pan[i * LD + cj] = src[(size_t)i * n + k0 + cj];
+    for (int i = tid; i < n; i += blockDim.x) rowmap[i] = i;
     __syncthreads();
     // ---- factor the panel
     for (int t = 0; t < bw; ++t) {
@@ -181,10 +234,9 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
         redi[wid] = bi;
       }
       __syncthreads();
-      S bv = lane < nwarp ? redv[lane] : S(-1);
-      int p = lane < nwarp ? redi[lane] : n;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
+      S bv = redv[lane & (nwarp - 1)];  // nwarp is a power of two
+      int p = redi[lane & (nwarp - 1)];
+      for (int o = nwarp >> 1; o > 0; o >>= 1) {
         const S ov = shfl_xor_any(bv, o);
         const int oi = __shfl_xor_sync(0xffffffffu, p, o);
         if (ov > bv || (ov == bv && oi < p)) {
@@ -194,21 +246,25 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
       }
       if (p >= n) p = k;
       const S pv = pan[p * LD + t];
-      const S ipv = pv != S(0) ? S(1) / pv : S(0);
-      if (tid == 0) {
-        piv[t] = p;
-        perm[k] = p;
-        if (pv == S(0)) sing = 1;
-        ld += ::log(::fabs((double)pv));
-        if (pv < S(0)) neg ^= 1;
-        if (p != k) neg ^= 1;
+      if (tid == k % (int)blockDim.x) pv_keep[k / (int)blockDim.x] = (double)pv;
+      if (wid == 0) {  // the inverse pivot (31: beyond the warps' entries) and the scaled pivot row
+        const S iv = pv != S(0) ? S(1) / pv : S(0);
+        if (lane == 0) {
+          redv[31] = iv;
+          piv[t] = p;
+          perm[k] = p;
+          if (pv == S(0)) sing = 1;
+          if (pv < S(0)) neg ^= 1;
+          if (p != k) neg ^= 1;
+        }
+        if (lane < bw) {
+          const S y = pan[p * LD + lane];
+          rk[lane] = pan[k * LD + lane];
+          rp[lane] = y;
+          rj[lane] = y * iv;
+        }
       }
       for (int i = (INV ? 0 : k) + tid; i < n; i += blockDim.x) colk[i] = pan[(i == k ? p : (i == p ? k : i)) * LD + t];
-      for (int j = tid; j < bw; j += blockDim.x) {
-        rk[j] = pan[k * LD + j];
-        rp[j] = pan[p * LD + j];
-        rj[j] = rp[j] * ipv;
-      }
       if (p != k)  // earlier transforms follow the interchange
         for (int s2 = tid; s2 < t; s2 += blockDim.x) {
           const S tk = W[k * LD + s2];
@@ -216,31 +272,25 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
           W[p * LD + s2] = tk;
         }
       __syncthreads();
-      if (INV) {  // Gauss-Jordan: every row of the panel columns not yet eliminated (the eliminated ones are
-                  // rebuilt from W~ after the panel)
-        const int nc = bw - t - 1;
-        if (nc > 0) {
-          const float inc = 1.f / (float)nc;
-          for (int e = tid; e < n * nc; e += blockDim.x) {
-            int i = (int)((float)e * inc);
-            if (i * nc > e) --i;
-            else if ((i + 1) * nc <= e) ++i;
-            const int j = t + 1 + (e - i * nc);
-            S* el = pan + i * LD + j;
-            *el = i == k ? rj[j] : df_sub_mul(i == p ? rk[j] : *el, colk[i], rj[j]);
+      const S ipv = redv[31];
+      // Gauss-Jordan: every row of the panel columns not yet eliminated (the eliminated ones are rebuilt from W~ after
+      // the panel).  LU: rows k.. of the panel columns right of the pivot (rows above k do not change).
+      if (cg < ncg)
+        for (int i = prow; i < n; i += nr32 > (int)blockDim.x ? (int)blockDim.x : nr32) {
+          S* row = pan + i * LD;
+          const S ci = INV || i >= k ? colk[i] : S(0);
+          const S ml = INV ? ci : (i > k ? ci * ipv : S(0));
+          if (INV) {
+            for (int j2 = t + 1 + cg; j2 < bw; j2 += ncg)
+              row[j2] = i == k ? rj[j2] : df_sub_mul(i == p ? rk[j2] : row[j2], ml, rj[j2]);
+          } else if (i >= k) {
+            for (int j2 = t + 1 + cg; j2 < bw; j2 += ncg) {
+              const S old = i == k ? rp[j2] : (i == p ? rk[j2] : row[j2]);
+              row[j2] = i > k ? df_sub_mul(old, ml, rp[j2]) : old;
+            }
           }
+          if (cg == 0) W[i * LD + t] = INV ? (i == k ? S(1) - ipv : ci * ipv) : ml;
         }
-      } else {  // LU: rows k.. of the panel columns right of the pivot (rows above k do not change)
-        const int nc = bw - t - 1, nr = n - k;
-        for (int e = tid; e < nr * nc; e += blockDim.x) {
-          const int ii = e / nc, i = k + ii, j = t + 1 + (e - ii * nc);
-          S* el = pan + i * LD + j;
-          const S old = i == k ? rp[j] : (i == p ? rk[j] : *el);
-          *el = i > k ? df_sub_mul(old, colk[i] * ipv, rp[j]) : old;
-        }
-      }
-      for (int i = tid; i < n; i += blockDim.x)
-        W[i * LD + t] = INV ? (i == k ? S(1) - ipv : colk[i] * ipv) : (i > k ? colk[i] * ipv : S(0));
       __syncthreads();
     }
     // ---- L^-1 (one lane per column s: Li[t][s] = -sum_{u=s}^{t-1} L[t][u] Li[u][s]) and W~ = W L^-1
@@ -252,7 +302,6 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
       }
     }
     if (tid == 0) {  // the panel's row interchanges as one permutation
-      for (int i = 0; i < n; ++i) rowmap[i] = i;
       for (int t = 0; t < bw; ++t) {
         const int q = piv[t];
         const int tmp = rowmap[k0 + t];
@@ -283,11 +332,21 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
     // order, rows padded to an even length) is staged over the panel buffer, which is free now; each thread
     // owns a pair of adjacent columns and walks its rows two at a time (2 x 2 tiles: three shared loads per
     // four products), reading the interchanged rows of src and writing dst (no in-place hazard).
+    // For double-FP32 a pair of columns is staged as (hi, hi, lo, lo), the operands of the packed update.
     S* Y = pan;
     const int ldy = n + (n & 1);
     for (int t = 0; t < bw; ++t) {
       const S* yr = src + (size_t)rowmap[k0 + t] * n;
-      for (int c = (INV ? 0 : k0 + bw) + tid; c < n; c += blockDim.x) Y[t * ldy + c] = yr[c];
+      for (int c = (INV ? 0 : k0 + bw) + tid; c < n; c += blockDim.x) {
+        if constexpr (std::is_same<S, df64>::value) {
+          const df64 y = yr[c];
+          float* q = reinterpret_cast<float*>(Y + t * ldy + (c & ~1)) + (c & 1);
+          q[0] = y.hi;
+          q[2] = y.lo;
+        } else {
+          Y[t * ldy + c] = yr[c];
+        }
+      }
     }
     __syncthreads();
     {
@@ -303,56 +362,53 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
           const S a00 = s0[0], a10 = s1[0];
           const S a01 = c1 ? s0[1] : S(0), a11 = c1 ? s1[1] : S(0);
           const S *w0 = W + i * LD, *w1 = W + (i + rn2) * LD;
-          SubDot<S> d00, d01, d10, d11;
+          PairDot<S> d0, d1;
           if (bw == BW) {
 #pragma unroll
             for (int t = 0; t < BW; ++t) {
-              S y0, y1;
-              ld_pair(Y + t * ldy + c, y0, y1);
-              const S wa = w0[t], wb = w1[t];
-              d00.add(wa, y0);
-              d01.add(wa, y1);
-              d10.add(wb, y0);
-              d11.add(wb, y1);
+              const typename PairDot<S>::Y y(Y + t * ldy + c);
+              d0.add(w0[t], y);
+              d1.add(w1[t], y);
             }
           } else {
             for (int t = 0; t < bw; ++t) {
-              S y0, y1;
-              ld_pair(Y + t * ldy + c, y0, y1);
-              const S wa = w0[t], wb = w1[t];
-              d00.add(wa, y0);
-              d01.add(wa, y1);
-              d10.add(wb, y0);
-              d11.add(wb, y1);
+              const typename PairDot<S>::Y y(Y + t * ldy + c);
+              d0.add(w0[t], y);
+              d1.add(w1[t], y);
             }
           }
           S* o0 = dst + (size_t)i * n + c;
           S* o1 = dst + (size_t)(i + rn2) * n + c;
-          o0[0] = d00.finish(a00);
-          o1[0] = d10.finish(a10);
+          o0[0] = d0.finish0(a00);
+          o1[0] = d1.finish0(a10);
           if (c1) {
-            o0[1] = d01.finish(a01);
-            o1[1] = d11.finish(a11);
+            o0[1] = d0.finish1(a01);
+            o1[1] = d1.finish1(a11);
           }
         }
         if (i < n) {
           const S* s0 = src + (size_t)rowmap[i] * n + c;
           const S a00 = s0[0], a01 = c1 ? s0[1] : S(0);
           const S* w0 = W + i * LD;
-          SubDot<S> d00, d01;
-          for (int t = 0; t < bw; ++t) {
-            S y0, y1;
-            ld_pair(Y + t * ldy + c, y0, y1);
-            d00.add(w0[t], y0);
-            d01.add(w0[t], y1);
-          }
+          PairDot<S> d0;
+          for (int t = 0; t < bw; ++t) d0.add(w0[t], typename PairDot<S>::Y(Y + t * ldy + c));
           S* o0 = dst + (size_t)i * n + c;
-          o0[0] = d00.finish(a00);
-          if (c1) o0[1] = d01.finish(a01);
+          o0[0] = d0.finish0(a00);
+          if (c1) o0[1] = d0.finish1(a01);
         }
       }
     }
     __syncthreads();  // dst complete before the next panel reads it
+  }
+  {
+    double* lg = reinterpret_cast<double*>(pan);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (tid + q * (int)blockDim.x < n) lg[tid + q * blockDim.x] = ::log(::fabs(pv_keep[q]));
+    __syncthreads();
+    if (tid == 0)
+      for (int k = 0; k < n; ++k) ld += lg[k];
+    __syncthreads();  // the panel buffer is staged over next
   }
   if (tid == 0) {
     logdet[mat] = ld;
@@ -362,8 +418,9 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
   if (INV) {
     // undo the row interchanges on the columns: final column jc holds working column src(jc)
     int* srcc = reinterpret_cast<int*>(colk);
+    for (int q = tid; q < n; q += blockDim.x) srcc[q] = q;
+    __syncthreads();
     if (tid == 0) {
-      for (int q = 0; q < n; ++q) srcc[q] = q;
       for (int k = n - 1; k >= 0; --k) {
         const int p = perm[k];
         if (p != k) {

@@ -1379,7 +1379,7 @@ fire_status grad_chunk_run(const fire_problem* p, cudaStream_t s, const float* R
     auto kern = k_gj_global<S, T, T, true>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return FIRE_ERR_CUDA;
-    kern<<<Wc * NDET, GJG_THREADS_DECL, smem, s>>>(B(P.A), (const T*)nullptr, n, reinterpret_cast<S*>(ws + P.gjw),
+    kern<<<Wc * NDET, gjg_threads(n), smem, s>>>(B(P.A), (const T*)nullptr, n, reinterpret_cast<S*>(ws + P.gjw),
                                                     reinterpret_cast<double*>(ws + P.ld),
                                                     reinterpret_cast<double*>(ws + P.sd), nullptr, B(P.Ainv), status);
   }

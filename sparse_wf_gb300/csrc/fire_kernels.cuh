@@ -41,7 +41,10 @@ __global__ void k_env_coef(const T* r, const float* R, const T* sp, int n, int n
 template <typename S, typename TI, typename TO, bool INV>
 __global__ void k_gj_global(const TI* A, const TI* A_lo, int n, S* work, double* logdet, double* sign, double* cond, TO* Ainv,
                             int32_t* status);
-constexpr int GJG_BW_DECL = 16, GJG_THREADS_DECL = 512;
+constexpr int GJG_BW_DECL = 16;
+// Threads per matrix of k_gj_global (a power of two warps; n <= 2 threads holds for every n): where a step's rows fill them.
+// LU / inverse of 1024 matrices at n = 82 and 2048 at n = 10 decided the lower lines, 612 at n = 322 the upper.
+inline int gjg_threads(int n) { return n <= 32 ? 32 : (n <= 128 ? 128 : (n <= 224 ? 256 : 512)); }
 template <typename T, int NT, int CLO, int CHI>
 __global__ void k_detlap(Nbr nb, Layout L, const T* Jp, const T* Ainv, const T* lapA, double* grad, double* lap,
                          int32_t* status);
