@@ -10,6 +10,7 @@
 //                messages Gamma_ij * silu(e_ij + h_ct[i] + h_nb[j]) with 6 tangents (center and
 //                neighbour coordinates) are summed into h[i]; d msg / d r_j becomes the Jacobian row of
 //                the pair (i, j) and d msg / d r_i accumulates into the self row.
+#include "fire_f32x2.cuh"
 #include "fire_internal.cuh"
 
 namespace fire {
@@ -93,54 +94,182 @@ __device__ __forceinline__ FLv<T, NT> fl_load(const T* src, int stride) {
   return a;
 }
 
-// Edge features and the filter of one edge, computed by one warp.  NT = 3: e-n edge (tangents =
-// electron coordinates); NT = 6: e-e edge (tangents 0..2 center, 3..5 neighbour).  Writes
-// beta[8] to sB[v * 8 + c] and the log-scaled features to sS[v * 4 + k], v over the stored rows.
-template <typename T, int NT, int NENV>
-__device__ __forceinline__ void edge_filter_warp(const T diff[3], const T* K /*[4][16]*/, const T* bias /*[16]*/,
-                                                 const T* inv_scale /*[NENV]*/, const T* dir_W /*[16][8]*/,
-                                                 const T* dir_b /*[8]*/, const T* env_W /*[NENV][8]*/,
-                                                 T inv_cutoff, FLv<T, NT>* wS /*[16]*/, FLv<T, NT>* wE /*[32]*/,
-                                                 T* sB, T* sS) {
-  constexpr int NV = NVr<NT>::v;
-  const int lane = threadIdx.x & 31;
-  // distance carrier
-  const T s2 = diff[0] * diff[0] + diff[1] * diff[1] + diff[2] * diff[2];
-  const T d = dsqrt(s2);
-  FLv<T, NT> fd;
-  fd.x = d;
-  fl_zero(fd);
-  fd.x = d;
+// Components of a carrier stored side by side (x, j[NT], l), padded to an even number.
+template <int NT>
+struct NVp {
+  static constexpr int v = NT > 0 ? (NT + 3) / 2 * 2 : 1;
+};
+template <typename T, int NT>
+__device__ __forceinline__ void fl_put(T* dst, const FLv<T, NT>& a) {
+  dst[0] = a.x;
   if (NT > 0) {
-    const T id = T(1) / d;
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      fd.j[t] = diff[t] * id;
-      if (NT == 6) fd.j[3 + t] = -diff[t] * id;
-    }
-    fd.l = (NT == 6 ? T(4) : T(2)) * id;
+    for (int t = 0; t < NT; ++t) dst[1 + t] = a.j[t];
+    dst[1 + NT] = a.l;
+    if (NVp<NT>::v > NT + 2) dst[NVp<NT>::v - 1] = T(0);
   }
-  auto feat = [&](int k) -> FLv<T, NT> {
-    if (k == 0) return fd;
+}
+template <typename T, int NT>
+__device__ __forceinline__ FLv<T, NT> fl_get(const T* src) {
+  FLv<T, NT> a;
+  a.x = src[0];
+  a.l = T(0);
+  if (NT > 0) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) a.j[t] = src[1 + t];
+    a.l = src[1 + NT];
+  }
+  return a;
+}
+// sum_c w[c] s_c over C carriers stored one after another (16-byte aligned), each component one chain of fused
+// multiply-adds over ascending c.  The block reads the same carriers for 256 features: 16-byte shared loads, in FP32 two
+// components per packed operation (scalar loads of every component were what these kernels waited for).
+template <typename T, int NT, int C>
+__device__ __forceinline__ FLv<T, NT> fl_dot(const T* s, const T (&w)[C]) {
+  constexpr int VP = NVp<NT>::v;
+  FLv<T, NT> r;
+  if constexpr (sizeof(T) == 4 && NT > 0) {
+    f32x2 acc[VP / 2];
+#pragma unroll
+    for (int v = 0; v < VP / 2; ++v) acc[v] = 0ull;
+#pragma unroll
+    for (int c = 0; c < C; c += 2) {  // two carriers: a whole number of 16-byte loads
+      f32x2 q[VP];
+#pragma unroll
+      for (int u = 0; u < VP / 2; ++u) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(s + c * VP + 4 * u);
+        q[2 * u] = x.x;
+        q[2 * u + 1] = x.y;
+      }
+      const f32x2 w0 = pack2(w[c], w[c]), w1 = pack2(w[c + 1], w[c + 1]);
+#pragma unroll
+      for (int v = 0; v < VP / 2; ++v) acc[v] = fma2(w0, q[v], acc[v]);
+#pragma unroll
+      for (int v = 0; v < VP / 2; ++v) acc[v] = fma2(w1, q[VP / 2 + v], acc[v]);
+    }
+    float e[VP];
+#pragma unroll
+    for (int v = 0; v < VP / 2; ++v) unpack2(acc[v], e[2 * v], e[2 * v + 1]);
+    r.x = e[0];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) r.j[t] = e[1 + t];
+    r.l = e[1 + NT];
+  } else {
+    constexpr int PER = 16 / sizeof(T);
+    T e[VP];
+#pragma unroll
+    for (int v = 0; v < VP; ++v) e[v] = T(0);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      T q[VP];
+      if constexpr (NT == 0) {
+        if (c % PER == 0) {  // PER carriers of one component per load
+          struct __align__(16) V {
+            T a[PER];
+          };
+          const V x = *reinterpret_cast<const V*>(s + c);
+#pragma unroll
+          for (int u = 0; u < PER; ++u)
+            if (c + u < C) e[0] = e[0] + w[c + u] * x.a[u];
+        }
+      } else {
+#pragma unroll
+        for (int v = 0; v < VP; v += 2) {
+          const double2 x = *reinterpret_cast<const double2*>(s + c * VP + v);
+          q[v] = x.x;
+          q[v + 1] = x.y;
+        }
+#pragma unroll
+        for (int v = 0; v < VP; ++v) e[v] += w[c] * q[v];
+      }
+    }
+    fl_zero(r);
+    r.x = e[0];
+    if constexpr (NT > 0) {
+#pragma unroll
+      for (int t = 0; t < NT; ++t) r.j[t] = e[1 + t];
+      r.l = e[1 + NT];
+    }
+  }
+  return r;
+}
+
+// Edges that a warp filters together, and edges staged per batch (8 warps): fewer where carriers of doubles would not fit
+// 48 KB of shared memory.
+template <typename T, int NT>
+struct EdgeBatch {
+  static constexpr int FE = sizeof(T) == 8 && NT > 0 ? 2 : 4, EB = 8 * FE;
+};
+
+// Scratch of one warp's filters.
+template <typename T, int NT, int NENV>
+struct FilterWs {
+  static constexpr int FE = EdgeBatch<T, NT>::FE;
+  FLv<T, NT> d[FE], S[FE][F0], E[FE][NENV];
+  T diff[FE][3];
+};
+// Weights of one edge's filter (PairwiseFilter, model/utils.py:393-433).
+template <typename T>
+struct FilterW {
+  const T *K /*[4][16]*/, *bias /*[16]*/, *inv_scale /*[NENV]*/, *dir_W /*[16][8]*/, *dir_b /*[8]*/, *env_W /*[NENV][8]*/;
+};
+// Edge features and filters of ne <= EdgeBatch::FE edges, computed by one warp: every step's (edge, unit) pairs are spread over the
+// lanes (one edge at a time left 16, 8 or 4 of them working, and repeated the distance and its logarithm).  NT = 3: e-n edge
+// (tangents = electron coordinates); NT = 6: e-e edge (tangents 0..2 center, 3..5 neighbour).  ws.diff holds the
+// differences; weights(e) gives the edge's weights.  Writes beta[8] of edge e to sB + e * 8 VP and its log-scaled
+// features to sS + e * 4 VP (carriers of VP components).
+template <typename T, int NT, int NENV, typename WF>
+__device__ __forceinline__ void edge_filters(int ne, WF weights, T inv_cutoff, FilterWs<T, NT, NENV>& ws, T* sB, T* sS) {
+  constexpr int VP = NVp<NT>::v;
+  const int lane = threadIdx.x & 31;
+  auto feat = [&](int e, int k) -> FLv<T, NT> {
+    if (k == 0) return ws.d[e];
     FLv<T, NT> f;
     fl_zero(f);
-    f.x = diff[k - 1];
+    f.x = ws.diff[e][k - 1];
     if (NT > 0) {
-      f.j[k - 1] = T(1);
-      if (NT == 6) f.j[k + 2] = T(-1);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        f.j[t] = t == k - 1 ? T(1) : T(0);
+        if (NT == 6) f.j[3 + t] = t == k - 1 ? T(-1) : T(0);
+      }
     }
     return f;
   };
-  if (lane < F0) {
+  if (lane < ne) {  // distance carriers
+    const T* diff = ws.diff[lane];
+    const T s2 = diff[0] * diff[0] + diff[1] * diff[1] + diff[2] * diff[2];
+    const T d = dsqrt(s2);
+    FLv<T, NT> fd;
+    fl_zero(fd);
+    fd.x = d;
+    if (NT > 0) {
+      const T id = T(1) / d;
+#pragma unroll
+      for (int t = 0; t < 3; ++t) {
+        fd.j[t] = diff[t] * id;
+        if (NT == 6) fd.j[3 + t] = -diff[t] * id;
+      }
+      fd.l = (NT == 6 ? T(4) : T(2)) * id;
+    }
+    ws.d[lane] = fd;
+  }
+  __syncwarp();
+  for (int q = lane; q < ne * F0; q += 32) {
+    const int e = q / F0, l = q % F0;
+    const FilterW<T> w = weights(e);
     FLv<T, NT> pre;
     fl_zero(pre);
-    pre.x = bias[lane];
+    pre.x = w.bias[l];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) fl_axpy(pre, K[k * F0 + lane], feat(k));
-    wS[lane] = fl_silu(pre);
+    for (int k = 0; k < 4; ++k) fl_axpy(pre, w.K[k * F0 + l], feat(e, k));
+    ws.S[e][l] = fl_silu(pre);
   }
-  if (lane < NENV) {
-    const T a = inv_scale[lane];
+  for (int q = lane; q < ne * NENV; q += 32) {
+    const int e = q / NENV, l = q % NENV;
+    const FLv<T, NT> fd = ws.d[e];
+    const T d = fd.x;
+    const T a = weights(e).inv_scale[l];
     const T u = d * a;
     const T g = dexp(-u * u);
     const T g1 = T(-2) * u * a * g;
@@ -149,22 +278,12 @@ __device__ __forceinline__ void edge_filter_warp(const T diff[3], const T* K /*[
     cutoff3(d * inv_cutoff, c, c1, c2);
     c1 *= inv_cutoff;
     c2 *= inv_cutoff * inv_cutoff;
-    wE[lane] = fl_apply(fd, g * c, g1 * c + g * c1, g2 * c + T(2) * g1 * c1 + g * c2);
+    ws.E[e][l] = fl_apply(fd, g * c, g1 * c + g * c1, g2 * c + T(2) * g1 * c1 + g * c2);
   }
-  __syncwarp();
-  if (lane < F1) {
-    FLv<T, NT> dirv, env8;
-    fl_zero(dirv);
-    fl_zero(env8);
-    dirv.x = dir_b[lane];
-#pragma unroll
-    for (int l = 0; l < F0; ++l) fl_axpy(dirv, dir_W[l * F1 + lane], wS[l]);
-#pragma unroll 8
-    for (int k = 0; k < NENV; ++k) fl_axpy(env8, env_W[k * F1 + lane], wE[k]);
-    const FLv<T, NT> beta = fl_mul(dirv, env8);
-    fl_store(sB + lane, F1, beta);
-  } else if (lane < F1 + 4) {
-    const int k = lane - F1;
+  if (lane < ne * 4) {  // log-scaled features
+    const int e = lane >> 2, k = lane & 3;
+    const FLv<T, NT> fd = ws.d[e];
+    const T d = fd.x;
     const T lp = dlog1p(d);
     FLv<T, NT> sf;
     if (k == 0) {
@@ -176,26 +295,36 @@ __device__ __forceinline__ void edge_filter_warp(const T diff[3], const T* K /*[
       const T psi = lp * id;
       const T psi1 = L1 * id - lp * id * id;
       const T psi2 = L2 * id - T(2) * L1 * id * id + T(2) * lp * id * id * id;
-      sf = fl_mul(feat(k), fl_apply(fd, psi, psi1, psi2));
+      sf = fl_mul(feat(e, k), fl_apply(fd, psi, psi1, psi2));
     }
-    fl_store(sS + k, 4, sf);
+    fl_put(sS + (e * 4 + k) * VP, sf);
   }
   __syncwarp();
-  (void)NV;
+  if (lane < ne * F1) {
+    const int e = lane / F1, c = lane % F1;
+    const FilterW<T> w = weights(e);
+    FLv<T, NT> dirv, env8;
+    fl_zero(dirv);
+    fl_zero(env8);
+    dirv.x = w.dir_b[c];
+#pragma unroll
+    for (int l = 0; l < F0; ++l) fl_axpy(dirv, w.dir_W[l * F1 + c], ws.S[e][l]);
+#pragma unroll 8
+    for (int k = 0; k < NENV; ++k) fl_axpy(env8, w.env_W[k * F1 + c], ws.E[e][k]);
+    fl_put(sB + (e * F1 + c) * VP, fl_mul(dirv, env8));
+  }
+  __syncwarp();
 }
-
-constexpr int EB = 32;  // edges staged per batch
 
 // One CTA (256 threads, thread = feature) per electron.  Output E5 [G][NV][F] (x, jac xyz, lap).
 template <typename T, int NT>
 __global__ void __launch_bounds__(256) k_elec_init(const T* __restrict__ r, const float* __restrict__ R,
                                                    Nbr nb, Weights<T> W, T inv_cutoff1, T* __restrict__ E5) {
-  constexpr int NV = NVr<NT>::v;
-  __shared__ T sB[EB][NV * F1];
-  __shared__ T sS[EB][NV * 4];
+  constexpr int NV = NVr<NT>::v, VP = NVp<NT>::v, FE = EdgeBatch<T, NT>::FE, EB = EdgeBatch<T, NT>::EB;
+  __shared__ __align__(16) T sB[EB * F1 * VP];
+  __shared__ __align__(16) T sS[EB * 4 * VP];
   __shared__ int sJ[EB];
-  __shared__ FLv<T, NT> wS[8][F0];
-  __shared__ FLv<T, NT> wE[8][NENV_EN];
+  __shared__ FilterWs<T, NT, NENV_EN> fw[8];
   __shared__ T red[32 * 6];
   const int g = blockIdx.x, f = threadIdx.x, lane = f & 31, wid = f >> 5;
   const int ne = nb.en_cnt[g];
@@ -211,38 +340,40 @@ __global__ void __launch_bounds__(256) k_elec_init(const T* __restrict__ r, cons
   FLv<T, NT> h;
   fl_zero(h);
   for (int e0 = 0; e0 < ne; e0 += EB) {
-    const int nbe = min(EB, ne - e0);
-    for (int e = wid; e < nbe; e += 8) {
-      const int J = eidx[e0 + e];
-      const T diff[3] = {rx - (T)R[3 * J], ry - (T)R[3 * J + 1], rz - (T)R[3 * J + 2]};
-      edge_filter_warp<T, NT, NENV_EN>(diff, W.w[FIRE_P_EN_KERNEL] + J * 4 * F0, W.w[FIRE_P_EN_BIAS] + J * F0,
-                                       W.w[PR_EN_INVSCALE] + J * NENV_EN, W.w[FIRE_P_EI_DIR_W],
-                                       W.w[FIRE_P_EI_DIR_B], W.w[FIRE_P_EI_ENV_W], inv_cutoff1, wS[wid], wE[wid],
-                                       sB[e], sS[e]);
-      if (lane == 0) sJ[e] = J;
+    const int nbe = min(EB, ne - e0), e1 = wid * FE, mine = min(FE, nbe - e1);  // this warp's edges of the batch
+    if (mine > 0) {
+      if (lane < mine) {
+        const int J = eidx[e0 + e1 + lane];
+        sJ[e1 + lane] = J;
+        fw[wid].diff[lane][0] = rx - (T)R[3 * J];
+        fw[wid].diff[lane][1] = ry - (T)R[3 * J + 1];
+        fw[wid].diff[lane][2] = rz - (T)R[3 * J + 2];
+      }
+      __syncwarp();
+      edge_filters<T, NT, NENV_EN>(
+          mine,
+          [&](int e) {
+            const int J = sJ[e1 + e];
+            return FilterW<T>{W.w[FIRE_P_EN_KERNEL] + J * 4 * F0, W.w[FIRE_P_EN_BIAS] + J * F0,
+                              W.w[PR_EN_INVSCALE] + J * NENV_EN, W.w[FIRE_P_EI_DIR_W], W.w[FIRE_P_EI_DIR_B],
+                              W.w[FIRE_P_EI_ENV_W]};
+          },
+          inv_cutoff1, fw[wid], sB + e1 * F1 * VP, sS + e1 * 4 * VP);
     }
     __syncthreads();
     const T* hn = W.w[FIRE_P_EN_NUC_EMB];
+    T emb = hn[sJ[0] * F + f];
     for (int e = 0; e < nbe; ++e) {
-      FLv<T, NT> G, E;
-      fl_zero(G);
-      fl_zero(E);
-#pragma unroll
-      for (int c = 0; c < F1; ++c) {
-        const FLv<T, NT> b = fl_load<T, NT>(&sB[e][c], F1);
-        fl_axpy(G, wg[c], b);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const FLv<T, NT> s = fl_load<T, NT>(&sS[e][k], 4);
-        fl_axpy(E, we[k], s);
-      }
-      E.x += hn[sJ[e] * F + f];
+      const T emb_next = e + 1 < nbe ? hn[sJ[e + 1] * F + f] : T(0);
+      const FLv<T, NT> G = fl_dot<T, NT, F1>(sB + e * F1 * VP, wg);
+      FLv<T, NT> E = fl_dot<T, NT, 4>(sS + e * 4 * VP, we);
+      E.x += emb;
       const FLv<T, NT> m = fl_mul(G, E);
       h.x += m.x;
       h.l += m.l;
 #pragma unroll
       for (int t = 0; t < NT; ++t) h.j[t] += m.j[t];
+      emb = emb_next;
     }
     __syncthreads();
   }
@@ -327,6 +458,14 @@ __global__ void k_silu5(T* __restrict__ Z, int G) {
   fl_store(Z + g * NV * F + f, F, fl_silu(a));
 }
 
+template <typename T>
+__device__ __forceinline__ FilterW<T> ee_filter(const Weights<T>& W, bool same) {
+  return same ? FilterW<T>{W.w[FIRE_P_EESAME_KERNEL], W.w[FIRE_P_EESAME_BIAS], W.w[PR_EESAME_INVSCALE],
+                           W.w[FIRE_P_EESAME_DIR_W], W.w[FIRE_P_EESAME_DIR_B], W.w[FIRE_P_EESAME_ENV_W]}
+              : FilterW<T>{W.w[FIRE_P_EEDIFF_KERNEL], W.w[FIRE_P_EEDIFF_BIAS], W.w[PR_EEDIFF_INVSCALE],
+                           W.w[FIRE_P_EEDIFF_DIR_W], W.w[FIRE_P_EEDIFF_DIR_B], W.w[FIRE_P_EEDIFF_ENV_W]};
+}
+
 // One CTA (256 threads) per center electron g.  E5o: [G][NV][5F] = h0 | ct_same | ct_diff | nb_same | nb_diff.
 // Outputs X [G][F], Lp [G][F] (if NT) and the Jacobian plane Jp [3 * positions][F] (if NT).
 template <typename T, int NT>
@@ -335,12 +474,11 @@ __global__ void __launch_bounds__(256) k_edge_contract(const T* __restrict__ r, 
                                                        T* __restrict__ Lp, T* __restrict__ Jp) {
   constexpr int NV = NVr<NT>::v;       // rows of the electron carriers (NT_e = 3 tangents)
   constexpr int NT6 = NT > 0 ? 6 : 0;  // pair carriers
-  constexpr int NV6 = NVr<NT6>::v;
-  __shared__ T sB[EB][NV6 * F1];
-  __shared__ T sS[EB][NV6 * 4];
+  constexpr int VP = NVp<NT6>::v, FE = EdgeBatch<T, NT6>::FE, EB = EdgeBatch<T, NT6>::EB;
+  __shared__ __align__(16) T sB[EB * F1 * VP];
+  __shared__ __align__(16) T sS[EB * 4 * VP];
   __shared__ int sj[EB];
-  __shared__ FLv<T, NT6> wS[8][F0];
-  __shared__ FLv<T, NT6> wE[8][NENV_EE];
+  __shared__ FilterWs<T, NT6, NENV_EE> fw[8];
   const int g = blockIdx.x, f = threadIdx.x, lane = f & 31, wid = f >> 5;
   const int n = nb.n, w = g / n, i = g - w * n;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
@@ -370,41 +508,42 @@ __global__ void __launch_bounds__(256) k_edge_contract(const T* __restrict__ r, 
   T ax = T(0), al = T(0), aj[3] = {T(0), T(0), T(0)};
   const long q0 = NT > 0 ? (long)L.pos_off[w] + rp[i] + i : 0;
   for (int k0 = 0; k0 < deg; k0 += EB) {
-    const int nbe = min(EB, deg - k0);
-    for (int e = wid; e < nbe; e += 8) {
-      const int j = nbl[k0 + e];
-      const int gj = w * n + j;
-      const T diff[3] = {rx - r[3 * gj], ry - r[3 * gj + 1], rz - r[3 * gj + 2]};
-      const bool same = (j < nb.n_up) == si;
-      if (same)
-        edge_filter_warp<T, NT6, NENV_EE>(diff, W.w[FIRE_P_EESAME_KERNEL], W.w[FIRE_P_EESAME_BIAS],
-                                          W.w[PR_EESAME_INVSCALE], W.w[FIRE_P_EESAME_DIR_W],
-                                          W.w[FIRE_P_EESAME_DIR_B], W.w[FIRE_P_EESAME_ENV_W], inv_c, wS[wid],
-                                          wE[wid], sB[e], sS[e]);
-      else
-        edge_filter_warp<T, NT6, NENV_EE>(diff, W.w[FIRE_P_EEDIFF_KERNEL], W.w[FIRE_P_EEDIFF_BIAS],
-                                          W.w[PR_EEDIFF_INVSCALE], W.w[FIRE_P_EEDIFF_DIR_W],
-                                          W.w[FIRE_P_EEDIFF_DIR_B], W.w[FIRE_P_EEDIFF_ENV_W], inv_c, wS[wid],
-                                          wE[wid], sB[e], sS[e]);
-      if (lane == 0) sj[e] = same ? j : -1 - j;
+    const int nbe = min(EB, deg - k0), e1 = wid * FE, mine = min(FE, nbe - e1);  // this warp's edges of the batch
+    if (mine > 0) {
+      if (lane < mine) {
+        const int j = nbl[k0 + e1 + lane], gj = w * n + j;
+        sj[e1 + lane] = (j < nb.n_up) == si ? j : -1 - j;
+        fw[wid].diff[lane][0] = rx - r[3 * gj];
+        fw[wid].diff[lane][1] = ry - r[3 * gj + 1];
+        fw[wid].diff[lane][2] = rz - r[3 * gj + 2];
+      }
+      __syncwarp();
+      edge_filters<T, NT6, NENV_EE>(mine, [&](int e) { return ee_filter(W, sj[e1 + e] >= 0); }, inv_c, fw[wid],
+                                    sB + e1 * F1 * VP, sS + e1 * 4 * VP);
     }
     __syncthreads();
+    // message map of edge e's neighbour
+    auto nb_row = [&](int e) {
+      const int code = sj[e], j = code >= 0 ? code : -1 - code;
+      return E5o + (size_t)(w * n + j) * NV * 5 * F + (code >= 0 ? 3 : 4) * F + f;
+    };
+    FLv<T, NT> hn = fl_load<T, NT>(nb_row(0), 5 * F);
     for (int e = 0; e < nbe; ++e) {
-      const int code = sj[e];
-      const bool same = code >= 0;
-      const int j = same ? code : -1 - code;
-      const int s = same ? 0 : 1;
+      const bool same = sj[e] >= 0;
+      FLv<T, NT> next = hn;
+      if (e + 1 < nbe) next = fl_load<T, NT>(nb_row(e + 1), 5 * F);  // in flight while this edge is summed
       FLv<T, NT6> G, E;
-      fl_zero(G);
-      fl_zero(E);
-#pragma unroll
-      for (int c = 0; c < F1; ++c) fl_axpy(G, wg[s][c], fl_load<T, NT6>(&sB[e][c], F1));
-#pragma unroll
-      for (int k = 0; k < 4; ++k) fl_axpy(E, we[s][k], fl_load<T, NT6>(&sS[e][k], 4));
-      E.x += be[s];
+      if (same) {
+        G = fl_dot<T, NT6, F1>(sB + e * F1 * VP, wg[0]);
+        E = fl_dot<T, NT6, 4>(sS + e * 4 * VP, we[0]);
+        E.x += be[0];
+      } else {
+        G = fl_dot<T, NT6, F1>(sB + e * F1 * VP, wg[1]);
+        E = fl_dot<T, NT6, 4>(sS + e * 4 * VP, we[1]);
+        E.x += be[1];
+      }
       // u = e + h_ct[i] (tangents 0..2) + h_nb[j] (tangents 3..5)
       const FLv<T, NT>& ct = same ? cts : ctd;
-      const FLv<T, NT> hn = fl_load<T, NT>(E5o + (size_t)(w * n + j) * NV * 5 * F + (same ? 3 : 4) * F + f, 5 * F);
       FLv<T, NT6> u = E;
       u.x += ct.x + hn.x;
       if (NT > 0) {
@@ -425,6 +564,7 @@ __global__ void __launch_bounds__(256) k_edge_contract(const T* __restrict__ r, 
 #pragma unroll
         for (int t = 0; t < 3; ++t) Jp[(3 * q + t) * F + f] = msg.j[3 + t];
       }
+      hn = next;
     }
     __syncthreads();
   }
@@ -447,11 +587,11 @@ __global__ void __launch_bounds__(256) k_lr_contract(const T* __restrict__ rn, i
                                                      const int* __restrict__ S_cnt, int KS,
                                                      Weights<T> W, const T* __restrict__ E5, const T* __restrict__ E5p,
                                                      T* __restrict__ HS) {
-  __shared__ T sB[EB][F1];
-  __shared__ T sS[EB][4];
+  constexpr int FE = EdgeBatch<T, 0>::FE, EB = EdgeBatch<T, 0>::EB;
+  __shared__ __align__(16) T sB[EB * F1];
+  __shared__ __align__(16) T sS[EB * 4];
   __shared__ int sj[EB];
-  __shared__ FLv<T, 0> wS[8][F0];
-  __shared__ FLv<T, 0> wE[8][NENV_EE];
+  __shared__ FilterWs<T, 0, NENV_EE> fw[8];
   __shared__ int snb[ELOC_MAX_EL];
   __shared__ int wcnt[8];
   const int slot = blockIdx.x, w = blockIdx.y, f = threadIdx.x, lane = f & 31, wid = f >> 5;
@@ -504,33 +644,32 @@ __global__ void __launch_bounds__(256) k_lr_contract(const T* __restrict__ rn, i
   const T h0 = ec[f], cts = ec[F + f], ctd = ec[2 * F + f];
   T ax = T(0);
   for (int k0 = 0; k0 < deg; k0 += EB) {
-    const int nbe = min(EB, deg - k0);
-    for (int q = wid; q < nbe; q += 8) {
-      const int j = snb[k0 + q];
-      const T diff[3] = {rx - rw[3 * j], ry - rw[3 * j + 1], rz - rw[3 * j + 2]};
-      const bool same = (j < n_up) == si;
-      if (same)
-        edge_filter_warp<T, 0, NENV_EE>(diff, W.w[FIRE_P_EESAME_KERNEL], W.w[FIRE_P_EESAME_BIAS],
-                                        W.w[PR_EESAME_INVSCALE], W.w[FIRE_P_EESAME_DIR_W], W.w[FIRE_P_EESAME_DIR_B],
-                                        W.w[FIRE_P_EESAME_ENV_W], inv_c, wS[wid], wE[wid], sB[q], sS[q]);
-      else
-        edge_filter_warp<T, 0, NENV_EE>(diff, W.w[FIRE_P_EEDIFF_KERNEL], W.w[FIRE_P_EEDIFF_BIAS],
-                                        W.w[PR_EEDIFF_INVSCALE], W.w[FIRE_P_EEDIFF_DIR_W], W.w[FIRE_P_EEDIFF_DIR_B],
-                                        W.w[FIRE_P_EEDIFF_ENV_W], inv_c, wS[wid], wE[wid], sB[q], sS[q]);
-      if (lane == 0) sj[q] = same ? j : -1 - j;
+    const int nbe = min(EB, deg - k0), e1 = wid * FE, mine = min(FE, nbe - e1);  // this warp's edges of the batch
+    if (mine > 0) {
+      if (lane < mine) {
+        const int j = snb[k0 + e1 + lane];
+        sj[e1 + lane] = (j < n_up) == si ? j : -1 - j;
+        fw[wid].diff[lane][0] = rx - rw[3 * j];
+        fw[wid].diff[lane][1] = ry - rw[3 * j + 1];
+        fw[wid].diff[lane][2] = rz - rw[3 * j + 2];
+      }
+      __syncwarp();
+      edge_filters<T, 0, NENV_EE>(mine, [&](int e) { return ee_filter(W, sj[e1 + e] >= 0); }, inv_c, fw[wid],
+                                  sB + e1 * F1, sS + e1 * 4);
     }
     __syncthreads();
     for (int q = 0; q < nbe; ++q) {
       const int code = sj[q];
       const bool same = code >= 0;
       const int j = same ? code : -1 - code;
-      const int s = same ? 0 : 1;
-      T G = T(0), E = T(0);
-#pragma unroll
-      for (int u = 0; u < F1; ++u) G += wg[s][u] * sB[q][u];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) E += we[s][u] * sS[q][u];
-      E += be[s];
+      T G, E;
+      if (same) {
+        G = fl_dot<T, 0, F1>(sB + q * F1, wg[0]).x;
+        E = fl_dot<T, 0, 4>(sS + q * 4, we[0]).x + be[0];
+      } else {
+        G = fl_dot<T, 0, F1>(sB + q * F1, wg[1]).x;
+        E = fl_dot<T, 0, 4>(sS + q * 4, we[1]).x + be[1];
+      }
       const T* ej = e5row(j);
       const T u = E + ((same ? cts : ctd) + ej[(same ? 3 : 4) * F + f]);
       T y, d1, d2;
