@@ -595,8 +595,10 @@ struct Ctx {
   // other neighbouring float.  log|psi| hardly sees that (10^-8); a local energy near a node, where the terms cancel to 10^-4
   // and less, moved by up to 10^-4 of itself.  A local energy keeps the sums it always had.
   bool pair = false;
-  // the refinement pass's FP64 value path: its envelope rows by k_gemm_env_df
-  bool env_df = false;
+  // the refinement pass's FP64 value path: plain FP64 sums instead of sliced ones, envelope rows by k_gemm_env_df.  Its walkers'
+  // orbital matrices have condition numbers up to 10^11, which turned the two's difference (10^-16, the sliced sums being the
+  // more exact) into up to 7 10^-5 of a batch's largest energies.
+  bool refine64 = false;
   TcWeights tcw[TC_COUNT];
   const unsigned char* slw[SLW_COUNT];  // sliced weights
   template <typename U>
@@ -629,6 +631,16 @@ void setup_ctx(Ctx<T>& c, bool fl) {
     c.L.cap_pos = c.Wc * (p->n_el + p->cap_pairs);
   } else {
     std::memset(&c.L, 0, sizeof(c.L));
+  }
+}
+
+// The refinement pass's chunks hold a device-counted number of walkers (Nbr::live): their rows only.  g.M is a whole number
+// of rows per walker; Jacobian rows carry their own count (pos_off, of the same walkers).
+template <typename T>
+void live_rows(const Ctx<T>& c, GemmP<T>& g) {
+  if (c.nb.live && !g.M_dev) {
+    g.M_dev = c.nb.live;
+    g.M_scale = g.M / c.Wc;
   }
 }
 
@@ -673,7 +685,8 @@ SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, const unsigned char* 
 }
 // SL_F64: mode is an EpiMode; SL_PAIR (hi + lo value rows): a CompMode
 template <typename T>
-cudaError_t sl_gemm(const Ctx<T>& c, int mode, const SlCall<T>& q) {
+cudaError_t sl_gemm(const Ctx<T>& c, int mode, SlCall<T> q) {
+  for (int g = 0; g < q.nseg; ++g) live_rows(c, q.p[g]);
   Prof pr(sizeof(T) == 4 ? "gemm_comp" : "gemm", c.s);
   unsigned char* scratch = c.template buf<unsigned char>(c.P.sl);
   int k;
@@ -688,8 +701,9 @@ cudaError_t sl_gemm(const Ctx<T>& c, int mode, const SlCall<T>& q) {
 template <typename T, int MODE>
 cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
   if constexpr (sizeof(T) == 8) {
-    if (sl_id >= 0) return sl_gemm(c, MODE, sl_call(g, c.slw[sl_id]));
+    if (sl_id >= 0 && !c.refine64) return sl_gemm(c, MODE, sl_call(g, c.slw[sl_id]));
   }
+  live_rows(c, g);
   // profile stages: "gemm_tc" the mixed path's tensor-core contractions, "gemm" the others
   const bool tc = sizeof(T) == 4 && c.mixed && tc_id >= 0;
   Prof pr(tc ? "gemm_tc" : "gemm", c.s);
@@ -705,7 +719,8 @@ cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
 
 // hi + lo value rows by the CUDA cores: low parts into C_lo / read from env_lo, row stride ld_lo
 template <int MODE>
-cudaError_t gemm_comp(const Ctx<float>& c, const GemmP<float>& g, float* C_lo, const float* env_lo, long ld_lo) {
+cudaError_t gemm_comp(const Ctx<float>& c, GemmP<float> g, float* C_lo, const float* env_lo, long ld_lo) {
+  live_rows(c, g);
   Prof pr("gemm_comp", c.s);
   g_nlaunch++;
   return launch_gemm_comp<MODE>(g, C_lo, env_lo, ld_lo, c.s);
@@ -942,10 +957,11 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     };
     cudaError_t e = cudaSuccess;
     if constexpr (sizeof(T) == 8) {
-      if (!c.env_df) {
+      if (!c.refine64) {
         e = sl_gemm(c, EPI_ENV, both(NV));
       } else {
-        e = each(both(NV), [&](const GemmP<T>& g, int) {
+        e = each(both(NV), [&](GemmP<T> g, int) {
+          live_rows(c, g);
           Prof pg("gemm", c.s);
           g_nlaunch++;
           return launch_gemm_env_df(g, c.s);
@@ -967,7 +983,9 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   g.ldb = DN; g.bias = c.W.w[FIRE_P_ORB_UP_B]; g.bias2 = c.W.w[FIRE_P_ORB_DN_B];
   g.C = c.template buf<T>(c.P.Apl); g.ldc = DN; g.M = G; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.aux0 = c.template buf<T>(c.P.rawx); g.aux1 = env; g.ld_aux = DN; g.env_nv = NV;
-  if (sizeof(T) == 8 || c.pair) {
+  if (c.refine64) {
+    gemm<T, EPI_ORB_X>(c, g);
+  } else if (sizeof(T) == 8 || c.pair) {
     SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN], 1);
     q.map_a = 1;
     if constexpr (sizeof(T) == 4) {
@@ -1053,7 +1071,7 @@ cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, 
   g_nlaunch++;
   kern<<<c.Wc * NDET, gjg_threads(n), smem, c.s>>>(A, A_lo, n, c.template buf<S>(c.P.gjw),
                                                       c.template buf<double>(c.P.ld), c.template buf<double>(c.P.sd),
-                                                      cond, Ainv, c.status);
+                                                      cond, Ainv, c.nb.live, c.status);
   return cudaPeekAtLastError();
 }
 
@@ -1383,7 +1401,8 @@ __global__ void k_refine_gather(const T* __restrict__ r, int n, const int32_t* _
 // (embedding, update, envelopes, orbitals) of their positions, then the chunk evaluation of the same positions with
 // those orbital matrices eliminated in FP64 and the derivative planes on the FP32 CUDA cores; the results go to the
 // walkers' rows.  The list is evaluated in passes of KC <= Wc walkers (the batch's chunk size, so that they fit
-// the workspace); a pass whose walkers are all beyond the count exits in its assembly.
+// the workspace); a pass's kernels leave the walkers beyond the device's count alone (Nbr::live), so that a capacity well
+// above it costs the launches only.
 template <typename T>
 cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const float* R, const float* Z,
                         const void* prepared, const T* r, void* logpsi, void* sign, void* eloc,
@@ -1407,8 +1426,9 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
                                        ws + L.c64, KC, false);
     c64.w0 = 0;
     c64.Wc = KC;
-    c64.env_df = true;
+    c64.refine64 = true;
     c64.r = r64;
+    c64.nb.live = sub_cnt + j;
     setup_ctx(c64, false);
     stage_neighbors(c64, false);
     stage_embedding<double, 0>(c64);
@@ -1418,6 +1438,7 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     c.w0 = 0;
     c.Wc = KC;
     c.r = r_ref;
+    c.nb.live = sub_cnt + j;
     Refine sub = rf;
     sub.idx = rf.idx + k0;
     sub.cnt = sub_cnt + j;

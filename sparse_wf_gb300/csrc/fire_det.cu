@@ -147,11 +147,12 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
                                                              int n, S* __restrict__ work,
                                                              double* __restrict__ logdet, double* __restrict__ sign,
                                                              double* __restrict__ cond, TO* __restrict__ Ainv,
-                                                             int32_t* status) {
+                                                             const int* __restrict__ live, int32_t* status) {
   extern __shared__ __align__(16) unsigned char gj_smem[];
   constexpr int BW = GJG_BW, LD = GJG_BW + 1;  // shared rows padded: column walks spread over the banks
   const int mat = blockIdx.x;
   const int w = mat / NDET, d = mat - w * NDET;
+  if (live && w >= *live) return;
   // two working copies per matrix: every panel reads one and writes the other
   S* Mb[2] = {work + (size_t)mat * n * n, work + ((size_t)gridDim.x + mat) * n * n};
   S* pan = reinterpret_cast<S*>(gj_smem);  // [n][LD] the panel, then each chunk of other columns
@@ -514,6 +515,7 @@ __global__ void __launch_bounds__(NT) k_detlap(Nbr nb, Layout L, const T* __rest
   extern __shared__ __align__(16) unsigned char dl_smem[];
   const int n = nb.n, nA = ainv_ld(n);
   const int m = blockIdx.x, d = blockIdx.y, w = blockIdx.z;
+  if (!walker_live(nb, w)) return;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
   if (rp[n] > nb.cap_p) return;
   const int cnt = rp[m + 1] - rp[m] + 1;
@@ -698,17 +700,17 @@ template __global__ void k_env_coef<double, 1>(const double*, const float*, cons
 template __global__ void k_env_coef<double, 5>(const double*, const float*, const double*, int, int, int, int,
                                                int, double*);
 template __global__ void k_gj_global<df64, float, float, false>(const float*, const float*, int, df64*, double*, double*, double*,
-                                                                 float*, int32_t*);
+                                                                 float*, const int*, int32_t*);
 template __global__ void k_gj_global<df64, float, float, true>(const float*, const float*, int, df64*, double*, double*, double*,
-                                                                float*, int32_t*);
+                                                                float*, const int*, int32_t*);
 // FP64 elimination of FP64 orbital matrices with the inverse in FP32 (the refinement pass of the FP32 / mixed local
 // energy, whose determinant Laplacian reads an FP32 inverse)
 template __global__ void k_gj_global<double, double, float, true>(const double*, const double*, int, double*, double*, double*,
-                                                                   double*, float*, int32_t*);
+                                                                   double*, float*, const int*, int32_t*);
 template __global__ void k_gj_global<double, double, double, true>(const double*, const double*, int, double*, double*, double*,
-                                                                    double*, double*, int32_t*);
+                                                                    double*, double*, const int*, int32_t*);
 template __global__ void k_gj_global<double, double, double, false>(const double*, const double*, int, double*, double*, double*,
-                                                                     double*, double*, int32_t*);
+                                                                     double*, double*, const int*, int32_t*);
 template __global__ void k_detlap<float, 128, 0, DL_CSPLIT>(Nbr, Layout, const float*, const float*, const float*,
                                                             double*, double*, int32_t*);
 template __global__ void k_detlap<float, 256, DL_CSPLIT, DL_CMAX>(Nbr, Layout, const float*, const float*,

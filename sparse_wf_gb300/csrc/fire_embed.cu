@@ -327,6 +327,7 @@ __global__ void __launch_bounds__(256) k_elec_init(const T* __restrict__ r, cons
   __shared__ FilterWs<T, NT, NENV_EN> fw[8];
   __shared__ T red[32 * 6];
   const int g = blockIdx.x, f = threadIdx.x, lane = f & 31, wid = f >> 5;
+  if (!walker_live(nb, g / nb.n)) return;
   const int ne = nb.en_cnt[g];
   const int* eidx = nb.en_idx + (size_t)g * nb.cap_nuc;
   const T rx = r[3 * g], ry = r[3 * g + 1], rz = r[3 * g + 2];
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(256) k_edge_contract(const T* __restrict__ r, 
   __shared__ FilterWs<T, NT6, NENV_EE> fw[8];
   const int g = blockIdx.x, f = threadIdx.x, lane = f & 31, wid = f >> 5;
   const int n = nb.n, w = g / n, i = g - w * n;
+  if (!walker_live(nb, w)) return;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
   const int P = rp[n];
   if (P > nb.cap_p) return;

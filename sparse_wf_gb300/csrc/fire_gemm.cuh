@@ -50,8 +50,6 @@ struct GemmP {
   int row_skip;          // tensor-core path: rows with row % row_skip == 0 are not stored (0: none)
 };
 
-constexpr int GBM = 128, GBN = 128, GBK = 8, GTHREADS = 256;
-
 template <typename T>
 __device__ __forceinline__ int gemm_node(const GemmP<T>& p, int row) {
   return p.node_map ? p.node_map[row / p.node_div] : row / p.node_div;
@@ -111,167 +109,10 @@ __device__ __forceinline__ void gemm_store(const GemmP<T>& p, int row, int col, 
   }
 }
 
-template <typename T, int MODE>
-__global__ void __launch_bounds__(GTHREADS) k_gemm(GemmP<T> p) {
-  __shared__ __align__(16) T As[2][GBK][GBM];
-  __shared__ __align__(16) T Bs[2][GBK][GBN];
-  extern __shared__ __align__(16) unsigned char gemm_dyn[];  // SILU_J: [GBM][GBN + 1] squares
-  __shared__ int row_node[GBM];
-
-  int rows = p.M;
-  if (p.M_dev) rows = min(rows, p.M_scale * (*p.M_dev));
-  const int m0 = blockIdx.y * GBM, n0 = blockIdx.x * GBN;
-  if (m0 >= rows) return;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-
-  // spin composition of the tile (per-spin weights)
-  int passes = 1, first_spin = 0;
-  if (p.B2) {
-    int up = 0, dn = 0;
-    if (tid < GBM && m0 + tid < rows) {
-      const int node = gemm_node(p, m0 + tid);
-      if ((node % p.n_el) < p.n_up) up = 1; else dn = 1;
-    }
-    up = __syncthreads_or(up);
-    dn = __syncthreads_or(dn);
-    first_spin = up ? 0 : 1;
-    passes = up + dn;
-  }
-  if (MODE == EPI_SILU_J) {
-    if (tid < GBM) row_node[tid] = (m0 + tid < rows) ? gemm_node(p, m0 + tid) : -1;
-  }
-
-  for (int pass = 0; pass < passes; ++pass) {
-    const int spin = first_spin + pass;
-    const T* Bp = spin == 0 ? p.B : p.B2;
-    T acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) acc[i][j] = T(0);
-
-    // global -> register staging: A: row a_r, k a_k..a_k+3; B: k b_k, cols b_c..b_c+3
-    const int a_r = tid >> 1, a_k = (tid & 1) * 4;
-    const int b_k = tid >> 5, b_c = (tid & 31) * 4;
-    T ra[4], rb[4];
-    // FP32 with 16-byte aligned rows: one vector load per operand whenever the 4 elements are in range
-    const bool va = sizeof(T) == 4 && p.lda % 4 == 0 && (reinterpret_cast<uintptr_t>(p.A) & 15) == 0;
-    const bool vb = sizeof(T) == 4 && p.ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(Bp) & 15) == 0;
-    auto load_tile = [&](int k0) {
-      const int gr = m0 + a_r;
-      if (va && gr < rows && k0 + a_k + 3 < p.K) {
-        const float4 q = *reinterpret_cast<const float4*>(p.A + (long)gr * p.lda + k0 + a_k);
-        ra[0] = q.x; ra[1] = q.y; ra[2] = q.z; ra[3] = q.w;
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int gk = k0 + a_k + u;
-          ra[u] = (gr < rows && gk < p.K) ? p.A[(long)gr * p.lda + gk] : T(0);
-        }
-      }
-      const int gk = k0 + b_k;
-      if (vb && gk < p.K && n0 + b_c + 3 < p.N) {
-        const float4 q = *reinterpret_cast<const float4*>(Bp + (long)gk * p.ldb + n0 + b_c);
-        rb[0] = q.x; rb[1] = q.y; rb[2] = q.z; rb[3] = q.w;
-      } else {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int gc = n0 + b_c + u;
-          rb[u] = (gk < p.K && gc < p.N) ? Bp[(long)gk * p.ldb + gc] : T(0);
-        }
-      }
-    };
-    auto store_tile = [&](int buf) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) As[buf][a_k + u][a_r] = ra[u];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) Bs[buf][b_k][b_c + u] = rb[u];
-    };
-    load_tile(0);
-    store_tile(0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < p.K; k0 += GBK) {
-      const bool more = k0 + GBK < p.K;
-      if (more) load_tile(k0 + GBK);
-#pragma unroll
-      for (int kk = 0; kk < GBK; ++kk) {
-        T a[8], b[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          a[i] = As[buf][kk][ty * 4 + i];
-          a[4 + i] = As[buf][kk][64 + ty * 4 + i];
-          b[i] = Bs[buf][kk][tx * 4 + i];
-          b[4 + i] = Bs[buf][kk][64 + tx * 4 + i];
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[i][j] += a[i] * b[j];
-      }
-      if (more) {
-        store_tile(buf ^ 1);
-        __syncthreads();
-        buf ^= 1;
-      }
-    }
-
-    // ---- epilogue
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int lr = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
-      const int row = m0 + lr;
-      if (row >= rows) continue;
-      if (p.B2) {
-        const int node = gemm_node(p, row);
-        const int s = ((node % p.n_el) < p.n_up) ? 0 : 1;
-        if (s != spin) continue;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int col = n0 + ((j < 4) ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-        if (col < p.N) gemm_store<T, MODE>(p, row, col, acc[i][j], spin);
-      }
-    }
-    if (MODE == EPI_SILU_J) {
-      // segmented sum of acc^2 over rows of the same center, one atomic per (segment, column)
-      T* sq = reinterpret_cast<T*>(gemm_dyn);
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int lr = (i < 4) ? ty * 4 + i : 64 + ty * 4 + (i - 4);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int lc = (j < 4) ? tx * 4 + j : 64 + tx * 4 + (j - 4);
-          sq[lr * (GBN + 1) + lc] = acc[i][j] * acc[i][j];
-        }
-      }
-      __syncthreads();
-      // 256 threads: column lc = tid & 127, rows half (tid >> 7)
-      const int lc = tid & (GBN - 1), half = tid >> 7;
-      const int col = n0 + lc;
-      if (col < p.N) {
-        int cur = -1;
-        T s = T(0);
-        for (int lr = half * 64; lr < half * 64 + 64; ++lr) {
-          const int nd = row_node[lr];
-          if (nd != cur) {
-            if (cur >= 0) atomic_add(&p.aux2[(long)cur * p.ld_aux + col], s);
-            cur = nd;
-            s = T(0);
-          }
-          if (nd >= 0) s += sq[lr * (GBN + 1) + lc];
-        }
-        if (cur >= 0) atomic_add(&p.aux2[(long)cur * p.ld_aux + col], s);
-      }
-    }
-    if (pass + 1 < passes) __syncthreads();
-  }
-}
-
-__device__ __forceinline__ void cp_async_n(void* dst, const void* src, int bytes, bool ok) {  // bytes 4 or 16, zero fill
+__device__ __forceinline__ void cp_async_n(void* dst, const void* src, int bytes, bool ok) {  // bytes 4, 8 or 16, zero fill
   const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst));
   if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(ok ? 16 : 0) : "memory");
+  else if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 template <int N>
@@ -477,6 +318,117 @@ inline cudaError_t launch_gemm_f(const GemmP<float>& p, cudaStream_t s) {
   return cudaPeekAtLastError();
 }
 
+// FP64 contraction on the CUDA cores (the refinement pass, the low-rank blocks, narrow layers): every output one chain of fused
+// multiply-adds over ascending k.  Bound by the FP64 pipe, which GB300 has at 1/64 of the FP32 rate: 128 x 128 outputs per CTA
+// at K = N = 256 kept an SM for 1.05 ms while the others idled.  16 x 16 outputs per CTA, 2 x 2 per thread: small enough that
+// any row count loads the SMs evenly, and two warps per CTA hide the chain.  At K = N = 256 with 160 / 600 / 2050 / 16400 rows
+// 48 / 110 / 271 / 1751 us (the pipe alone: 18 / 68 / 233 / 1861 at 1.9 GHz); 32 x 32 with 2 x 2 per thread 72 / 135 / 265 /
+// 1727, 16 x 16 with 4 x 4, half a warp, 150 / 246 / 645 / 3557.
+constexpr int DG_BM = 16, DG_RT = 2, DG_K = 16, DG_ST = 3, DG_LA = DG_K + 2, DG_THREADS = (DG_BM / DG_RT) * (DG_BM / DG_RT);
+constexpr int DG_STAGE = DG_BM * DG_LA + DG_K * DG_BM;
+template <int MODE>
+__global__ void __launch_bounds__(DG_THREADS) k_gemm_d(GemmP<double> p) {
+  constexpr int BM = DG_BM, RT = DG_RT, NT = DG_THREADS, TX = BM / RT, LA = DG_LA, DK = DG_K, ST = DG_ST;
+  __shared__ __align__(16) double sm[ST * DG_STAGE];
+  int rows = p.M;
+  if (p.M_dev) rows = min(rows, p.M_scale * (*p.M_dev));
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BM;
+  if (m0 >= rows) return;
+  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  int passes = 1, first_spin = 0;
+  if (p.B2) {  // per-spin weights: a pass per spin present in the tile
+    int up = 0, dn = 0;
+    for (int r = tid; r < BM && m0 + r < rows; r += NT) {
+      if ((gemm_node(p, m0 + r) % p.n_el) < p.n_up) up = 1; else dn = 1;
+    }
+    up = __syncthreads_or(up);
+    dn = __syncthreads_or(dn);
+    first_spin = up ? 0 : 1;
+    passes = up + dn;
+  }
+  const bool va = p.lda % 2 == 0 && p.K % 2 == 0 && (reinterpret_cast<uintptr_t>(p.A) & 15) == 0;
+  for (int pass = 0; pass < passes; ++pass) {
+    const int spin = first_spin + pass, ks = (p.K + DK - 1) / DK;
+    const double* Bp = spin == 0 ? p.B : p.B2;
+    auto fetch = [&](int st) {
+      if (st < ks) {
+        double* As = sm + (st % ST) * DG_STAGE;
+        double* Bs = As + BM * LA;
+        const int k0 = st * DK;
+        if (va) {
+          for (int e = tid; e < BM * DK / 2; e += NT) {
+            const int r = e / (DK / 2), k = e % (DK / 2) * 2;
+            const bool ok = m0 + r < rows && k0 + k < p.K;
+            cp_async_n(As + r * LA + k, ok ? p.A + (long)(m0 + r) * p.lda + k0 + k : p.A, 16, ok);
+          }
+        } else {
+          for (int e = tid; e < BM * DK; e += NT) {
+            const int r = e / DK, k = e % DK;
+            const bool ok = m0 + r < rows && k0 + k < p.K;
+            cp_async_n(As + r * LA + k, ok ? p.A + (long)(m0 + r) * p.lda + k0 + k : p.A, 8, ok);
+          }
+        }
+        for (int e = tid; e < DK * BM; e += NT) {
+          const int k = e / BM, c = e % BM;
+          const bool ok = k0 + k < p.K && n0 + c < p.N;
+          cp_async_n(Bs + k * BM + c, ok ? Bp + (long)(k0 + k) * p.ldb + n0 + c : Bp, 8, ok);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[RT][RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 0; j < RT; ++j) acc[i][j] = 0.0;
+#pragma unroll
+    for (int st = 0; st < ST - 1; ++st) fetch(st);
+    for (int st = 0; st < ks; ++st) {
+      cp_async_left<ST - 2>();
+      __syncthreads();  // stage st has landed for everyone, and everyone has left stage st - 1
+      fetch(st + ST - 1);
+      const double* As = sm + (st % ST) * DG_STAGE + ty * RT * LA;
+      const double* Bs = sm + (st % ST) * DG_STAGE + BM * LA + tx * RT;
+#pragma unroll 4
+      for (int k = 0; k < DK; ++k) {
+        double b[RT];
+#pragma unroll
+        for (int j = 0; j < RT; j += 2) {
+          const double2 v = *reinterpret_cast<const double2*>(Bs + k * BM + j);
+          b[j] = v.x;
+          b[j + 1] = v.y;
+        }
+#pragma unroll
+        for (int i = 0; i < RT; ++i) {
+          const double a = As[i * LA + k];
+#pragma unroll
+          for (int j = 0; j < RT; ++j) acc[i][j] = fma(a, b[j], acc[i][j]);
+        }
+      }
+    }
+    cp_async_left<0>();
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      const int row = m0 + ty * RT + i;
+      if (row >= rows) continue;
+      if (p.B2 && (((gemm_node(p, row) % p.n_el) < p.n_up) ? 0 : 1) != spin) continue;
+#pragma unroll
+      for (int j = 0; j < RT; ++j) {
+        const int col = n0 + tx * RT + j;
+        if (col < p.N) gemm_store<double, MODE>(p, row, col, acc[i][j], spin);
+      }
+    }
+    if (pass + 1 < passes) __syncthreads();
+  }
+}
+template <int MODE>
+inline cudaError_t launch_gemm_d(const GemmP<double>& p, cudaStream_t s) {
+  const dim3 grid((p.M + DG_BM - 1) / DG_BM, (p.N + DG_BM - 1) / DG_BM);
+  if (grid.y == 0 || grid.x == 0) return cudaSuccess;
+  k_gemm_d<MODE><<<grid, DG_THREADS, 0, s>>>(p);
+  return cudaPeekAtLastError();
+}
+
 template <typename T, int MODE>
 inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
@@ -487,16 +439,10 @@ inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
     if (tiles(128) >= 1200) return launch_gemm_f<MODE, 128>(p, s);
     if (tiles(64) >= 800) return launch_gemm_f<MODE, 64>(p, s);
     return launch_gemm_f<MODE, 32>(p, s);
+  } else if constexpr (MODE == EPI_PLAIN || MODE == EPI_SILU_X || MODE == EPI_ORB_X || MODE == EPI_ENV) {
+    return launch_gemm_d<MODE>(p, s);
   } else {
-    dim3 grid((p.N + GBN - 1) / GBN, (p.M + GBM - 1) / GBM);
-    size_t dyn = (MODE == EPI_SILU_J) ? sizeof(T) * GBM * (GBN + 1) : 0;
-    if (dyn > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(k_gemm<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-      if (e != cudaSuccess) return e;
-    }
-    if (grid.y == 0 || grid.x == 0) return cudaSuccess;
-    k_gemm<T, MODE><<<grid, GTHREADS, dyn, s>>>(p);
-    return cudaPeekAtLastError();
+    return cudaErrorInvalidValue;  // FP64 derivative rows: the sliced contraction
   }
 }
 
@@ -580,7 +526,8 @@ __global__ void __launch_bounds__(CTHREADS, 2) k_gemm_comp(GemmP<float> p, float
   __shared__ __align__(16) float Csg[CBN];        // per column: 3 * 2^eb, the grid spacing 2^(eb-22), 16 bits(3 * 2^eb)
   __shared__ __align__(16) float Cg[CBN];
   __shared__ __align__(16) unsigned Cs16[CBN];
-  const int rows = p.M;
+  int rows = p.M;
+  if (p.M_dev) rows = min(rows, p.M_scale * (*p.M_dev));
   const int m0 = blockIdx.y * CBM, n0 = blockIdx.x * CBN;
   if (m0 >= rows) return;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
@@ -811,7 +758,8 @@ __global__ void __launch_bounds__(CTHREADS) k_gemm_env_df(GemmP<double> p) {
   __shared__ __align__(16) float Ah[2][CBK][CBM];
   __shared__ __align__(16) float Al[2][CBK][CBM];
   __shared__ __align__(16) float Bs[2][CBK][CBN];
-  const int rows = p.M;
+  int rows = p.M;
+  if (p.M_dev) rows = min(rows, p.M_scale * (*p.M_dev));
   const int m0 = blockIdx.y * CBM, n0 = blockIdx.x * CBN;
   if (m0 >= rows) return;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;

@@ -1381,7 +1381,7 @@ fire_status grad_chunk_run(const fire_problem* p, cudaStream_t s, const float* R
       return FIRE_ERR_CUDA;
     kern<<<Wc * NDET, gjg_threads(n), smem, s>>>(B(P.A), (const T*)nullptr, n, reinterpret_cast<S*>(ws + P.gjw),
                                                     reinterpret_cast<double*>(ws + P.ld),
-                                                    reinterpret_cast<double*>(ws + P.sd), nullptr, B(P.Ainv), status);
+                                                    reinterpret_cast<double*>(ws + P.sd), nullptr, B(P.Ainv), nullptr, status);
   }
   // ---- forward: Jastrow
   mm<T>(s, G, F, F, B(P.hf), F, W.w[FIRE_P_ATT_Q_W], F, W.w[FIRE_P_ATT_Q_B], B(P.q), F);

@@ -17,7 +17,11 @@ struct Nbr {
   int* en_cnt;  // [W, n]        e-n neighbours (capped at cap_nuc)
   int* en_idx;  // [W, n, cap_nuc] nucleus indices, ascending
   int* counts;  // [W, 4]        n_pairs_same, n_pairs_diff, n_triplets, n_neighbours_en
+  const int* live = nullptr;  // device count of the chunk's walkers to evaluate (the first of them), or nullptr: all
 };
+
+// whether walker w of a chunk is evaluated
+__device__ __forceinline__ bool walker_live(const Nbr& nb, int w) { return !nb.live || w < *nb.live; }
 
 // Sparse forward-Laplacian layout of a chunk ("positions" = Jacobian rows of NodeWithFwdLap,
 // sparse_fwd_lap.py:14-22).  Per walker w the positions of center i are

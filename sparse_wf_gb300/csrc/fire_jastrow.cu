@@ -33,6 +33,27 @@ __device__ __forceinline__ void act3(T z, T& f, T& f1, T& f2) {
 }
 
 // FLM: forward-Laplacian mode (X, J, L planes) or value mode (X only).
+// warp_sum of NC values (a power of two) at once: in every exchange a lane keeps half of the values it still holds, so that
+// NC + log2(32 / NC) - 1 shuffles do the work of 5 NC; the same pairs are added as in warp_sum.  Lane l returns value
+// l / (32 / NC).
+template <typename T, int NC>
+__device__ __forceinline__ T warp_sums(T (&v)[NC], int lane) {
+#pragma unroll
+  for (int h = NC / 2, o = 16; o > 0; h /= 2, o /= 2) {
+    if (h > 0) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int c = 0; c < h; ++c) {
+        const T send = up ? v[c] : v[c + h], keep = up ? v[c + h] : v[c];
+        v[c] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+  return v[0];
+}
+
 template <typename T, int NC, int ACT, bool FLM>
 __global__ void __launch_bounds__(256) k_narrow(const T* __restrict__ X, const T* __restrict__ Jp,
                                                 const T* __restrict__ Lp, Nbr nb, Layout L, const T* __restrict__ Wn,
@@ -43,11 +64,13 @@ __global__ void __launch_bounds__(256) k_narrow(const T* __restrict__ X, const T
   // weights staged in shared memory (the FP64 validation build reads them through L1 instead, to stay
   // within the static shared-memory limit)
   constexpr bool kSmemW = sizeof(T) == 4;
-  __shared__ T Ws_s[kSmemW ? F * NC : 1];
+  constexpr int LW = kSmemW && NC >= 16 ? NC + 4 : NC;  // row length of the staged weights: no bank conflicts
+  __shared__ __align__(16) T Ws_s[kSmemW ? F * LW : 1];
   __shared__ T zr[NARROW_MAXROWS][NC];
   const T* Ws = kSmemW ? Ws_s : Wn;
   const int g = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n = nb.n, w = g / n, i = g - w * n;
+  if (!walker_live(nb, w)) return;
   int cnt = 0;
   long q0 = 0;
   if (FLM) {
@@ -61,7 +84,7 @@ __global__ void __launch_bounds__(256) k_narrow(const T* __restrict__ X, const T
     q0 = (long)L.pos_off[w] + rp[i] + i;
   }
   if (kSmemW)
-    for (int e = tid; e < F * NC; e += blockDim.x) Ws_s[e] = Wn[e];
+    for (int e = tid; e < F * NC; e += blockDim.x) Ws_s[e / NC * LW + e % NC] = Wn[e];
   __syncthreads();
   const int nrows = FLM ? 3 * cnt + 2 : 1;
   for (int rr = wid; rr < nrows; rr += 8) {
@@ -77,13 +100,10 @@ __global__ void __launch_bounds__(256) k_narrow(const T* __restrict__ X, const T
       const int f = lane + 32 * u;
       const T v = src[f];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) acc[c] += v * Ws[f * NC + c];
+      for (int c = 0; c < NC; ++c) acc[c] += v * Ws[f * LW + c];
     }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      const T s = warp_sum(acc[c]);
-      if (lane == 0) zr[rr][c] = s;
-    }
+    const T s = warp_sums<T, NC>(acc, lane);
+    if ((lane & (32 / NC - 1)) == 0) zr[rr][lane / (32 / NC)] = s;
   }
   __syncthreads();
   if (tid < NC) {
@@ -115,6 +135,7 @@ template <typename T, bool FLM>
 __global__ void k_mlp_sum(Nbr nb, Layout L, const T* __restrict__ Xo, const T* __restrict__ Jo,
                           const T* __restrict__ Lo, T* __restrict__ ox, T* __restrict__ ol, T* __restrict__ oj) {
   const int w = blockIdx.x, n = nb.n, tid = threadIdx.x;
+  if (!walker_live(nb, w)) return;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
   if (rp[n] > nb.cap_p) return;
   __shared__ T red[32 * 4];
@@ -163,6 +184,7 @@ __global__ void __launch_bounds__(256) k_att_sums(Nbr nb, Layout L, const T* __r
                                                   const T* __restrict__ VL, T* __restrict__ Ax, T* __restrict__ Al,
                                                   T* __restrict__ AJ) {
   const int m = blockIdx.x, w = blockIdx.y, n = nb.n, tid = threadIdx.x;
+  if (!walker_live(nb, w)) return;
   const int r = tid >> 4;
   const size_t gm = (size_t)w * n + m;
   const int sm = m < nb.n_up ? 0 : 1;

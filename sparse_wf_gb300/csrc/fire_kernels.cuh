@@ -40,7 +40,7 @@ __global__ void k_env_coef(const T* r, const float* R, const T* sp, int n, int n
                            T* coef);
 template <typename S, typename TI, typename TO, bool INV>
 __global__ void k_gj_global(const TI* A, const TI* A_lo, int n, S* work, double* logdet, double* sign, double* cond, TO* Ainv,
-                            int32_t* status);
+                            const int* live, int32_t* status);
 constexpr int GJG_BW_DECL = 16;
 // Threads per matrix of k_gj_global (a power of two warps; n <= 2 threads holds for every n): where a step's rows fill them.
 // LU / inverse of 1024 matrices at n = 82 and 2048 at n = 10 decided the lower lines, 612 at n = 322 the upper.

@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(512) k_neighbors(const T* __restrict__ r, cons
                                                    int32_t* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int w = blockIdx.x;
+  if (!walker_live(nb, w)) return;
   const int n = nb.n, n_up = nb.n_up, N = nb.N;
   T* sr = reinterpret_cast<T*>(smem_raw);
   int* sdeg = reinterpret_cast<int*>(sr + 3 * n);
@@ -323,7 +324,7 @@ __global__ void k_pos_scan(Nbr nb, int* __restrict__ pos_off) {
   for (int w0 = 0; w0 < nb.W; w0 += blockDim.x) {
     const int w = w0 + threadIdx.x;
     int v = 0;
-    if (w < nb.W) v = n + min(nb.rowptr[(size_t)w * (n + 1) + n], nb.cap_p);
+    if (w < nb.W && walker_live(nb, w)) v = n + min(nb.rowptr[(size_t)w * (n + 1) + n], nb.cap_p);
     // block inclusive scan (blockDim = 1024)
     __shared__ int buf[1024];
     buf[threadIdx.x] = v;
@@ -345,6 +346,7 @@ __global__ void k_pos_scan(Nbr nb, int* __restrict__ pos_off) {
 // Fills pos_ctr / pos_dep / dep_pos (one CTA per walker).
 __global__ void __launch_bounds__(256) k_layout(Nbr nb, Layout L) {
   const int w = blockIdx.x, n = nb.n;
+  if (!walker_live(nb, w)) return;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
   const int P = rp[n];
   if (P > nb.cap_p) return;

@@ -119,7 +119,7 @@ struct SliceArgs {
   long lda[2];
   int M[2];
   const int* M_dev;
-  int M_scale;
+  int M_scale[2];
   int row0, row1;  // this pass's rows of every segment
   int K, nkb, n_el;
   int ns[2], soff[2];  // ns > 0: row q is row (q / ns) n_el + soff + q % ns of A
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
   __shared__ U part[SLR_WARPS][32];
   const int g = blockIdx.z, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int rows = a.M[g];
-  if (a.M_dev) rows = min(rows, a.M_scale * *a.M_dev);
+  if (a.M_dev) rows = min(rows, a.M_scale[g] * *a.M_dev);
   rows = min(rows, a.row1) - a.row0;  // of this pass
   const int ql = blockIdx.x * 32 + lane, q = a.row0 + ql;
   if ((int)blockIdx.x * 32 >= (rows + 127) / 128 * 128) return;
@@ -736,7 +736,6 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
   a.env_lo = c.env_lo;
   a.ld_lo = c.ld_lo;
   r.M_dev = p0.M_dev;
-  r.M_scale = p0.M_scale;
   r.K = p0.K;
   r.nkb = a.tl.nkb;
   r.n_el = p0.n_el;
@@ -763,6 +762,7 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
     r.lda[g] = p.lda;
     r.a_bs[g] = c.a_bs[g];
     r.M[g] = p.M;
+    r.M_scale[g] = p.M_scale;
     r.ns[g] = c.map_a ? c.ns[g] : 0;
     r.soff[g] = c.soff[g];
     r.out[g] = const_cast<unsigned char*>(a.At[g]);

@@ -139,8 +139,9 @@ class FireWaveFunction:
         cap_n = static.n_neighbours_en if static is not None else 1
         cap_r = 0
         if refine and self.refine:
-            # the last call's count padded; at least 2 % of the batch (and 2 walkers)
-            cap_r = min(int(n_walkers), max(self._refine_cap, 2, -(-2 * int(n_walkers) // 100)))
+            # the last call's count padded; at least a quarter of the batch (unused capacity costs launches only, a call
+            # that finds more is repeated)
+            cap_r = min(int(n_walkers), max(self._refine_cap, 2, -(-int(n_walkers) // 4)))
         return _lib.Problem(self.n_electrons, self.n_up, self.n_nuclei, int(n_walkers), self.cutoff,
                             self.cutoff_1el, max(1, int(cap_p)), max(1, int(cap_n)), _lib.PREC[self.precision],
                             self.chunk_walkers, cap_r, float(self.refine_ratio), float(self.refine_kappa),
