@@ -132,6 +132,23 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
+// 8 consecutive floats through L2: one 32-byte load when wide (32-byte aligned), else two of 16
+__device__ __forceinline__ void ldg8(const float* p, bool wide, float (&x)[8]) {
+  if (wide) {
+    asm volatile("ld.global.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]), "=f"(x[4]), "=f"(x[5]), "=f"(x[6]), "=f"(x[7])
+                 : "l"(p));
+  } else {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(p)), b = __ldcg(reinterpret_cast<const float4*>(p) + 1);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+  }
+}
+// asks for a contiguous range in L2 (16-byte aligned address, size a multiple of 16)
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t r[16];
   asm volatile(
@@ -144,24 +161,31 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+// 16 columns of two accumulators, one wait
+__device__ __forceinline__ void tmem_ld16x2(uint32_t ta, uint32_t tb, float (&a)[16], float (&b)[16]) {
+  uint32_t r[16], q[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%32];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%33];\n"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(q[0]),
+        "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]), "=r"(q[9]),
+        "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+      : "r"(ta), "r"(tb)
+      : "memory");
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    a[k] = __uint_as_float(r[k]);
+    b[k] = __uint_as_float(q[k]);
+  }
+}
+
 // byte offset of element (row, k) in a canonical no-swizzle K-major tile (BF16)
 __device__ __forceinline__ uint32_t tc_off(int row, int k) {
   return (uint32_t)((row & 7) * 16 + (row >> 3) * TC_SBO + (k & 7) * 2 + (k >> 3) * TC_LBO);
 }
 
-// 16-byte global -> shared asynchronous copy (zero fill when !ok), commit and wait (n copies groups may stay
-// in flight, n <= 3)
-__device__ __forceinline__ void cp_async16_tc(void* dst, const void* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit_tc() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_tc(int n) {
-  if (n <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
-  else if (n == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-  else if (n == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
-  else asm volatile("cp.async.wait_group 3;" ::: "memory");
-}
 // Scaled-grid split (the A-resident kernel, K <= 256).  A row of A (or a column of W) whose largest magnitude is in
 // [2^e, 2^(e+1)) is scaled by 2^(7 - e) (exactly), so its values lie in (-256, 256); each scaled value x is split
 // into hi = rint(x), an integer of magnitude <= 256, and lo = x - hi (exact in FP32, |lo| <= 1/2), both stored in
@@ -199,7 +223,9 @@ __host__ __device__ inline int grid_hb(int K) {
 }
 __device__ __forceinline__ void split_grid_f16x2(float a, float b, float inv, uint32_t& hi, uint32_t& lo) {
   const float xa = a * inv, xb = b * inv;
-  const float ha = rintf(xa), hb = rintf(xb);
+  // rint of a magnitude below 2^22 by adding and subtracting 1.5 2^23: two additions where rintf goes through the
+  // conversion unit
+  const float ha = (xa + 12582912.f) - 12582912.f, hb = (xb + 12582912.f) - 12582912.f;
   const __half2 h = __floats2half2_rn(ha, hb);
   const __half2 l = __floats2half2_rn(xa - ha, xb - hb);
   hi = *reinterpret_cast<const uint32_t*>(&h);
@@ -339,8 +365,7 @@ __device__ __forceinline__ void tc_val16(const GemmP<float>& p, int row, int nod
 template <int MODE>
 __device__ __forceinline__ void tc_epilogue_tile(const GemmP<float>& p, int rows, int m0, int n0, uint32_t tacc,
                                                  int spin_filter, int tma, const CUtensorMap* tmC, float* stg,
-                                                 int& nst, int warp, int lane, bool two_acc = false,
-                                                 float row_sc = 1.f, const float* col_sc = nullptr) {
+                                                 int& nst, int warp, int lane) {
   const int quad = warp & 3, half = warp >> 2;
   const int row = m0 + quad * 32 + lane;
   const bool valid = row < rows;
@@ -359,19 +384,6 @@ __device__ __forceinline__ void tc_epilogue_tile(const GemmP<float>& p, int rows
   for (int c0 = half * (TCP_BN / 2); c0 < (half + 1) * (TCP_BN / 2); c0 += 16) {
     float v[16];
     tmem_ld16(base + (uint32_t)c0, v);
-    if (two_acc) {  // the exact hi x hi sums plus the cross terms, TCP_BN columns further on
-      float v2[16];
-      tmem_ld16(base + (uint32_t)(TCP_BN + c0), v2);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) v[k] += v2[k];
-    }
-    if (col_sc) {  // undo the scaled-grid split: row scale times column scale (powers of two: exact)
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int col = n0 + c0 + k;
-        v[k] *= row_sc * (col < p.N ? col_sc[col] : 0.f);
-      }
-    }
     const int spin = spin_filter < 0 ? 0 : spin_filter;
     const bool full = n0 + c0 + 15 < p.N;
     const bool use_tma = tma_warp && full;
@@ -680,7 +692,15 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) k_gemm_tcs(GemmP<float> p, con
 // 128-column x 64-deep tile, hi and lo planes, already in the canonical K-major layout: k-groups 2048 bytes
 // apart, 8-row groups 128 bytes apart).  A is a ring of 64-deep blocks: block kb is released once the MMAs of
 // the last column tile have read it, so the next row tile's conversion overlaps the current tile's tail.
-// Warp roles: 0-7 epilogue, 8-11 A converters, 12 (lane 0) MMA issuer, 13 (lane 0) weight loader.
+// Warp roles: 0-7 epilogue, 8-15 A converters, 16 MMA issuer, 17 (lane 0) weight loader.
+// A passes from L2 through registers: a row's grid needs its largest magnitude before its first value is split, so the
+// converters read a row tile twice, once ahead of time for the magnitudes (after a bulk prefetch into L2) and once, a
+// block ahead of the MMAs, to split.  The first version copied raw rows into the A ring, waited for all of the tile and
+// split in place: its four converter warps kept the chain of load, maximum, barrier and split serial.  What bounds it now:
+// the operands the MMAs read fill the shared memory's bandwidth (8 KB per 64 cycles), which the epilogue's staging shares;
+// without the epilogue 922500 x 256 x 256 takes 400 us (HBM alone: 278).  Before / after, with the plain epilogue 720 / 505
+// us, with the silu epilogue and its per-center sums 780 / 710, with the orbital one (N = 328) 1120 / 917.  Slower or no
+// gain: 16 epilogue and 4 converter warps (764, 944, 1097), weight stages of half the depth (510, 709, 936).
 // Splitting: every row of A (and, at preparation, every column of the weights) is scaled and split on the grid of
 // its own largest magnitude (split_grid_f16x2, FP16 operands), so that the hi x hi products of a row and a column are
 // integers and their sum over K <= 256 is exact in FP32 whatever order and rounding the tensor core's accumulation
@@ -688,20 +708,205 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) k_gemm_tcs(GemmP<float> p, con
 // of the result, so their accumulation rounding is ~2^-32 of it); the epilogue adds the two and applies the row and
 // column scales.  (a_lo w_lo is kept: on the grid lo reaches half a step, 2^-8 of the row's largest value, so the
 // term is ~2^-16 of a product.)  The per-element error is ~2^-20 of the row's (column's) largest value.
-constexpr int TCA_THREADS = 448, TCA_KB = 4, TCA_BSTAGES = 2;
+//
+// Epilogue of one row tile's 128-column tiles, per warp (TMEM lane quadrant warp % 4, column half warp / 4): what does not
+// depend on the column is found once per row tile (TcaRows).  Per 16-column chunk the first operand row and the column
+// scales are fetched before the accumulators are read, both accumulators under one wait, and the squares of a chunk are
+// all read back before the first is summed: the epilogue is a chain of latencies with two warps per scheduler to hide them.
+struct TcaRows {
+  int row, node;
+  bool valid, mine, self, tma_warp;
+  uint32_t brk;     // bit 2 i: row 2 i + (lane / 16) begins another center's run
+  int first, last;  // centers of this half-warp's first and last runs
+  int runs;         // most ends of runs within a half-warp
+  bool merge;       // both half-warps' last runs belong to one center
+};
+template <int MODE>
+__device__ __forceinline__ TcaRows tca_rows(const GemmP<float>& p, int rows, int m0, int spin_filter, int tma, int* nodes,
+                                            int warp, int lane) {
+  TcaRows t;
+  t.row = m0 + (warp & 3) * 32 + lane;
+  t.valid = t.row < rows;
+  t.node = t.valid ? gemm_node(p, t.row) : -1;
+  t.mine = t.valid && !(p.row_skip > 0 && t.row % p.row_skip == 0);
+  if (t.mine && spin_filter >= 0) t.mine = ((((t.node % p.n_el) < p.n_up) ? 0 : 1) == spin_filter);
+  t.tma_warp = tma != 0 && __all_sync(0xffffffffu, t.mine);
+  t.self = MODE == EPI_ORB_J && t.valid && p.dep_map[t.row / 3] == t.node;
+  if (MODE == EPI_SILU_J) {
+    const int h = lane >> 4, before = __shfl_up_sync(0xffffffffu, t.node, 2);
+    t.brk = (__ballot_sync(0xffffffffu, lane >= 2 && t.node != before) >> h) & 0x55555555u;
+    t.first = __shfl_sync(0xffffffffu, t.node, h);
+    t.last = __shfl_sync(0xffffffffu, t.node, 30 + h);
+    const int ends = __popc(t.brk);
+    t.runs = max(ends, __shfl_xor_sync(0xffffffffu, ends, 16));
+    t.merge = __shfl_xor_sync(0xffffffffu, t.last, 16) == t.last;
+    __syncwarp();
+    nodes[lane] = t.node;
+    __syncwarp();
+  }
+  return t;
+}
+template <int MODE>
+__device__ __forceinline__ void tca_epilogue_tile(const GemmP<float>& p, const TcaRows& t, int n0, uint32_t tacc, int spin_filter,
+                                                  const CUtensorMap* tmC, float* stg, const int* nodes, int& nst, int warp,
+                                                  int lane, float row_sc, const float* col_sc) {
+  const int quad = warp & 3, half = warp >> 2, spin = spin_filter < 0 ? 0 : spin_filter;
+  const uint32_t base = tacc + ((uint32_t)(quad * 32) << 16);
+  const float* arow = nullptr;  // silu' of the row's center; its envelope values and their derivatives
+  if (MODE == EPI_SILU_J) arow = p.aux1 + (long)max(t.node, 0) * p.ld_aux;
+  if (MODE == EPI_ORB_J) arow = p.aux1 + (long)max(t.node, 0) * 5 * p.ld_aux;
+  for (int c0 = half * (TCP_BN / 2); c0 < (half + 1) * (TCP_BN / 2); c0 += 16) {
+    const int col0 = n0 + c0;
+    if (col0 >= p.N) break;
+    const bool full = col0 + 15 < p.N, use_tma = t.tma_warp && full;
+    float4 w[4], cs[4];
+    if (MODE == EPI_SILU_J || MODE == EPI_ORB_J) {
+      if (full && t.mine) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = ld4(arow + col0 + 4 * u);
+      }
+    }
+    if (full) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) cs[u] = __ldg(reinterpret_cast<const float4*>(col_sc + col0) + u);
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = col0 + 4 * u;
+        cs[u] = make_float4(c < p.N ? col_sc[c] : 0.f, c + 1 < p.N ? col_sc[c + 1] : 0.f, c + 2 < p.N ? col_sc[c + 2] : 0.f,
+                            c + 3 < p.N ? col_sc[c + 3] : 0.f);
+      }
+    }
+    float v[16];
+    {
+      float v2[16];
+      tmem_ld16x2(base + (uint32_t)c0, base + (uint32_t)(TCP_BN + c0), v, v2);  // exact hi x hi sums, cross terms
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {  // row scale times column scale (powers of two: exact)
+        v[4 * u] = (v[4 * u] + v2[4 * u]) * (row_sc * cs[u].x);
+        v[4 * u + 1] = (v[4 * u + 1] + v2[4 * u + 1]) * (row_sc * cs[u].y);
+        v[4 * u + 2] = (v[4 * u + 2] + v2[4 * u + 2]) * (row_sc * cs[u].z);
+        v[4 * u + 3] = (v[4 * u + 3] + v2[4 * u + 3]) * (row_sc * cs[u].w);
+      }
+    }
+    float* sb = stg + (size_t)(warp * 2 + (nst & 1)) * 32 * 16;  // this chunk's staging buffer
+    if (use_tma || MODE == EPI_SILU_J) {
+      if (lane == 0 && nst >= 2) tma_wait_read1();  // the store from this buffer two chunks ago has read it
+      __syncwarp();
+    }
+    if (MODE == EPI_SILU_J) {
+      // squared pre-activation values through the staging buffer (in the 64-byte swizzle of the stores: conflict-free both
+      // ways): lanes 0-15 sum the even rows of column lane % 16, lanes 16-31 the odd rows, one atomic per center run; the
+      // last runs of the two half-warps merge when they belong to the same center
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        *reinterpret_cast<float4*>(sb + lane * 16 + 4 * (u ^ ((lane >> 1) & 3))) =
+            t.valid ? make_float4(v[4 * u] * v[4 * u], v[4 * u + 1] * v[4 * u + 1], v[4 * u + 2] * v[4 * u + 2], v[4 * u + 3] * v[4 * u + 3])
+                    : make_float4(0.f, 0.f, 0.f, 0.f);
+      __syncwarp();
+      const int c = lane & 15, h = lane >> 4, col = col0 + c;
+      float q[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) q[i] = sb[(2 * i + h) * 16 + (c ^ ((i & 3) << 2))];
+      float s2 = 0.f;
+      if (t.runs <= 1) {  // at most one center ends in either half: no branch per row
+        float first = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if ((t.brk >> (2 * i)) & 1) {
+            first = s2;
+            s2 = 0.f;
+          }
+          s2 += q[i];
+        }
+        if (t.brk && t.first >= 0 && col < p.N) atomicAdd(&p.aux2[(long)t.first * p.ld_aux + col], first);
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < 16; ++i) {
+          if ((t.brk >> (2 * i)) & 1) {
+            const int cur = nodes[2 * (i - 1) + h];
+            if (cur >= 0 && col < p.N) atomicAdd(&p.aux2[(long)cur * p.ld_aux + col], s2);
+            s2 = 0.f;
+          }
+          s2 += sb[(2 * i + h) * 16 + (c ^ ((i & 3) << 2))];
+        }
+      }
+      __syncwarp();
+      const float s2o = __shfl_xor_sync(0xffffffffu, s2, 16);
+      if (t.merge) s2 = h ? 0.f : s2 + s2o;
+      if (t.last >= 0 && col < p.N && !(t.merge && h)) atomicAdd(&p.aux2[(long)t.last * p.ld_aux + col], s2);
+    }
+    if (full && t.mine) {
+      float4 o[4];
+      if (MODE == EPI_SILU_J) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          o[u] = make_float4(v[4 * u] * w[u].x, v[4 * u + 1] * w[u].y, v[4 * u + 2] * w[u].z, v[4 * u + 3] * w[u].w);
+      } else if (MODE == EPI_ORB_J) {
+        if (t.self) {
+          const int a = t.row % 3;
+          float4 raw[4], ej[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            raw[u] = ld4(p.aux3 + (long)t.node * p.ld_aux + col0 + 4 * u);
+            ej[u] = ld4(arow + (1 + a) * p.ld_aux + col0 + 4 * u);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            o[u] = make_float4(raw[u].x * ej[u].x + w[u].x * v[4 * u], raw[u].y * ej[u].y + w[u].y * v[4 * u + 1],
+                               raw[u].z * ej[u].z + w[u].z * v[4 * u + 2], raw[u].w * ej[u].w + w[u].w * v[4 * u + 3]);
+            st4(p.aux2 + ((long)t.node * 3 + a) * p.ld_aux + col0 + 4 * u,
+                make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]));
+          }
+        } else {
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            o[u] = make_float4(w[u].x * v[4 * u], w[u].y * v[4 * u + 1], w[u].z * v[4 * u + 2], w[u].w * v[4 * u + 3]);
+        }
+      } else {
+        tc_val16<MODE>(p, t.row, t.node, col0, v, spin, o);
+      }
+      if (use_tma) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)  // the tensor map's 64-byte swizzle (staging buffers are 512-byte aligned)
+          *reinterpret_cast<float4*>(sb + lane * 16 + 4 * (u ^ ((lane >> 1) & 3))) = o[u];
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) st4(p.C + (long)t.row * p.ldc + col0 + 4 * u, o[u]);
+      }
+    } else if (t.mine) {
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) {
+        const int col = col0 + j;
+        if (col + 3 < p.N) tc_store4<MODE>(p, t.row, t.node, col, v + j, spin);
+        else
+          for (int e = 0; e < 4; ++e)
+            if (col + e < p.N) gemm_store<float, MODE>(p, t.row, col + e, v[j + e], spin);
+      }
+    }
+    if (use_tma) {
+      proxy_fence();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(tmC, smem_u32(sb), col0, t.row);
+        tma_commit();
+      }
+      ++nst;
+    }
+  }
+}
+constexpr int TCA_THREADS = 576, TCA_KB = 4, TCA_BSTAGES = 2;
 struct TcaCfg {
   static constexpr int A_BYTES = TC_BM * TC_BK * 2;  // one BF16 plane of a 128 x 64 block
   static constexpr int A_BLOCK = 2 * A_BYTES;        // hi + lo
   static constexpr int B_BLOCK = 2 * TCP_BN * TC_BK * 2;  // one tiled weight block (hi + lo)
   static constexpr int STG_BYTES = TcCfg::STG_BYTES;
-  // row exponent codes (int16): the converters' halves [row tile parity][k half][128 rows], then the rows' codes for
-  // the epilogue [row tile mod 4][128 rows]
-  static constexpr int RMAX_BYTES = 2 * 2 * TC_BM * 2 + 4 * TC_BM * 2;
+  // the rows' exponent codes (int16) [row tile mod 4][128 rows], the epilogue warps' rows' centers (int32) [8][32]
+  static constexpr int RMAX_BYTES = 4 * TC_BM * 2 + 8 * 32 * 4;
   static constexpr int TOTAL = TCA_KB * A_BLOCK + TCA_BSTAGES * B_BLOCK + STG_BYTES + RMAX_BYTES + 256;
 };
 struct TcaBar {
   uint64_t afull[TCA_KB], aempty[TCA_KB], bfull[TCA_BSTAGES], bempty[TCA_BSTAGES], tfull[2], tempty[2];
-  uint64_t rmax;      // the converters' row maxima of a row tile are complete
   uint64_t rsfull[4];  // the row codes of row tile t (slot t mod 4) are written
   uint32_t tmem;
   int abort;
@@ -716,8 +921,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
   unsigned char* ares = tc_smem;                                   // [kb][hi, lo][128 x 64], LBO 128, SBO 1024
   unsigned char* bst = tc_smem + TCA_KB * TcaCfg::A_BLOCK;         // [stage][hi, lo][8 k-groups][128 rows][16 B]
   float* stg = reinterpret_cast<float*>(bst + TCA_BSTAGES * TcaCfg::B_BLOCK);
-  int16_t* rpart = reinterpret_cast<int16_t*>(bst + TCA_BSTAGES * TcaCfg::B_BLOCK + TcaCfg::STG_BYTES);
-  int16_t* rcode = rpart + 2 * 2 * TC_BM;
+  int16_t* rcode = reinterpret_cast<int16_t*>(bst + TCA_BSTAGES * TcaCfg::B_BLOCK + TcaCfg::STG_BYTES);
   TcaBar* bars = reinterpret_cast<TcaBar*>(bst + TCA_BSTAGES * TcaCfg::B_BLOCK + TcaCfg::STG_BYTES +
                                            TcaCfg::RMAX_BYTES);
   volatile int* abort = &bars->abort;
@@ -732,7 +936,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
 
   if (tid == 0) {
     for (int k = 0; k < TCA_KB; ++k) {
-      mbar_init(smem_u32(&bars->afull[k]), 128);
+      mbar_init(smem_u32(&bars->afull[k]), 8);
       mbar_init(smem_u32(&bars->aempty[k]), 1);
     }
     for (int s2 = 0; s2 < TCA_BSTAGES; ++s2) {
@@ -743,12 +947,11 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
       mbar_init(smem_u32(&bars->tfull[b]), 1);
       mbar_init(smem_u32(&bars->tempty[b]), 256);
     }
-    mbar_init(smem_u32(&bars->rmax), 128);
-    for (int q = 0; q < 4; ++q) mbar_init(smem_u32(&bars->rsfull[q]), 128);
+    for (int q = 0; q < 4; ++q) mbar_init(smem_u32(&bars->rsfull[q]), 8);
     bars->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 12) {  // two accumulator pairs (exact hi x hi sums, cross terms): all 512 columns
+  if (warp == 16) {  // two accumulator pairs (exact hi x hi sums, cross terms): all 512 columns
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem)),
                  "r"(4 * TCP_BN));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -760,108 +963,95 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
   const uint32_t tmem = bars->tmem;
   long bc_issued = 0;  // weight blocks issued (loader lane)
 
-  if (warp >= 8 && warp < 12) {
-    // ------------------------------------------------------------------ A converters (128 threads)
-    // Each thread owns 8 (row, 8-deep k-group) items of every 64-deep block: one 16-byte core-matrix row in the hi
-    // plane and the same row in the lo plane.  The FP32 values of an item (32 bytes) are copied asynchronously
-    // straight into those two rows (first 4 into the hi row, last 4 into the lo row) as soon as the block's slot
-    // is free, then split in place by the same thread: no other thread touches these bytes, so the thread's own
-    // cp.async wait is the only synchronisation.  A row tile's copies are all issued before its first block is
-    // split, so its HBM latency is paid about once per row tile, not once per block.
-    const int lt = tid - 256, lw = lt >> 5, r8 = lane & 7, kq8 = lane >> 3;
-    long ua = 0;
-    for (int m = blockIdx.x; m < mt && !*abort; m += gridDim.x) {
-      if (skip(m)) continue;
-      const int m0 = m * TC_BM;
-      int issued = 0;
+  if (warp >= 8 && warp < 16) {
+    // ------------------------------------------------------------------ A converters (256 threads)
+    // Warp w owns rows 16 w .. 16 w + 15 of every row tile, from their largest magnitudes to their core-matrix rows, so
+    // the converters never wait for one another.  A lane holds 8 consecutive k (a 32-byte load): an instruction reads one
+    // full line of 8 rows, and its split halves fill 512 contiguous bytes of each plane.
+    const int cw = warp - 8, r8 = lane & 7, kq8 = lane >> 3;
+    const bool wide = p.lda % 8 == 0 && (reinterpret_cast<uintptr_t>(p.A) & 31) == 0;
+    auto load = [&](int m, int kb, float (&x)[4][8]) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int gr = m * TC_BM + cw * 16 + (i >> 1) * 8 + r8, gk = kb * TC_BK + (i & 1) * 32 + kq8 * 8;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[i][k] = 0.f;
+        if (gr < rows && gk < p.K) ldg8(p.A + (long)gr * p.lda + gk, wide, x[i]);  // K % 8 == 0
+      }
+    };
+    // the grid of this warp's rows of row tile m (the u-th of this CTA): the exponent of the largest magnitude over K, the
+    // code for the epilogue into slot u mod 4 (the epilogue of row tile u - 4 finished before the MMAs of row tile u - 2,
+    // whose completion released the A blocks that row tile u - 1 was converted into)
+    auto grid = [&](int m, long u, float (&inv)[2]) {
+      float mx[2] = {0.f, 0.f};
+#pragma unroll 2
       for (int kb = 0; kb < nk; ++kb) {
-        if (ua > 0 && !tc_wait(&bars->aempty[kb], (uint32_t)((ua - 1) & 1), abort)) break;
-        unsigned char* a_hi = ares + kb * TcaCfg::A_BLOCK;
-        unsigned char* a_lo = a_hi + TcaCfg::A_BYTES;
-        const int k0 = kb * TC_BK;
+        float x[4][8];
+        load(m, kb, x);
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int blk = lw + 4 * it;  // (8-row group, k half)
-          const int r = (blk >> 1) * 8 + r8, kk = (blk & 1) * 32 + kq8 * 8;
-          const int gr = m0 + r, gk = k0 + kk;
-          const bool ok = gr < rows && gk < p.K;  // K % 8 == 0: the whole k-group is inside
-          const float* src = ok ? p.A + (long)gr * p.lda + gk : p.A;
-          const uint32_t off = tc_off(r, kk);
-          cp_async16_tc(a_hi + off, src, ok);
-          cp_async16_tc(a_lo + off, src + 4, ok);
-        }
-        cp_async_commit_tc();
-        ++issued;
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) mx[i >> 1] = fmaxf(mx[i >> 1], fabsf(x[i][k]));
       }
-      if (issued < nk) break;  // aborted
-      // the grid of every row: the exponent of its largest magnitude over K.  A row's k-groups belong to lanes r8,
-      // r8 + 8, r8 + 16, r8 + 24 of two warps (k halves lw & 1); each warp writes its half's code, and the converters
-      // meet on an mbarrier (bounded wait) before reading the other half's.  The buffer alternates between row tiles:
-      // a warp writing row tile t + 2 has passed the barrier of t + 1, so every reader of t is done.
-      cp_async_wait_tc(0);
-      float mx[8];
+      int16_t* codes = rcode + (u & 3) * TC_BM + cw * 16 + r8;
 #pragma unroll
-      for (int it = 0; it < 8; ++it) mx[it] = 0.f;
-      for (int kb = 0; kb < nk; ++kb) {
-        const unsigned char* a_hi = ares + kb * TcaCfg::A_BLOCK;
-        const unsigned char* a_lo = a_hi + TcaCfg::A_BYTES;
-#pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int blk = lw + 4 * it;
-          const uint32_t off = tc_off((blk >> 1) * 8 + r8, (blk & 1) * 32 + kq8 * 8);
-          const float4 x = *reinterpret_cast<const float4*>(a_hi + off);
-          const float4 y = *reinterpret_cast<const float4*>(a_lo + off);
-          mx[it] = fmaxf(mx[it], fmaxf(fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))),
-                                       fmaxf(fmaxf(fabsf(y.x), fabsf(y.y)), fmaxf(fabsf(y.z), fabsf(y.w)))));
-        }
-      }
-      int16_t* part = rpart + (ua & 1) * 2 * TC_BM;
-#pragma unroll
-      for (int it = 0; it < 8; ++it) {
-        mx[it] = fmaxf(mx[it], __shfl_xor_sync(0xffffffffu, mx[it], 8));
-        mx[it] = fmaxf(mx[it], __shfl_xor_sync(0xffffffffu, mx[it], 16));
-        if (kq8 == 0) part[(lw & 1) * TC_BM + ((lw + 4 * it) >> 1) * 8 + r8] = (int16_t)grid_code(mx[it]);
-      }
-      tc_arrive(&bars->rmax);
-      if (!tc_wait(&bars->rmax, (uint32_t)(ua & 1), abort)) break;
-      // the rows' codes for the epilogue (slot ua mod 4; the epilogue of row tile ua - 4 finished before the MMAs of
-      // row tile ua - 1, whose completion released these A blocks), published by an mbarrier of their own
-      int16_t* codes = rcode + (ua & 3) * TC_BM;
-      float inv[8];
-#pragma unroll
-      for (int it = 0; it < 8; ++it) {
-        const int r = ((lw + 4 * it) >> 1) * 8 + r8;
-        const int code = max((int)part[r], (int)part[TC_BM + r]);
+      for (int g = 0; g < 2; ++g) {
+        mx[g] = fmaxf(mx[g], __shfl_xor_sync(0xffffffffu, mx[g], 8));
+        mx[g] = fmaxf(mx[g], __shfl_xor_sync(0xffffffffu, mx[g], 16));
+        const int code = grid_code(mx[g]);
         float sc;
-        grid_scales(code, inv[it], sc);
-        if (kq8 == 0 && (lw & 1) == 0) codes[r] = (int16_t)code;
+        grid_scales(code, inv[g], sc);
+        if (kq8 == 0) codes[8 * g] = (int16_t)code;
       }
-      tc_arrive(&bars->rsfull[ua & 3]);
-      for (int kb = 0; kb < nk; ++kb) {
-        unsigned char* a_hi = ares + kb * TcaCfg::A_BLOCK;
-        unsigned char* a_lo = a_hi + TcaCfg::A_BYTES;
+      __syncwarp();
+      if (lane == 0) tc_arrive(&bars->rsfull[u & 3]);
+    };
+    auto next = [&](int m) {
+      do m += gridDim.x;
+      while (m < mt && skip(m));
+      return m;
+    };
+    int m = blockIdx.x;
+    if (skip(m)) m = next(m);
+    float inv[2];
+    if (m < mt) grid(m, 0, inv);
+    for (long ua = 0; m < mt; ++ua) {
+      const int m2 = next(m);
+      if (m2 < mt && lane == 0 && p.lda == p.K) {  // the next row tile's rows of this warp towards L2
+        const int r0 = m2 * TC_BM + cw * 16, nr = min(16, rows - r0);
+        if (nr > 0) l2_prefetch(p.A + (long)r0 * p.lda, (uint32_t)(nr * p.K * 4));
+      }
+      float x[2][4][8];
+      load(m, 0, x[0]);
+      bool live = true;
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int blk = lw + 4 * it;
-          const int r = (blk >> 1) * 8 + r8, kk = (blk & 1) * 32 + kq8 * 8;
-          const uint32_t off = tc_off(r, kk);
-          const float4 x = *reinterpret_cast<const float4*>(a_hi + off);
-          const float4 y = *reinterpret_cast<const float4*>(a_lo + off);
+      for (int kb = 0; kb < TCA_KB; ++kb) {
+        if (kb >= nk) break;
+        if (kb + 1 < nk) load(m, kb + 1, x[(kb + 1) & 1]);
+        if (ua > 0) live = __all_sync(0xffffffffu, tc_wait(&bars->aempty[kb], (uint32_t)((ua - 1) & 1), abort));
+        if (!live) break;
+        unsigned char* a_hi = ares + kb * TcaCfg::A_BLOCK;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float(&v)[8] = x[kb & 1][i];
           uint4 hi, lo;
-          split_grid_f16x2(x.x, x.y, inv[it], hi.x, lo.x);
-          split_grid_f16x2(x.z, x.w, inv[it], hi.y, lo.y);
-          split_grid_f16x2(y.x, y.y, inv[it], hi.z, lo.z);
-          split_grid_f16x2(y.z, y.w, inv[it], hi.w, lo.w);
-          *reinterpret_cast<uint4*>(a_hi + off) = hi;
-          *reinterpret_cast<uint4*>(a_lo + off) = lo;
+          split_grid_f16x2(v[0], v[1], inv[i >> 1], hi.x, lo.x);
+          split_grid_f16x2(v[2], v[3], inv[i >> 1], hi.y, lo.y);
+          split_grid_f16x2(v[4], v[5], inv[i >> 1], hi.z, lo.z);
+          split_grid_f16x2(v[6], v[7], inv[i >> 1], hi.w, lo.w);
+          unsigned char* d = a_hi + tc_off(cw * 16 + (i >> 1) * 8 + r8, (i & 1) * 32 + kq8 * 8);
+          *reinterpret_cast<uint4*>(d) = hi;
+          *reinterpret_cast<uint4*>(d + TcaCfg::A_BYTES) = lo;
         }
         proxy_fence();
-        tc_arrive(&bars->afull[kb]);
+        __syncwarp();
+        if (lane == 0) tc_arrive(&bars->afull[kb]);
       }
-      ++ua;
+      if (!live) break;
+      if (m2 < mt) grid(m2, ua + 1, inv);
+      m = m2;
     }
-    cp_async_wait_tc(0);
-  } else if (warp == 13) {
+  } else if (warp == 17) {
     // ------------------------------------------------------------------ weight loader
     if (lane == 0) {
       long bc = 0;
@@ -879,65 +1069,67 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
           }
       }
     }
-  } else if (warp == 12) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t idesc = tc_idesc_f16<TCP_BN>();
-      const uint32_t a0 = smem_u32(ares), b0 = smem_u32(bst);
-      long ua = 0, bc = 0, uc = 0;
-      for (int m = blockIdx.x; m < mt && !*abort; m += gridDim.x) {
-        if (skip(m)) continue;
-        for (int j = 0; j < nt && !*abort; ++j) {
-          const int b = (int)(uc & 1);
-          const long ub = uc >> 1;
-          if (ub > 0 && !tc_wait(&bars->tempty[b], (uint32_t)((ub - 1) & 1), abort)) break;
-          tc_fence_after();
-          const uint32_t acc_t = tmem + (uint32_t)(b * 2 * TCP_BN);  // hi x hi sums; cross terms TCP_BN further
-          for (int kb = 0; kb < nk; ++kb, ++bc) {
-            if (j == 0 && !tc_wait(&bars->afull[kb], (uint32_t)(ua & 1), abort)) break;
-            const int s2 = (int)(bc % TCA_BSTAGES);
-            if (!tc_wait(&bars->bfull[s2], (uint32_t)((bc / TCA_BSTAGES) & 1), abort)) break;
-            tc_fence_after();
-            const uint32_t ah = a0 + kb * TcaCfg::A_BLOCK, al = ah + TcaCfg::A_BYTES;
-            const uint32_t bh = b0 + s2 * TcaCfg::B_BLOCK, bl = bh + TcaCfg::B_BLOCK / 2;
+  } else if (warp == 16) {
+    // ------------------------------------------------------------------ MMA issuer (the whole warp, one elected lane)
+    const uint32_t idesc = tc_idesc_f16<TCP_BN>();
+    const uint32_t a0 = smem_u32(ares), b0 = smem_u32(bst);
+    long ua = 0, bc = 0, uc = 0;
+    bool live = true;
+    auto wait = [&](uint64_t* bar, long parity) {
+      live = __all_sync(0xffffffffu, tc_wait(bar, (uint32_t)(parity & 1), abort));
+      if (live) tc_fence_after();
+      return live;
+    };
+    for (int m = blockIdx.x; m < mt && live; m += gridDim.x) {
+      if (skip(m)) continue;
+      for (int j = 0; j < nt && live; ++j) {
+        const int b = (int)(uc & 1);
+        const long ub = uc >> 1;
+        if (ub > 0 && !wait(&bars->tempty[b], ub - 1)) break;
+        const uint32_t acc_t = tmem + (uint32_t)(b * 2 * TCP_BN);  // hi x hi sums; cross terms TCP_BN further
+        for (int kb = 0; kb < nk; ++kb, ++bc) {
+          if (j == 0 && !wait(&bars->afull[kb], ua)) break;
+          const int s2 = (int)(bc % TCA_BSTAGES);
+          if (!wait(&bars->bfull[s2], bc / TCA_BSTAGES)) break;
+          const uint64_t dah = tc_desc(a0 + kb * TcaCfg::A_BLOCK), dal = dah + (TcaCfg::A_BYTES >> 4);
+          const uint64_t dbh = tc_desc_s(b0 + s2 * TcaCfg::B_BLOCK, 2048, 128), dbl = dbh + (TcaCfg::B_BLOCK >> 5);
 #pragma unroll
-            for (int kk = 0; kk < TC_BK / 16; ++kk) {
-              const uint32_t sa = kk * 2 * TC_LBO, sb = kk * 2 * 2048;
-              const uint64_t dah = tc_desc(ah + sa), dal = tc_desc(al + sa);
-              const uint64_t dbh = tc_desc_s(bh + sb, 2048, 128), dbl = tc_desc_s(bl + sb, 2048, 128);
-              tc_mma(acc_t, dah, dbh, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-              tc_mma(acc_t + TCP_BN, dah, dbl, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-              tc_mma(acc_t + TCP_BN, dal, dbh, idesc, 1u);
-              tc_mma(acc_t + TCP_BN, dal, dbl, idesc, 1u);
-            }
-            tc_commit(smem_u32(&bars->bempty[s2]));
-            if (j == nt - 1) tc_commit(smem_u32(&bars->aempty[kb]));
+          for (int kk = 0; kk < TC_BK / 16; ++kk) {
+            const uint64_t sa = kk * 2 * (TC_LBO >> 4), sb = kk * 2 * (2048 >> 4);
+            const uint32_t more = (kb > 0 || kk > 0) ? 1u : 0u;
+            tc_mma_elect(acc_t, dah + sa, dbh + sb, idesc, more);
+            tc_mma_elect(acc_t + TCP_BN, dah + sa, dbl + sb, idesc, more);
+            tc_mma_elect(acc_t + TCP_BN, dal + sa, dbh + sb, idesc, 1u);
+            tc_mma_elect(acc_t + TCP_BN, dal + sa, dbl + sb, idesc, 1u);
           }
-          if (*abort) break;
-          tc_commit(smem_u32(&bars->tfull[b]));
-          ++uc;
+          tc_commit_elect(smem_u32(&bars->bempty[s2]));
+          if (j == nt - 1) tc_commit_elect(smem_u32(&bars->aempty[kb]));
         }
-        ++ua;
+        if (!live) break;
+        tc_commit_elect(smem_u32(&bars->tfull[b]));
+        ++uc;
       }
+      ++ua;
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-7, 256 threads)
     long uc = 0, ue = 0;
     int nst = 0;
+    int* nodes = reinterpret_cast<int*>(rcode + 4 * TC_BM) + warp * 32;  // this warp's rows' centers
     for (int m = blockIdx.x; m < mt && !*abort; m += gridDim.x) {
       if (skip(m)) continue;
-      const int m0 = m * TC_BM;
       // this thread's row scale (the converters' code of row m0 + 32 (warp % 4) + lane)
       if (!tc_wait(&bars->rsfull[ue & 3], (uint32_t)((ue >> 2) & 1), abort)) break;
       float inv_unused, row_sc;
       grid_scales((int)rcode[(ue & 3) * TC_BM + (warp & 3) * 32 + lane], inv_unused, row_sc);
       ++ue;
+      const TcaRows tr = tca_rows<MODE>(p, rows, m * TC_BM, spin_filter, tma, nodes, warp, lane);
       for (int j = 0; j < nt && !*abort; ++j) {
         const int b = (int)(uc & 1);
         if (!tc_wait(&bars->tfull[b], (uint32_t)((uc >> 1) & 1), abort)) break;
         tc_fence_after();
-        tc_epilogue_tile<MODE>(p, rows, m0, j * TCP_BN, tmem + (uint32_t)(b * 2 * TCP_BN), spin_filter, tma, &tmC,
-                               stg, nst, warp, lane, true, row_sc, col_sc);
+        tca_epilogue_tile<MODE>(p, tr, j * TCP_BN, tmem + (uint32_t)(b * 2 * TCP_BN), spin_filter, &tmC, stg, nodes, nst,
+                                warp, lane, row_sc, col_sc);
         tc_fence_before();
         tc_arrive(&bars->tempty[b]);
         ++uc;
@@ -947,7 +1139,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
   }
   __syncthreads();
   if (*abort && tid == 0) set_flag(status, FIRE_FLAG_TIMEOUT);
-  if (*abort && warp == 13 && lane == 0) {
+  if (*abort && warp == 17 && lane == 0) {
     // bounded drain: weight copies still in flight must land before the CTA's shared memory goes away
     for (long q = bc_issued > TCA_BSTAGES ? bc_issued - TCA_BSTAGES : 0; q < bc_issued; ++q) {
       const uint32_t a = smem_u32(&bars->bfull[q % TCA_BSTAGES]);
@@ -963,7 +1155,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
       }
     }
   }
-  if (*abort && warp == 12 && lane == 0) {
+  if (*abort && warp == 16 && lane == 0) {
     // bounded drain: an MMA still in flight must finish before tensor memory is released
     for (int s2 = 0; s2 < TCA_BSTAGES; ++s2) {
       const uint32_t a = smem_u32(&bars->bempty[s2]);
@@ -985,7 +1177,7 @@ __global__ void __launch_bounds__(TCA_THREADS, 1) k_gemm_tca(GemmP<float> p, con
   }
   __syncthreads();
   tc_fence_after();
-  if (warp == 12) {
+  if (warp == 16) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(4 * TCP_BN));
   }
 }
