@@ -18,7 +18,7 @@
 
 namespace fire {
 
-enum EpiMode { EPI_PLAIN = 0, EPI_SILU_X, EPI_SILU_J, EPI_SILU_L, EPI_ORB_X, EPI_ORB_J, EPI_ORB_L, EPI_ENV };
+enum EpiMode { EPI_PLAIN = 0, EPI_SILU_X, EPI_SILU_J, EPI_SILU_L, EPI_ORB_X, EPI_ORB_J, EPI_ORB_L, EPI_ENV, EPI_ACC };  // EPI_ACC: added to C
 
 template <typename T>
 struct GemmP {
@@ -61,6 +61,8 @@ __device__ __forceinline__ void gemm_store(const GemmP<T>& p, int row, int col, 
     T v = acc;
     if (p.bias && p.bias_period > 0 && (row % p.bias_period) == 0) v += p.bias[col];
     p.C[(long)row * p.ldc + col] = v;
+  } else if (MODE == EPI_ACC) {
+    p.C[(long)row * p.ldc + col] += acc;
   } else if (MODE == EPI_SILU_X) {
     // value plane; with aux0 set it also writes silu'(z) (aux0) and silu''(z) (aux2), which the
     // Jacobian and Laplacian epilogues of the same layer read instead of re-evaluating them per row
@@ -126,19 +128,21 @@ __device__ __forceinline__ void cp_async_left() {  // at most N groups of this t
 // the packed FMA rate (large tiles: 45 TFLOP/s) or, with few rows, by the chain of stages: a small tile then puts more SMs to
 // work.
 constexpr int FGS = 4;
-template <int BM>
+template <int BM, bool BT = false>
 struct FgCfg {
   static constexpr int BN = BM, TM = BM >= 64 ? 8 : 4, THREADS = (BM / TM) * (BN / TM);
   static constexpr int FGK = BM == 32 ? 32 : 16;
   static constexpr int FGA = FGK + 4;  // row length of the A tile (k contiguous, rows on different banks)
-  static constexpr int STAGE = BM * FGA + FGK * BN;  // floats
+  static constexpr int STAGE = BM * FGA + (BT ? BN * FGA : FGK * BN);  // floats
   static constexpr int SQ = BM * (BN + 1);
   static constexpr size_t smem(bool sq) { return sizeof(float) * (sq && SQ > FGS * STAGE ? SQ : FGS * STAGE); }
 };
 
-template <int MODE, int BM>
+// BT: B is the transpose of p.B [N, K] (p.ldb); its tile is kept like A's, k contiguous, and a thread's columns lie TX apart
+// so that their rows are read without bank conflicts.
+template <int MODE, int BM, bool BT = false>
 __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 ? 7 : 1)) k_gemm_f(GemmP<float> p) {
-  using Cf = FgCfg<BM>;
+  using Cf = FgCfg<BM, BT>;
   constexpr int BN = Cf::BN, TM = Cf::TM, NT = Cf::THREADS, H = BM / 2;  // H: rows (columns) between a thread's two halves
   constexpr int TX = BN / TM, FGK = Cf::FGK, FGA = Cf::FGA;
   extern __shared__ __align__(16) float fg_smem[];  // [stage][A: BM x FGA, B: FGK x BN]; at the end the squares of SILU_J
@@ -150,6 +154,7 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
   // rows and columns of the thread: groups of 4, with 8 x 8 a second group half a tile further
   auto rloc = [&](int i) { return (i & 3) + ty * 4 + (i >> 2) * H; };
+  auto cloc = [&](int j) { return BT ? tx + j * TX : (j & 3) + tx * 4 + (j >> 2) * H; };
 
   // spin composition of the tile (per-spin weights)
   int passes = 1, first_spin = 0;
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
   for (int pass = 0; pass < passes; ++pass) {
     const int spin = first_spin + pass;
     const float* Bp = spin == 0 ? p.B : p.B2;
-    const bool vb = p.ldb % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(Bp) & 15) == 0;
+    const bool vb = p.ldb % 4 == 0 && (BT ? p.K : p.N) % 4 == 0 && (reinterpret_cast<uintptr_t>(Bp) & 15) == 0;
     f32x2 acc[TM][TM / 2];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
@@ -197,7 +202,13 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
             cp_async_n(As + r * FGA + k, ok ? p.A + (long)(m0 + r) * p.lda + k0 + k : p.A, 4, ok);
           }
         }
-        if (vb) {
+        if (BT) {
+          for (int e = tid; e < BN * FGK / (vb ? 4 : 1); e += NT) {
+            const int w = vb ? 4 : 1, c = e / (FGK / w), k = e % (FGK / w) * w;
+            const bool ok = n0 + c < p.N && k0 + k < p.K;
+            cp_async_n(Bs + c * FGA + k, ok ? Bp + (long)(n0 + c) * p.ldb + k0 + k : Bp, 4 * w, ok);
+          }
+        } else if (vb) {
 #pragma unroll
           for (int u = 0; u < FGK * BN / 4 / NT; ++u) {
             const int e = tid + u * NT, k = e / (BN / 4), c = (e % (BN / 4)) * 4;
@@ -230,9 +241,21 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
           const float4 q = *reinterpret_cast<const float4*>(As + rloc(i) * FGA + kq);
           a[i][0] = q.x; a[i][1] = q.y; a[i][2] = q.z; a[i][3] = q.w;
         }
+        float bt[BT ? TM : 1][4];
+        if (BT) {
+#pragma unroll
+          for (int j = 0; j < TM; ++j) {
+            const float4 q = *reinterpret_cast<const float4*>(Bs + cloc(j) * FGA + kq);
+            bt[BT ? j : 0][0] = q.x; bt[BT ? j : 0][1] = q.y; bt[BT ? j : 0][2] = q.z; bt[BT ? j : 0][3] = q.w;
+          }
+        }
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           f32x2 b[TM / 2];
+          if (BT) {
+#pragma unroll
+            for (int j = 0; j < TM / 2; ++j) b[j] = pack2(bt[BT ? 2 * j : 0][kk], bt[BT ? 2 * j + 1 : 0][kk]);
+          } else
 #pragma unroll
           for (int h = 0; h < TM / 4; ++h) {
             const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(Bs + (kq + kk) * BN + tx * 4 + h * H);
@@ -262,11 +285,11 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
       }
 #pragma unroll
       for (int j = 0; j < TM / 2; ++j) {
-        const int col = n0 + (j & 1) * 2 + tx * 4 + (j >> 1) * H;
+        const int cx = n0 + cloc(2 * j), cy = n0 + cloc(2 * j + 1);
         float x, y;
         unpack2(acc[i][j], x, y);
-        if (col < p.N) gemm_store<float, MODE>(p, row, col, x, spin);
-        if (col + 1 < p.N) gemm_store<float, MODE>(p, row, col + 1, y, spin);
+        if (cx < p.N) gemm_store<float, MODE>(p, row, cx, x, spin);
+        if (cy < p.N) gemm_store<float, MODE>(p, row, cy, y, spin);
       }
     }
     if (MODE == EPI_SILU_J || pass + 1 < passes) __syncthreads();  // everyone has left the tiles
@@ -306,15 +329,15 @@ __global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 
   }
 }
 
-template <int MODE, int BM>
+template <int MODE, int BM, bool BT = false>
 inline cudaError_t launch_gemm_f(const GemmP<float>& p, cudaStream_t s) {
-  using Cf = FgCfg<BM>;
+  using Cf = FgCfg<BM, BT>;
   const dim3 grid((p.N + Cf::BN - 1) / Cf::BN, (p.M + BM - 1) / BM);
   const size_t smem = Cf::smem(MODE == EPI_SILU_J);
-  const cudaError_t e = cudaFuncSetAttribute(k_gemm_f<MODE, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = cudaFuncSetAttribute(k_gemm_f<MODE, BM, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (grid.y == 0 || grid.x == 0) return cudaSuccess;
-  k_gemm_f<MODE, BM><<<grid, Cf::THREADS, smem, s>>>(p);
+  k_gemm_f<MODE, BM, BT><<<grid, Cf::THREADS, smem, s>>>(p);
   return cudaPeekAtLastError();
 }
 
@@ -429,16 +452,16 @@ inline cudaError_t launch_gemm_d(const GemmP<double>& p, cudaStream_t s) {
   return cudaPeekAtLastError();
 }
 
-template <typename T, int MODE>
+template <typename T, int MODE, bool BT = false>
 inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
     auto tiles = [&](int b) { return (long)((p.N + b - 1) / b) * ((p.M + b - 1) / b); };
     // Where the lines lie (us at K = 256, tiles of 128 / 64 / 32): 184500 x 256 587 / 655 / 732, 20992 x 1280 303 / 306 / 408,
     // 20992 x 256 90 / 79 / 91, 6400 x 1288 117 / 107 / 137, 6400 x 256 38 / 38 / 34, 2560 x 256 38 / 27 / 20,
     // 160 x 256 38 / 26 / 9 (the scalar 128 x 128 kernel before: 877, 441, 120, 160, 42, 42, 41)
-    if (tiles(128) >= 1200) return launch_gemm_f<MODE, 128>(p, s);
-    if (tiles(64) >= 800) return launch_gemm_f<MODE, 64>(p, s);
-    return launch_gemm_f<MODE, 32>(p, s);
+    if (tiles(128) >= 1200) return launch_gemm_f<MODE, 128, BT>(p, s);
+    if (tiles(64) >= 800) return launch_gemm_f<MODE, 64, BT>(p, s);
+    return launch_gemm_f<MODE, 32, BT>(p, s);
   } else if constexpr (MODE == EPI_PLAIN || MODE == EPI_SILU_X || MODE == EPI_ORB_X || MODE == EPI_ENV) {
     return launch_gemm_d<MODE>(p, s);
   } else {

@@ -15,7 +15,7 @@
 //   messages     the e-e pairs' Gamma * silu(e + m_ct + m_nb) (new_sparse_model.py:83-131), their filters and
 //                the cutoff parameter;
 //   ElecInit     Dense 1280, SiLU, GLU, LayerNorm and the e-n edges with the per-nucleus filter parameters.
-// Dense layers are row-major GEMMs on the CUDA cores (gk_mm).  Every weight gradient is a per-walker reduction over
+// Dense layers are row-major GEMMs on the CUDA cores (k_gemm_f; FP64: gk_mm).  Every weight gradient is a per-walker reduction over
 // that walker's rows (gk_wgrad: X^T Y and the column sums of Y for a bias), written straight into the walker's
 // gradient row, which has the layout of the parameter blob (fire_param_layout).
 //
@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "fire_df64.cuh"
+#include "fire_gemm.cuh"
 #include "fire_internal.cuh"
 #include "fire_kernels.cuh"
 
@@ -47,6 +48,7 @@ __host__ __device__ inline long sm_row(int w, int i, int Wc, int nu, int nd) {
 }
 
 // ------------------------------------------------------------------------------------------ GEMMs
+// FP64 (the FP64 pipe bounds it; FP32 goes through k_gemm_f):
 // C[M, N] (ldc) = A[M, K] (lda) op(B) (+ bias) (+ C when acc); op(B) = B [K, N] (ldb), or with BT the transpose of
 // B [N, K] (ldb).  64 x 64 tiles, 16-deep k steps, 256 threads with 4 x 4 outputs each; every load bounds-checked.
 template <typename T, bool BT>
@@ -133,7 +135,7 @@ struct WgP {
   T* bias;   // optional: column sums of Y at bias + w * ldw + n
 };
 
-// Per-walker X^T Y (K x N) over the walker's rows, with the column sums of Y as an extra row when bias is set.
+// FP64: per-walker X^T Y (K x N) over the walker's rows, with the column sums of Y as an extra row when bias is set.
 // Grid (N tiles, K tiles, walkers); each output element is written by one thread (deterministic).
 template <typename T>
 __global__ void __launch_bounds__(256) gk_wgrad(WgP<T> p) {
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(256) gk_wgrad(WgP<T> p) {
   }
 }
 
-// The same reduction for K + (bias ? 1 : 0) <= 16 over many rows (the edge and pair filters' 4- to 16-row weights):
+// The same reduction (FP64) for K + (bias ? 1 : 0) <= 16 over many rows (the edge and pair filters' 4- to 16-row weights):
 // one CTA per 64 columns and walker, 4 row groups of 64 threads; each thread keeps its column's K sums in registers
 // (the X row is a broadcast load, the Y row a coalesced one) and the row groups are summed through shared memory.
 template <typename T>
@@ -238,6 +240,243 @@ __global__ void __launch_bounds__(256) gk_wgrad_skinny(WgP<T> p) {
       p.out[(long)w * p.ldw + (long)(k / p.grp) * p.grp_stride + (long)(k % p.grp) * p.ldo + nc] = v;
     else if (k == p.K && p.bias)
       p.bias[(long)w * p.ldw + nc] = v;
+  }
+}
+
+// FP32 forms of the two reductions above.
+//
+// gk_wgrad_f: 64 x 64 outputs per CTA; 32 rows per stage, copied asynchronously two stages ahead, 8 of them to each of 4 groups
+// of 64 threads, which hold 8 x 8 outputs each and add up at the end (in a fixed order).  gk_wgrad was bound by its shared
+// loads (8 words for 16 products) and, with the pair rows (2207 rows per walker, 64 to 128 CTAs), by one chain of load,
+// barrier and sum: 82 rows x 256 x 256 of 64 walkers 61 -> 33 us, 2207 x 74 x 49 379 -> 149 us.
+constexpr int WGF_R = 32, WGF_ST = 3;
+__global__ void __launch_bounds__(256, 2) gk_wgrad_f(WgP<float> p) {
+  __shared__ __align__(16) float sm[WGF_ST * 2 * WGF_R * 64];  // [stage][X, Y][row][64]; at the end three groups' outputs
+  const int tid = threadIdx.x, g = tid >> 6, tx = tid & 7, ty = (tid >> 3) & 7;
+  const int n0 = blockIdx.x * 64, k0 = blockIdx.y * 64, w = blockIdx.z;
+  const int r0 = p.s[0].rows, rows = r0 + p.s[1].rows;
+  const long b0 = p.s[0].base + (long)w * p.s[0].wstride, b1 = p.s[1].base + (long)w * p.s[1].wstride - r0;
+  const bool vx = p.ldx % 4 == 0 && p.K % 4 == 0 && (reinterpret_cast<uintptr_t>(p.X) & 15) == 0;
+  const bool vy = p.ldy % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.Y) & 15) == 0;
+  const int ns = (rows + WGF_R - 1) / WGF_R;
+  auto copy = [&](float* dst, const float* src, long ld, int c0, int C, bool vec, int st) {
+    const int wd = vec ? 4 : 1;
+    for (int e = tid; e < WGF_R * 64 / wd; e += 256) {
+      const int rr = e / (64 / wd), c = e % (64 / wd) * wd, r = st * WGF_R + rr;
+      const bool ok = r < rows && c0 + c < C;
+      cp_async_n(dst + rr * 64 + c, ok ? src + ((r < r0 ? b0 : b1) + r) * ld + c0 + c : src, 4 * wd, ok);
+    }
+  };
+  auto fetch = [&](int st) {
+    if (st < ns) {
+      float* d = sm + (st % WGF_ST) * 2 * WGF_R * 64;
+      copy(d, p.X, p.ldx, k0, p.K, vx, st);
+      copy(d + WGF_R * 64, p.Y, p.ldy, n0, p.N, vy, st);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  f32x2 acc[8][4], bias[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    bias[j] = 0ull;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i][j] = 0ull;
+  }
+  const bool sum = p.bias && blockIdx.y == 0 && ty == 0;
+#pragma unroll
+  for (int st = 0; st < WGF_ST - 1; ++st) fetch(st);
+  for (int st = 0; st < ns; ++st) {
+    cp_async_left<WGF_ST - 2>();
+    __syncthreads();  // stage st has landed for everyone, and everyone has left stage st - 1
+    fetch(st + WGF_ST - 1);
+    const float* xs = sm + (st % WGF_ST) * 2 * WGF_R * 64 + g * 8 * 64 + ty * 4;
+    const float* ys = sm + (st % WGF_ST) * 2 * WGF_R * 64 + (WGF_R + g * 8) * 64 + tx * 4;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const float4 xa = *reinterpret_cast<const float4*>(xs + r * 64), xb = *reinterpret_cast<const float4*>(xs + r * 64 + 32);
+      const ulonglong2 ya = *reinterpret_cast<const ulonglong2*>(ys + r * 64);
+      const ulonglong2 yb = *reinterpret_cast<const ulonglong2*>(ys + r * 64 + 32);
+      const float x[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+      const f32x2 y[4] = {ya.x, ya.y, yb.x, yb.y};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fma2(pack2(x[i], x[i]), y[j], acc[i][j]);
+      if (sum) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bias[j] = add2(bias[j], y[j]);
+      }
+    }
+  }
+  cp_async_left<0>();
+  __syncthreads();
+  auto kl = [&](int i) { return ty * 4 + (i & 3) + (i >> 2) * 32; };
+  auto nl = [&](int j) { return tx * 4 + (j & 1) * 2 + (j >> 1) * 32; };
+  if (g > 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<f32x2*>(sm + ((g - 1) * 64 + kl(i)) * 64 + nl(j)) = acc[i][j];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int k = k0 + kl(i);
+    if (g > 0 || k >= p.K) continue;
+    float* o = p.out + (long)w * p.ldw + (long)(k / p.grp) * p.grp_stride + (long)(k % p.grp) * p.ldo + n0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f32x2 v = acc[i][j];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v = add2(v, *reinterpret_cast<const f32x2*>(sm + (q * 64 + kl(i)) * 64 + nl(j)));
+      float a, b;
+      unpack2(v, a, b);
+      if (n0 + nl(j) < p.N) o[nl(j)] = a;
+      if (n0 + nl(j) + 1 < p.N) o[nl(j) + 1] = b;
+    }
+  }
+  if (!p.bias || blockIdx.y > 0) return;
+  __syncthreads();
+  if (sum && g > 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<f32x2*>(sm + (g - 1) * 64 + nl(j)) = bias[j];
+  }
+  __syncthreads();
+  if (sum && g == 0) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f32x2 v = bias[j];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) v = add2(v, *reinterpret_cast<const f32x2*>(sm + q * 64 + nl(j)));
+      float a, b;
+      unpack2(v, a, b);
+      if (n0 + nl(j) < p.N) p.bias[(long)w * p.ldw + n0 + nl(j)] = a;
+      if (n0 + nl(j) + 1 < p.N) p.bias[(long)w * p.ldw + n0 + nl(j) + 1] = b;
+    }
+  }
+}
+
+// gk_wgrad_skinny_f<KS>: K + (bias ? 1 : 0) <= KS; 64 columns per CTA, 4 per thread, 32 row groups of 16 threads whose sums
+// meet by a shuffle and then through shared memory.  The Y rows (145 MB for the pair rows of 64 walkers) are read once and
+// bound it; one column per thread and 4 row groups kept too few loads in flight: 340 -> 104 us.
+template <int KS>
+__global__ void __launch_bounds__(512) gk_wgrad_skinny_f(WgP<float> p) {
+  __shared__ float red[16][4][64];
+  const int tid = threadIdx.x, c = (tid & 15) * 4, rg = tid >> 4, warp = tid >> 5, lane = tid & 31;
+  const int nc = blockIdx.x * 64 + c, w = blockIdx.z;
+  const bool vy = p.ldy % 4 == 0 && p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(p.Y) & 15) == 0;
+  const bool vx = p.ldx % 4 == 0 && p.K % 4 == 0 && (reinterpret_cast<uintptr_t>(p.X) & 15) == 0;
+  float acc[KS][4];
+#pragma unroll
+  for (int k = 0; k < KS; ++k)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[k][j] = 0.f;
+#pragma unroll
+  for (int sg = 0; sg < 2; ++sg) {
+    const long rb = p.s[sg].base + (long)w * p.s[sg].wstride;
+#pragma unroll 4
+    for (int r = rg; r < p.s[sg].rows; r += 32) {
+      const float* x = p.X + (rb + r) * p.ldx;
+      const float* yr = p.Y + (rb + r) * p.ldy + nc;
+      float y[4];
+      if (vy) {
+        const float4 q = nc < p.N ? __ldg(reinterpret_cast<const float4*>(yr)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        y[0] = q.x; y[1] = q.y; y[2] = q.z; y[3] = q.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y[j] = nc + j < p.N ? yr[j] : 0.f;
+      }
+      float xv[KS];
+#pragma unroll
+      for (int k = 0; k < KS; k += 4) {
+        if (vx && k < p.K) {
+          const float4 q = __ldg(reinterpret_cast<const float4*>(x + k));
+          xv[k] = q.x; xv[k + 1] = q.y; xv[k + 2] = q.z; xv[k + 3] = q.w;
+        } else {
+#pragma unroll
+          for (int t = k; t < k + 4; ++t) xv[t] = t < p.K ? __ldg(x + t) : (t == p.K && p.bias ? 1.f : 0.f);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[k][j] = fmaf(xv[k], y[j], acc[k][j]);
+    }
+  }
+#pragma unroll
+  for (int kq = 0; kq < KS; kq += 4) {
+    if (kq > 0) __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float v = acc[kq + k][j] + __shfl_xor_sync(0xffffffffu, acc[kq + k][j], 16);
+        if (lane < 16) red[warp][k][c + j] = v;
+      }
+    __syncthreads();
+    if (tid < 256) {
+      const int k = kq + (tid >> 6), n = blockIdx.x * 64 + (tid & 63);
+      float v = 0.f;
+#pragma unroll
+      for (int q = 0; q < 16; ++q) v += red[q][tid >> 6][tid & 63];
+      if (n < p.N) {
+        if (k < p.K)
+          p.out[(long)w * p.ldw + (long)(k / p.grp) * p.grp_stride + (long)(k % p.grp) * p.ldo + n] = v;
+        else if (k == p.K && p.bias)
+          p.bias[(long)w * p.ldw + n] = v;
+      }
+    }
+  }
+}
+
+// C[M, N] (ldc) = A[M, K] (lda) times the transpose of B [N, K] (ldb), N <= 8, K <= 512, rows of A and B 16-byte aligned: a warp
+// takes 4 rows, its lanes 4 consecutive k each, and the 32 dot products meet in 31 shuffles, one result per lane.  Reading A
+// bounds it; the tiled contraction spent 64 columns on 8: 141000 x 8 x 256 175 -> 61 us.
+constexpr int MMN_K = 512;
+__global__ void __launch_bounds__(256) gk_mm_narrow(long M, int N, int K, const float* __restrict__ A, long lda,
+                                                    const float* __restrict__ B, long ldb, float* __restrict__ C, long ldc) {
+  __shared__ __align__(16) float sB[8][MMN_K];
+  for (int e = threadIdx.x; e < 8 * K; e += 256) {
+    const int n = e / K, k = e % K;
+    sB[n][k] = n < N ? B[(long)n * ldb + k] : 0.f;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (long m0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; m0 < M; m0 += (long)gridDim.x * 32) {
+    f32x2 acc[4][8];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int n = 0; n < 8; ++n) acc[r][n] = 0ull;
+    for (int k = lane * 4; k < K; k += 128) {
+      ulonglong2 x[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        x[r] = make_ulonglong2(0ull, 0ull);
+        if (m0 + r < M) x[r] = __ldg(reinterpret_cast<const ulonglong2*>(A + (m0 + r) * lda + k));
+      }
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(&sB[n][k]);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r][n] = fma2(x[r].y, b.y, fma2(x[r].x, b.x, acc[r][n]));
+      }
+    }
+    float v[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) {
+      float a, b;
+      unpack2(acc[q >> 3][q & 7], a, b);
+      v[q] = a + b;
+    }
+#pragma unroll
+    for (int h = 16; h >= 1; h >>= 1) {
+      const bool up = (lane & h) != 0;
+#pragma unroll
+      for (int q = 0; q < h; ++q) v[q] = (up ? v[q + h] : v[q]) + __shfl_xor_sync(0xffffffffu, up ? v[q] : v[q + h], h);
+    }
+    const long m = m0 + (lane >> 3);
+    if (m < M && (lane & 7) < N) C[m * ldc + (lane & 7)] = v[0];
   }
 }
 
@@ -1266,8 +1505,24 @@ template <typename T, bool BT = false>
 void mm(cudaStream_t s, long M, int N, int K, const T* A, long lda, const T* B, long ldb, const T* bias, T* C,
         long ldc, int acc = 0) {
   if (M <= 0 || N <= 0) return;
-  dim3 grid((unsigned)((M + 63) / 64), (unsigned)((N + 63) / 64));
-  gk_mm<T, BT><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, bias, C, ldc, acc);
+  if constexpr (sizeof(T) == 4) {
+    const bool al = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0;
+    // few columns, rows enough to fill the SMs' warps twice (608 CTAs of 8 warps, 4 rows each); below that the 32 x 32 tiles
+    // of k_gemm_f take 12 us at any row count
+    if (BT && N <= 8 && K <= MMN_K && M >= 4096 && !bias && !acc && K % 4 == 0 && lda % 4 == 0 && al) {
+      gk_mm_narrow<<<(unsigned)std::min<long>((M + 31) / 32, 608), 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
+      return;
+    }
+    GemmP<float> g;
+    std::memset(&g, 0, sizeof(g));
+    g.A = A; g.lda = lda; g.B = B; g.ldb = ldb; g.bias = bias; g.bias_period = bias ? 1 : 0; g.C = C; g.ldc = ldc;
+    g.M = (int)M; g.N = N; g.K = K; g.node_div = 1; g.M_scale = 1;
+    if (acc) launch_gemm<float, EPI_ACC, BT>(g, s);
+    else launch_gemm<float, EPI_PLAIN, BT>(g, s);
+  } else {
+    dim3 grid((unsigned)((M + 63) / 64), (unsigned)((N + 63) / 64));
+    gk_mm<T, BT><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, bias, C, ldc, acc);
+  }
 }
 // dX = dY W^T for a layer Y = X W with W [K, N] row-major
 template <typename T>
@@ -1280,11 +1535,21 @@ void wgrad(cudaStream_t s, int Wc, WgP<T> p) {
   const int Ke = p.K + (p.bias ? 1 : 0);
   if (p.grp <= 0) p.grp = p.K > 0 ? p.K : 1;
   if (Ke <= 16) {
-    gk_wgrad_skinny<T><<<dim3((unsigned)((p.N + 63) / 64), 1, (unsigned)Wc), 256, 0, s>>>(p);
+    const dim3 grid((unsigned)((p.N + 63) / 64), 1, (unsigned)Wc);
+    if constexpr (sizeof(T) == 4) {
+      if (Ke <= 8) gk_wgrad_skinny_f<8><<<grid, 512, 0, s>>>(p);
+      else gk_wgrad_skinny_f<16><<<grid, 512, 0, s>>>(p);
+    } else {
+      gk_wgrad_skinny<T><<<grid, 256, 0, s>>>(p);
+    }
     return;
   }
-  dim3 grid((unsigned)((p.N + 63) / 64), (unsigned)((Ke + 63) / 64), (unsigned)Wc);
-  gk_wgrad<T><<<grid, 256, 0, s>>>(p);
+  if constexpr (sizeof(T) == 4) {
+    gk_wgrad_f<<<dim3((unsigned)((p.N + 63) / 64), (unsigned)((p.K + 63) / 64), (unsigned)Wc), 256, 0, s>>>(p);
+  } else {
+    dim3 grid((unsigned)((p.N + 63) / 64), (unsigned)((Ke + 63) / 64), (unsigned)Wc);
+    gk_wgrad<T><<<grid, 256, 0, s>>>(p);
+  }
 }
 // a dense layer's weight (K x N, blob slot wslot) and bias (bslot, or < 0) gradient of walker rows Seg(s)
 template <typename T>
