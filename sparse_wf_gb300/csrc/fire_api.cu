@@ -1275,11 +1275,14 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
   }
   cudaMemsetAsync(c.template buf<double>(c.P.dlap), 0, sizeof(double) * c.Wc * NDET, c.s);
   {
-    // FP32: dependencies with at most DL_CSPLIT positions in 128-thread CTAs (4 per SM), the rest in 256-thread
-    // CTAs; each launch leaves the other's dependencies alone.  FP64: one 256-thread launch.
+    // Dependencies with at most DL_CSPLIT positions (FP64: DL_DSPLIT) in 128-thread CTAs (4 per SM), the rest in 256-thread
+    // CTAs; each launch leaves the other's dependencies alone, and n electrons have at most n positions.  The second launch
+    // finds few: its CTAs walk over the dependencies (32 CTAs per SM in all), where a CTA for each took 305 us to find none
+    // among 111000.
     Prof pr("detlap", c.s);
-    const dim3 grid(c.p->n_el, NDET, c.Wc);
-    auto go = [&](auto kern, int threads, int chi) {
+    const int wd = NDET * c.Wc, n = c.p->n_el;
+    auto go = [&](auto kern, int threads, int chi, int walk) {
+      const dim3 grid(walk ? std::min(n, std::max(1, 4864 / wd)) : n, NDET, c.Wc);
       const size_t smem = sizeof(T) * (size_t)dl_smem_elems(chi);
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       g_nlaunch++;
@@ -1288,10 +1291,12 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
                                          c.template buf<double>(c.P.dlap), c.status);
     };
     if constexpr (sizeof(T) == 4) {
-      go(k_detlap<T, 128, 0, DL_CSPLIT>, 128, DL_CSPLIT);
-      go(k_detlap<T, 256, DL_CSPLIT, DL_CMAX>, 256, DL_CMAX);
+      if (n <= DL_DSPLIT) go(k_detlap<T, 128, 0, DL_DSPLIT>, 128, DL_DSPLIT, 0);  // less shared memory: 8 CTAs per SM
+      else go(k_detlap<T, 128, 0, DL_CSPLIT>, 128, DL_CSPLIT, 0);
+      if (n > DL_CSPLIT) go(k_detlap<T, 256, DL_CSPLIT, DL_CMAX>, 256, DL_CMAX, 1);
     } else {
-      go(k_detlap<T, 256, 0, DL_CMAX>, 256, DL_CMAX);
+      go(k_detlap<T, 128, 0, DL_DSPLIT>, 128, DL_DSPLIT, 0);
+      if (n > DL_DSPLIT) go(k_detlap<T, 256, DL_DSPLIT, DL_CMAX>, 256, DL_CMAX, 0);
     }
   }
   stage_jastrow<T, 3>(c);

@@ -15,6 +15,8 @@
 //               gives d log det / d r_m = sum_i B[(i,m)][i] and the triplet term
 //               -sum_xyz sum_{i,k} B[(i,m)][k] B[(k,m)][i]; the first Laplacian term tr(lap A A^-1) is
 //               accumulated row by row.
+#include <type_traits>
+
 #include "fire_df64.cuh"
 #include "fire_f32x2.cuh"
 #include "fire_internal.cuh"
@@ -479,11 +481,16 @@ __global__ void __launch_bounds__(GJG_THREADS, 2) k_gj_global(const TI* __restri
 // (J rows and rows of the transposed inverse), in 16-byte quads of x = o + sh where sh = (d n) mod 4 makes the
 // J rows of determinant d 16-byte aligned; the inverse rows carry the same shift and zeros outside o in [0, n),
 // which cancel the neighbouring columns the J quads pick up.  Chunks of DL_OC x are copied asynchronously
-// (cp.async) into a ring of DL_STAGES shared-memory buffers, rows of DL_LD elements; each thread accumulates 4 x 4 tiles
-// whose rows (r, r + TR, r + 2 TR, r + 3 TR) and columns (k, k + TC, ...) are strided, so that a warp's 16-byte
-// loads hit consecutive rows: 8 shared loads per 64 FMAs, no bank conflicts.  The result tile reuses the
-// staging memory.
+// (cp.async) into a ring of DL_STAGES shared-memory buffers, rows of DL_LD elements; each thread accumulates one TH x 4 tile
+// whose rows (r, r + TR, r + 2 TR, ...) and columns (k, k + TC, ...) are strided, so that a warp's 16-byte
+// loads hit consecutive rows, no bank conflicts.  The result tile reuses the staging memory.
+// TH is the smallest height with a tile per thread at most: with 4 x 4 tiles, 25 positions made 133 tiles of 128 threads,
+// so that one scheduler ran two rounds, and 10 positions 24 tiles of 256 (FP64).  The triplet sums were bound by the FP64
+// pipe (two conversions and a product per element at 2 per cycle and SM): of FP32 factors they are now exact three-term
+// FP32 expansions.  Before / after, 341 walkers of 82 electrons (25 positions each): 3710 -> 2970 us;
+// 171 walkers of 322: 5440 -> 4270; FP64, 512 walkers of 10 electrons: 2790 -> 327.
 static_assert(3 * DL_CMAX * (DL_CMAX + 1) <= dl_smem_elems(DL_CMAX), "result tile inside the staging buffers");
+static_assert(3 * DL_DSPLIT * (DL_DSPLIT + 1) <= dl_smem_elems(DL_DSPLIT), "result tile inside the staging buffers");
 static_assert(3 * DL_CSPLIT * (DL_CSPLIT + 1) <= dl_smem_elems(DL_CSPLIT), "result tile inside the staging buffers");
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32_det(dst)), "l"(src), "r"(ok ? 16 : 0)
@@ -503,6 +510,46 @@ __device__ __forceinline__ void ld_quad(const double* p, double (&v)[4]) {
   const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
+// One thread's TH x 4 tile of B over one chunk, ascending in the contracted index.
+template <int TH, int QPR, typename T>
+__device__ __forceinline__ void dl_chunk(const T* Jb, const T* Ac, int TR, int TC, T (&acc)[TH * 4]) {
+#pragma unroll 2
+  for (int qx = 0; qx < QPR; ++qx) {
+    T b[4][4];
+#pragma unroll
+    for (int y = 0; y < 4; ++y) ld_quad(Ac + TC * y * DL_LD + 4 * qx, b[y]);
+#pragma unroll
+    for (int j = 0; j < TH; ++j) {
+      T a[4];
+      ld_quad(Jb + TR * j * DL_LD + 4 * qx, a);
+#pragma unroll
+      for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int o = 0; o < 4; ++o) acc[4 * j + y] += a[o] * b[y][o];
+    }
+  }
+}
+// Sum of products: in double, or of FP32 factors as the exact products' three-term expansion (each addition's and each
+// product's rounding error is kept; what is lost is below 2^-70 of the largest partial sum, a double loses 2^-53).  An FP32
+// overflow makes the sum non-finite: the caller then sums in double.
+template <typename T>
+struct DlSum {
+  double s = 0.0;
+  __device__ __forceinline__ void add(T a, T b) { s += a * b; }
+  __device__ __forceinline__ double value() const { return s; }
+};
+template <>
+struct DlSum<float> {
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+  __device__ __forceinline__ void add(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    const df64 h = df_two_sum(s0, p), l = df_two_sum(s1, fmaf(a, b, -p)), m = df_two_sum(l.hi, h.lo);
+    s0 = h.hi;
+    s1 = m.hi;
+    s2 += l.lo + m.lo;
+  }
+  __device__ __forceinline__ double value() const { return (double)s0 + ((double)s1 + (double)s2); }
+};
 // NT threads; jobs with CLO < cnt <= CHI (the others are left to the other instance; cnt > DL_CMAX reports a
 // pair overflow)
 template <typename T, int NT, int CLO, int CHI>
@@ -510,160 +557,131 @@ __global__ void __launch_bounds__(NT) k_detlap(Nbr nb, Layout L, const T* __rest
                                                const T* __restrict__ AinvT, const T* __restrict__ lapA,
                                                double* __restrict__ grad, double* __restrict__ lap, int32_t* status) {
   constexpr int JROWS = dl_jrows(CHI), STAGE = dl_stage_elems(CHI), BLD = CHI + 1;
-  constexpr int MAXT = ((3 * CHI + 3) / 4 * ((CHI + 3) / 4) + NT - 1) / NT;  // 4 x 4 tiles per thread
-  constexpr int RPT = (4 * CHI + NT - 1) / NT;                              // staged rows per thread
   extern __shared__ __align__(16) unsigned char dl_smem[];
   const int n = nb.n, nA = ainv_ld(n);
-  const int m = blockIdx.x, d = blockIdx.y, w = blockIdx.z;
+  const int d = blockIdx.y, w = blockIdx.z;
   if (!walker_live(nb, w)) return;
   const int* rp = nb.rowptr + (size_t)w * (n + 1);
   if (rp[n] > nb.cap_p) return;
-  const int cnt = rp[m + 1] - rp[m] + 1;
-  if (cnt <= CLO) return;
-  if (cnt > CHI) {
-    if (CHI == DL_CMAX && threadIdx.x == 0) set_flag(status, FIRE_FLAG_PAIR_OVERFLOW);
-    return;
-  }
   T* stg = reinterpret_cast<T*>(dl_smem);  // [DL_STAGES][J rows JROWS, inverse rows CHI + 4][DL_LD]
   T* Bm = reinterpret_cast<T*>(dl_smem);   // [3 * CHI][BLD] after the main loop
-  __shared__ long qrow[3 * CHI];           // element index of x = 0 of J row rr
-  __shared__ int is[CHI];
+  __shared__ const T* prow[4 * CHI];       // x = 0 of the R J rows, then of the cnt inverse rows
+  __shared__ double rs[NT / 32];
   const int tid = threadIdx.x;
   const int off = L.pos_off[w];
-  const int s0 = off + rp[m] + m;
+  const T* Ab = AinvT + ((size_t)w * NDET + d) * n * nA;
   const long ldj = (long)NDET * n;
   const int sh = (d * n) & 3, XN = (sh + n + 3) & ~3;
-  for (int k = tid; k < cnt; k += blockDim.x) {
-    const int q = L.dep_pos[s0 + k];
-    is[k] = L.pos_ctr[q] - w * n;
-    for (int t = 0; t < 3; ++t) qrow[3 * k + t] = (3L * q + t) * ldj + (long)d * n - sh;
-  }
-  __syncthreads();
-  const int R = 3 * cnt;
-  const T* Ab = AinvT + ((size_t)w * NDET + d) * n * nA;
-  constexpr int QPR = DL_OC / 4;           // quads per row and chunk
-  constexpr int CPQ = 4 * sizeof(T) / 16;  // 16-byte copies per quad
-  constexpr int EPC = 16 / sizeof(T);      // elements per copy
-  // staging: thread tid owns rows tid, tid + NT, ... of the R J rows followed by the cnt inverse rows is[k],
-  // for the whole job
-  const T* srow[RPT];
-  int drow[RPT];
-#pragma unroll
-  for (int q = 0; q < RPT; ++q) {
-    const int row = tid + q * NT;
-    srow[q] = Ab;
-    drow[q] = -1;
-    if (row < R) {
-      srow[q] = Jp + qrow[row];
-      drow[q] = row * DL_LD;
-    } else if (row < R + cnt) {
-      srow[q] = Ab + (size_t)is[row - R] * nA;
-      drow[q] = (JROWS + row - R) * DL_LD;
+  constexpr int EPC = 16 / sizeof(T), CPR = DL_OC / EPC;  // elements per 16-byte copy, copies per row and chunk
+  constexpr int QPR = DL_OC / 4;                          // quads per row and chunk
+  for (int m = blockIdx.x; m < n; m += gridDim.x) {
+    const int cnt = rp[m + 1] - rp[m] + 1;
+    if (cnt <= CLO) continue;
+    if (cnt > CHI) {
+      if (CHI == DL_CMAX && tid == 0) set_flag(status, FIRE_FLAG_PAIR_OVERFLOW);
+      continue;
     }
-  }
-  auto stage = [&](int buf, int x0) {
-#pragma unroll
-    for (int q = 0; q < RPT; ++q) {
-      if (drow[q] < 0) continue;
-      T* dst = stg + (size_t)buf * STAGE + drow[q];
-#pragma unroll
-      for (int qx = 0; qx < QPR; ++qx) {
-        const int x = x0 + 4 * qx;
-        const bool ok = x < XN;
-#pragma unroll
-        for (int h = 0; h < CPQ; ++h) cp_async16(dst + 4 * qx + h * EPC, ok ? srow[q] + x + h * EPC : Ab, ok);
-      }
+    const int s0 = off + rp[m] + m, R = 3 * cnt;
+    __syncthreads();  // the last job's sums have been read
+    for (int k = tid; k < cnt; k += NT) {
+      const int q = L.dep_pos[s0 + k];
+      for (int t = 0; t < 3; ++t) prow[3 * k + t] = Jp + (3L * q + t) * ldj + (long)d * n - sh;
+      prow[R + k] = Ab + (size_t)(L.pos_ctr[q] - w * n) * nA;
     }
-  };
-  const int TR = (R + 3) / 4, TC = (cnt + 3) / 4, ntile = TR * TC;
-  T acc[MAXT][16];
-#pragma unroll
-  for (int u = 0; u < MAXT; ++u)
-#pragma unroll
-    for (int e = 0; e < 16; ++e) acc[u][e] = T(0);
-  // DL_STAGES - 1 chunks ahead; one commit group per chunk (empty past the end), one barrier per chunk: the
-  // buffer restaged after the barrier of chunk ch held chunk ch - 1, which every thread has finished
-  const int nch = (XN + DL_OC - 1) / DL_OC;
-#pragma unroll
-  for (int c = 0; c < DL_STAGES - 1; ++c) {
-    if (c < nch) stage(c, c * DL_OC);
-    cp_async_commit();
-  }
-  for (int ch = 0; ch < nch; ++ch) {
-    cp_async_wait<DL_STAGES - 2>();
     __syncthreads();
-    {
-      const int nx = ch + DL_STAGES - 1;
-      if (nx < nch) stage(nx % DL_STAGES, nx * DL_OC);
-      cp_async_commit();
+    // staging: CPR neighbouring lanes copy one row's chunk, so that a warp touches 4 lines (2 of doubles) per copy; a thread
+    // per row touched 32 and kept the load unit's tag stage busy for a third of the time
+    auto stage = [&](int buf, int x0) {
+#pragma unroll 4
+      for (int e = tid; e < (R + cnt) * CPR; e += NT) {
+        const int row = e / CPR, c = e % CPR * EPC;
+        const bool ok = x0 + c < XN;
+        cp_async16(stg + (size_t)buf * STAGE + (row < R ? row : JROWS + row - R) * DL_LD + c, ok ? prow[row] + x0 + c : Ab, ok);
+      }
+    };
+    const int TC = (cnt + 3) / 4;
+    const int nch = (XN + DL_OC - 1) / DL_OC;
+    // DL_STAGES - 1 chunks ahead; one commit group per chunk (empty past the end), one barrier per chunk: the
+    // buffer restaged after the barrier of chunk ch held chunk ch - 1, which every thread has finished
+    auto contract = [&](auto th) {
+      constexpr int TH = decltype(th)::value;
+      const int TR = (R + TH - 1) / TH, r0 = tid / TC, k0 = tid - r0 * TC;
+      T acc[TH * 4];
+#pragma unroll
+      for (int q = 0; q < TH * 4; ++q) acc[q] = T(0);
+#pragma unroll
+      for (int c = 0; c < DL_STAGES - 1; ++c) {
+        if (c < nch) stage(c, c * DL_OC);
+        cp_async_commit();
+      }
+      for (int ch = 0; ch < nch; ++ch) {
+        cp_async_wait<DL_STAGES - 2>();
+        __syncthreads();
+        const int nx = ch + DL_STAGES - 1;
+        if (nx < nch) stage(nx % DL_STAGES, nx * DL_OC);
+        cp_async_commit();
+        const T* Jb = stg + (size_t)(ch % DL_STAGES) * STAGE;
+        if (r0 < TR) dl_chunk<TH, QPR>(Jb + r0 * DL_LD, Jb + (JROWS + k0) * DL_LD, TR, TC, acc);
+      }
+      cp_async_wait<0>();
+      __syncthreads();  // every chunk consumed: the result tile overwrites the staging buffers
+      if (r0 < TR) {
+#pragma unroll
+        for (int j = 0; j < TH; ++j)
+#pragma unroll
+          for (int y = 0; y < 4; ++y) {
+            const int r = r0 + TR * j, k = k0 + TC * y;
+            if (r < R && k < cnt) Bm[r * BLD + k] = acc[4 * j + y];
+          }
+      }
+    };
+    const int rt = NT / TC;  // tile rows that the CTA's threads hold
+    if (R <= rt) contract(std::integral_constant<int, 1>());
+    else if (R <= 2 * rt) contract(std::integral_constant<int, 2>());
+    else if (R <= 4 * rt) contract(std::integral_constant<int, 4>());
+    else if (R <= 5 * rt) contract(std::integral_constant<int, 5>());
+    else if (R <= 6 * rt) contract(std::integral_constant<int, 6>());
+    else if (R <= 8 * rt) contract(std::integral_constant<int, 8>());
+    else contract(std::integral_constant<int, 12>());
+    __syncthreads();
+    // triplet term: sum_t sum_{k, k2} B[(k, t)][k2] * B[(k2, t)][k], a warp per row (k, t);  gradient: sum_k B[(k, t)][k];
+    // tr(lap A A^-1) row m: sum_o lapA[m][o] Ainv[o][m]
+    const int lane = tid & 31;
+    const T* lrow = lapA + ((size_t)w * n + m) * ldj + (long)d * n;
+    const T* irow = Ab + (size_t)m * nA + sh;
+    DlSum<T> tl, tr;
+    for (int rr = tid >> 5; rr < R; rr += NT / 32) {
+      const int k = rr / 3, t = rr - 3 * k;
+      for (int k2 = lane; k2 < cnt; k2 += 32) tl.add(Bm[rr * BLD + k2], Bm[(3 * k2 + t) * BLD + k]);
     }
-    const T* Jb = stg + (size_t)(ch % DL_STAGES) * STAGE;
-    const T* Ac = Jb + JROWS * DL_LD;
-#pragma unroll
-    for (int u = 0; u < MAXT; ++u) {
-      const int t = tid + u * NT;
-      if (t < ntile) {
-        const int r0 = t / TC, k0 = t - r0 * TC;
-#pragma unroll 2
-        for (int qx = 0; qx < QPR; ++qx) {
-          T a[4][4], b[4][4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) ld_quad(Jb + (r0 + TR * j) * DL_LD + 4 * qx, a[j]);
-#pragma unroll
-          for (int y = 0; y < 4; ++y) ld_quad(Ac + (k0 + TC * y) * DL_LD + 4 * qx, b[y]);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int y = 0; y < 4; ++y)
-#pragma unroll
-              for (int o = 0; o < 4; ++o) acc[u][4 * j + y] += a[j][o] * b[y][o];
+    for (int o = tid; o < n; o += NT) tr.add(lrow[o], irow[o]);
+    double v = tr.value() - tl.value();
+    if (sizeof(T) == 4) {
+      if (__syncthreads_or(!isfinite(v))) {  // factors beyond 10^19, an infinity or a NaN: in double
+        DlSum<double> tl2, tr2;
+        for (int rr = tid >> 5; rr < R; rr += NT / 32) {
+          const int k = rr / 3, t = rr - 3 * k;
+          for (int k2 = lane; k2 < cnt; k2 += 32) tl2.add((double)Bm[rr * BLD + k2], (double)Bm[(3 * k2 + t) * BLD + k]);
         }
+        for (int o = tid; o < n; o += NT) tr2.add((double)lrow[o], (double)irow[o]);
+        v = tr2.value() - tl2.value();
       }
     }
-  }
-  cp_async_wait<0>();
-  __syncthreads();  // every chunk consumed: the result tile overwrites the staging buffers
-#pragma unroll
-  for (int u = 0; u < MAXT; ++u) {
-    const int t = tid + u * NT;
-    if (t < ntile) {
-      const int r0 = t / TC, k0 = t - r0 * TC;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int y = 0; y < 4; ++y) {
-          const int r = r0 + TR * j, k = k0 + TC * y;
-          if (r < R && k < cnt) Bm[r * BLD + k] = acc[u][4 * j + y];
-        }
+    v = warp_sum(v);
+    if (lane == 0) rs[tid >> 5] = v;
+    if (tid < 96) {  // kept in double: near a node |grad log psi|^2 is ~1e4 |E_loc|
+      const int t = tid >> 5;
+      double gsum = 0.0;
+      for (int k = lane; k < cnt; k += 32) gsum += (double)Bm[(3 * k + t) * BLD + k];
+      gsum = warp_sum(gsum);
+      if (lane == 0) grad[(((size_t)w * NDET + d) * n + m) * 3 + t] = gsum;
     }
-  }
-  __syncthreads();
-  // triplet term: sum_t sum_{k, k2} B[(k, t)][k2] * B[(k2, t)][k];  gradient: sum_k B[(k, t)][k]
-  double tl = 0.0;
-  const int nel = R * cnt;
-  for (int e = tid; e < nel; e += blockDim.x) {
-    const int rr = e / cnt, k2 = e - rr * cnt;
-    const int k = rr / 3, t = rr - 3 * k;
-    tl += (double)Bm[rr * BLD + k2] * (double)Bm[(3 * k2 + t) * BLD + k];
-  }
-  // tr(lap A A^-1) row m: sum_o lapA[m][o] Ainv[o][m]
-  double tr = 0.0;
-  for (int o = tid; o < n; o += blockDim.x)
-    tr += (double)lapA[((size_t)w * n + m) * ldj + (long)d * n + o] * (double)Ab[(size_t)m * nA + sh + o];
-  double v = tr - tl;
-  v = warp_sum(v);
-  __shared__ double rs[NT / 32];
-  if ((tid & 31) == 0) rs[tid >> 5] = v;
-  __syncthreads();
-  if (tid == 0) {
-    double sum = 0.0;
-    for (int q = 0; q < NT / 32; ++q) sum += rs[q];
-    atomicAdd(&lap[w * NDET + d], sum);
-  }
-  if (tid < 3) {
-    double gsum = 0.0;  // kept in double: near a node |grad log psi|^2 is ~1e4 |E_loc|
-    for (int k = 0; k < cnt; ++k) gsum += (double)Bm[(3 * k + tid) * BLD + k];
-    grad[(((size_t)w * NDET + d) * n + m) * 3 + tid] = gsum;
+    __syncthreads();
+    if (tid == 0) {
+      double sum = 0.0;
+      for (int q = 0; q < NT / 32; ++q) sum += rs[q];
+      atomicAdd(&lap[w * NDET + d], sum);
+    }
   }
 }
 
@@ -711,11 +729,15 @@ template __global__ void k_gj_global<double, double, double, true>(const double*
                                                                     double*, double*, const int*, int32_t*);
 template __global__ void k_gj_global<double, double, double, false>(const double*, const double*, int, double*, double*, double*,
                                                                      double*, double*, const int*, int32_t*);
+template __global__ void k_detlap<float, 128, 0, DL_DSPLIT>(Nbr, Layout, const float*, const float*, const float*,
+                                                            double*, double*, int32_t*);
 template __global__ void k_detlap<float, 128, 0, DL_CSPLIT>(Nbr, Layout, const float*, const float*, const float*,
                                                             double*, double*, int32_t*);
 template __global__ void k_detlap<float, 256, DL_CSPLIT, DL_CMAX>(Nbr, Layout, const float*, const float*,
                                                                   const float*, double*, double*, int32_t*);
-template __global__ void k_detlap<double, 256, 0, DL_CMAX>(Nbr, Layout, const double*, const double*,
+template __global__ void k_detlap<double, 128, 0, DL_DSPLIT>(Nbr, Layout, const double*, const double*,
+                                                            const double*, double*, double*, int32_t*);
+template __global__ void k_detlap<double, 256, DL_DSPLIT, DL_CMAX>(Nbr, Layout, const double*, const double*,
                                                             const double*, double*, double*, int32_t*);
 
 }  // namespace fire

@@ -65,8 +65,8 @@ constexpr int ENV_TC_KMAX = 4096;
 // k_detlap staging: up to chi positions per dependency (3 J rows each, DL_CMAX at most), contraction chunks of
 // DL_OC elements in shared-memory rows of DL_LD (16-byte aligned; consecutive rows on distinct bank quads); + 4
 // rows because a thread's strided tile rows may run past the last one; DL_STAGES chunks in flight.  Jobs with
-// at most DL_CSPLIT positions run in small CTAs (128 threads, 4 per SM), the rest in 256-thread CTAs.
-constexpr int DL_CMAX = 64, DL_CSPLIT = 44, DL_OC = 32, DL_LD = DL_OC + 4, DL_STAGES = 2;
+// at most DL_CSPLIT (FP64: DL_DSPLIT) positions run in small CTAs (128 threads, 4 per SM), the rest in 256-thread CTAs.
+constexpr int DL_CMAX = 64, DL_CSPLIT = 44, DL_DSPLIT = 20, DL_OC = 32, DL_LD = DL_OC + 4, DL_STAGES = 2;
 __host__ __device__ constexpr int dl_jrows(int chi) { return 3 * chi + 4; }
 __host__ __device__ constexpr int dl_stage_elems(int chi) { return (dl_jrows(chi) + chi + 4) * DL_LD; }
 __host__ __device__ constexpr int dl_smem_elems(int chi) { return DL_STAGES * dl_stage_elems(chi); }
