@@ -1234,13 +1234,59 @@ cudaError_t chunk_logpsi(Ctx<T>& c, void* logpsi, void* sign, int w0_out) {
 }
 
 // Ill-conditioned walkers of a local-energy call: the first pass appends them to idx (count cnt, capacity cap);
-// the refinement pass evaluates the chunk of their positions with the orbital matrices of c64 (FP64 values of the
-// same walkers) and writes its results to their rows.
+// the refinement pass evaluates the chunk of their positions with the inverses and determinants of FP64 orbital
+// matrices and writes its results to their rows.
 struct Refine {
   int32_t* idx = nullptr;
   int32_t* cnt = nullptr;
   int cap = 0;
-  const Ctx<double>* c64 = nullptr;
+  bool refined = false;         // this is the refinement: the inverses and determinants are made from FP64 values
+  cudaEvent_t ready = nullptr;  // ... on another stream, which this marks (nullptr: on the chunk's own)
+};
+
+// A stream of its own for work that may overlap the caller's, for the length of one call: work forked from `main` starts
+// when it is enqueued there, mark() returns the event that `main` waits for, and whatever is left joins `main` at the end, so
+// that the caller's buffers are the caller's again by stream order.  While `main` is being captured, or if no stream or
+// event can be had, s is `main` itself.
+struct SideStream {
+  cudaStream_t main, s;
+  cudaEvent_t ev = nullptr;
+  explicit SideStream(cudaStream_t m) : main(m), s(m) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(m, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // creation does not touch a capture of another thread
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaStream_t t = nullptr;
+    if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+      ev = nullptr;
+      cudaGetLastError();
+    } else if (cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaEventDestroy(ev);
+      ev = nullptr;
+      cudaGetLastError();
+    } else {
+      s = t;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
+  void fork() {
+    if (s == main) return;
+    cudaEventRecord(ev, main);
+    cudaStreamWaitEvent(s, ev, 0);
+  }
+  cudaEvent_t mark() {
+    if (s == main) return nullptr;
+    cudaEventRecord(ev, s);
+    return ev;
+  }
+  ~SideStream() {
+    if (s == main) return;
+    cudaStreamWaitEvent(main, mark(), 0);
+    cudaEventDestroy(ev);  // both are released once their work is done
+    cudaStreamDestroy(s);
+  }
+  SideStream(const SideStream&) = delete;
+  SideStream& operator=(const SideStream&) = delete;
 };
 
 template <typename T>
@@ -1257,15 +1303,8 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
     Prof pr("gauss_jordan", c.s);
     if constexpr (sizeof(T) == 8) {
       launch_gjg<double, T, T, true>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, c.template buf<T>(c.P.Ainv));
-    } else if (rf.c64) {
-      const Ctx<double>& c64 = *rf.c64;
-      launch_gjg<double, double, T, true>(c64, c64.template buf<double>(c64.P.Apl), (const double*)nullptr,
-                                          c.template buf<T>(c.P.Ainv));
-      const size_t nb = sizeof(double) * (size_t)c.Wc * NDET;
-      cudaMemcpyAsync(c.template buf<double>(c.P.ld), c64.template buf<double>(c64.P.ld), nb,
-                      cudaMemcpyDeviceToDevice, c.s);
-      cudaMemcpyAsync(c.template buf<double>(c.P.sd), c64.template buf<double>(c64.P.sd), nb,
-                      cudaMemcpyDeviceToDevice, c.s);
+    } else if (rf.refined) {
+      if (rf.ready) cudaStreamWaitEvent(c.s, rf.ready, 0);
     } else {
       // the condition numbers of the orbital matrices feed the ill-conditioned test of the assembly
       launch_gjg<df64, T, T, true>(c, c.template buf<T>(c.P.Apl), c.template buf<T>(c.P.Apl_lo),
@@ -1309,7 +1348,7 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
   o.sign = sign;
   o.eloc = eloc;
   if (dbg) o.dbg = *dbg;
-  if (rf.c64) {  // refinement pass: walker w of the chunk is batch walker idx[w]
+  if (rf.refined) {  // refinement pass: walker w of the chunk is batch walker idx[w]
     o.wmap = rf.idx;
     o.wcnt = rf.cnt;
   } else if (rf.idx) {
@@ -1423,10 +1462,19 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
   pr_.chunk_walkers = KC;
   pr_.precision = FIRE_PREC_FP32;  // derivative planes on the CUDA cores in FP32 (the float slots are shared)
   Prof pr("refine", s);
+  SideStream side(s);
   for (int k0 = 0, j = 0; k0 < KF; k0 += KC, ++j) {
     g_nlaunch++;
     k_refine_gather<T><<<KC, 128, 0, s>>>(r, n, rf.idx, rf.cnt, KF, k0, KC, r_ref, r64, sub_cnt + j, status);
-    Ctx<double> c64 = make_ctx<double>(&p64, s, R, Z,
+    Ctx<T> c = make_ctx<T>(&pr_, s, R, Z, prepared, status, ws, KC, true);
+    c.w0 = 0;
+    c.Wc = KC;
+    c.r = r_ref;
+    c.nb.live = sub_cnt + j;
+    // FP64 values, determinants and inverses: bound by the FP64 pipe, while the FP32 planes of the same walkers are bound by
+    // the FP32 one; the two meet at the determinants' Laplacian (each has a workspace of its own but for the results)
+    side.fork();
+    Ctx<double> c64 = make_ctx<double>(&p64, side.s, R, Z,
                                        reinterpret_cast<const unsigned char*>(prepared) + prep64_offset(p), status,
                                        ws + L.c64, KC, false);
     c64.w0 = 0;
@@ -1439,15 +1487,21 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     stage_embedding<double, 0>(c64);
     stage_update<double, 0>(c64);
     stage_orbitals<double, 0>(c64);
-    Ctx<T> c = make_ctx<T>(&pr_, s, R, Z, prepared, status, ws, KC, true);
-    c.w0 = 0;
-    c.Wc = KC;
-    c.r = r_ref;
-    c.nb.live = sub_cnt + j;
+    {
+      Prof pr_gj("gauss_jordan", side.s);
+      launch_gjg<double, double, T, true>(c64, c64.template buf<double>(c64.P.Apl), (const double*)nullptr,
+                                          c.template buf<T>(c.P.Ainv));
+      const size_t nb = sizeof(double) * (size_t)KC * NDET;
+      cudaMemcpyAsync(c.template buf<double>(c.P.ld), c64.template buf<double>(c64.P.ld), nb, cudaMemcpyDeviceToDevice,
+                      side.s);
+      cudaMemcpyAsync(c.template buf<double>(c.P.sd), c64.template buf<double>(c64.P.sd), nb, cudaMemcpyDeviceToDevice,
+                      side.s);
+    }
     Refine sub = rf;
     sub.idx = rf.idx + k0;
     sub.cnt = sub_cnt + j;
-    sub.c64 = &c64;
+    sub.refined = true;
+    sub.ready = side.mark();
     const cudaError_t e = chunk_eloc<T>(c, logpsi, sign, eloc, dbg, sub);
     if (e != cudaSuccess) return e;
   }
