@@ -244,6 +244,25 @@ __global__ void k_lr_env_add(long total, T* __restrict__ env_p, const T* __restr
   if (i < total) env_p[i] += env_d[i];
 }
 
+// four consecutive values of a 16-byte aligned row
+__device__ __forceinline__ void lr_quad(const float* p, float (&v)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+}
+__device__ __forceinline__ void lr_quad(const double* p, double (&v)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+// magnitudes of pivot candidates and their order (a double-FP32 number's high part decides unless equal)
+__device__ __forceinline__ double lr_abs(double x) { return fabs(x); }
+__device__ __forceinline__ df64 lr_abs(df64 x) { return x.hi < 0.f ? df64(-x.hi, -x.lo) : x; }
+__device__ __forceinline__ bool lr_less(double a, double b) { return a < b; }
+__device__ __forceinline__ bool lr_less(df64 a, df64 b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
+__device__ __forceinline__ double lr_shfl_xor(double x, int o) { return __shfl_xor_sync(kFull, x, o); }
+__device__ __forceinline__ df64 lr_shfl_xor(df64 x, int o) {
+  return df64(__shfl_xor_sync(kFull, x.hi, o), __shfl_xor_sync(kFull, x.lo, o));
+}
+
 // One CTA (256 threads) per (determinant d, walker w).  rawS [W][KS][DN]: raw orbital rows of S; env, Apl
 // [W][n][DN]: the state's envelope and orbital-matrix rows; env_p [W][KM][DN]: the envelope rows of the moved
 // electrons moved[w][0..KM) after the move.  B: the
@@ -251,7 +270,8 @@ __global__ void k_lr_env_add(long total, T* __restrict__ env_p, const T* __restr
 // Writes V [W][NDET][KS][n] (A'[S] - A[S]), Minv [W][NDET][KS][KS] (double) and the proposal's slogdet
 // (ld_p, sd_p) = (ld + log|det M|, sd sign(det M)).  A set larger than KS (flagged by k_lr_select) gives sign 0:
 // the proposal is rejected.  Dynamic shared memory: KS * KS doubles (M, inverted in place) + 2 * KS * 33 elements
-// of T (the staged V and B[S] columns).
+// of T (the staged V and B[S] columns).  Bound by the chain of its elimination steps: 256 walkers of 10 electrons 113 ->
+// 34 us, 128 of 322 470 -> 216 us.
 template <typename T>
 __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const int* __restrict__ S_cnt, int KS,
                                                 int n, const int* __restrict__ moved, int KM, const T* __restrict__ rawS,
@@ -270,7 +290,8 @@ __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const
   T* Bt = Vt + (size_t)KS * 33;                                // [KS][33]
   __shared__ int sS[LR_KMAX];
   __shared__ int perm[LR_KMAX];
-  __shared__ SE fac[LR_KMAX];
+  __shared__ SE fac[LR_KMAX], piv[LR_KMAX];
+  __shared__ double plog[LR_KMAX];
   __shared__ int piv_row;
   const int d = blockIdx.x, w = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int cnt = S_cnt[w];
@@ -285,17 +306,24 @@ __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const
   const int k = cnt;
   const int DN = NDET * n, nA = ainv_ld(n), sh = (d * n) & 3;
   for (int a = tid; a < k; a += blockDim.x) sS[a] = S[(size_t)w * KS + a];
-  for (int q = tid; q < k * k; q += blockDim.x) Ms[q] = (q / k == q % k) ? SE(1.0) : SE(0.0);
+  // a warp per row, its lanes over the columns, in every loop below
+  for (int a = wid; a < k; a += 8)
+    for (int b = lane; b < k; b += 32) Ms[a * k + b] = a == b ? SE(1.0) : SE(0.0);
   __syncthreads();
   // V rows: A'[S] - A[S] (the orbital-matrix rows are raw * envelope, as in the value path)
   T* Vw = V + md * KS * n;
-  for (long q = tid; q < (long)k * n; q += blockDim.x) {
-    const int a = (int)(q / n), o = (int)(q - (long)a * n), c = sS[a];
+  for (int a = wid; a < k; a += 8) {
+    const int c = sS[a];
     const T* er = env + ((size_t)w * n + c) * DN;
     for (int t = 0; t < KM; ++t)
       if (moved[(size_t)w * KM + t] == c) er = env_p + ((size_t)w * KM + t) * DN;
-    const T an = rawS[((size_t)w * KS + a) * DN + (size_t)d * n + o] * er[(size_t)d * n + o];
-    Vw[(size_t)a * n + o] = an - Apl[((size_t)w * n + c) * DN + (size_t)d * n + o];
+    er += (size_t)d * n;
+    const T* rs = rawS + ((size_t)w * KS + a) * DN + (size_t)d * n;
+    const T* ap = Apl + ((size_t)w * n + c) * DN + (size_t)d * n;
+    for (int o = lane; o < n; o += 32) {
+      const T an = rs[o] * er[o];
+      Vw[(size_t)a * n + o] = an - ap[o];
+    }
   }
   __syncthreads();
   // M = I + V A^-1[:, S]: (A^-1)[o][S_b] = B[S_b][o]; 32 orbitals per pass
@@ -307,36 +335,35 @@ __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const
       Bt[a * 33 + oo] = o < n ? Bw[(size_t)sS[a] * nA + o] : T(0);
     }
     __syncthreads();
-    for (int q = tid; q < k * k; q += blockDim.x) {
-      const int a = q / k, b = q - a * k;
-      T s = T(0);
+    for (int a = wid; a < k; a += 8)
+      for (int b = lane; b < k; b += 32) {
+        T s = T(0);
 #pragma unroll 8
-      for (int oo = 0; oo < 32; ++oo) s += Vt[a * 33 + oo] * Bt[b * 33 + oo];
-      Ms[q] += SE(s);
-    }
+        for (int oo = 0; oo < 32; ++oo) s += Vt[a * 33 + oo] * Bt[b * 33 + oo];
+        Ms[a * k + b] += SE(s);
+      }
     __syncthreads();
   }
   // in-place Gauss-Jordan with row pivoting: after step t row t holds the pivot row of the inverse; the row swaps
   // are undone on the columns at the end.  det M = (-1)^swaps prod(pivots).
-  double ldet = 0.0;
   int neg = 0;
   bool singular = false;
   for (int t = 0; t < k; ++t) {
     if (wid == 0) {
-      double best = -1.0;
+      SE best = SE(-1.0);
       int bi = t;
       for (int i = t + lane; i < k; i += 32) {
-        const double v = fabs((double)Ms[i * k + t]);
-        if (v > best) {
+        const SE v = lr_abs(Ms[i * k + t]);
+        if (lr_less(best, v)) {
           best = v;
           bi = i;
         }
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
-        const double ob = __shfl_xor_sync(kFull, best, o);
+        const SE ob = lr_shfl_xor(best, o);
         const int oi = __shfl_xor_sync(kFull, bi, o);
-        if (ob > best || (ob == best && oi < bi)) {
+        if (lr_less(best, ob) || (!lr_less(ob, best) && oi < bi)) {
           best = ob;
           bi = oi;
         }
@@ -347,37 +374,46 @@ __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const
       }
     }
     __syncthreads();
+    // the swap of rows t and p, the scaled pivot row and the factors, read before any of them is written
     const int p = piv_row;
-    if (p != t) {
-      for (int q = tid; q < k; q += blockDim.x) {
-        const SE x = Ms[t * k + q];
-        Ms[t * k + q] = Ms[p * k + q];
-        Ms[p * k + q] = x;
-      }
-      neg ^= 1;
-    }
-    __syncthreads();
-    const SE pv = Ms[t * k + t];
-    const double pvd = (double)pv;
-    if (pvd == 0.0) {
+    const SE pv = Ms[p * k + t];
+    if ((double)pv == 0.0) {
       singular = true;
       break;
     }
-    ldet += log(fabs(pvd));
-    if (pvd < 0.0) neg ^= 1;
+    if (p != t) neg ^= 1;
+    if ((double)pv < 0.0) neg ^= 1;
     const SE ip = SE(1.0) / pv;
-    __syncthreads();
-    for (int q = tid; q < k; q += blockDim.x) {
-      Ms[t * k + q] = q == t ? ip : Ms[t * k + q] * ip;
-      fac[q] = q == t ? SE(0.0) : Ms[q * k + t];
+    SE x, y, f;
+    const int q = tid;  // k <= LR_KMAX < 256
+    if (q < k) {
+      x = Ms[p * k + q];
+      y = Ms[t * k + q];
+      f = q == t ? SE(0.0) : Ms[(q == p ? t : q) * k + t];
     }
     __syncthreads();
-    for (int q = tid; q < k * k; q += blockDim.x) {
-      const int i = q / k, c = q - i * k;
+    if (q < k) {
+      if (p != t) Ms[p * k + q] = y;
+      Ms[t * k + q] = q == t ? ip : x * ip;
+      fac[q] = f;
+      if (q == t) piv[t] = pv;
+    }
+    __syncthreads();
+    for (int i = wid; i < k; i += 8) {
       if (i == t) continue;
-      Ms[q] = c == t ? -(fac[i] * Ms[t * k + t]) : df_sub_mul(Ms[q], fac[i], Ms[t * k + c]);
+      for (int c = lane; c < k; c += 32)
+        Ms[i * k + c] = c == t ? -(fac[i] * Ms[t * k + t]) : df_sub_mul(Ms[i * k + c], fac[i], Ms[t * k + c]);
     }
     __syncthreads();
+  }
+  // the pivots' logarithms, all at once (in the loop every thread took each: the FP64 pipe's two results per cycle made
+  // them most of a step), summed in their order
+  double ldet = 0.0;
+  if (!singular) {
+    if (tid < k) plog[tid] = log(fabs((double)piv[tid]));
+    __syncthreads();
+    if (tid == 0)
+      for (int t = 0; t < k; ++t) ldet += plog[t];
   }
   if (!singular) {
     for (int t = k - 1; t >= 0; --t) {
@@ -392,10 +428,8 @@ __global__ void __launch_bounds__(256) k_lr_det(const int* __restrict__ S, const
     }
   }
   double* Mo = Minv + md * KS * KS;
-  for (int q = tid; q < k * k; q += blockDim.x) {
-    const int a = q / k, b = q - a * k;
-    Mo[(size_t)a * KS + b] = singular ? 0.0 : (double)Ms[q];
-  }
+  for (int a = wid; a < k; a += 8)
+    for (int b = lane; b < k; b += 32) Mo[(size_t)a * KS + b] = singular ? 0.0 : (double)Ms[a * k + b];
   if (tid == 0) {
     ld_p[md] = ld[md] + (singular ? 0.0 : ldet);
     sd_p[md] = singular ? 0.0 : (neg ? -sd[md] : sd[md]);
@@ -619,7 +653,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_lr_wb_apply(const int* __restrict__ accf, const int* __restrict__ S_cnt,
                                                      int KS, int n, T* __restrict__ B, const T* __restrict__ Zb,
                                                      const T* __restrict__ Qb) {
-  __shared__ T Zs[32][33];
+  __shared__ __align__(16) T Zs[32][36];
   __shared__ T Qs[32][33];
   const int w = blockIdx.z, d = blockIdx.y, i0 = blockIdx.x * 32, tid = threadIdx.x, jj = tid & 31, g = tid >> 5;
   if (!accf[w]) return;
@@ -634,15 +668,22 @@ __global__ void __launch_bounds__(256) k_lr_wb_apply(const int* __restrict__ acc
     for (int a0 = 0; a0 < k; a0 += 32) {
       for (int q = tid; q < 32 * 32; q += blockDim.x) {
         const int rr = q >> 5, cc = q & 31;
-        Zs[rr][cc] = (i0 + rr < n && a0 + cc < k) ? Zw[(size_t)(i0 + rr) * KS + a0 + cc] : T(0);
+        if (j0 == 0 || k > 32) Zs[rr][cc] = (i0 + rr < n && a0 + cc < k) ? Zw[(size_t)(i0 + rr) * KS + a0 + cc] : T(0);
         Qs[rr][cc] = (a0 + rr < k && j0 + cc < n) ? Qw[(size_t)(a0 + rr) * n + j0 + cc] : T(0);
       }
       __syncthreads();
-#pragma unroll 8
-      for (int aa = 0; aa < 32; ++aa) {
-        const T qv = Qs[aa][jj];
+#pragma unroll 4
+      for (int aa = 0; aa < 32; aa += 4) {
+        const T q0 = Qs[aa][jj], q1 = Qs[aa + 1][jj], q2 = Qs[aa + 2][jj], q3 = Qs[aa + 3][jj];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) acc[t] += Zs[g + 8 * t][aa] * qv;
+        for (int t = 0; t < 4; ++t) {
+          T z[4];
+          lr_quad(&Zs[g + 8 * t][aa], z);
+          acc[t] += z[0] * q0;
+          acc[t] += z[1] * q1;
+          acc[t] += z[2] * q2;
+          acc[t] += z[3] * q3;
+        }
       }
       __syncthreads();
     }
