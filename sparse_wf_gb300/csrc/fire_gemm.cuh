@@ -141,7 +141,7 @@ struct FgCfg {
 // BT: B is the transpose of p.B [N, K] (p.ldb); its tile is kept like A's, k contiguous, and a thread's columns lie TX apart
 // so that their rows are read without bank conflicts.
 template <int MODE, int BM, bool BT = false>
-__global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 ? 7 : 1)) k_gemm_f(GemmP<float> p) {
+__global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 ? 7 : 6)) k_gemm_f(GemmP<float> p) {
   using Cf = FgCfg<BM, BT>;
   constexpr int BN = Cf::BN, TM = Cf::TM, NT = Cf::THREADS, H = BM / 2;  // H: rows (columns) between a thread's two halves
   constexpr int TX = BN / TM, FGK = Cf::FGK, FGA = Cf::FGA;
@@ -456,11 +456,11 @@ template <typename T, int MODE, bool BT = false>
 inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
     auto tiles = [&](int b) { return (long)((p.N + b - 1) / b) * ((p.M + b - 1) / b); };
-    // Where the lines lie (us at K = 256, tiles of 128 / 64 / 32): 184500 x 256 587 / 655 / 732, 20992 x 1280 303 / 306 / 408,
-    // 20992 x 256 90 / 79 / 91, 6400 x 1288 117 / 107 / 137, 6400 x 256 38 / 38 / 34, 2560 x 256 38 / 27 / 20,
-    // 160 x 256 38 / 26 / 9 (the scalar 128 x 128 kernel before: 877, 441, 120, 160, 42, 42, 41)
+    // Where the lines lie (us at K = 256, tiles of 128 / 64 / 32): 184500 x 256 588 / 657 / 733, 20992 x 1280 302 / 305 / 358,
+    // 20992 x 256 90 / 79 / 78, 6400 x 256 38 / 38 / 30, 2560 x 256 38 / 27 / 16, 160 x 256 38 / 26 / 9 (the scalar 128 x 128
+    // kernel before: 880, 441, 120, 42, 42, 41).  Slower: 256 x 128 outputs, 16 x 8 per thread (814 and 399 on the first two).
     if (tiles(128) >= 1200) return launch_gemm_f<MODE, 128, BT>(p, s);
-    if (tiles(64) >= 800) return launch_gemm_f<MODE, 64, BT>(p, s);
+    if (tiles(64) >= 1600) return launch_gemm_f<MODE, 64, BT>(p, s);
     return launch_gemm_f<MODE, 32, BT>(p, s);
   } else if constexpr (MODE == EPI_PLAIN || MODE == EPI_SILU_X || MODE == EPI_ORB_X || MODE == EPI_ENV) {
     return launch_gemm_d<MODE>(p, s);
