@@ -257,6 +257,7 @@ struct SlArgs {
   const unsigned char* Bt[2];
   size_t Bt_bs, b_code;
   SlTile tl;
+  int pw;  // 16-column pieces of a column tile per unit of work
   int row0, row1;  // this pass's rows of every segment
   int ns[2], soff[2], spin[2];
   const int* tile_mask;
@@ -463,15 +464,19 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
       rows[g] = max(0, min(rows[g], a.row1) - a.row0);
       mt[g] = (rows[g] + 127) / 128;
     }
-  const int t0 = a.batch * mt[0] * nt, total = t0 + a.batch * mt[1] * nt;
+  // a column tile may be split into ncp parts of pw pieces of 16 columns, each its own unit of work (few rows)
+  const int np = nc / 16, pw = a.pw, ncp = (np + pw - 1) / pw, nu = nt * ncp;
+  const int t0 = a.batch * mt[0] * nu, total = t0 + a.batch * mt[1] * nu;
   if ((int)blockIdx.x >= total) return;
-  // tile t: segment, batch block, row tile, column tile (column tiles of a row tile run next to each other: its slices
-  // come from L2)
-  auto decode = [&](int t, int& g, int& b, int& m, int& n) -> bool {
+  // unit t: segment, batch block, row tile, column tile and the first piece in it (column tiles of a row tile run next to
+  // each other: its slices come from L2)
+  auto decode = [&](int t, int& g, int& b, int& m, int& n, int& p0) -> bool {
     g = t >= t0 ? 1 : 0;
     if (g) t -= t0;
-    n = t % nt;
-    const int r = t / nt;
+    n = t % nu;
+    const int r = t / nu;
+    p0 = n % ncp * pw;
+    n /= ncp;
     m = r % mt[g];
     b = r / mt[g];
     return !a.tile_mask || ((a.tile_mask[a.row0 / 128 + m] >> a.spin[g]) & 1);
@@ -504,8 +509,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     // ------------------------------------------------------------------ loader
     if (lane == 0) {
       for (int t = blockIdx.x; t < total && !*abort; t += gridDim.x) {
-        int g, b, m, n;
-        if (!decode(t, g, b, m, n)) continue;
+        int g, b, m, n, p0;
+        if (!decode(t, g, b, m, n, p0)) continue;
         const unsigned char* as = a.At[g] + (size_t)b * a.At_bs[g] + (size_t)m * nkb * Sm::A_STEP;
         const unsigned char* bs = a.Bt[g] + (size_t)b * a.Bt_bs + (size_t)n * nkb * Sm::B_STEP;
         for (int kb = 0; kb < nkb; ++kb) {
@@ -521,12 +526,12 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer (warp-uniform; one lane issues)
-    const uint32_t idesc = (1u << 4) | ((uint32_t)(nc >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
     long kc = 0, uc = 0;
     bool live = true;
     for (int t = blockIdx.x; t < total && live; t += gridDim.x) {
-      int g, b, m, n;
-      if (!decode(t, g, b, m, n)) continue;
+      int g, b, m, n, p0;
+      if (!decode(t, g, b, m, n, p0)) continue;
+      const uint32_t idesc = (1u << 4) | ((uint32_t)(2 * min(pw, np - p0)) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
       for (int kb = 0; kb < nkb; ++kb, ++kc) {
         const bool start = kb % SL_KCH == 0;
         if (start && uc > 0) {
@@ -539,7 +544,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
         if (!live) break;
         tc_fence_after();
         const uint64_t da = tc_desc_s(s0 + q * Sm::STAGE, 2048, 128);
-        const uint64_t db = tc_desc_s(s0 + q * Sm::STAGE + Sm::A_STEP, 16 * Fm::NMAX, 128);
+        const uint64_t db = tc_desc_s(s0 + q * Sm::STAGE + Sm::A_STEP + p0 * 256, 16 * Fm::NMAX, 128);  // 16 columns: 256 bytes
 #pragma unroll
         for (int i = 0; i < NS; ++i)
 #pragma unroll
@@ -555,15 +560,16 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     }
   } else {
     // ------------------------------------------------------------------ epilogue (warps 0-7)
-    const int quad = warp & 3, half = warp >> 2, np = nc / 16;
+    const int quad = warp & 3, half = warp >> 2;
     const uint32_t tq = tmem + ((uint32_t)(quad * 32) << 16);
     long uc = 0;
     bool live = true;  // warp-uniform
     for (int t = blockIdx.x; t < total && live; t += gridDim.x) {
-      int g, b, m, n;
-      if (!decode(t, g, b, m, n)) continue;
+      int g, b, m, n, p0;
+      if (!decode(t, g, b, m, n, p0)) continue;
       const GemmP<T>& p = a.p[g];
-      const int M = a.row0 + rows[g], N = p.N, l0 = m * 128 + quad * 32, m0 = a.row0 + l0, n0 = n * nc;
+      const int M = a.row0 + rows[g], N = p.N, l0 = m * 128 + quad * 32, m0 = a.row0 + l0, n0 = n * nc + p0 * 16;
+      const int nl = min(pw, np - p0);  // pieces of this unit
       const int* bc = reinterpret_cast<const int*>(a.Bt[g] + (size_t)b * a.Bt_bs + a.b_code);
       const int rc = a.ac[g][b * a.ac_bs[g] + l0 + lane];
       SlAcc<KIND> acc;
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
 #pragma unroll
         for (int ci = 0; ci < SlAcc<KIND>::NC; ++ci) {  // pieces half, half + 2, ... of the tile's columns
           const int c = half + 2 * ci;
-          if (c < np) sl_drain(acc, ci, tq + (uint32_t)(c * 16), k0 == 0);
+          if (c < nl) sl_drain(acc, ci, tq + (uint32_t)(c * 16), k0 == 0);
         }
         tc_fence_before();
         tc_arrive(&bars->tempty);
@@ -601,7 +607,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
 #pragma unroll
       for (int ci = 0; ci < SlAcc<KIND>::NC; ++ci) {
         const int c = half + 2 * ci;
-        if (c >= np) continue;
+        if (c >= nl) continue;
         const int col = n0 + c * 16 + cl;
         const int cc = col < N ? bc[col] : SL_ZERO;
         if constexpr (KIND == SL_PAIR) {
@@ -785,7 +791,12 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
     }
     const dim3 gr((unsigned)(sl_rows(rows) / 32), (unsigned)c.batch, (unsigned)sliced);
     k_slice_rows<KIND, T><<<gr, 32 * SLR_WARPS, 0, s>>>(r);
-    k_gemm_sl<KIND, MODE><<<(unsigned)std::min<long>(tiles, sms), SL_THREADS, smem, s>>>(a, status);
+    // Few tiles: parts of two pieces or of one, as long as each gets an SM of its own (an MMA of 16 columns takes 36 cycles
+    // where 64 take 48, and a unit's epilogue goes with its columns): 160 rows x 256 x 256 26 -> 20 us.
+    const int np = a.tl.nc / 16;
+    a.pw = tiles * np <= sms ? 1 : (tiles * ((np + 1) / 2) <= sms ? std::min(2, np) : np);
+    const long units = tiles * ((np + a.pw - 1) / a.pw);
+    k_gemm_sl<KIND, MODE><<<(unsigned)std::min<long>(units, sms), SL_THREADS, smem, s>>>(a, status);
     launched += 2;
   }
   return cudaPeekAtLastError() == cudaSuccess ? launched : -1;
