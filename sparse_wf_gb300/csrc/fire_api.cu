@@ -4,7 +4,7 @@
 // wave_function.py:165-181 + hamiltonian.py:69-81):
 //   neighbours -> layout -> ElecInit (edges, LayerNorm) -> GLU/Dense/Dense GEMMs on [x, jac, lap]
 //   -> e-e edges + messages -> update MLP (2 x silu layers) -> envelopes -> orbitals
-//   -> FP64 Gauss-Jordan -> determinant Laplacian -> attention Jastrow -> MLP Jastrow -> assembly.
+//   -> double-FP32 or FP64 Gauss-Jordan -> determinant Laplacian -> attention Jastrow -> MLP Jastrow -> assembly.
 // The value path (log|psi|, the MCMC building block) runs the same stages without tangents.
 #include <algorithm>
 #include <cmath>

@@ -1,7 +1,8 @@
 // fire_gemm.cuh -- CUDA-core GEMM C = A[M,K] * B[K,N] with fused forward-Laplacian epilogues.
 //
-// This is the contraction engine of the FP32 and FP64 paths.  Every dense layer of the sparse
-// forward Laplacian (sparse_fwd_lap.py:160-225) is applied to three "planes" of one node:
+// k_gemm_f: FP32 (derivative planes of the FP32 path, plain value rows, gradients); k_gemm_d: FP64 (the refinement's values,
+// narrow layers; fire_sliced.cu has the FP64 build's wide ones); k_gemm_comp: the FP32 local energy's compensated value
+// rows; k_gemm_env_df: the refinement's envelope rows.  Every dense layer of the sparse forward Laplacian (sparse_fwd_lap.py:160-225) is applied to three "planes" of one node:
 //   X plane  [nodes, K]        values            (bias added)
 //   J plane  [3 * positions, K] Jacobian rows    (sorted by center)
 //   L plane  [nodes, K]        Laplacians

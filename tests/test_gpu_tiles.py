@@ -68,6 +68,18 @@ def test_tiles_of_batch_sizes():
         assert abs(float(big[w]) - want) <= 2e-5 * scale
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_parts_of_column_tiles(precision):
+    """log|psi| of 16, 200 and 2000 walkers of 10 electrons: column tiles in parts of one and of two pieces, and whole; the
+    sums are exact either way, so that the walkers' values agree to the rounding of their type."""
+    mol = systems.hydrogen_chain(10, 1.8)
+    wf, p, _ = _model(mol, precision)
+    r = systems.init_electrons(mol, 2000, 13)
+    a, b, c = (wf.signed(p, r[:w], wf.get_static_input(r[:w]))[1][:16].double().cpu().numpy() for w in (16, 200, 2000))
+    tol = (1e-12 if precision == "fp64" else 1e-6) * np.maximum(1.0, np.abs(a))
+    assert np.all(np.abs(b - a) <= tol) and np.all(np.abs(c - a) <= tol)
+
+
 @pytest.mark.parametrize("walkers", [1, 3, 40])
 def test_every_walker_refined(walkers):
     """More walkers refined than the first pass's room (a quarter of the batch): the call runs again with room for all."""
