@@ -164,29 +164,27 @@ void tc_offsets(const fire_problem* p, size_t float_bytes, size_t* off) {
 // Weights of the sliced contractions (fire_sliced.cuh), cut when the parameters are prepared: for the value path of the FP32
 // and mixed builds (SL_PAIR, without the attention readout's), for every layer in FP64 (SL_F64).
 enum SlSlot {
-  SLW_GLU, SLW_DENSE, SLW_OUT, SLW_UPD1, SLW_UPD2, SLW_ORB_UP, SLW_ORB_DN, SLW_V, SLW_JMLP1, SLW_JMLP2, SLW_ENV_UP,
-  SLW_ENV_DN, SLW_READ1, SLW_READ2, SLW_COUNT
+  SLW_GLU, SLW_DENSE, SLW_OUT, SLW_UPD1, SLW_UPD2, SLW_ORB_UP, SLW_ORB_DN, SLW_V, SLW_JMLP1, SLW_JMLP2, SLW_READ1,
+  SLW_READ2, SLW_COUNT
 };
 struct SlSrc {
-  int slot, K, N, batch;
+  int slot, K, N;
 };
 SlSrc sl_src(int k, const fire_problem* p) {
-  const int DN = NDET * p->n_el, K8 = NENV_ORB * p->n_nuc;
+  const int DN = NDET * p->n_el;
   switch (k) {
-    case SLW_GLU: return {FIRE_P_EI_GLU_W, F, 2 * F, 1};
-    case SLW_DENSE: return {FIRE_P_EI_DENSE_W, F, F, 1};
-    case SLW_OUT: return {FIRE_P_EI_OUT_W, F, 5 * F, 1};
-    case SLW_UPD1: return {PR_UPD1_W_S0, F, F, 1};
-    case SLW_UPD2: return {FIRE_P_UPD2_W, F, F, 1};
-    case SLW_ORB_UP: return {PR_ORB_UP_W_S1, F, DN, 1};
-    case SLW_ORB_DN: return {PR_ORB_DN_W_S1, F, DN, 1};
-    case SLW_V: return {PR_V_W_S1, F, F, 1};
-    case SLW_JMLP1: return {PR_JMLP1_W_S1, F, F, 1};
-    case SLW_JMLP2: return {FIRE_P_JMLP2_W, F, F, 1};
-    case SLW_ENV_UP: return {PR_ENV_UP_PI, K8, p->n_el, NDET};
-    case SLW_ENV_DN: return {PR_ENV_DN_PI, K8, p->n_el, NDET};
-    case SLW_READ1: return {FIRE_P_ATT_OUT1_W, 2 * F, F, 1};
-    default: return {FIRE_P_ATT_OUT2_W, F, F, 1};
+    case SLW_GLU: return {FIRE_P_EI_GLU_W, F, 2 * F};
+    case SLW_DENSE: return {FIRE_P_EI_DENSE_W, F, F};
+    case SLW_OUT: return {FIRE_P_EI_OUT_W, F, 5 * F};
+    case SLW_UPD1: return {PR_UPD1_W_S0, F, F};
+    case SLW_UPD2: return {FIRE_P_UPD2_W, F, F};
+    case SLW_ORB_UP: return {PR_ORB_UP_W_S1, F, DN};
+    case SLW_ORB_DN: return {PR_ORB_DN_W_S1, F, DN};
+    case SLW_V: return {PR_V_W_S1, F, F};
+    case SLW_JMLP1: return {PR_JMLP1_W_S1, F, F};
+    case SLW_JMLP2: return {FIRE_P_JMLP2_W, F, F};
+    case SLW_READ1: return {FIRE_P_ATT_OUT1_W, 2 * F, F};
+    default: return {FIRE_P_ATT_OUT2_W, F, F};
   }
 }
 // Byte offsets of the sliced weights behind the slots of T (and, in the mixed path, the tensor-core weights);
@@ -206,8 +204,8 @@ void sl_offsets(const fire_problem* p, size_t* off) {
     off[k] = o;
     if (k == SLW_COUNT) break;
     const SlSrc q = sl_src(k, p);
-    if (sizeof(T) == 8) o += q.batch * sl_w_bytes<SL_F64>(q.K, q.N);
-    else if (k < SLW_READ1) o += q.batch * sl_w_bytes<SL_PAIR>(q.K, q.N);
+    if (sizeof(T) == 8) o += sl_w_bytes<SL_F64>(q.K, q.N);
+    else if (k < SLW_READ1) o += sl_w_bytes<SL_PAIR>(q.K, q.N);
   }
 }
 
@@ -244,11 +242,9 @@ struct Plan {
 template <int KIND>
 size_t sl_plan_bytes(const fire_problem* p, size_t W, bool fl) {
   const long n = p->n_el, nu = p->n_up, ms = std::max<long>(nu, n - nu), w = (long)W;
-  const int K8 = NENV_ORB * p->n_nuc;
   const long nv = fl ? 5 : 1;
   size_t b = sl_scratch_bytes<KIND>(w * n * nv, F);
   b = std::max(b, sl_scratch_bytes<KIND>(w * ms, F, 2));
-  b = std::max(b, sl_scratch_bytes<KIND>(w * ms * nv, K8, 2 * NDET));
   if (KIND == SL_F64) b = std::max(b, sl_scratch_bytes<KIND>(w * (fl ? 3 * n : 1), 2 * F));
   if (fl) b = std::max(b, sl_scratch_bytes<KIND>(3 * w * (n + p->cap_pairs), F));
   return b;
@@ -551,8 +547,8 @@ fire_status prepare_impl(cudaStream_t s, const fire_problem* p, const float* blo
     if (sizeof(T) == 4 && k >= SLW_READ1) continue;
     unsigned char* dst = reinterpret_cast<unsigned char*>(prepared) + so[k];
     g_nlaunch++;
-    if constexpr (sizeof(T) == 4) sl_prepare_pair(out + off[q.slot], q.K, q.N, q.batch, dst, s);
-    else sl_prepare_f64(out + off[q.slot], q.K, q.N, q.batch, dst, s);
+    if constexpr (sizeof(T) == 4) sl_prepare_pair(out + off[q.slot], q.K, q.N, dst, s);
+    else sl_prepare_f64(out + off[q.slot], q.K, q.N, dst, s);
   }
   return launch_status(__func__);
 }
@@ -660,22 +656,20 @@ SlCall<T> sl_call(const GemmP<T>& g, const unsigned char* w) {
   SlCall<T> q;
   std::memset(&q, 0, sizeof(q));
   q.nseg = 1;
-  q.batch = 1;
   q.p[0] = g;
   q.w[0] = w;
   return q;
 }
-// ... of both spins' rows (rows_per_el per electron, the walkers' electrons of a spin in a row), each with its own weight.
+// ... of both spins' rows (the walkers' electrons of a spin one after another), each with its own weight.
 template <typename T>
-SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, const unsigned char* w_up, const unsigned char* w_dn,
-                       int rows_per_el) {
+SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, const unsigned char* w_up, const unsigned char* w_dn) {
   SlCall<T> q = sl_call(g, w_up);
   const int nu = c.p->n_up, nd = c.p->n_el - nu;
   q.nseg = 2;
   q.p[1] = g;
   q.w[1] = w_dn;
-  q.p[0].M = c.Wc * nu * rows_per_el;
-  q.p[1].M = c.Wc * nd * rows_per_el;
+  q.p[0].M = c.Wc * nu;
+  q.p[1].M = c.Wc * nd;
   q.p[0].n_el = q.p[1].n_el = c.p->n_el;
   q.ns[0] = nu;
   q.ns[1] = nd;
@@ -922,58 +916,55 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   }
   // The rest of the envelope rows: in FP64 all of them (the refinement pass's by k_gemm_env_df), in FP32 the derivative rows
   // (with their value rows) and the Metropolis blocks' value rows by the plain contraction, then the value rows hi + lo (hi
-  // into the carrier, lo into env_lo).  The sliced contractions take both spins and all determinants in one launch.
+  // into the carrier, lo into env_lo).  Not by the sliced contraction: an electron's coefficients fall from 1 at its own
+  // nucleus to e^-100 at far ones, and an orbital with no weight near the electron is the sum of the small ones alone, which
+  // a grid laid for the row's largest value has cut off (12 protons 4 bohr apart, every orbital on its own: errors of log|psi|
+  // of 6e-3 in FP64 and 0.4 in FP32 where these sums leave 1e-9 and 5e-4).
   {
     const bool tc_ok = sizeof(T) == 4 && c.mixed && NENV_ORB * N <= ENV_TC_KMAX;
     const int nvc = tc_ok ? 1 : NV;  // coefficient rows per electron
     const long K8 = (long)N * NENV_ORB;
-    auto both = [&](int nvr) {  // nvr: rows taken per electron
+    auto rows = [&](int s, int nvr) {  // a spin's rows for the first determinant, nvr per electron
+      const int ns = s == 0 ? nu : n - nu;
       GemmP<T> g = gp0<T>();
-      g.lda = K8 * (nvc / nvr); g.C = env; g.ldc = (long)DN * (NV / nvr); g.N = n; g.K = (int)K8; g.n_el = n;
-      g.env_nv = nvr;
-      SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ENV_UP], c.slw[SLW_ENV_DN], nvr);
-      q.batch = NDET;
-      q.p[0].A = c.template buf<T>(c.P.coef_up);
-      q.p[1].A = c.template buf<T>(c.P.coef_dn);
-      q.a_bs[0] = (long)c.Wc * nu * nvc * K8;
-      q.a_bs[1] = (long)c.Wc * (n - nu) * nvc * K8;
-      q.c_bs = q.lo_bs = n;
-      q.ld_lo = DN;
-      return q;
+      g.A = c.template buf<T>(s == 0 ? c.P.coef_up : c.P.coef_dn);
+      g.lda = K8 * (nvc / nvr); g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI]; g.ldb = n; g.C = env;
+      g.ldc = (long)DN * (NV / nvr); g.M = c.Wc * ns * nvr; g.N = n; g.K = (int)K8; g.n_el = n;
+      g.env_ns = ns; g.env_soff = s == 0 ? 0 : nu; g.env_nv = nvr;
+      return g;
     };
-    // go(contraction of one spin's rows for one determinant, determinant) over all of them
-    auto each = [&](const SlCall<T>& q, auto go) -> cudaError_t {
+    auto a_bs = [&](int s) { return (long)c.Wc * (s == 0 ? nu : n - nu) * nvc * K8; };  // coefficients of a determinant
+    // go(contraction) over the spins and determinants
+    auto each = [&](int nvr, auto go) -> cudaError_t {
       for (int s = 0; s < 2; ++s)
-        for (int d = 0; d < NDET && q.p[s].M > 0; ++d) {
-          GemmP<T> g = q.p[s];
-          g.A += d * q.a_bs[s];
-          g.B = c.W.w[s == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (long)d * K8 * n; g.ldb = n;
-          g.C += d * q.c_bs;
-          g.env_ns = q.ns[s]; g.env_soff = q.soff[s];
-          const cudaError_t e = go(g, d);
+        for (int d = 0; d < NDET; ++d) {
+          GemmP<T> g = rows(s, nvr);
+          if (g.M == 0) continue;
+          g.A += d * a_bs(s);
+          g.B += d * K8 * n;
+          g.C += (long)d * n;
+          const cudaError_t e = go(g);
           if (e != cudaSuccess) return e;
         }
       return cudaSuccess;
     };
     cudaError_t e = cudaSuccess;
     if constexpr (sizeof(T) == 8) {
-      if (!c.refine64) {
-        e = sl_gemm(c, EPI_ENV, both(NV));
-      } else {
-        e = each(both(NV), [&](GemmP<T> g, int) {
-          live_rows(c, g);
-          Prof pg("gemm", c.s);
-          g_nlaunch++;
-          return launch_gemm_env_df(g, c.s);
-        });
-      }
+      e = each(NV, [&](GemmP<T> g) {
+        if (!c.refine64) return gemm<T, EPI_ENV>(c, g);
+        live_rows(c, g);
+        Prof pg("gemm", c.s);
+        g_nlaunch++;
+        return launch_gemm_env_df(g, c.s);
+      });
     } else {
-      if (nvc > 1 || (!c.comp && !tc_ok)) e = each(both(nvc), [&](const GemmP<T>& g, int) { return gemm<T, EPI_ENV>(c, g); });
+      if (nvc > 1 || (!c.comp && !tc_ok)) e = each(nvc, [&](const GemmP<T>& g) { return gemm<T, EPI_ENV>(c, g); });
       if (e == cudaSuccess && c.comp) {
-        SlCall<T> q = both(1);
-        q.C_lo = c.template buf<float>(c.P.env_lo);
-        if (c.pair) e = sl_gemm(c, COMP_ENV, q);
-        else e = each(q, [&](const GemmP<T>& g, int d) { return gemm_comp<COMP_ENV>(c, g, q.C_lo + (long)d * n, nullptr, DN); });
+        CompEnvP q{{rows(0, 1), rows(1, 1)}, {a_bs(0), a_bs(1)}, K8 * n, n};
+        for (int s = 0; s < 2; ++s) live_rows(c, q.p[s]);
+        Prof pg("gemm_comp", c.s);
+        g_nlaunch++;
+        e = launch_gemm_comp_env(q, c.template buf<float>(c.P.env_lo), DN, c.s);
       }
     }
     if (e != cudaSuccess) return e;
@@ -986,8 +977,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   if (c.refine64) {
     gemm<T, EPI_ORB_X>(c, g);
   } else if (sizeof(T) == 8 || c.pair) {
-    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN], 1);
-    q.map_a = 1;
+    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN]);
     if constexpr (sizeof(T) == 4) {
       q.C_lo = c.template buf<float>(c.P.Apl_lo);
       q.env_lo = c.template buf<float>(c.P.env_lo);
@@ -1046,8 +1036,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     }
   }
   if constexpr (sizeof(T) == 8) {
-    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN], 1);
-    q.map_a = 1;
+    SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN]);
     return sl_gemm(c, EPI_ORB_L, q);
   } else {
     gemm<T, EPI_ORB_L>(c, g, TC_ORB_UP);

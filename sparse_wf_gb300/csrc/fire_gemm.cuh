@@ -526,8 +526,9 @@ __device__ __forceinline__ void comp_grid_row(float m, float& inv, float& sc) {
   sc = __int_as_float((127 + ea) << 23);
 }
 
-// The CUDA-core form of the hi + lo value rows, for the local energy (Ctx::pair in fire_api.cu says why).  The exact part of every product is summed on a power-of-two grid instead of by a TwoSum per product (Ogita,
-// Rump and Oishi's Dot2), in the spirit of Rump's error-free extraction against a fixed power of two:
+// The CUDA-core form of the hi + lo value rows: all of a local energy's (Ctx::pair in fire_api.cu says why) and every
+// envelope value row (stage_orbitals).  The exact part of every product is summed on a power-of-two grid instead of by a
+// TwoSum per product (Ogita, Rump and Oishi's Dot2), in the spirit of Rump's error-free extraction against a fixed power of two:
 //   - each column of B is bounded over the whole K by |b| < 2^eb, and each row of a staged 16-k tile of A is
 //     scaled by a power of two so that |a'| < 1 (the row's scale 2^ea kept beside the tile);
 //   - t = fma(a', b, 3 * 2^eb) then lies in [2^(eb+1), 2^(eb+2)], where floats are evenly spaced by G = 2^(eb-22),
@@ -541,8 +542,8 @@ __device__ __forceinline__ void comp_grid_row(float m, float& inv, float& sc) {
 // memory (A transposed and scaled per row), the next tile prefetched into registers while the current one is
 // summed.  Before the first tile every pass bounds its 64 columns of B over the whole K.
 template <int MODE>
-__global__ void __launch_bounds__(CTHREADS, 2) k_gemm_comp(GemmP<float> p, float* __restrict__ C_lo,
-                                                           const float* __restrict__ env_lo, long ld_lo) {
+__device__ __forceinline__ void gemm_comp_tile(const GemmP<float>& p, float* __restrict__ C_lo,
+                                               const float* __restrict__ env_lo, long ld_lo) {
   __shared__ __align__(16) float As[2][CBK][CBM];
   __shared__ __align__(16) float Bs[2][CBK][CBN];
   __shared__ __align__(16) float Asc[2][CBM];     // 2^ea of every row of the staged A tile
@@ -772,6 +773,27 @@ __global__ void __launch_bounds__(CTHREADS, 2) k_gemm_comp(GemmP<float> p, float
   }
 }
 
+template <int MODE>
+__global__ void __launch_bounds__(CTHREADS, 2) k_gemm_comp(GemmP<float> p, float* __restrict__ C_lo,
+                                                           const float* __restrict__ env_lo, long ld_lo) {
+  gemm_comp_tile<MODE>(p, C_lo, env_lo, ld_lo);
+}
+// Envelope value rows (COMP_ENV) of both spins and every determinant: blockIdx.z = spin NDET + determinant, whose
+// coefficients, weights and columns of C and C_lo lie a_bs[spin], b_bs and c_bs elements further on.
+struct CompEnvP {
+  GemmP<float> p[2];
+  long a_bs[2], b_bs, c_bs;
+};
+template <int V = 0>  // a template so that every translation unit that includes this header may hold it
+__global__ void __launch_bounds__(CTHREADS, 2) k_gemm_comp_env(CompEnvP q, float* __restrict__ C_lo, long ld_lo) {
+  const int s = blockIdx.z / NDET, d = blockIdx.z % NDET;
+  GemmP<float> p = s == 0 ? q.p[0] : q.p[1];
+  p.A += d * (s == 0 ? q.a_bs[0] : q.a_bs[1]);
+  p.B += d * q.b_bs;
+  p.C += d * q.c_bs;
+  gemm_comp_tile<COMP_ENV>(p, C_lo + d * q.c_bs, nullptr, ld_lo);
+}
+
 // Envelope value rows of the refinement pass (EPI_ENV's row map, env_nv = 1) on the FP32 pipes: A holds FP64
 // coefficients, B weights whose values are exact in FP32 (the float32 parameter blob's), C is FP64.  Each a is split
 // into a_hi + a_lo floats; a_hi b by Dot2 (as in k_gemm_comp), a_lo b by FP32 FMAs into the low accumulator, and the
@@ -870,6 +892,14 @@ inline cudaError_t launch_gemm_comp(const GemmP<float>& p, float* C_lo, const fl
   dim3 grid((p.N + CBN - 1) / CBN, (p.M + CBM - 1) / CBM);
   if (grid.y == 0 || grid.x == 0) return cudaSuccess;
   k_gemm_comp<MODE><<<grid, CTHREADS, 0, s>>>(p, C_lo, env_lo, ld_lo);
+  return cudaPeekAtLastError();
+}
+
+inline cudaError_t launch_gemm_comp_env(const CompEnvP& q, float* C_lo, long ld_lo, cudaStream_t s) {
+  const int M = q.p[0].M > q.p[1].M ? q.p[0].M : q.p[1].M;
+  const dim3 grid((q.p[0].N + CBN - 1) / CBN, (M + CBM - 1) / CBM, 2 * NDET);
+  if (grid.y == 0 || grid.x == 0) return cudaSuccess;
+  k_gemm_comp_env<0><<<grid, CTHREADS, 0, s>>>(q, C_lo, ld_lo);
   return cudaPeekAtLastError();
 }
 

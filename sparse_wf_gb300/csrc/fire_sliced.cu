@@ -123,11 +123,8 @@ struct SliceArgs {
   int row0, row1;  // this pass's rows of every segment
   int K, nkb, n_el;
   int ns[2], soff[2];  // ns > 0: row q is row (q / ns) n_el + soff + q % ns of A
-  long a_bs[2];
   unsigned char* out[2];
-  size_t out_bs[2];
   int* code[2];
-  long code_bs[2];
 };
 
 // 32 rows per CTA (lane = row), warps over the 8-deep k-groups: every load takes a 32- or 64-byte piece of 32 rows, every
@@ -139,7 +136,7 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
   constexpr int NS = SlFmt<KIND>::NS;
   using U = typename Mag<T>::U;
   __shared__ U part[SLR_WARPS][32];
-  const int g = blockIdx.z, b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int rows = a.M[g];
   if (a.M_dev) rows = min(rows, a.M_scale[g] * *a.M_dev);
   rows = min(rows, a.row1) - a.row0;  // of this pass
@@ -147,8 +144,8 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
   if ((int)blockIdx.x * 32 >= (rows + 127) / 128 * 128) return;
   const bool ok = ql < rows;
   const long src = a.ns[g] > 0 ? (long)(q / a.ns[g]) * a.n_el + a.soff[g] + q % a.ns[g] : (long)q;
-  const T* p = a.A[g] + b * a.a_bs[g] + (ok ? src : 0) * a.lda[g];
-  const bool vec = (a.lda[g] * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.A[g] + b * a.a_bs[g]) & 15) == 0;
+  const T* p = a.A[g] + (ok ? src : 0) * a.lda[g];
+  const bool vec = (a.lda[g] * sizeof(T)) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.A[g]) & 15) == 0;
   const int nkg = 2 * a.nkb;
   const bool keep = nkg <= SLR_KEEP * SLR_WARPS;
   T v[SLR_KEEP][8];
@@ -176,9 +173,9 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
 #pragma unroll
   for (int w = 0; w < SLR_WARPS; ++w) mx = max(mx, part[w][lane]);
   const int code = sl_code(mx);
-  if (warp == 0) a.code[g][b * a.code_bs[g] + ql] = code;
+  if (warp == 0) a.code[g][ql] = code;
   // [128-row tile][16-deep step][slice][k-group][128 rows][16 bytes]
-  unsigned char* out = a.out[g] + b * a.out_bs[g] + (size_t)(ql >> 7) * a.nkb * NS * 4096 + (ql & 127) * 16;
+  unsigned char* out = a.out[g] + (size_t)(ql >> 7) * a.nkb * NS * 4096 + (ql & 127) * 16;
   auto put = [&](const T (&x)[8], int kg) {
     store_slices<KIND>(x, code, out + (size_t)(kg >> 1) * NS * 4096 + (kg & 1) * 2048, 4096);
   };
@@ -201,15 +198,13 @@ __global__ void __launch_bounds__(32 * SLR_WARPS) k_slice_rows(SliceArgs<T> a) {
 // then N column exponents.  32 columns per CTA (lane = column), warps over k.
 template <int KIND, typename T>
 __global__ void __launch_bounds__(256) k_slice_w(const T* __restrict__ W, int K, int N, SlTile tl,
-                                                 unsigned char* __restrict__ out, size_t code_off, size_t bytes) {
+                                                 unsigned char* __restrict__ out, size_t code_off) {
   constexpr int NS = SlFmt<KIND>::NS;
   using U = typename Mag<T>::U;
   __shared__ U part[8][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
   const bool ok = c < N;
-  W += (size_t)blockIdx.y * K * N;
-  out += (size_t)blockIdx.y * bytes;
   U mx = 0;
 #pragma unroll 8
   for (int k = warp; k < K; k += 8) mx = max(mx, ok ? (U)mag_bits(W[(size_t)k * N + c]) : (U)0);
@@ -248,20 +243,17 @@ constexpr int SL_THREADS = 320;  // warps 0-7 epilogue, 8 loader, 9 MMA issuer
 
 template <typename T>
 struct SlArgs {
-  int nseg, batch;
+  int nseg;
   GemmP<T> p[2];
   const unsigned char* At[2];
   const int* ac[2];
-  size_t At_bs[2];
-  long ac_bs[2];
   const unsigned char* Bt[2];
-  size_t Bt_bs, b_code;
+  size_t b_code;
   SlTile tl;
   int pw;  // 16-column pieces of a column tile per unit of work
   int row0, row1;  // this pass's rows of every segment
   int ns[2], soff[2], spin[2];
   const int* tile_mask;
-  long c_bs, lo_bs;
   float* C_lo;
   const float* env_lo;
   long ld_lo;
@@ -333,16 +325,14 @@ __device__ __forceinline__ float sl_scale(int code) {
 
 // Element-wise epilogues of the hi + lo results (CompMode); row: row of C, q: row of the segment.
 template <int MODE>
-__device__ __forceinline__ void sl_store_pair(const SlArgs<float>& a, const GemmP<float>& p, int spin, int b, int q, long row,
+__device__ __forceinline__ void sl_store_pair(const SlArgs<float>& a, const GemmP<float>& p, int spin, int q, long row,
                                               int col, float h, float l) {
-  if (MODE != COMP_ENV) {
-    const float* bias = spin == 1 ? p.bias2 : p.bias;
-    if (bias && (MODE != COMP_PLAIN || (p.bias_period > 0 && q % p.bias_period == 0))) {
-      float s, e;
-      two_sum(h, bias[col], s, e);
-      h = s;
-      l += e;
-    }
+  const float* bias = spin == 1 ? p.bias2 : p.bias;
+  if (bias && (MODE != COMP_PLAIN || (p.bias_period > 0 && q % p.bias_period == 0))) {
+    float s, e;
+    two_sum(h, bias[col], s, e);
+    h = s;
+    l += e;
   }
   float s, e;  // normalised pair: s = fl(h + l)
   two_sum(h, l, s, e);
@@ -358,9 +348,6 @@ __device__ __forceinline__ void sl_store_pair(const SlArgs<float>& a, const Gemm
     } else {
       p.C[row * p.ldc + col] = silu(s);
     }
-  } else if (MODE == COMP_ENV) {
-    p.C[b * a.c_bs + row * p.ldc + col] = s;
-    a.C_lo[b * a.lo_bs + row * a.ld_lo + col] = e;
   } else {  // COMP_ORB: raw orbital times envelope, hi + lo
     p.aux0[row * p.ld_aux + col] = s;
     const float eh = p.aux1[row * p.env_nv * p.ld_aux + col], el = a.env_lo[row * a.ld_lo + col];
@@ -466,19 +453,17 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     }
   // a column tile may be split into ncp parts of pw pieces of 16 columns, each its own unit of work (few rows)
   const int np = nc / 16, pw = a.pw, ncp = (np + pw - 1) / pw, nu = nt * ncp;
-  const int t0 = a.batch * mt[0] * nu, total = t0 + a.batch * mt[1] * nu;
+  const int t0 = mt[0] * nu, total = t0 + mt[1] * nu;
   if ((int)blockIdx.x >= total) return;
-  // unit t: segment, batch block, row tile, column tile and the first piece in it (column tiles of a row tile run next to
-  // each other: its slices come from L2)
-  auto decode = [&](int t, int& g, int& b, int& m, int& n, int& p0) -> bool {
+  // unit t: segment, row tile, column tile and the first piece in it (column tiles of a row tile run next to each other: its
+  // slices come from L2)
+  auto decode = [&](int t, int& g, int& m, int& n, int& p0) -> bool {
     g = t >= t0 ? 1 : 0;
     if (g) t -= t0;
     n = t % nu;
-    const int r = t / nu;
+    m = t / nu;
     p0 = n % ncp * pw;
     n /= ncp;
-    m = r % mt[g];
-    b = r / mt[g];
     return !a.tile_mask || ((a.tile_mask[a.row0 / 128 + m] >> a.spin[g]) & 1);
   };
 
@@ -509,10 +494,10 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     // ------------------------------------------------------------------ loader
     if (lane == 0) {
       for (int t = blockIdx.x; t < total && !*abort; t += gridDim.x) {
-        int g, b, m, n, p0;
-        if (!decode(t, g, b, m, n, p0)) continue;
-        const unsigned char* as = a.At[g] + (size_t)b * a.At_bs[g] + (size_t)m * nkb * Sm::A_STEP;
-        const unsigned char* bs = a.Bt[g] + (size_t)b * a.Bt_bs + (size_t)n * nkb * Sm::B_STEP;
+        int g, m, n, p0;
+        if (!decode(t, g, m, n, p0)) continue;
+        const unsigned char* as = a.At[g] + (size_t)m * nkb * Sm::A_STEP;
+        const unsigned char* bs = a.Bt[g] + (size_t)n * nkb * Sm::B_STEP;
         for (int kb = 0; kb < nkb; ++kb) {
           const int q = (int)(issued % STAGES);
           const long use = issued / STAGES;
@@ -529,8 +514,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     long kc = 0, uc = 0;
     bool live = true;
     for (int t = blockIdx.x; t < total && live; t += gridDim.x) {
-      int g, b, m, n, p0;
-      if (!decode(t, g, b, m, n, p0)) continue;
+      int g, m, n, p0;
+      if (!decode(t, g, m, n, p0)) continue;
       const uint32_t idesc = (1u << 4) | ((uint32_t)(2 * min(pw, np - p0)) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
       for (int kb = 0; kb < nkb; ++kb, ++kc) {
         const bool start = kb % SL_KCH == 0;
@@ -565,13 +550,13 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
     long uc = 0;
     bool live = true;  // warp-uniform
     for (int t = blockIdx.x; t < total && live; t += gridDim.x) {
-      int g, b, m, n, p0;
-      if (!decode(t, g, b, m, n, p0)) continue;
+      int g, m, n, p0;
+      if (!decode(t, g, m, n, p0)) continue;
       const GemmP<T>& p = a.p[g];
       const int M = a.row0 + rows[g], N = p.N, l0 = m * 128 + quad * 32, m0 = a.row0 + l0, n0 = n * nc + p0 * 16;
       const int nl = min(pw, np - p0);  // pieces of this unit
-      const int* bc = reinterpret_cast<const int*>(a.Bt[g] + (size_t)b * a.Bt_bs + a.b_code);
-      const int rc = a.ac[g][b * a.ac_bs[g] + l0 + lane];
+      const int* bc = reinterpret_cast<const int*>(a.Bt[g] + a.b_code);
+      const int rc = a.ac[g][l0 + lane];
       SlAcc<KIND> acc;
       for (int k0 = 0; k0 < nkb; k0 += SL_KCH) {
         live = __all_sync(0xffffffffu, tc_wait(&bars->tfull, (uint32_t)(uc & 1), abort));
@@ -591,14 +576,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
       // lane's row of the segment: its row in C (-1: none), for FP32 its scale.
       const int cl = lane & 15, hl = lane >> 4, q0 = m0 + lane;
       int crow = q0 < M ? q0 : -1;
-      if (KIND == SL_F64 && MODE == EPI_ENV) {
-        if (q0 < M) {
-          const int rr = q0 / p.env_nv, e = (rr / a.ns[g]) * p.n_el + a.soff[g] + rr % a.ns[g];
-          crow = e * p.env_nv + (q0 - p.env_nv * rr);
-        }
-      } else if (a.ns[g] > 0 && q0 < M) {
-        crow = (q0 / a.ns[g]) * p.n_el + a.soff[g] + q0 % a.ns[g];
-      }
+      if (a.ns[g] > 0 && q0 < M) crow = (q0 / a.ns[g]) * p.n_el + a.soff[g] + q0 % a.ns[g];
       if (KIND == SL_F64 && MODE == EPI_ORB_J && crow >= 0 &&
           (((gemm_node(p, crow) % p.n_el) < p.n_up) ? 0 : 1) != a.spin[g])
         crow = -1;
@@ -625,7 +603,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
             const int r = 2 * i + hl, row = __shfl_sync(0xffffffffu, crow, r);
             const float sc = __shfl_sync(0xffffffffu, rs, r);
             if (row >= 0 && col < N)
-              sl_store_pair<MODE>(a, p, a.spin[g], b, m0 + r, (long)row, col, sh[r * 17 + cl] * sc * cs,
+              sl_store_pair<MODE>(a, p, a.spin[g], m0 + r, (long)row, col, sh[r * 17 + cl] * sc * cs,
                                   sl[r * 17 + cl] * sc * cs);
           }
         } else {
@@ -656,10 +634,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_gemm_sl(const __grid_constant
               }
               s2 += x * x;
             }
-            if (row >= 0 && col < N) {
-              if constexpr (MODE == EPI_ENV) p.C[b * a.c_bs + (long)row * p.ldc + col] = x;
-              else gemm_store<double, MODE>(p, row, col, x, a.spin[g]);
-            }
+            if (row >= 0 && col < N) gemm_store<double, MODE>(p, row, col, x, a.spin[g]);
           }
           if constexpr (MODE == EPI_SILU_J) {
             if (cur >= 0 && col < N) atomic_add(&p.aux2[(long)cur * p.ld_aux + col], s2);
@@ -725,19 +700,15 @@ template <int KIND, int MODE>
 int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, int32_t* status, cudaStream_t s) {
   using T = typename SlFmt<KIND>::T;
   const GemmP<T>& p0 = c.p[0];
-  if (c.nseg < 1 || c.nseg > 2 || c.batch < 1 || p0.K < 1 || p0.N < 1) return -1;
+  if (c.nseg < 1 || c.nseg > 2 || p0.K < 1 || p0.N < 1) return -1;
   SlArgs<T> a;
   SliceArgs<T> r;
   std::memset(&a, 0, sizeof(a));
   std::memset(&r, 0, sizeof(r));
   a.nseg = c.nseg;
-  a.batch = c.batch;
   a.tl = sl_tile(p0.K, p0.N, SlFmt<KIND>::NMAX);
-  a.Bt_bs = sl_w_bytes<KIND>(p0.K, p0.N);
   a.b_code = sl_w_code_offset<KIND>(p0.K, p0.N);
   a.tile_mask = c.tile_mask;
-  a.c_bs = c.c_bs;
-  a.lo_bs = c.lo_bs;
   a.C_lo = c.C_lo;
   a.env_lo = c.env_lo;
   a.ld_lo = c.ld_lo;
@@ -745,11 +716,11 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
   r.K = p0.K;
   r.nkb = a.tl.nkb;
   r.n_el = p0.n_el;
-  const int sliced = c.share_a ? 1 : c.nseg, blocks = sliced * c.batch;
+  const int sliced = c.share_a ? 1 : c.nseg;
   long mmax = 0;
   for (int g = 0; g < c.nseg; ++g) mmax = std::max<long>(mmax, c.p[g].M);
   if (mmax == 0) return 0;
-  const long pass = sl_pass_rows(mmax, blocks);
+  const long pass = sl_pass_rows(mmax, sliced);
   const size_t a_bytes = sl_a_bytes<KIND>(pass, p0.K), block = (a_bytes + (size_t)pass * 4 + 255) / 256 * 256;
   for (int g = 0; g < c.nseg; ++g) {
     const GemmP<T>& p = c.p[g];
@@ -760,21 +731,16 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
     a.ns[g] = c.ns[g];
     a.soff[g] = c.soff[g];
     a.spin[g] = c.spin[g];
-    a.At[g] = scratch + (size_t)q * c.batch * block;
-    a.At_bs[g] = block;
+    a.At[g] = scratch + (size_t)q * block;
     a.ac[g] = reinterpret_cast<const int*>(a.At[g] + a_bytes);
-    a.ac_bs[g] = (long)(block / 4);
     r.A[g] = p.A;
     r.lda[g] = p.lda;
-    r.a_bs[g] = c.a_bs[g];
     r.M[g] = p.M;
     r.M_scale[g] = p.M_scale;
-    r.ns[g] = c.map_a ? c.ns[g] : 0;
+    r.ns[g] = c.ns[g];
     r.soff[g] = c.soff[g];
     r.out[g] = const_cast<unsigned char*>(a.At[g]);
-    r.out_bs[g] = block;
     r.code[g] = const_cast<int*>(a.ac[g]);
-    r.code_bs[g] = a.ac_bs[g];
   }
   constexpr int smem = SlSmem<KIND>::TOTAL;
   if (cudaFuncSetAttribute(k_gemm_sl<KIND, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
@@ -786,10 +752,10 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
     long tiles = 0, rows = 0;
     for (int g = 0; g < c.nseg; ++g) {
       const long m = std::max<long>(0, std::min<long>(c.p[g].M, a.row1) - r0);
-      tiles += (long)c.batch * ((m + 127) / 128) * a.tl.nt;
+      tiles += ((m + 127) / 128) * a.tl.nt;
       rows = std::max(rows, m);
     }
-    const dim3 gr((unsigned)(sl_rows(rows) / 32), (unsigned)c.batch, (unsigned)sliced);
+    const dim3 gr((unsigned)(sl_rows(rows) / 32), (unsigned)sliced);
     k_slice_rows<KIND, T><<<gr, 32 * SLR_WARPS, 0, s>>>(r);
     // Few tiles: parts of two pieces or of one, as long as each gets an SM of its own (an MMA of 16 columns takes 36 cycles
     // where 64 take 48, and a unit's epilogue goes with its columns): 160 rows x 256 x 256 26 -> 20 us.
@@ -803,10 +769,9 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
 }
 
 template <int KIND>
-cudaError_t sl_prepare(const typename SlFmt<KIND>::T* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
+cudaError_t sl_prepare(const typename SlFmt<KIND>::T* W, int K, int N, unsigned char* out, cudaStream_t s) {
   const SlTile t = sl_tile(K, N, SlFmt<KIND>::NMAX);
-  const dim3 grid((unsigned)((t.nt * t.nc + 31) / 32), (unsigned)batch);
-  k_slice_w<KIND><<<grid, 256, 0, s>>>(W, K, N, t, out, sl_w_code_offset<KIND>(K, N), sl_w_bytes<KIND>(K, N));
+  k_slice_w<KIND><<<(unsigned)((t.nt * t.nc + 31) / 32), 256, 0, s>>>(W, K, N, t, out, sl_w_code_offset<KIND>(K, N));
   return cudaPeekAtLastError();
 }
 
@@ -825,11 +790,11 @@ __global__ void k_sl_tile_mask(GemmP<double> p, int* mask) {
 
 }  // namespace
 
-cudaError_t sl_prepare_pair(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
-  return sl_prepare<SL_PAIR>(W, K, N, batch, out, s);
+cudaError_t sl_prepare_pair(const float* W, int K, int N, unsigned char* out, cudaStream_t s) {
+  return sl_prepare<SL_PAIR>(W, K, N, out, s);
 }
-cudaError_t sl_prepare_f64(const double* W, int K, int N, int batch, unsigned char* out, cudaStream_t s) {
-  return sl_prepare<SL_F64>(W, K, N, batch, out, s);
+cudaError_t sl_prepare_f64(const double* W, int K, int N, unsigned char* out, cudaStream_t s) {
+  return sl_prepare<SL_F64>(W, K, N, out, s);
 }
 
 void sl_tile_mask(const GemmP<double>& p, int* mask, cudaStream_t s) {
@@ -840,7 +805,6 @@ int sl_gemm_pair(int mode, const SlCall<float>& c, unsigned char* scratch, int32
   switch (mode) {
     case COMP_PLAIN: return sl_launch<SL_PAIR, COMP_PLAIN>(c, scratch, status, s);
     case COMP_SILU: return sl_launch<SL_PAIR, COMP_SILU>(c, scratch, status, s);
-    case COMP_ENV: return sl_launch<SL_PAIR, COMP_ENV>(c, scratch, status, s);
     case COMP_ORB: return sl_launch<SL_PAIR, COMP_ORB>(c, scratch, status, s);
     default: return -1;
   }
@@ -855,7 +819,6 @@ int sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32
     case EPI_ORB_X: return sl_launch<SL_F64, EPI_ORB_X>(c, scratch, status, s);
     case EPI_ORB_J: return sl_launch<SL_F64, EPI_ORB_J>(c, scratch, status, s);
     case EPI_ORB_L: return sl_launch<SL_F64, EPI_ORB_L>(c, scratch, status, s);
-    case EPI_ENV: return sl_launch<SL_F64, EPI_ENV>(c, scratch, status, s);
     default: return -1;
   }
 }

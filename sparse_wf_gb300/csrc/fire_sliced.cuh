@@ -7,13 +7,15 @@
 // exact in FP16, so a product of two of them is an integer and the tensor core's FP32 accumulator sums up to 256 of them
 // exactly, whatever order and rounding it uses.  Products are grouped by their level l = i + j (their common scale is
 // 2^(-bits l)); levels l < NS are computed, each in a tensor-memory accumulator of its own, and the epilogue puts them
-// together.  Two formats:
+// together.  Two formats (an operand's bits count from its row's or column's largest value, so the error is relative to the
+// product of the two largest magnitudes, not to the terms: rows whose large values meet zero weights are not for this, see
+// stage_orbitals for the envelopes):
 //   SL_PAIR  FP32 operands, 6 slices (8 + 5 x 9 bits), 21 MMAs per product; the result is a hi + lo float pair.  The slices
 //            hold 53 bits below the row's largest value.  Five slices of 9 bits (15 MMAs) left errors up to 10 times those
 //            of the compensated dot product on the CUDA cores (k_gemm_comp).
 //   SL_F64   FP64 operands, 8 slices of 8 bits, 36 MMAs per product; the levels are put together in integer arithmetic and
-//            rounded once.  64 bits below the largest value: 11 more than an FP64 number has, for rows whose values spread
-//            over many powers of two (envelope coefficients; 7 slices left errors up to twice FP64's own there).
+//            rounded once.  63 bits below the largest value, 10 more than an FP64 number has (7 slices left errors up to
+//            twice FP64's own).  FP64 denormals count as zero.
 // Sums of the first levels stay below 2^24, the range of exact integers: SL_PAIR's first slice is at most 2^7 in magnitude
 // (2 x 256 x 2^7 x 2^8 for level 1), SL_F64's all are ((l + 1) 256 x 2^14 for level l <= 3).  From level 2 (3) on an
 // accumulator could lose its lowest bit if every product had the same sign and nearly the largest size, at 2^-17 (2^-32)
@@ -82,45 +84,41 @@ template <int KIND>
 inline size_t sl_a_bytes(long M, int K) {  // slices of M rows (whole 128-row tiles)
   return (size_t)sl_rows(M) * ((K + 15) / 16) * 32 * SlFmt<KIND>::NS;
 }
-// Row tiles of one pass over all segments and batch blocks: one per SM, as many whole tiles as that leaves to each of the
-// `blocks` segments and batch blocks.
+// Row tiles of one pass over all segments: one per SM, as many whole tiles as that leaves to each of the `segs` segments.
 constexpr int SL_SMS = 152;
-inline long sl_pass_rows(long M, int blocks) {
-  return std::min<long>(sl_rows(M), 128 * std::max<long>(1, SL_SMS / blocks));
+inline long sl_pass_rows(long M, int segs) {
+  return std::min<long>(sl_rows(M), 128 * std::max<long>(1, SL_SMS / segs));
 }
-// scratch of a contraction's A: the slices of a pass, then one exponent per row, for every segment and batch block (M: the
-// larger segment's rows)
+// scratch of a contraction's A: the slices of a pass, then one exponent per row, for every segment (M: the larger segment's
+// rows)
 template <int KIND>
-inline size_t sl_scratch_bytes(long M, int K, int blocks = 1) {
-  const long r = sl_pass_rows(M, blocks);
-  return (size_t)blocks * ((sl_a_bytes<KIND>(r, K) + (size_t)r * 4 + 255) / 256 * 256);
+inline size_t sl_scratch_bytes(long M, int K, int segs = 1) {
+  const long r = sl_pass_rows(M, segs);
+  return (size_t)segs * ((sl_a_bytes<KIND>(r, K) + (size_t)r * 4 + 255) / 256 * 256);
 }
 
 // One contraction, or two that differ in their rows and weights (the spins).  Segment g multiplies its own rows
-// (p[g].A, M, lda ...) by its own weight; `batch` blocks per segment (the determinants of the envelopes) advance A, W, C
-// and C_lo by the strides below.  ns[g] > 0: row q of the segment is row (q / ns) n_el + soff + q % ns of C and of the
-// per-row operands (and of A, if map_a); 0: row q.
+// (p[g].A, M, lda ...) by its own weight.  ns[g] > 0: row q of the segment is row (q / ns) n_el + soff + q % ns of A, of C and
+// of the per-row operands; 0: row q.
 template <typename T>
 struct SlCall {
-  int nseg, batch;
+  int nseg;
   GemmP<T> p[2];
-  const unsigned char* w[2];  // sliced weights (sl_w_bytes each; batch block b follows b of them)
+  const unsigned char* w[2];  // sliced weights
   int ns[2], soff[2];
-  int map_a;
   int spin[2];                // bias2 instead of bias for 1; ORB_J: the rows' spin that the segment stores
   int share_a;                // both segments read the same rows: sliced once
   const int* tile_mask;       // ORB_J: spins present in every 128-row tile
-  long a_bs[2], c_bs, lo_bs;  // elements from one batch block to the next
   float* C_lo;
   const float* env_lo;
   long ld_lo;
 };
-cudaError_t sl_prepare_pair(const float* W, int K, int N, int batch, unsigned char* out, cudaStream_t s);
-cudaError_t sl_prepare_f64(const double* W, int K, int N, int batch, unsigned char* out, cudaStream_t s);
+cudaError_t sl_prepare_pair(const float* W, int K, int N, unsigned char* out, cudaStream_t s);
+cudaError_t sl_prepare_f64(const double* W, int K, int N, unsigned char* out, cudaStream_t s);
 // spins present in every 128-row tile (bit 0 up, bit 1 down) of a contraction's rows
 void sl_tile_mask(const GemmP<double>& p, int* mask, cudaStream_t s);
 // mode: CompMode for hi + lo pairs, EpiMode for FP64.  scratch: sl_scratch_bytes over the call's segments (one if
-// they share A) and batch blocks, 256-byte aligned.  Returns the number of kernels launched, or -1 on an error.
+// they share A), 256-byte aligned.  Returns the number of kernels launched, or -1 on an error.
 int sl_gemm_pair(int mode, const SlCall<float>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
 int sl_gemm_f64(int mode, const SlCall<double>& c, unsigned char* scratch, int32_t* status, cudaStream_t s);
 
