@@ -162,7 +162,8 @@ void tc_offsets(const fire_problem* p, size_t float_bytes, size_t* off) {
 }
 
 // Weights of the sliced contractions (fire_sliced.cuh), cut when the parameters are prepared: for the value path of the FP32
-// and mixed builds (SL_PAIR, without the attention readout's), for every layer in FP64 (SL_F64).
+// and mixed builds (SL_PAIR, without the attention readout's), for every layer in the FP64 build (SL_F64).  The FP64 copy in
+// an FP32 or mixed buffer has none: the refinement pass, its only reader, sums in plain FP64.
 enum SlSlot {
   SLW_GLU, SLW_DENSE, SLW_OUT, SLW_UPD1, SLW_UPD2, SLW_ORB_UP, SLW_ORB_DN, SLW_V, SLW_JMLP1, SLW_JMLP2, SLW_READ1,
   SLW_READ2, SLW_COUNT
@@ -250,7 +251,9 @@ size_t sl_plan_bytes(const fire_problem* p, size_t W, bool fl) {
   return b;
 }
 
-Plan make_plan(const fire_problem* p, int Wc, bool fl) {
+// sliced: with room for the slices of the contractions (a value path, or the FP64 build's local energy; not the FP32 local
+// energy nor the refinement's FP64 value path)
+Plan make_plan(const fire_problem* p, int Wc, bool fl, bool sliced = true) {
   Plan P;
   std::memset(&P, 0, sizeof(P));
   const size_t es = elem_size(p);
@@ -341,9 +344,11 @@ Plan make_plan(const fire_problem* p, int Wc, bool fl) {
     take(P.JMl, W * 2, es);
     take(P.JMj, W * 3 * n * 2, es);
   }
-  // two working copies per matrix for the Gauss-Jordan / LU kernel; the sliced contractions before and after it (all of
-  // FP64, the value path in FP32) cut their rows into the same bytes
-  const size_t slb = es == 8 ? sl_plan_bytes<SL_F64>(p, W, fl) : sl_plan_bytes<SL_PAIR>(p, W, false);
+  // two working copies per matrix for the Gauss-Jordan / LU kernel; the sliced contractions before and after it cut their
+  // rows into the same bytes
+  size_t slb = 0;
+  if (sliced && es == 8) slb = sl_plan_bytes<SL_F64>(p, W, fl);
+  else if (sliced && !fl) slb = sl_plan_bytes<SL_PAIR>(p, W, false);
   take(P.gjw, std::max(2 * W * NDET * n * n * 8, slb), 1);
   P.sl = P.gjw;
   take(P.enn, 1, 8);
@@ -386,7 +391,7 @@ RefineLayout refine_layout(const fire_problem* p, int KC) {
   const size_t n3 = (size_t)KC * p->n_el * 3;
   auto up = [](size_t x) { return (x + 255) / 256 * 256; };
   L.c64 = up(make_plan(&pr, KC, true).total);
-  L.r_ref = up(L.c64 + make_plan(&p64, KC, false).total);
+  L.r_ref = up(L.c64 + make_plan(&p64, KC, false, false).total);
   L.r64 = up(L.r_ref + n3 * elem_size(p));
   L.total = up(L.r64 + n3 * 8);
   return L;
@@ -495,7 +500,7 @@ inline unsigned nblk(long n, int t = 256) { return (unsigned)((n + t - 1) / t); 
 
 template <typename T>
 fire_status prepare_impl(cudaStream_t s, const fire_problem* p, const float* blob, const int64_t* boff,
-                         void* prepared) {
+                         void* prepared, bool sliced = true) {
   int64_t off[PR_COUNT + 1];
   prep_offsets(p, off);
   T* out = reinterpret_cast<T*>(prepared);
@@ -542,7 +547,7 @@ fire_status prepare_impl(cudaStream_t s, const fire_problem* p, const float* blo
                                 out + off[PR_SCALARS]);
   size_t so[SLW_COUNT + 1];
   sl_offsets<T>(p, so);
-  for (int k = 0; k < SLW_COUNT; ++k) {
+  for (int k = 0; sliced && k < SLW_COUNT; ++k) {
     const SlSrc q = sl_src(k, p);
     if (sizeof(T) == 4 && k >= SLW_READ1) continue;
     unsigned char* dst = reinterpret_cast<unsigned char*>(prepared) + so[k];
@@ -596,7 +601,7 @@ struct Ctx {
   // more exact) into up to 7 10^-5 of a batch's largest energies.
   bool refine64 = false;
   TcWeights tcw[TC_COUNT];
-  const unsigned char* slw[SLW_COUNT];  // sliced weights
+  const unsigned char* slw[SLW_COUNT];  // sliced weights (null in a context that does not read them)
   template <typename U>
   U* buf(size_t off) const {
     return reinterpret_cast<U*>(ws + off);
@@ -1360,16 +1365,10 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
   return cudaPeekAtLastError();
 }
 
-template <typename T>
-void set_sliced(Ctx<T>& c, const fire_problem* p, const void* prepared) {
-  size_t so[SLW_COUNT + 1];
-  sl_offsets<T>(p, so);
-  for (int k = 0; k < SLW_COUNT; ++k) c.slw[k] = reinterpret_cast<const unsigned char*>(prepared) + so[k];
-}
-
+// pair: a value path of FP32 or mixed whose value planes are sliced; refine64: the refinement pass's FP64 value path
 template <typename T>
 Ctx<T> make_ctx(const fire_problem* p, cudaStream_t s, const float* R, const float* Z, const void* prepared,
-                int32_t* status, void* ws, int Wmax, bool fl) {
+                int32_t* status, void* ws, int Wmax, bool fl, bool pair = false, bool refine64 = false) {
   Ctx<T> c;
   c.p = p;
   c.s = s;
@@ -1380,9 +1379,14 @@ Ctx<T> make_ctx(const fire_problem* p, cudaStream_t s, const float* R, const flo
   c.W = make_weights<T>(p, prepared);
   c.status = status;
   c.ws = reinterpret_cast<unsigned char*>(ws);
-  c.P = make_plan(p, Wmax, fl);
+  c.P = make_plan(p, Wmax, fl, !refine64);
   c.mixed = p->precision == FIRE_PREC_MIXED;
-  set_sliced(c, p, prepared);
+  c.pair = pair && sizeof(T) == 4;
+  c.refine64 = refine64;
+  size_t so[SLW_COUNT + 1];
+  sl_offsets<T>(p, so);
+  for (int k = 0; k < SLW_COUNT; ++k)
+    c.slw[k] = c.pair || (sizeof(T) == 8 && !refine64) ? reinterpret_cast<const unsigned char*>(prepared) + so[k] : nullptr;
   if (c.mixed) {
     int64_t off[PR_COUNT + 1];
     prep_offsets(p, off);
@@ -1465,10 +1469,9 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     side.fork();
     Ctx<double> c64 = make_ctx<double>(&p64, side.s, R, Z,
                                        reinterpret_cast<const unsigned char*>(prepared) + prep64_offset(p), status,
-                                       ws + L.c64, KC, false);
+                                       ws + L.c64, KC, false, false, true);
     c64.w0 = 0;
     c64.Wc = KC;
-    c64.refine64 = true;
     c64.r = r64;
     c64.nb.live = sub_cnt + j;
     setup_ctx(c64, false);
@@ -1537,8 +1540,7 @@ fire_status run_logpsi(const fire_problem* p, cudaStream_t s, const float* R, co
                        const void* r, void* sign, void* logpsi, void* ws, size_t wsb, int32_t* status) {
   const int Wc = choose_chunk(p, wsb, false);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
-  Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false);
-  c.pair = true;
+  Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false, true);
   const T* rr = reinterpret_cast<const T*>(r);
   for (int w0 = 0; w0 < p->n_walkers; w0 += Wc) {
     c.w0 = w0;
@@ -1554,8 +1556,7 @@ fire_status run_embedding(const fire_problem* p, cudaStream_t s, const float* R,
                           const void* r, void* hc, void* hu, void* ws, size_t wsb, int32_t* status) {
   const int Wc = choose_chunk(p, wsb, false);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
-  Ctx<T> c = make_ctx<T>(p, s, R, nullptr, prepared, status, ws, Wc, false);
-  c.pair = true;
+  Ctx<T> c = make_ctx<T>(p, s, R, nullptr, prepared, status, ws, Wc, false, true);
   const T* rr = reinterpret_cast<const T*>(r);
   for (int w0 = 0; w0 < p->n_walkers; w0 += Wc) {
     c.w0 = w0;
@@ -2002,8 +2003,7 @@ fire_status run_ecp(const fire_problem* p, cudaStream_t s, const float* R, const
                     void* out, int32_t* static_max, void* ws, size_t wsb, int32_t* status) {
   const int Wc = choose_chunk_lr(p, wsb, KS);
   if (Wc <= 0) return FIRE_ERR_WORKSPACE;
-  Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false);
-  c.pair = true;
+  Ctx<T> c = make_ctx<T>(p, s, R, Z, prepared, status, ws, Wc, false, true);
   const LrPlan Q = make_lr_plan(p, Wc, KS);
   const EcpQuad qt = ecp_quadratures();
   T* rr = const_cast<T*>(reinterpret_cast<const T*>(r));  // read only: nothing is committed
@@ -2108,17 +2108,23 @@ fire_status fire_param_layout(const fire_problem* prob, int64_t* offsets) {
 
 fire_status fire_prepared_size(const fire_problem* prob, size_t* bytes) {
   if (!valid(prob) || !bytes) return FIRE_ERR_INVALID;
-  const fire_problem p64 = refine_problem64(prob, 1);
-  size_t so[SLW_COUNT + 1];
-  sl_offsets<double>(&p64, so);
-  *bytes = so[SLW_COUNT] + (prob->precision != FIRE_PREC_FP64 ? prep64_offset(prob) : 0);
+  if (prob->precision == FIRE_PREC_FP64) {
+    size_t so[SLW_COUNT + 1];
+    sl_offsets<double>(prob, so);
+    *bytes = so[SLW_COUNT];
+  } else {
+    int64_t off[PR_COUNT + 1];
+    prep_offsets(prob, off);
+    *bytes = prep64_offset(prob) + (size_t)off[PR_COUNT] * 8;
+  }
   return FIRE_OK;
 }
 
 fire_status fire_workspace_size(const fire_problem* prob, int32_t chunk, size_t* bytes) {
   if (!valid(prob) || !bytes) return FIRE_ERR_INVALID;
   const int c = chunk > 0 ? std::min(chunk, prob->n_walkers) : prob->n_walkers;
-  *bytes = eloc_ws_bytes(prob, c, nullptr);
+  // the value paths take the same workspace (in a batch of a few walkers their slices are more than the local energy's planes)
+  *bytes = std::max(eloc_ws_bytes(prob, c, nullptr), make_plan(prob, c, false).total);
   return FIRE_OK;
 }
 
@@ -2138,7 +2144,7 @@ fire_status fire_prepare_params(void* stream, const fire_problem* prob, const fl
   if (st == FIRE_OK) {  // the FP64 copy of the refinement pass
     const fire_problem p64 = refine_problem64(prob, 1);
     st = prepare_impl<double>(s, &p64, blob, offsets_host,
-                              reinterpret_cast<unsigned char*>(prepared) + prep64_offset(prob));
+                              reinterpret_cast<unsigned char*>(prepared) + prep64_offset(prob), false);
   }
   if (st != FIRE_OK || prob->precision != FIRE_PREC_MIXED) return st;
   int64_t off[PR_COUNT + 1];

@@ -724,7 +724,7 @@ int sl_launch(const SlCall<typename SlFmt<KIND>::T>& c, unsigned char* scratch, 
   const size_t a_bytes = sl_a_bytes<KIND>(pass, p0.K), block = (a_bytes + (size_t)pass * 4 + 255) / 256 * 256;
   for (int g = 0; g < c.nseg; ++g) {
     const GemmP<T>& p = c.p[g];
-    if (p.K != p0.K || p.N != p0.N) return -1;
+    if (p.K != p0.K || p.N != p0.N || !c.w[g]) return -1;
     const int q = c.share_a ? 0 : g;  // whose slices
     a.p[g] = p;
     a.Bt[g] = c.w[g];
