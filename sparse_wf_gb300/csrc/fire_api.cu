@@ -15,6 +15,7 @@
 
 #include "fire_gemm.cuh"
 #include "fire_kernels.cuh"
+#include "fire_passes.h"
 #include "fire_sliced.cuh"
 
 using namespace fire;
@@ -407,11 +408,30 @@ size_t eloc_ws_bytes(const fire_problem* p, int Wc, size_t* list_off) {
   return KF > 0 ? t + ((size_t)(2 * KF + 1) * 4 + 255) / 256 * 256 : t;
 }
 
-// A pass of c walkers reduced to whole rounds of the elimination where that fills the GPU with two CTAs per SM (512 threads,
-// gjg_threads): 153 walkers of 322 electrons are 612 matrices, three rounds of 304 where 152 walkers take two.
+// Dynamic shared memory of k_gj_global (eight-byte elements): two panel buffers, the panel's small arrays, two index lists.
+size_t gjg_smem(int n) {
+  constexpr int BW = GJG_BW_DECL;
+  return 8 * (2 * (size_t)n * (BW + 1) + BW * BW + n + 3 * BW) + sizeof(int) * (2 * (size_t)n + BW);
+}
+// Matrices that the local energy's elimination has on this GPU at once (0: cannot be asked).
+int elimination_places(const fire_problem* p) {
+  int dev = 0, sms = 0, per = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  const size_t smem = gjg_smem(p->n_el);
+  auto ask = [&](auto kern) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+           cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, gjg_threads(p->n_el), smem) == cudaSuccess;
+  };
+  const bool ok = p->precision == FIRE_PREC_FP64 ? ask(k_gj_global<double, double, double, true>)
+                                                 : ask(k_gj_global<df64, float, float, true>);
+  return ok ? per * sms : 0;
+}
+// A pass of c walkers reduced to whole rounds of the elimination where that saves rounds (fire_passes.h).  Only for the large
+// matrices (512 threads each), whose rounds are long beside what a pass costs.
 int whole_rounds(const fire_problem* p, int c) {
-  constexpr int ROUND = 2 * SL_SMS / NDET;  // walkers of a round
-  return gjg_threads(p->n_el) == 512 && c > ROUND ? c - c % ROUND : c;
+  if (gjg_threads(p->n_el) < 512 || c >= p->n_walkers) return c;
+  return pass_walkers(p->n_walkers, c, NDET, elimination_places(p));
 }
 
 int choose_chunk(const fire_problem* p, size_t ws_bytes, bool fl) {
@@ -434,7 +454,7 @@ int choose_chunk(const fire_problem* p, size_t ws_bytes, bool fl) {
     const int mid = (lo + hi + 1) / 2;
     if (need(mid) <= ws_bytes) lo = mid; else hi = mid - 1;
   }
-  return fl && lo < p->n_walkers ? whole_rounds(p, lo) : lo;
+  return fl ? whole_rounds(p, lo) : lo;
 }
 
 // ------------------------------------------------------------------------------ prepare kernels
@@ -1055,9 +1075,8 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
 template <typename S, typename TI, typename TO, bool INV>
 cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, double* cond = nullptr) {
   const int n = c.p->n_el;
-  constexpr int BW = GJG_BW_DECL;
-  const size_t smem =
-      sizeof(S) * (2 * (size_t)n * (BW + 1) + BW * BW + n + 3 * BW) + sizeof(int) * (2 * (size_t)n + BW);
+  static_assert(sizeof(S) == 8, "gjg_smem");
+  const size_t smem = gjg_smem(n);
   auto kern = k_gj_global<S, TI, TO, INV>;
   // always opt in: the kernel's static shared memory adds to the dynamic size
   const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
