@@ -824,14 +824,14 @@ cudaError_t stage_embedding(Ctx<T>& c) {
   g.M = G * NV; g.N = 2 * F; g.K = F;
   ei_gemm<T>(c, g, NV, TC_EI_GLU, SLW_GLU);
   g_nlaunch++;
-  k_glu<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, E5a, G);
+  k_glu<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, E5a, G, n, c.nb.live);
   g = gp0<T>();
   g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_DENSE_W]; g.ldb = F; g.C = Z1; g.ldc = F;
   g.bias = c.W.w[FIRE_P_EI_DENSE_B]; g.bias_period = NV;
   g.M = G * NV; g.N = F; g.K = F;
   ei_gemm<T>(c, g, NV, TC_EI_DENSE, SLW_DENSE);
   g_nlaunch++;
-  k_silu5<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, G);
+  k_silu5<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, G, n, c.nb.live);
   g = gp0<T>();
   g.A = Z1; g.lda = F; g.B = c.W.w[FIRE_P_EI_OUT_W]; g.ldb = 5 * F; g.C = E5o; g.ldc = 5 * F;
   g.bias = c.W.w[FIRE_P_EI_OUT_B]; g.bias_period = NV;
@@ -913,13 +913,12 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     const bool tc_ok = sizeof(T) == 4 && c.mixed && NENV_ORB * N <= ENV_TC_KMAX;
     const bool tc_env = tc_ok && NV > 1;
     const bool tc_val = tc_ok && NV == 1 && !c.comp;
-    const int nvc = tc_env ? 1 : NV;  // coefficient rows per electron
     if (!tc_val) {
       g_nlaunch++;
       if (tc_env)
-        k_env_coef<T, 1><<<nblk(tot), 256, 0, c.s>>>(c.r, c.R, sp, n, ns, s == 0 ? 0 : nu, N, c.Wc, coef);
+        k_env_coef<T, 1><<<nblk(tot), 256, 0, c.s>>>(c.r, c.R, sp, n, ns, s == 0 ? 0 : nu, N, c.Wc, coef, c.nb.live);
       else
-        k_env_coef<T, NV><<<nblk(tot), 256, 0, c.s>>>(c.r, c.R, sp, n, ns, s == 0 ? 0 : nu, N, c.Wc, coef);
+        k_env_coef<T, NV><<<nblk(tot), 256, 0, c.s>>>(c.r, c.R, sp, n, ns, s == 0 ? 0 : nu, N, c.Wc, coef, c.nb.live);
     }
     for (int d = 0; d < NDET; ++d) {
       if constexpr (sizeof(T) == 4) {
@@ -1139,7 +1138,7 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
   k_readout_in<T, FLM><<<Wc, 512, 0, c.s>>>(n, c.template buf<T>(c.P.Ax), FLM ? c.template buf<T>(c.P.Al) : nullptr,
                                             FLM ? c.template buf<T>(c.P.AJ) : nullptr, c.template buf<T>(c.P.RX),
                                             FLM ? c.template buf<T>(c.P.RJ) : nullptr,
-                                            FLM ? c.template buf<T>(c.P.RL) : nullptr);
+                                            FLM ? c.template buf<T>(c.P.RL) : nullptr, c.nb.live);
   // readout MLP 512 -> 256 -> 256 -> 2 on the dense carrier (node = walker, tangents 3n)
   const Planes RI{c.P.RX, c.P.RJ, c.P.RL}, R1{c.P.R1X, c.P.R1J, c.P.R1L}, R2{c.P.R2X, c.P.R2J, c.P.R2L};
   {
@@ -1457,8 +1456,8 @@ __global__ void k_refine_gather(const T* __restrict__ r, int n, const int32_t* _
 // (embedding, update, envelopes, orbitals) of their positions, then the chunk evaluation of the same positions with
 // those orbital matrices eliminated in FP64 and the derivative planes on the FP32 CUDA cores; the results go to the
 // walkers' rows.  The list is evaluated in passes of KC <= Wc walkers (the batch's chunk size, so that they fit
-// the workspace); a pass's kernels leave the walkers beyond the device's count alone (Nbr::live), so that a capacity well
-// above it costs the launches only.
+// the workspace).  A pass's kernels leave the walkers beyond the device's count alone (Nbr::live); what a capacity above it
+// costs is their launches, grids that find nothing to do, and a few cleared sums.
 template <typename T>
 cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const float* R, const float* Z,
                         const void* prepared, const T* r, void* logpsi, void* sign, void* eloc,
@@ -1817,13 +1816,13 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
     g.M = ME; g.N = 2 * F; g.K = F;
     gemm<T, EPI_PLAIN>(c, g);
     g_nlaunch++;
-    k_glu<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, E5a, ME);
+    k_glu<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, E5a, ME, 1, nullptr);
     g = gp0<T>();
     g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_DENSE_W]; g.ldb = F; g.C = Z1; g.ldc = F;
     g.bias = c.W.w[FIRE_P_EI_DENSE_B]; g.bias_period = 1; g.M = ME; g.N = F; g.K = F;
     gemm<T, EPI_PLAIN>(c, g);
     g_nlaunch++;
-    k_silu5<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, ME);
+    k_silu5<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, ME, 1, nullptr);
     g = gp0<T>();
     g.A = Z1; g.lda = F; g.B = c.W.w[FIRE_P_EI_OUT_W]; g.ldb = 5 * F; g.C = c.template buf<T>(Q.E5p);
     g.ldc = 5 * F; g.bias = c.W.w[FIRE_P_EI_OUT_B]; g.bias_period = 1; g.M = ME; g.N = 5 * F; g.K = F;
@@ -1920,7 +1919,7 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
                                      c.template buf<T>(Q.oS), c.template buf<T>(c.P.Ax), c.template buf<T>(c.P.JMx));
     g_nlaunch++;
     k_readout_in<T, false><<<Wc, 512, 0, s>>>(n, c.template buf<T>(c.P.Ax), nullptr, nullptr,
-                                              c.template buf<T>(c.P.RX), nullptr, nullptr);
+                                              c.template buf<T>(c.P.RX), nullptr, nullptr, nullptr);
     readout_value<T>(c);
   }
   // log|psi'| and the Metropolis test

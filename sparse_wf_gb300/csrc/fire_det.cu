@@ -26,7 +26,8 @@ namespace fire {
 // coef layout: [det][rows = (w * n_s + i) * NV + v][N * 8]
 template <typename T, int NV>
 __global__ void k_env_coef(const T* __restrict__ r, const float* __restrict__ R, const T* __restrict__ sp,
-                           int n, int n_s, int s_off, int N, int Wn, T* __restrict__ coef) {
+                           int n, int n_s, int s_off, int N, int Wn, T* __restrict__ coef,
+                           const int* __restrict__ live) {
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;  // over (w * n_s + i, I, k)
   const long total = (long)Wn * n_s * N * NENV_ORB;
   if (idx >= total) return;
@@ -34,6 +35,7 @@ __global__ void k_env_coef(const T* __restrict__ r, const float* __restrict__ R,
   const int I = (int)((idx / NENV_ORB) % N);
   const long rr = idx / ((long)NENV_ORB * N);
   const int w = (int)(rr / n_s), i = (int)(rr % n_s);
+  if (live && w >= *live) return;
   const long g = (long)w * n + s_off + i;
   const T dx = r[3 * g] - (T)R[3 * I], dy = r[3 * g + 1] - (T)R[3 * I + 1], dz = r[3 * g + 2] - (T)R[3 * I + 2];
   const T rho = dsqrt(dx * dx + dy * dy + dz * dz);
@@ -710,13 +712,13 @@ __global__ void k_orb_lap(float* __restrict__ lapA, const float* __restrict__ en
 }
 
 template __global__ void k_env_coef<float, 1>(const float*, const float*, const float*, int, int, int, int, int,
-                                              float*);
+                                              float*, const int*);
 template __global__ void k_env_coef<float, 5>(const float*, const float*, const float*, int, int, int, int, int,
-                                              float*);
+                                              float*, const int*);
 template __global__ void k_env_coef<double, 1>(const double*, const float*, const double*, int, int, int, int,
-                                               int, double*);
+                                               int, double*, const int*);
 template __global__ void k_env_coef<double, 5>(const double*, const float*, const double*, int, int, int, int,
-                                               int, double*);
+                                               int, double*, const int*);
 template __global__ void k_gj_global<df64, float, float, false>(const float*, const float*, int, df64*, double*, double*, double*,
                                                                  float*, const int*, int32_t*);
 template __global__ void k_gj_global<df64, float, float, true>(const float*, const float*, int, df64*, double*, double*, double*,

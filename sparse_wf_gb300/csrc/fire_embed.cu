@@ -434,14 +434,16 @@ __global__ void __launch_bounds__(256) k_elec_init(const T* __restrict__ r, cons
   fl_store(E5 + (size_t)g * NV * F + f, F, y);
 }
 
-// out[g][v][f] = a * silu(gate) with a = Z[g][v][f], gate = Z[g][v][F + f]   (GatedLinearUnit)
+// out[g][v][f] = a * silu(gate) with a = Z[g][v][f], gate = Z[g][v][F + f]   (GatedLinearUnit).  n rows per walker; live: as
+// Nbr::live
 template <typename T, int NT>
-__global__ void k_glu(const T* __restrict__ Z, T* __restrict__ out, int G) {
+__global__ void k_glu(const T* __restrict__ Z, T* __restrict__ out, int G, int n, const int* __restrict__ live) {
   constexpr int NV = NVr<NT>::v;
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)G * F) return;
   const long g = idx / F;
   const int f = (int)(idx - g * F);
+  if (live && g >= (long)*live * n) return;
   const FLv<T, NT> a = fl_load<T, NT>(Z + g * NV * 2 * F + f, 2 * F);
   const FLv<T, NT> b = fl_load<T, NT>(Z + g * NV * 2 * F + F + f, 2 * F);
   fl_store(out + g * NV * F + f, F, fl_mul(a, fl_silu(b)));
@@ -449,12 +451,13 @@ __global__ void k_glu(const T* __restrict__ Z, T* __restrict__ out, int G) {
 
 // in-place silu on carriers [G][NV][F]
 template <typename T, int NT>
-__global__ void k_silu5(T* __restrict__ Z, int G) {
+__global__ void k_silu5(T* __restrict__ Z, int G, int n, const int* __restrict__ live) {
   constexpr int NV = NVr<NT>::v;
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long)G * F) return;
   const long g = idx / F;
   const int f = (int)(idx - g * F);
+  if (live && g >= (long)*live * n) return;
   const FLv<T, NT> a = fl_load<T, NT>(Z + g * NV * F + f, F);
   fl_store(Z + g * NV * F + f, F, fl_silu(a));
 }
@@ -690,8 +693,8 @@ template __global__ void k_lr_contract<double>(const double*, int, int, double, 
 
 #define FIRE_INST_EMBED(T, NT)                                                                              \
   template __global__ void k_elec_init<T, NT>(const T*, const float*, Nbr, Weights<T>, T, T*);            \
-  template __global__ void k_glu<T, NT>(const T*, T*, int);                                                 \
-  template __global__ void k_silu5<T, NT>(T*, int);                                                         \
+  template __global__ void k_glu<T, NT>(const T*, T*, int, int, const int*);                                                 \
+  template __global__ void k_silu5<T, NT>(T*, int, int, const int*);                                                         \
   template __global__ void k_edge_contract<T, NT>(const T*, Nbr, Layout, Weights<T>, const T*, T*, T*, T*);
 FIRE_INST_EMBED(float, 0)
 FIRE_INST_EMBED(float, 3)

@@ -250,8 +250,10 @@ __global__ void __launch_bounds__(256) k_att_sums(Nbr nb, Layout L, const T* __r
 template <typename T, bool FLM>
 __global__ void __launch_bounds__(512) k_readout_in(int n, const T* __restrict__ Ax, const T* __restrict__ Al,
                                                     const T* __restrict__ AJ, T* __restrict__ RX,
-                                                    T* __restrict__ RJ, T* __restrict__ RL) {
+                                                    T* __restrict__ RJ, T* __restrict__ RL,
+                                                    const int* __restrict__ live) {
   const int w = blockIdx.x, slot = threadIdx.x;  // slot = s * 256 + r * 16 + d
+  if (live && w >= *live) return;
   const int s = slot >> 8, rd = slot & 255, r = rd >> 4;
   const T* ax = Ax + ((size_t)w * 2 + s) * 272;
   const T N = ax[256 + r], V = ax[rd];
@@ -591,8 +593,8 @@ __global__ void k_stats(const T* __restrict__ e, int B, double* __restrict__ out
                                                const T*, T*, T*, T*);                                            \
   template __global__ void k_att_sums<T, false>(Nbr, Layout, const T*, const T*, const T*, const T*, const T*,    \
                                                 const T*, T*, T*, T*);                                           \
-  template __global__ void k_readout_in<T, true>(int, const T*, const T*, const T*, T*, T*, T*);                  \
-  template __global__ void k_readout_in<T, false>(int, const T*, const T*, const T*, T*, T*, T*);                 \
+  template __global__ void k_readout_in<T, true>(int, const T*, const T*, const T*, T*, T*, T*, const int*);                  \
+  template __global__ void k_readout_in<T, false>(int, const T*, const T*, const T*, T*, T*, T*, const int*);                 \
   template __global__ void k_assemble<T, true>(int, int, int, int, const T*, const float*, const float*,          \
                                                Weights<T>, const double*, const double*, const double*,          \
                                                const double*, const T*, const T*, const T*, const T*, const T*,   \

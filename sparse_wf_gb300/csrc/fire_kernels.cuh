@@ -22,9 +22,9 @@ __global__ void k_layout(Nbr nb, Layout L);
 template <typename T, int NT>
 __global__ void k_elec_init(const T* r, const float* R, Nbr nb, Weights<T> W, T inv_cutoff1, T* E5);
 template <typename T, int NT>
-__global__ void k_glu(const T* Z, T* out, int G);
+__global__ void k_glu(const T* Z, T* out, int G, int n, const int* live);
 template <typename T, int NT>
-__global__ void k_silu5(T* Z, int G);
+__global__ void k_silu5(T* Z, int G, int n, const int* live);
 template <typename T, int NT>
 __global__ void k_edge_contract(const T* r, Nbr nb, Layout L, Weights<T> W, const T* E5o, T* X, T* Lp, T* Jp);
 template <typename T>
@@ -37,7 +37,7 @@ __global__ void k_lr_contract(const T* rn, int n, int n_up, T cutoff, const int*
 __global__ void k_orb_lap(float* lapA, const float* env, const float* raw, const float* rjs, long G, int DN);
 template <typename T, int NV>
 __global__ void k_env_coef(const T* r, const float* R, const T* sp, int n, int n_s, int s_off, int N, int Wn,
-                           T* coef);
+                           T* coef, const int* live);
 template <typename S, typename TI, typename TO, bool INV>
 __global__ void k_gj_global(const TI* A, const TI* A_lo, int n, S* work, double* logdet, double* sign, double* cond, TO* Ainv,
                             const int* live, int32_t* status);
@@ -61,7 +61,7 @@ template <typename T, bool FLM>
 __global__ void k_att_sums(Nbr nb, Layout L, const T* aX, const T* aJ, const T* aL, const T* VX, const T* VJ,
                            const T* VL, T* Ax, T* Al, T* AJ);
 template <typename T, bool FLM>
-__global__ void k_readout_in(int n, const T* Ax, const T* Al, const T* AJ, T* RX, T* RJ, T* RL);
+__global__ void k_readout_in(int n, const T* Ax, const T* Al, const T* AJ, T* RX, T* RJ, T* RL, const int* live);
 template <typename T, bool FLM>
 __global__ void k_assemble(int n, int n_up, int N, int w0, const T* r, const float* R, const float* Z,
                            Weights<T> W, const double* ld, const double* sd, const double* dgrad, const double* dlap,
