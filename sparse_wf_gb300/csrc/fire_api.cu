@@ -397,13 +397,25 @@ RefineLayout refine_layout(const fire_problem* p, int KC) {
   L.total = up(L.r64 + n3 * 8);
   return L;
 }
+// Walkers of a refinement pass beside chunks of Wc walkers: the most that fit the chunk's workspace (one at least), so that
+// room for refined walkers takes none of its own.
+int refine_chunk(const fire_problem* p, int Wc) {
+  const size_t ws = make_plan(p, Wc, true).total;
+  int lo = 1, hi = std::min(refine_walkers(p), Wc);
+  if (hi <= 1 || refine_layout(p, hi).total <= ws) return hi;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (refine_layout(p, mid).total <= ws) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
 // Total workspace of the local energy with chunks of Wc walkers: the larger of the chunk plan and the refinement
-// pass (in passes of at most Wc walkers), then the list of ill-conditioned walkers (KF indices, their count and
-// one count per pass), which lives through both.
+// pass, then the list of ill-conditioned walkers (KF indices, their count and one count per pass), which lives through
+// both.
 size_t eloc_ws_bytes(const fire_problem* p, int Wc, size_t* list_off) {
   const int KF = refine_walkers(p);
   size_t t = make_plan(p, Wc, true).total;
-  if (KF > 0) t = std::max(t, refine_layout(p, std::min(KF, Wc)).total);
+  if (KF > 0) t = std::max(t, refine_layout(p, refine_chunk(p, Wc)).total);
   if (list_off) *list_off = t;
   return KF > 0 ? t + ((size_t)(2 * KF + 1) * 4 + 255) / 256 * 256 : t;
 }
@@ -1455,14 +1467,13 @@ __global__ void k_refine_gather(const T* __restrict__ r, int n, const int32_t* _
 // The refinement pass over the ill-conditioned walkers of the batch (rf.idx, rf.cnt): the FP64 value path
 // (embedding, update, envelopes, orbitals) of their positions, then the chunk evaluation of the same positions with
 // those orbital matrices eliminated in FP64 and the derivative planes on the FP32 CUDA cores; the results go to the
-// walkers' rows.  The list is evaluated in passes of KC <= Wc walkers (the batch's chunk size, so that they fit
-// the workspace).  A pass's kernels leave the walkers beyond the device's count alone (Nbr::live); what a capacity above it
+// walkers' rows.  The list is evaluated in passes of KC walkers (refine_chunk).  A pass's kernels leave the walkers beyond the device's count alone (Nbr::live); what a capacity above it
 // costs is their launches, grids that find nothing to do, and a few cleared sums.
 template <typename T>
 cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const float* R, const float* Z,
                         const void* prepared, const T* r, void* logpsi, void* sign, void* eloc,
                         const fire_eloc_debug* dbg, unsigned char* ws, int32_t* status, Refine rf) {
-  const int KF = rf.cap, KC = std::min(KF, Wc), n = p->n_el;
+  const int KF = rf.cap, KC = refine_chunk(p, Wc), n = p->n_el;
   const RefineLayout L = refine_layout(p, KC);
   T* r_ref = reinterpret_cast<T*>(ws + L.r_ref);
   double* r64 = reinterpret_cast<double*>(ws + L.r64);
@@ -1475,11 +1486,12 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
   Prof pr("refine", s);
   SideStream side(s);
   for (int k0 = 0, j = 0; k0 < KF; k0 += KC, ++j) {
+    const int kc = std::min(KC, KF - k0);  // of this pass
     g_nlaunch++;
-    k_refine_gather<T><<<KC, 128, 0, s>>>(r, n, rf.idx, rf.cnt, KF, k0, KC, r_ref, r64, sub_cnt + j, status);
+    k_refine_gather<T><<<kc, 128, 0, s>>>(r, n, rf.idx, rf.cnt, KF, k0, kc, r_ref, r64, sub_cnt + j, status);
     Ctx<T> c = make_ctx<T>(&pr_, s, R, Z, prepared, status, ws, KC, true);
     c.w0 = 0;
-    c.Wc = KC;
+    c.Wc = kc;
     c.r = r_ref;
     c.nb.live = sub_cnt + j;
     // FP64 values, determinants and inverses: bound by the FP64 pipe, while the FP32 planes of the same walkers are bound by
@@ -1489,7 +1501,7 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
                                        reinterpret_cast<const unsigned char*>(prepared) + prep64_offset(p), status,
                                        ws + L.c64, KC, false, false, true);
     c64.w0 = 0;
-    c64.Wc = KC;
+    c64.Wc = kc;
     c64.r = r64;
     c64.nb.live = sub_cnt + j;
     setup_ctx(c64, false);
@@ -1501,7 +1513,7 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
       Prof pr_gj("gauss_jordan", side.s);
       launch_gjg<double, double, T, true>(c64, c64.template buf<double>(c64.P.Apl), (const double*)nullptr,
                                           c.template buf<T>(c.P.Ainv));
-      const size_t nb = sizeof(double) * (size_t)KC * NDET;
+      const size_t nb = sizeof(double) * (size_t)kc * NDET;
       cudaMemcpyAsync(c.template buf<double>(c.P.ld), c64.template buf<double>(c64.P.ld), nb, cudaMemcpyDeviceToDevice,
                       side.s);
       cudaMemcpyAsync(c.template buf<double>(c.P.sd), c64.template buf<double>(c64.P.sd), nb, cudaMemcpyDeviceToDevice,

@@ -139,9 +139,10 @@ class FireWaveFunction:
         cap_n = static.n_neighbours_en if static is not None else 1
         cap_r = 0
         if refine and self.refine:
-            # the last call's count padded; at least a quarter of the batch (unused capacity costs launches only, a call
-            # that finds more is repeated)
-            cap_r = min(int(n_walkers), max(self._refine_cap, 2, -(-int(n_walkers) // 4)))
+            # the last call's count padded; at least a quarter of the batch (a call that finds more is repeated), but not
+            # more than a pass: every pass of the refinement is launched, whatever it finds to do
+            per = self.chunk_walkers if self.chunk_walkers > 0 else int(n_walkers)
+            cap_r = min(int(n_walkers), max(self._refine_cap, 2, min(-(-int(n_walkers) // 4), per)))
         return _lib.Problem(self.n_electrons, self.n_up, self.n_nuclei, int(n_walkers), self.cutoff,
                             self.cutoff_1el, max(1, int(cap_p)), max(1, int(cap_n)), _lib.PREC[self.precision],
                             self.chunk_walkers, cap_r, float(self.refine_ratio), float(self.refine_kappa),

@@ -56,3 +56,21 @@ def test_workspace_serves_value_and_energy_calls(precision, walkers):
     assert size == sorted(size)
     tile = 128 * F * 2 * (8 if precision == "fp64" else 6)
     assert size[0] >= tile
+
+
+@pytest.mark.parametrize("precision", ["fp32", "mixed"])
+@pytest.mark.parametrize("mol,pairs,walkers,chunk", [(systems.alkane(40), 8000, 2048, 152), (systems.alkane(10), 1500, 2048, 610),
+                                                     (systems.hydrogen_chain(10, 1.8), 80, 512, 16), (systems.alkane(2), 200, 512, 3)])
+def test_room_for_refined_walkers_is_one_pass(mol, pairs, walkers, chunk, precision):
+    """Before any count is known the refinement has room for a quarter of the batch, but for no more than one pass (the least
+    room is two walkers), and a pass's workspace holds it."""
+    from sparse_wf_gb300.wavefunction import FireWaveFunction, StaticArgs
+
+    lib = _lib.load()
+    wf = FireWaveFunction(mol, precision=precision, device="cpu", chunk_walkers=chunk)
+    static = StaticArgs(pairs // 2, pairs - pairs // 2, 0, mol.n_nuc)
+    prob = wf._problem(walkers, static, refine=True)
+    assert 2 <= prob.refine_cap <= min(chunk, -(-walkers // 4))
+    bare = wf._problem(walkers, static)
+    room = _size(lib.fire_workspace_size, C.byref(prob), chunk) - _size(lib.fire_workspace_size, C.byref(bare), chunk)
+    assert room <= _align((2 * prob.refine_cap + 1) * 4)  # the list of walkers
