@@ -20,7 +20,8 @@ INCLUDE = ROOT / "include"
 LIB = PKG / "libfire.so"
 OBJ = ROOT / "_build" / "obj"
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-static-global-template-stub=false",
+# 2809: the value of a [[nodiscard]] function is dropped (the error codes of the stages)
+NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-static-global-template-stub=false", "-diag-error", "2809",
                      "-Xcompiler", "-fPIC", f"-I{INCLUDE}"]
 
 

@@ -31,6 +31,17 @@ fire_status launch_status(const char* where) {
   return FIRE_ERR_CUDA;
 }
 
+// The status of a call that a stage gave up: FIRE_ERR_CUDA also where the cause was a refused contraction, not a CUDA error.
+fire_status failed(const char* where) {
+  const fire_status s = launch_status(where);
+  return s == FIRE_OK ? FIRE_ERR_CUDA : s;
+}
+#define FIRE_TRY(...)                               \
+  do {                                              \
+    const cudaError_t fire_try_ = __VA_ARGS__;      \
+    if (fire_try_ != cudaSuccess) return fire_try_; \
+  } while (0)
+
 // ------------------------------------------------------------------------------ stage profiling
 struct ProfRec {
   const char* name;
@@ -716,7 +727,7 @@ SlCall<T> sl_spin_call(const Ctx<T>& c, const GemmP<T>& g, const unsigned char* 
 }
 // SL_F64: mode is an EpiMode; SL_PAIR (hi + lo value rows): a CompMode
 template <typename T>
-cudaError_t sl_gemm(const Ctx<T>& c, int mode, SlCall<T> q) {
+[[nodiscard]] cudaError_t sl_gemm(const Ctx<T>& c, int mode, SlCall<T> q) {
   for (int g = 0; g < q.nseg; ++g) live_rows(c, q.p[g]);
   Prof pr(sizeof(T) == 4 ? "gemm_comp" : "gemm", c.s);
   unsigned char* scratch = c.template buf<unsigned char>(c.P.sl);
@@ -730,9 +741,10 @@ cudaError_t sl_gemm(const Ctx<T>& c, int mode, SlCall<T> q) {
 // tc_id: tensor-core weight of the mixed path's derivative rows; sl_id: sliced weight in FP64; neither: the CUDA-core
 // contraction
 template <typename T, int MODE>
-cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
+[[nodiscard]] cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
   if constexpr (sizeof(T) == 8) {
     if (sl_id >= 0 && !c.refine64) return sl_gemm(c, MODE, sl_call(g, c.slw[sl_id]));
+    if constexpr (!gemm_d_mode(MODE)) return cudaErrorInvalidValue;  // derivative rows: the sliced contraction alone
   }
   live_rows(c, g);
   // profile stages: "gemm_tc" the mixed path's tensor-core contractions, "gemm" the others
@@ -745,12 +757,13 @@ cudaError_t gemm(const Ctx<T>& c, GemmP<T> g, int tc_id = -1, int sl_id = -1) {
       return gemm_tc(MODE, bn, g, c.tcw[tc_id], c.template buf<int>(c.P.tile_mask), c.status, c.s);
     }
   }
-  return launch_gemm<T, MODE>(g, c.s);
+  if constexpr (sizeof(T) == 4 || gemm_d_mode(MODE)) return launch_gemm<T, MODE>(g, c.s);
+  return cudaErrorInvalidValue;  // not reached
 }
 
 // hi + lo value rows by the CUDA cores: low parts into C_lo / read from env_lo, row stride ld_lo
 template <int MODE>
-cudaError_t gemm_comp(const Ctx<float>& c, GemmP<float> g, float* C_lo, const float* env_lo, long ld_lo) {
+[[nodiscard]] cudaError_t gemm_comp(const Ctx<float>& c, GemmP<float> g, float* C_lo, const float* env_lo, long ld_lo) {
   live_rows(c, g);
   Prof pr("gemm_comp", c.s);
   g_nlaunch++;
@@ -759,7 +772,7 @@ cudaError_t gemm_comp(const Ctx<float>& c, GemmP<float> g, float* C_lo, const fl
 
 // Value-plane contraction of a dense layer (EPI_PLAIN or EPI_SILU_X): hi + lo accuracy in the FP32 and mixed paths.
 template <typename T, int MODE>
-cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
+[[nodiscard]] cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
   if constexpr (sizeof(T) == 4) {
     static_assert(MODE == EPI_PLAIN || MODE == EPI_SILU_X, "value_gemm: plain or SiLU layers");
     if (c.comp && c.pair) return sl_gemm(c, MODE == EPI_PLAIN ? COMP_PLAIN : COMP_SILU, sl_call(g, c.slw[sl_id]));
@@ -772,7 +785,7 @@ cudaError_t value_gemm(const Ctx<T>& c, const GemmP<T>& g, int sl_id) {
 
 // neighbour lists (+ layout for the forward-Laplacian path)
 template <typename T>
-cudaError_t stage_neighbors(Ctx<T>& c, bool fl) {
+[[nodiscard]] cudaError_t stage_neighbors(Ctx<T>& c, bool fl) {
   Prof pr("neighbors", c.s);
   const int n = c.p->n_el;
   const size_t smem = 3 * n * sizeof(T) + (5 * n + 2) * sizeof(int);
@@ -796,7 +809,7 @@ cudaError_t stage_neighbors(Ctx<T>& c, bool fl) {
 // the tensor cores take the derivative rows (the value rows they also compute are not stored) and the
 // CUDA cores the value rows, read with a stride of NV rows: the value plane stays FP32.
 template <typename T>
-cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id, int sl_id) {
+[[nodiscard]] cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id, int sl_id) {
   if (NV == 1) return value_gemm<T, EPI_PLAIN>(c, g, sl_id);
   GemmP<T> gv = g;  // the value rows (every NV-th row), compensated in the FP32 and mixed paths
   gv.lda = g.lda * NV;
@@ -819,7 +832,7 @@ cudaError_t ei_gemm(Ctx<T>& c, const GemmP<T>& g, int NV, int tc_id, int sl_id) 
 }
 
 template <typename T, int NT>
-cudaError_t stage_embedding(Ctx<T>& c) {
+[[nodiscard]] cudaError_t stage_embedding(Ctx<T>& c) {
   constexpr int NV = NT > 0 ? NT + 2 : 1;
   const int n = c.p->n_el, G = c.Wc * n;
   T* E5a = c.template buf<T>(c.P.E5a);
@@ -834,21 +847,21 @@ cudaError_t stage_embedding(Ctx<T>& c) {
   GemmP<T> g = gp0<T>();
   g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_GLU_W]; g.ldb = 2 * F; g.C = Z1; g.ldc = 2 * F;
   g.M = G * NV; g.N = 2 * F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_GLU, SLW_GLU);
+  FIRE_TRY(ei_gemm<T>(c, g, NV, TC_EI_GLU, SLW_GLU));
   g_nlaunch++;
   k_glu<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, E5a, G, n, c.nb.live);
   g = gp0<T>();
   g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_DENSE_W]; g.ldb = F; g.C = Z1; g.ldc = F;
   g.bias = c.W.w[FIRE_P_EI_DENSE_B]; g.bias_period = NV;
   g.M = G * NV; g.N = F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_DENSE, SLW_DENSE);
+  FIRE_TRY(ei_gemm<T>(c, g, NV, TC_EI_DENSE, SLW_DENSE));
   g_nlaunch++;
   k_silu5<T, NT><<<nblk((long)G * F), 256, 0, c.s>>>(Z1, G, n, c.nb.live);
   g = gp0<T>();
   g.A = Z1; g.lda = F; g.B = c.W.w[FIRE_P_EI_OUT_W]; g.ldb = 5 * F; g.C = E5o; g.ldc = 5 * F;
   g.bias = c.W.w[FIRE_P_EI_OUT_B]; g.bias_period = NV;
   g.M = G * NV; g.N = 5 * F; g.K = F;
-  ei_gemm<T>(c, g, NV, TC_EI_OUT, SLW_OUT);
+  FIRE_TRY(ei_gemm<T>(c, g, NV, TC_EI_OUT, SLW_OUT));
   Prof pr("edge_contract", c.s);
   k_edge_contract<T, NT><<<G, 256, 0, c.s>>>(c.r, c.nb, c.L, c.W, E5o, c.template buf<T>(c.P.HX),
                                              NT ? c.template buf<T>(c.P.HL) : nullptr,
@@ -862,7 +875,7 @@ struct Planes {
 
 // Linear(F -> N) + SiLU on a sparse node (value path: X plane only)
 template <typename T>
-cudaError_t silu_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
+[[nodiscard]] cudaError_t silu_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
                        int rowsX, int rowsJcap, const int* rowsJdev, const int* node_map, int node_div, size_t zx,
                        size_t jsq, int tc_id, int sl_id) {
   GemmP<T> g = gp0<T>();
@@ -872,42 +885,42 @@ cudaError_t silu_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, c
     g.aux0 = c.template buf<T>(zx);
     g.aux2 = c.template buf<T>(c.P.Zx2);
   }
-  value_gemm<T, EPI_SILU_X>(c, g, sl_id);
+  FIRE_TRY(value_gemm<T, EPI_SILU_X>(c, g, sl_id));
   if (!fl) return cudaPeekAtLastError();
   cudaMemsetAsync(c.template buf<T>(jsq), 0, sizeof(T) * (size_t)rowsX * N, c.s);
   g = gp0<T>();
   g.A = c.template buf<T>(in.J); g.lda = K; g.B = Wt; g.ldb = N; g.C = c.template buf<T>(out.J); g.ldc = N;
   g.M = rowsJcap; g.M_dev = rowsJdev; g.M_scale = 3; g.N = N; g.K = K; g.node_map = node_map;
   g.node_div = node_div; g.aux1 = c.template buf<T>(zx); g.aux2 = c.template buf<T>(jsq); g.ld_aux = N;
-  gemm<T, EPI_SILU_J>(c, g, tc_id, sl_id);
+  FIRE_TRY(gemm<T, EPI_SILU_J>(c, g, tc_id, sl_id));
   g = gp0<T>();
   g.A = c.template buf<T>(in.L); g.lda = K; g.B = Wt; g.ldb = N; g.C = c.template buf<T>(out.L); g.ldc = N;
   g.M = rowsX; g.N = N; g.K = K; g.aux1 = c.template buf<T>(zx); g.aux0 = c.template buf<T>(c.P.Zx2);
   g.aux3 = c.template buf<T>(jsq); g.ld_aux = N;
-  gemm<T, EPI_SILU_L>(c, g, tc_id, sl_id);
+  FIRE_TRY(gemm<T, EPI_SILU_L>(c, g, tc_id, sl_id));
   return cudaPeekAtLastError();
 }
 
 // Linear(F -> N) without activation on a node (bias on X only)
 template <typename T>
-cudaError_t linear_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
+[[nodiscard]] cudaError_t linear_layer(Ctx<T>& c, bool fl, Planes in, Planes out, const T* Wt, const T* b, int K, int N,
                          int rowsX, int rowsJcap, const int* rowsJdev, int tc_id, int sl_id) {
   GemmP<T> g = gp0<T>();
   g.A = c.template buf<T>(in.X); g.lda = K; g.B = Wt; g.ldb = N; g.bias = b; g.bias_period = 1;
   g.C = c.template buf<T>(out.X); g.ldc = N; g.M = rowsX; g.N = N; g.K = K;
-  value_gemm<T, EPI_PLAIN>(c, g, sl_id);
+  FIRE_TRY(value_gemm<T, EPI_PLAIN>(c, g, sl_id));
   if (!fl) return cudaPeekAtLastError();
   g.A = c.template buf<T>(in.J); g.bias = nullptr; g.C = c.template buf<T>(out.J); g.M = rowsJcap;
   g.M_dev = rowsJdev; g.M_scale = rowsJdev ? 3 : 1;
-  gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id);
+  FIRE_TRY(gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id));
   g.A = c.template buf<T>(in.L); g.C = c.template buf<T>(out.L); g.M = rowsX; g.M_dev = nullptr; g.M_scale = 1;
-  gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id);
+  FIRE_TRY(gemm<T, EPI_PLAIN>(c, g, tc_id, sl_id));
   return cudaPeekAtLastError();
 }
 
 // envelopes + orbital matrices (+ their Jacobian/Laplacian planes)
 template <typename T, int NT>
-cudaError_t stage_orbitals(Ctx<T>& c) {
+[[nodiscard]] cudaError_t stage_orbitals(Ctx<T>& c) {
   constexpr int NV = NT > 0 ? NT + 2 : 1;
   const bool fl = NT > 0;
   const int n = c.p->n_el, nu = c.p->n_up, N = c.p->n_nuc, G = c.Wc * n, DN = NDET * n;
@@ -1011,7 +1024,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
   g.C = c.template buf<T>(c.P.Apl); g.ldc = DN; g.M = G; g.N = DN; g.K = F; g.n_el = n; g.n_up = nu;
   g.aux0 = c.template buf<T>(c.P.rawx); g.aux1 = env; g.ld_aux = DN; g.env_nv = NV;
   if (c.refine64) {
-    gemm<T, EPI_ORB_X>(c, g);
+    FIRE_TRY(gemm<T, EPI_ORB_X>(c, g));
   } else if (sizeof(T) == 8 || c.pair) {
     SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN]);
     if constexpr (sizeof(T) == 4) {
@@ -1023,9 +1036,9 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     if (e != cudaSuccess) return e;
   } else if constexpr (sizeof(T) == 4) {
     if (c.comp)
-      gemm_comp<COMP_ORB>(c, g, c.template buf<float>(c.P.Apl_lo), c.template buf<float>(c.P.env_lo), DN);
+      FIRE_TRY(gemm_comp<COMP_ORB>(c, g, c.template buf<float>(c.P.Apl_lo), c.template buf<float>(c.P.env_lo), DN));
     else
-      gemm<T, EPI_ORB_X>(c, g);
+      FIRE_TRY(gemm<T, EPI_ORB_X>(c, g));
   }
   if (!fl) return cudaPeekAtLastError();
   g = gp0<T>();
@@ -1048,7 +1061,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     const cudaError_t e = sl_gemm(c, EPI_ORB_J, q);
     if (e != cudaSuccess) return e;
   } else {
-    gemm<T, EPI_ORB_J>(c, g, TC_ORB_UP);
+    FIRE_TRY(gemm<T, EPI_ORB_J>(c, g, TC_ORB_UP));
   }
   g = gp0<T>();
   g.A = c.template buf<T>(c.P.B2L); g.lda = F; g.B = c.W.w[PR_ORB_UP_W_S1]; g.B2 = c.W.w[PR_ORB_DN_W_S1];
@@ -1075,7 +1088,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
     SlCall<T> q = sl_spin_call(c, g, c.slw[SLW_ORB_UP], c.slw[SLW_ORB_DN]);
     return sl_gemm(c, EPI_ORB_L, q);
   } else {
-    gemm<T, EPI_ORB_L>(c, g, TC_ORB_UP);
+    FIRE_TRY(gemm<T, EPI_ORB_L>(c, g, TC_ORB_UP));
   }
   return cudaPeekAtLastError();
 }
@@ -1084,7 +1097,7 @@ cudaError_t stage_orbitals(Ctx<T>& c) {
 // working matrix in the workspace (k_gj_global).  Its shared memory (two panel buffers of n x 17 eight-byte
 // elements plus ~2.5 KB) limits the inverse, and so the local energy, to ELOC_MAX_EL electrons.
 template <typename S, typename TI, typename TO, bool INV>
-cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, double* cond = nullptr) {
+[[nodiscard]] cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, double* cond = nullptr) {
   const int n = c.p->n_el;
   static_assert(sizeof(S) == 8, "gjg_smem");
   const size_t smem = gjg_smem(n);
@@ -1101,7 +1114,7 @@ cudaError_t launch_gjg(const Ctx<TI>& c, const TI* A, const TI* A_lo, TO* Ainv, 
 
 // Jastrow: attention (Q.keys narrow + V + sums + readout MLP) and MLP Jastrow; H and B1 are scratch.
 template <typename T, int NT>
-cudaError_t stage_jastrow(Ctx<T>& c) {
+[[nodiscard]] cudaError_t stage_jastrow(Ctx<T>& c) {
   constexpr bool FLM = NT > 0;
   const int n = c.p->n_el, G = c.Wc * n, Wc = c.Wc;
   const int Jcap = 3 * c.L.cap_pos;
@@ -1123,13 +1136,13 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
     g.C = c.template buf<T>(c.P.aJ); g.ldc = HEADS; g.M = Jcap; g.M_dev = Jdev; g.M_scale = 3; g.N = HEADS;
     g.K = F; g.node_map = c.L.pos_ctr; g.node_div = 3; g.aux1 = c.template buf<T>(c.P.aD1);
     g.aux2 = c.template buf<T>(c.P.ajsq); g.ld_aux = HEADS;
-    gemm<T, EPI_SILU_J>(c, g, TC_QK);
+    FIRE_TRY(gemm<T, EPI_SILU_J>(c, g, TC_QK));
     g = gp0<T>();
     g.A = c.template buf<T>(B2.L); g.lda = F; g.B = c.W.w[PR_QK_W_S1]; g.ldb = HEADS;
     g.C = c.template buf<T>(c.P.aL); g.ldc = HEADS; g.M = G; g.N = HEADS; g.K = F;
     g.aux1 = c.template buf<T>(c.P.aD1); g.aux0 = c.template buf<T>(c.P.aD2);
     g.aux3 = c.template buf<T>(c.P.ajsq); g.ld_aux = HEADS;
-    gemm<T, EPI_SILU_L>(c, g, TC_QK);
+    FIRE_TRY(gemm<T, EPI_SILU_L>(c, g, TC_QK));
   } else {
     g_nlaunch++;
     k_narrow<T, HEADS, 1, FLM><<<G, 256, 0, c.s>>>(
@@ -1138,7 +1151,7 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
         FLM ? c.template buf<T>(c.P.aJ) : nullptr, FLM ? c.template buf<T>(c.P.aL) : nullptr, c.status, nullptr,
         nullptr);
   }
-  linear_layer<T>(c, FLM, B2, B1, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, G, Jcap, Jdev, TC_V, SLW_V);
+  FIRE_TRY(linear_layer<T>(c, FLM, B2, B1, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, G, Jcap, Jdev, TC_V, SLW_V));
   cudaMemsetAsync(c.template buf<T>(c.P.Ax), 0, sizeof(T) * Wc * 2 * 272, c.s);
   if (FLM) cudaMemsetAsync(c.template buf<T>(c.P.Al), 0, sizeof(T) * Wc * 2 * 272, c.s);
   g_nlaunch++;
@@ -1156,7 +1169,7 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
   {
     GemmP<T> g = gp0<T>();
     // layer 1/2 with dense Jacobian rows: node of a J row = row / (3n)
-    auto dense_silu = [&](Planes in, Planes out, const T* Wt, const T* b, int K, int sl_id) {
+    auto dense_silu = [&](Planes in, Planes out, const T* Wt, const T* b, int K, int sl_id) -> cudaError_t {
       GemmP<T> q = gp0<T>();
       q.A = c.template buf<T>(in.X); q.lda = K; q.B = Wt; q.ldb = F; q.bias = b; q.C = c.template buf<T>(out.X);
       q.ldc = F; q.M = Wc; q.N = F; q.K = K; q.ld_aux = F;
@@ -1164,37 +1177,37 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
         q.aux0 = c.template buf<T>(c.P.Zr);
         q.aux2 = c.template buf<T>(c.P.Zr2);
       }
-      gemm<T, EPI_SILU_X>(c, q, -1, sl_id);
-      if (!FLM) return;
+      FIRE_TRY(gemm<T, EPI_SILU_X>(c, q, -1, sl_id));
+      if (!FLM) return cudaSuccess;
       cudaMemsetAsync(c.template buf<T>(c.P.jsqr), 0, sizeof(T) * Wc * F, c.s);
       q = gp0<T>();
       q.A = c.template buf<T>(in.J); q.lda = K; q.B = Wt; q.ldb = F; q.C = c.template buf<T>(out.J); q.ldc = F;
       q.M = Wc * 3 * n; q.N = F; q.K = K; q.node_div = 3 * n; q.aux1 = c.template buf<T>(c.P.Zr);
       q.aux2 = c.template buf<T>(c.P.jsqr); q.ld_aux = F;
-      gemm<T, EPI_SILU_J>(c, q, -1, sl_id);
+      FIRE_TRY(gemm<T, EPI_SILU_J>(c, q, -1, sl_id));
       q = gp0<T>();
       q.A = c.template buf<T>(in.L); q.lda = K; q.B = Wt; q.ldb = F; q.C = c.template buf<T>(out.L); q.ldc = F;
       q.M = Wc; q.N = F; q.K = K; q.aux1 = c.template buf<T>(c.P.Zr); q.aux0 = c.template buf<T>(c.P.Zr2);
       q.aux3 = c.template buf<T>(c.P.jsqr); q.ld_aux = F;
-      gemm<T, EPI_SILU_L>(c, q, -1, sl_id);
+      return gemm<T, EPI_SILU_L>(c, q, -1, sl_id);
     };
-    dense_silu(RI, R1, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F, SLW_READ1);
-    dense_silu(R1, R2, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F, SLW_READ2);
+    FIRE_TRY(dense_silu(RI, R1, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F, SLW_READ1));
+    FIRE_TRY(dense_silu(R1, R2, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F, SLW_READ2));
     g.A = c.template buf<T>(R2.X); g.lda = F; g.B = c.W.w[FIRE_P_ATT_OUT3_W]; g.ldb = 2; g.bias = c.W.w[FIRE_P_ATT_OUT3_B];
     g.bias_period = 1; g.C = c.template buf<T>(c.P.JAx); g.ldc = 2; g.M = Wc; g.N = 2; g.K = F;
-    gemm<T, EPI_PLAIN>(c, g);
+    FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
     if (FLM) {
       g.A = c.template buf<T>(R2.J); g.bias = nullptr; g.C = c.template buf<T>(c.P.JAj); g.M = Wc * 3 * n;
-      gemm<T, EPI_PLAIN>(c, g);
+      FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
       g.A = c.template buf<T>(R2.L); g.C = c.template buf<T>(c.P.JAl); g.M = Wc;
-      gemm<T, EPI_PLAIN>(c, g);
+      FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
     }
   }
   // MLP Jastrow: SparseMLP [256, 256, 2] (silu on every layer), * mlp_scale + [0, log_bias], sum over nodes
-  silu_layer<T>(c, FLM, B2, B1, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
-                c.P.Zx, c.P.jsq, TC_JMLP1, SLW_JMLP1);
-  silu_layer<T>(c, FLM, B1, H, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
-                c.P.Zx, c.P.jsq, TC_JMLP2, SLW_JMLP2);
+  FIRE_TRY(silu_layer<T>(c, FLM, B2, B1, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
+                c.P.Zx, c.P.jsq, TC_JMLP1, SLW_JMLP1));
+  FIRE_TRY(silu_layer<T>(c, FLM, B1, H, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3,
+                c.P.Zx, c.P.jsq, TC_JMLP2, SLW_JMLP2));
   g_nlaunch++;
   k_narrow<T, 2, 0, FLM><<<G, 256, 0, c.s>>>(
       c.template buf<T>(H.X), FLM ? c.template buf<T>(H.J) : nullptr, FLM ? c.template buf<T>(H.L) : nullptr, c.nb,
@@ -1211,37 +1224,37 @@ cudaError_t stage_jastrow(Ctx<T>& c) {
 
 // update MLP: H -> B1 -> B2 (scales[0] folded into the first weight, scales[1] into the consumers)
 template <typename T, int NT>
-cudaError_t stage_update(Ctx<T>& c) {
+[[nodiscard]] cudaError_t stage_update(Ctx<T>& c) {
   constexpr bool FLM = NT > 0;
   const int G = c.Wc * c.p->n_el;
   const int Jcap = 3 * c.L.cap_pos;
   const int* Jdev = FLM ? c.L.pos_off + c.Wc : nullptr;
   const Planes H{c.P.HX, c.P.HJ, c.P.HL}, B1{c.P.B1X, c.P.B1J, c.P.B1L}, B2{c.P.B2X, c.P.B2J, c.P.B2L};
   Prof pr("update_mlp", c.s);
-  silu_layer<T>(c, FLM, H, B1, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
-                c.P.jsq, TC_UPD1, SLW_UPD1);
-  silu_layer<T>(c, FLM, B1, B2, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
-                c.P.jsq, TC_UPD2, SLW_UPD2);
+  FIRE_TRY(silu_layer<T>(c, FLM, H, B1, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
+                c.P.jsq, TC_UPD1, SLW_UPD1));
+  FIRE_TRY(silu_layer<T>(c, FLM, B1, B2, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, G, Jcap, Jdev, c.L.pos_ctr, 3, c.P.Zx,
+                c.P.jsq, TC_UPD2, SLW_UPD2));
   return cudaPeekAtLastError();
 }
 
 // value path for one chunk: writes logpsi/sign via the assembly (indices w0 + w)
 template <typename T>
-cudaError_t chunk_logpsi(Ctx<T>& c, void* logpsi, void* sign, int w0_out) {
+[[nodiscard]] cudaError_t chunk_logpsi(Ctx<T>& c, void* logpsi, void* sign, int w0_out) {
   setup_ctx(c, false);
-  stage_neighbors(c, false);
-  stage_embedding<T, 0>(c);
-  stage_update<T, 0>(c);
-  stage_orbitals<T, 0>(c);
+  FIRE_TRY(stage_neighbors(c, false));
+  FIRE_TRY(stage_embedding<T, 0>(c));
+  FIRE_TRY(stage_update<T, 0>(c));
+  FIRE_TRY(stage_orbitals<T, 0>(c));
   // slogdet only: double-FP32 LU in the FP32 and mixed paths (FP64-class, like the inverse of the local
   // energy), native FP64 in the FP64 build
   Prof pr_lu("lu", c.s);
   if constexpr (sizeof(T) == 8)
-    launch_gjg<double, T, T, false>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, (T*)nullptr);
+    FIRE_TRY(launch_gjg<double, T, T, false>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, (T*)nullptr));
   else
-    launch_gjg<df64, T, T, false>(c, c.template buf<T>(c.P.Apl), c.comp ? c.template buf<T>(c.P.Apl_lo) : nullptr,
-                                  (T*)nullptr);
-  stage_jastrow<T, 0>(c);
+    FIRE_TRY(launch_gjg<df64, T, T, false>(c, c.template buf<T>(c.P.Apl), c.comp ? c.template buf<T>(c.P.Apl_lo) : nullptr,
+                                  (T*)nullptr));
+  FIRE_TRY(stage_jastrow<T, 0>(c));
   AssembleOut o;
   std::memset(&o, 0, sizeof(o));
   g_nlaunch++;
@@ -1314,26 +1327,26 @@ struct SideStream {
 };
 
 template <typename T>
-cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fire_eloc_debug* dbg,
+[[nodiscard]] cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fire_eloc_debug* dbg,
                        const Refine& rf = Refine()) {
   setup_ctx(c, true);
-  stage_neighbors(c, true);
-  stage_embedding<T, 3>(c);
-  stage_update<T, 3>(c);
-  stage_orbitals<T, 3>(c);
+  FIRE_TRY(stage_neighbors(c, true));
+  FIRE_TRY(stage_embedding<T, 3>(c));
+  FIRE_TRY(stage_update<T, 3>(c));
+  FIRE_TRY(stage_orbitals<T, 3>(c));
   {
     // orbital-matrix inverse: native FP64 in the FP64 build, double-FP32 (48-bit significand) otherwise; the
     // refinement pass eliminates the FP64 orbital matrices of its walkers in FP64
     Prof pr("gauss_jordan", c.s);
     if constexpr (sizeof(T) == 8) {
-      launch_gjg<double, T, T, true>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, c.template buf<T>(c.P.Ainv));
+      FIRE_TRY(launch_gjg<double, T, T, true>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, c.template buf<T>(c.P.Ainv)));
     } else if (rf.refined) {
       if (rf.ready) cudaStreamWaitEvent(c.s, rf.ready, 0);
     } else {
       // the condition numbers of the orbital matrices feed the ill-conditioned test of the assembly
-      launch_gjg<df64, T, T, true>(c, c.template buf<T>(c.P.Apl), c.template buf<T>(c.P.Apl_lo),
+      FIRE_TRY(launch_gjg<df64, T, T, true>(c, c.template buf<T>(c.P.Apl), c.template buf<T>(c.P.Apl_lo),
                                    c.template buf<T>(c.P.Ainv),
-                                   rf.idx ? c.template buf<double>(c.P.cond) : nullptr);
+                                   rf.idx ? c.template buf<double>(c.P.cond) : nullptr));
     }
   }
   cudaMemsetAsync(c.template buf<double>(c.P.dlap), 0, sizeof(double) * c.Wc * NDET, c.s);
@@ -1362,7 +1375,7 @@ cudaError_t chunk_eloc(Ctx<T>& c, void* logpsi, void* sign, void* eloc, const fi
       if (n > DL_DSPLIT) go(k_detlap<T, 256, DL_DSPLIT, DL_CMAX>, 256, DL_CMAX, 0);
     }
   }
-  stage_jastrow<T, 3>(c);
+  FIRE_TRY(stage_jastrow<T, 3>(c));
   AssembleOut o;
   std::memset(&o, 0, sizeof(o));
   g_nlaunch++;
@@ -1470,7 +1483,7 @@ __global__ void k_refine_gather(const T* __restrict__ r, int n, const int32_t* _
 // walkers' rows.  The list is evaluated in passes of KC walkers (refine_chunk).  A pass's kernels leave the walkers beyond the device's count alone (Nbr::live); what a capacity above it
 // costs is their launches, grids that find nothing to do, and a few cleared sums.
 template <typename T>
-cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const float* R, const float* Z,
+[[nodiscard]] cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const float* R, const float* Z,
                         const void* prepared, const T* r, void* logpsi, void* sign, void* eloc,
                         const fire_eloc_debug* dbg, unsigned char* ws, int32_t* status, Refine rf) {
   const int KF = rf.cap, KC = refine_chunk(p, Wc), n = p->n_el;
@@ -1505,14 +1518,14 @@ cudaError_t refine_pass(const fire_problem* p, int Wc, cudaStream_t s, const flo
     c64.r = r64;
     c64.nb.live = sub_cnt + j;
     setup_ctx(c64, false);
-    stage_neighbors(c64, false);
-    stage_embedding<double, 0>(c64);
-    stage_update<double, 0>(c64);
-    stage_orbitals<double, 0>(c64);
+    FIRE_TRY(stage_neighbors(c64, false));
+    FIRE_TRY(stage_embedding<double, 0>(c64));
+    FIRE_TRY(stage_update<double, 0>(c64));
+    FIRE_TRY(stage_orbitals<double, 0>(c64));
     {
       Prof pr_gj("gauss_jordan", side.s);
-      launch_gjg<double, double, T, true>(c64, c64.template buf<double>(c64.P.Apl), (const double*)nullptr,
-                                          c.template buf<T>(c.P.Ainv));
+      FIRE_TRY(launch_gjg<double, double, T, true>(c64, c64.template buf<double>(c64.P.Apl), (const double*)nullptr,
+                                          c.template buf<T>(c.P.Ainv)));
       const size_t nb = sizeof(double) * (size_t)kc * NDET;
       cudaMemcpyAsync(c.template buf<double>(c.P.ld), c64.template buf<double>(c64.P.ld), nb, cudaMemcpyDeviceToDevice,
                       side.s);
@@ -1553,12 +1566,12 @@ fire_status run_eloc(const fire_problem* p, cudaStream_t s, const float* R, cons
     c.w0 = w0;
     c.Wc = std::min(Wc, p->n_walkers - w0);
     c.r = rr + (size_t)w0 * p->n_el * 3;
-    if (chunk_eloc<T>(c, logpsi, sign, eloc, dbg, rf) != cudaSuccess) return launch_status("local_energy chunk");
+    if (chunk_eloc<T>(c, logpsi, sign, eloc, dbg, rf) != cudaSuccess) return failed("local_energy chunk");
   }
   if constexpr (sizeof(T) == 4) {
     if (rf.cap > 0 && refine_pass<T>(p, Wc, s, R, Z, prepared, rr, logpsi, sign, eloc, dbg,
                                      reinterpret_cast<unsigned char*>(ws), status, rf) != cudaSuccess)
-      return launch_status("local_energy refinement");
+      return failed("local_energy refinement");
   }
   g_nlaunch++;
   if (stats) k_stats<T><<<1, 1024, 0, s>>>(reinterpret_cast<const T*>(eloc), p->n_walkers, stats);
@@ -1576,7 +1589,7 @@ fire_status run_logpsi(const fire_problem* p, cudaStream_t s, const float* R, co
     c.w0 = w0;
     c.Wc = std::min(Wc, p->n_walkers - w0);
     c.r = rr + (size_t)w0 * p->n_el * 3;
-    if (chunk_logpsi<T>(c, logpsi, sign, w0) != cudaSuccess) return launch_status("logpsi chunk");
+    if (chunk_logpsi<T>(c, logpsi, sign, w0) != cudaSuccess) return failed("logpsi chunk");
   }
   return FIRE_OK;
 }
@@ -1593,9 +1606,8 @@ fire_status run_embedding(const fire_problem* p, cudaStream_t s, const float* R,
     c.Wc = std::min(Wc, p->n_walkers - w0);
     c.r = rr + (size_t)w0 * p->n_el * 3;
     setup_ctx(c, false);
-    stage_neighbors(c, false);
-    stage_embedding<T, 0>(c);
-    stage_update<T, 0>(c);
+    if (stage_neighbors(c, false) != cudaSuccess || stage_embedding<T, 0>(c) != cudaSuccess) return failed("embedding");
+    if (stage_update<T, 0>(c) != cudaSuccess) return failed("embedding");
     const size_t cnt = (size_t)c.Wc * p->n_el * F;
     if (hc)
       cudaMemcpyAsync(reinterpret_cast<T*>(hc) + (size_t)w0 * p->n_el * F, c.template buf<T>(c.P.HX),
@@ -1650,7 +1662,7 @@ fire_status run_mcmc(const fire_problem* p, cudaStream_t s, const float* R, cons
                                                           st, (T)width, seed, counter,
                                                           reinterpret_cast<const T*>(noise));
       c.r = rn;
-      if (chunk_logpsi<T>(c, lpn, nullptr, 0) != cudaSuccess) return launch_status("mcmc chunk");
+      if (chunk_logpsi<T>(c, lpn, nullptr, 0) != cudaSuccess) return failed("mcmc chunk");
       g_nlaunch++;
       k_accept<T><<<c.Wc, 128, 0, s>>>(rr, rn, reinterpret_cast<T*>(logpsi), lpn, n, w0, p->n_walkers, st, seed,
                                       counter, reinterpret_cast<const T*>(logu), n_accept, c.nb.counts, static_max,
@@ -1741,45 +1753,45 @@ int choose_chunk_lr(const fire_problem* p, size_t ws_bytes, int KS) {
 // the attention readout MLP 512 -> 256 -> 256 -> 2 on the value rows RX [W][512] -> JAx [W][2] (the value
 // path's part of stage_jastrow)
 template <typename T>
-void readout_value(Ctx<T>& c) {
+[[nodiscard]] cudaError_t readout_value(Ctx<T>& c) {
   const int Wc = c.Wc;
-  auto layer = [&](size_t in, size_t out, const T* Wt, const T* b, int K) {
+  auto layer = [&](size_t in, size_t out, const T* Wt, const T* b, int K) -> cudaError_t {
     GemmP<T> q = gp0<T>();
     q.A = c.template buf<T>(in); q.lda = K; q.B = Wt; q.ldb = F; q.bias = b; q.C = c.template buf<T>(out);
     q.ldc = F; q.M = Wc; q.N = F; q.K = K; q.ld_aux = F;
-    gemm<T, EPI_SILU_X>(c, q);
+    return gemm<T, EPI_SILU_X>(c, q);
   };
-  layer(c.P.RX, c.P.R1X, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F);
-  layer(c.P.R1X, c.P.R2X, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F);
+  FIRE_TRY(layer(c.P.RX, c.P.R1X, c.W.w[FIRE_P_ATT_OUT1_W], c.W.w[FIRE_P_ATT_OUT1_B], 2 * F));
+  FIRE_TRY(layer(c.P.R1X, c.P.R2X, c.W.w[FIRE_P_ATT_OUT2_W], c.W.w[FIRE_P_ATT_OUT2_B], F));
   GemmP<T> g = gp0<T>();
   g.A = c.template buf<T>(c.P.R2X); g.lda = F; g.B = c.W.w[FIRE_P_ATT_OUT3_W]; g.ldb = 2;
   g.bias = c.W.w[FIRE_P_ATT_OUT3_B]; g.bias_period = 1; g.C = c.template buf<T>(c.P.JAx); g.ldc = 2; g.M = Wc;
   g.N = 2; g.K = F;
-  gemm<T, EPI_PLAIN>(c, g);
+  return gemm<T, EPI_PLAIN>(c, g);
 }
 
 // State of one chunk: the value path with the inverse kept (Gauss-Jordan instead of the LU), the attention value
 // rows, and log|psi| (and its sign, if sign is not null) of the chunk's walkers into logpsi[w0_out + w]
 // (log_psi_with_state, wave_function.py:226-247).
 template <typename T>
-cudaError_t chunk_state(Ctx<T>& c, const LrPlan& Q, void* logpsi, void* sign, int w0_out) {
+[[nodiscard]] cudaError_t chunk_state(Ctx<T>& c, const LrPlan& Q, void* logpsi, void* sign, int w0_out) {
   setup_ctx(c, false);
-  stage_neighbors(c, false);
-  stage_embedding<T, 0>(c);
-  stage_update<T, 0>(c);
-  stage_orbitals<T, 0>(c);
+  FIRE_TRY(stage_neighbors(c, false));
+  FIRE_TRY(stage_embedding<T, 0>(c));
+  FIRE_TRY(stage_update<T, 0>(c));
+  FIRE_TRY(stage_orbitals<T, 0>(c));
   {
     Prof pr("gauss_jordan", c.s);
     if constexpr (sizeof(T) == 8)
-      launch_gjg<double, T, T, true>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, c.template buf<T>(Q.B));
+      FIRE_TRY(launch_gjg<double, T, T, true>(c, c.template buf<T>(c.P.Apl), (const T*)nullptr, c.template buf<T>(Q.B)));
     else
-      launch_gjg<df64, T, T, true>(c, c.template buf<T>(c.P.Apl),
-                                   c.comp ? c.template buf<T>(c.P.Apl_lo) : nullptr, c.template buf<T>(Q.B));
+      FIRE_TRY(launch_gjg<df64, T, T, true>(c, c.template buf<T>(c.P.Apl),
+                                   c.comp ? c.template buf<T>(c.P.Apl_lo) : nullptr, c.template buf<T>(Q.B)));
   }
-  stage_jastrow<T, 0>(c);
+  FIRE_TRY(stage_jastrow<T, 0>(c));
   const Planes B2{c.P.B2X, 0, 0}, VL{Q.vals, 0, 0};
-  linear_layer<T>(c, false, B2, VL, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, c.Wc * c.p->n_el, 0, nullptr,
-                  -1, SLW_V);
+  FIRE_TRY(linear_layer<T>(c, false, B2, VL, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, c.Wc * c.p->n_el, 0, nullptr,
+                  -1, SLW_V));
   AssembleOut o;
   std::memset(&o, 0, sizeof(o));
   o.logpsi = logpsi;
@@ -1796,7 +1808,7 @@ cudaError_t chunk_state(Ctx<T>& c, const LrPlan& Q, void* logpsi, void* sign, in
 // moved the electrons moved[w][0..KM) (the plan's moved buffer, padded with FIRE_NO_NEIGHBOUR), from the state; the
 // proposal's rows stay in the plan's scratch for the commit.
 template <typename T>
-cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32_t* static_max, T* sgn_out,
+[[nodiscard]] cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32_t* static_max, T* sgn_out,
                         int mover_spin = -1) {
   const fire_problem* p = c.p;
   const int n = p->n_el, nu = p->n_up, N = p->n_nuc, Wc = c.Wc, DN = NDET * n, rows = Wc * KS;
@@ -1826,19 +1838,19 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
     GemmP<T> g = gp0<T>();
     g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_GLU_W]; g.ldb = 2 * F; g.C = Z1; g.ldc = 2 * F;
     g.M = ME; g.N = 2 * F; g.K = F;
-    gemm<T, EPI_PLAIN>(c, g);
+    FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
     g_nlaunch++;
     k_glu<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, E5a, ME, 1, nullptr);
     g = gp0<T>();
     g.A = E5a; g.lda = F; g.B = c.W.w[FIRE_P_EI_DENSE_W]; g.ldb = F; g.C = Z1; g.ldc = F;
     g.bias = c.W.w[FIRE_P_EI_DENSE_B]; g.bias_period = 1; g.M = ME; g.N = F; g.K = F;
-    gemm<T, EPI_PLAIN>(c, g);
+    FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
     g_nlaunch++;
     k_silu5<T, 0><<<nblk((long)ME * F), 256, 0, s>>>(Z1, ME, 1, nullptr);
     g = gp0<T>();
     g.A = Z1; g.lda = F; g.B = c.W.w[FIRE_P_EI_OUT_W]; g.ldb = 5 * F; g.C = c.template buf<T>(Q.E5p);
     g.ldc = 5 * F; g.bias = c.W.w[FIRE_P_EI_OUT_B]; g.bias_period = 1; g.M = ME; g.N = 5 * F; g.K = F;
-    gemm<T, EPI_PLAIN>(c, g);
+    FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
   }
   // messages and update MLP of the changed centers
   g_nlaunch++;
@@ -1846,17 +1858,17 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
                                                 c.template buf<T>(c.P.E5o), c.template buf<T>(Q.E5p),
                                                 c.template buf<T>(Q.HS));
   const Planes HS{Q.HS, 0, 0}, B1S{Q.B1S, 0, 0}, hS{Q.hS, 0, 0};
-  silu_layer<T>(c, false, HS, B1S, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
-                0, -1, SLW_UPD1);
-  silu_layer<T>(c, false, B1S, hS, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
-                0, -1, SLW_UPD2);
+  FIRE_TRY(silu_layer<T>(c, false, HS, B1S, c.W.w[PR_UPD1_W_S0], c.W.w[FIRE_P_UPD1_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
+                0, -1, SLW_UPD1));
+  FIRE_TRY(silu_layer<T>(c, false, B1S, hS, c.W.w[FIRE_P_UPD2_W], c.W.w[FIRE_P_UPD2_B], F, F, rows, 0, nullptr, nullptr, 1, 0,
+                0, -1, SLW_UPD2));
   // raw orbital rows of the changed centers (both spins' contractions, then each row's own)
   for (int sp = 0; sp < 2; ++sp) {
     GemmP<T> g = gp0<T>();
     g.A = c.template buf<T>(Q.hS); g.lda = F; g.B = c.W.w[sp == 0 ? PR_ORB_UP_W_S1 : PR_ORB_DN_W_S1]; g.ldb = DN;
     g.bias = c.W.w[sp == 0 ? FIRE_P_ORB_UP_B : FIRE_P_ORB_DN_B]; g.bias_period = 1;
     g.C = c.template buf<T>(sp == 0 ? Q.rawU : Q.rawD); g.ldc = DN; g.M = rows; g.N = DN; g.K = F;
-    gemm<T, EPI_PLAIN>(c, g);
+    FIRE_TRY(gemm<T, EPI_PLAIN>(c, g));
   }
   g_nlaunch++;
   k_lr_orb<T><<<dim3(KS, Wc), 256, 0, s>>>(S, S_cnt, KS, nu, DN, c.template buf<T>(Q.rawU),
@@ -1878,7 +1890,7 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
         g.B = c.W.w[mover_spin == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (size_t)d * K8 * n; g.ldb = n;
         g.C = c.template buf<T>(Q.env_p) + (size_t)d * n; g.ldc = DN; g.M = ME; g.N = n;
         g.K = K8; g.n_el = 1; g.env_ns = 1; g.env_soff = 0; g.env_nv = 1;
-        gemm<T, EPI_ENV>(c, g);
+        FIRE_TRY(gemm<T, EPI_ENV>(c, g));
       }
     } else {
     for (int sp = 0; sp < 2; ++sp)
@@ -1888,7 +1900,7 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
         g.B = c.W.w[sp == 0 ? PR_ENV_UP_PI : PR_ENV_DN_PI] + (size_t)d * K8 * n; g.ldb = n;
         g.C = c.template buf<T>(sp == 0 ? Q.env_p : Q.env_pD) + (size_t)d * n; g.ldc = DN; g.M = ME; g.N = n;
         g.K = K8; g.n_el = 1; g.env_ns = 1; g.env_soff = 0; g.env_nv = 1;
-        gemm<T, EPI_ENV>(c, g);
+        FIRE_TRY(gemm<T, EPI_ENV>(c, g));
       }
     g_nlaunch++;
     k_lr_env_add<T><<<nblk((long)ME * DN), 256, 0, s>>>((long)ME * DN, c.template buf<T>(Q.env_p),
@@ -1914,11 +1926,11 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
                                                       c.template buf<T>(Q.aS), nullptr, nullptr, c.status, nullptr,
                                                       nullptr);
     const Planes vS{Q.vS, 0, 0};
-    linear_layer<T>(c, false, hS, vS, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, rows, 0, nullptr, -1, SLW_V);
-    silu_layer<T>(c, false, hS, HS, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, rows, 0, nullptr, nullptr, 1,
-                  0, 0, -1, SLW_JMLP1);
-    silu_layer<T>(c, false, HS, B1S, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, rows, 0, nullptr, nullptr,
-                  1, 0, 0, -1, SLW_JMLP2);
+    FIRE_TRY(linear_layer<T>(c, false, hS, vS, c.W.w[PR_V_W_S1], c.W.w[FIRE_P_ATT_V_B], F, F, rows, 0, nullptr, -1, SLW_V));
+    FIRE_TRY(silu_layer<T>(c, false, hS, HS, c.W.w[PR_JMLP1_W_S1], c.W.w[FIRE_P_JMLP1_B], F, F, rows, 0, nullptr, nullptr, 1,
+                  0, 0, -1, SLW_JMLP1));
+    FIRE_TRY(silu_layer<T>(c, false, HS, B1S, c.W.w[FIRE_P_JMLP2_W], c.W.w[FIRE_P_JMLP2_B], F, F, rows, 0, nullptr, nullptr,
+                  1, 0, 0, -1, SLW_JMLP2));
     g_nlaunch++;
     k_narrow<T, 2, 0, false><<<rows, 256, 0, s>>>(c.template buf<T>(Q.B1S), nullptr, nullptr, c.nb, c.L,
                                                   c.W.w[FIRE_P_JMLP3_W], c.W.w[FIRE_P_JMLP3_B],
@@ -1932,7 +1944,7 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
     g_nlaunch++;
     k_readout_in<T, false><<<Wc, 512, 0, s>>>(n, c.template buf<T>(c.P.Ax), nullptr, nullptr,
                                               c.template buf<T>(c.P.RX), nullptr, nullptr, nullptr);
-    readout_value<T>(c);
+    FIRE_TRY(readout_value<T>(c));
   }
   // log|psi'| and the Metropolis test
   AssembleOut o;
@@ -1951,7 +1963,7 @@ cudaError_t lr_evaluate(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, int32
 // state, the Metropolis test with the proposals' log ratios plr (may be null), and on acceptance the state's rows and
 // the Woodbury update of the inverse.
 template <typename T>
-cudaError_t lr_step(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, void* logpsi, int st, uint64_t seed,
+[[nodiscard]] cudaError_t lr_step(Ctx<T>& c, const LrPlan& Q, int KS, int KM, T* rr, void* logpsi, int st, uint64_t seed,
                     uint64_t counter, const void* logu, int32_t* n_accept, int32_t* static_max, const T* plr,
                     int mover_spin = -1) {
   const fire_problem* p = c.p;
@@ -2046,7 +2058,7 @@ fire_status run_ecp(const fire_problem* p, cudaStream_t s, const float* R, const
     T* sgn0 = c.template buf<T>(Q.sgn0);
     double* acc = c.template buf<double>(Q.ecp_acc);
     double* pt = c.template buf<double>(Q.ecp_pt);
-    if (chunk_state<T>(c, Q, lp0, sgn0, 0) != cudaSuccess) return launch_status("pseudopotential state");
+    if (chunk_state<T>(c, Q, lp0, sgn0, 0) != cudaSuccess) return failed("pseudopotential state");
     g_nlaunch++;
     k_ecp_local<T><<<c.Wc, 256, 0, s>>>(c.r, n, R, ecp, acc);
     for (int e = 0; e < n; ++e)
@@ -2055,7 +2067,7 @@ fire_status run_ecp(const fire_problem* p, cudaStream_t s, const float* R, const
         k_ecp_point<T><<<c.Wc, 128, 0, s>>>(c.r, c.template buf<T>(c.P.rn), n, e, k, R, ecp, qt, w0, seed, counter,
                                             reinterpret_cast<const T*>(rot), pt, c.template buf<int>(Q.moved));
         if (lr_evaluate<T>(c, Q, KS, 1, rr, static_max, c.template buf<T>(Q.sgn_p)) != cudaSuccess)
-          return launch_status("pseudopotential ratio");
+          return failed("pseudopotential ratio");
         g_nlaunch++;
         k_ecp_accum<T><<<nblk(c.Wc), 256, 0, s>>>(c.Wc, pt, c.template buf<T>(c.P.lpn), c.template buf<T>(Q.sgn_p),
                                                   lp0, sgn0, ecp, acc);
@@ -2090,7 +2102,7 @@ fire_status run_mcmc_lr(const fire_problem* p, cudaStream_t s, const float* R, c
     c.w0 = w0;
     c.Wc = std::min(Wc, p->n_walkers - w0);
     c.r = rr + (size_t)w0 * n * 3;
-    if (chunk_state<T>(c, Q, logpsi, nullptr, w0) != cudaSuccess) return launch_status("low-rank state");
+    if (chunk_state<T>(c, Q, logpsi, nullptr, w0) != cudaSuccess) return failed("low-rank state");
     int* moved = c.template buf<int>(Q.moved);
     T* plr = (kind == MC_JUMP || kind == MC_CLUSTER) ? c.template buf<T>(c.P.plr) : nullptr;
     const int KM = kind == MC_CLUSTER ? ck : 1;
@@ -2113,7 +2125,7 @@ fire_status run_mcmc_lr(const fire_problem* p, cudaStream_t s, const float* R, c
       const int mover_spin = mover < 0 ? -1 : (mover < p->n_up ? 0 : 1);
       if (lr_step<T>(c, Q, KS, KM, rr, logpsi, st, seed, counter, logu, n_accept, static_max, plr, mover_spin) !=
           cudaSuccess)
-        return launch_status("low-rank step");
+        return failed("low-rank step");
     }
   }
   return launch_status(__func__);
@@ -2564,7 +2576,7 @@ fire_status fire_profile_report(char* buf, size_t len) {
   if (!buf || len == 0) return FIRE_ERR_INVALID;
   std::vector<std::pair<const char*, std::pair<int, double>>> acc;
   for (auto& r : g_recs) {
-    if (cudaEventSynchronize(r.b) != cudaSuccess) return launch_status("profile");
+    if (cudaEventSynchronize(r.b) != cudaSuccess) return failed("profile");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, r.a, r.b);
     bool found = false;

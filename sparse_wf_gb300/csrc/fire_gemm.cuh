@@ -453,6 +453,8 @@ inline cudaError_t launch_gemm_d(const GemmP<double>& p, cudaStream_t s) {
   return cudaPeekAtLastError();
 }
 
+// modes that the FP64 contraction on the CUDA cores is built for
+constexpr bool gemm_d_mode(int mode) { return mode == EPI_PLAIN || mode == EPI_SILU_X || mode == EPI_ORB_X || mode == EPI_ENV; }
 template <typename T, int MODE, bool BT = false>
 inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
   if constexpr (sizeof(T) == 4) {
@@ -463,10 +465,9 @@ inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
     if (tiles(128) >= 1200) return launch_gemm_f<MODE, 128, BT>(p, s);
     if (tiles(64) >= 1600) return launch_gemm_f<MODE, 64, BT>(p, s);
     return launch_gemm_f<MODE, 32, BT>(p, s);
-  } else if constexpr (MODE == EPI_PLAIN || MODE == EPI_SILU_X || MODE == EPI_ORB_X || MODE == EPI_ENV) {
-    return launch_gemm_d<MODE>(p, s);
   } else {
-    return cudaErrorInvalidValue;  // FP64 derivative rows: the sliced contraction
+    static_assert(gemm_d_mode(MODE), "FP64 derivative rows: the sliced contraction");
+    return launch_gemm_d<MODE>(p, s);
   }
 }
 
