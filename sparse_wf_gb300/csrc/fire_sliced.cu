@@ -305,15 +305,15 @@ __device__ __forceinline__ double sl_assemble(long long h, uint32_t l, int e) {
   const int lz = __clz(x);
   x = __funnelshift_l(y, x, lz);
   y = __funnelshift_l(z, y, lz);
-  unsigned long long m = ((unsigned long long)x << 32) | y;  // bit 63 set; value = m 2^ex
-  const int ex = e + 32 - up - lz;
-  m = (m >> 11) + ((m >> 10) & 1);  // 53 bits (2^53 carries into the exponent below)
-  const int field = ex + 11 + 1075;
-  const long long sgn = neg & (long long)0x8000000000000000ull;
-  if (field > 0 && field < 2046)
-    return __longlong_as_double(sgn | (long long)(((unsigned long long)(field - 1) << 52) + m));
-  const double r = ldexp((double)m, ex + 11);
-  return neg ? -r : r;
+  const unsigned long long m = ((unsigned long long)x << 32) | y;  // bit 63 set
+  const int field = e + 32 - up - lz + 1086;  // the exponent's field; in a denormal more than 11 bits are rounded away
+  const int drop = field > 0 ? 11 : 12 - field;
+  unsigned long long q = 0;
+  if (drop < 64) q = m >> drop;
+  if (drop <= 64) q += (m >> (drop - 1)) & 1;
+  if (field > 0) q += (unsigned long long)(field - 1) << 52;  // a carry to 2^53 goes into the exponent
+  if (field > 2046) q = 0x7ff0000000000000ull;
+  return __longlong_as_double((neg & (long long)0x8000000000000000ull) | (long long)q);
 }
 
 // 2^(e - 6), the scale of a row or column of SL_PAIR
