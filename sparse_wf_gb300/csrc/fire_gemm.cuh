@@ -137,12 +137,16 @@ struct FgCfg {
   static constexpr int STAGE = BM * FGA + (BT ? BN * FGA : FGK * BN);  // floats
   static constexpr int SQ = BM * (BN + 1);
   static constexpr size_t smem(bool sq) { return sizeof(float) * (sq && SQ > FGS * STAGE ? SQ : FGS * STAGE); }
+  // CTAs per SM that the registers are shared out for: what 228 KB of shared memory (1 KB of each CTA's reserved) hold, and no
+  // more than 6 (a bound of 7 for the 64 x 64 tile, of which 6 fit, kept it at 128 registers and made it spill)
+  static constexpr int FIT = 228 * 1024 / (int)(smem(false) + 1024 + sizeof(int) * BM);
+  static constexpr int CTAS = BM == 128 ? 2 : (FIT < 6 ? FIT : 6);
 };
 
 // BT: B is the transpose of p.B [N, K] (p.ldb); its tile is kept like A's, k contiguous, and a thread's columns lie TX apart
 // so that their rows are read without bank conflicts.
 template <int MODE, int BM, bool BT = false>
-__global__ void __launch_bounds__(FgCfg<BM>::THREADS, BM == 128 ? 2 : (BM == 64 ? 7 : 6)) k_gemm_f(GemmP<float> p) {
+__global__ void __launch_bounds__(FgCfg<BM, BT>::THREADS, FgCfg<BM, BT>::CTAS) k_gemm_f(GemmP<float> p) {
   using Cf = FgCfg<BM, BT>;
   constexpr int BN = Cf::BN, TM = Cf::TM, NT = Cf::THREADS, H = BM / 2;  // H: rows (columns) between a thread's two halves
   constexpr int TX = BN / TM, FGK = Cf::FGK, FGA = Cf::FGA;
