@@ -926,7 +926,9 @@ __global__ void __launch_bounds__(256) gk_att_bwd(Weights<T> W, const T* __restr
     const T nm = nrm[((long)w * 2 + s) * HEADS + h];
     const T dXv = dX[(long)w * 2 * F + s * F + f];
     const T dV = dXv / nm;
-    T dn = -dXv * Vs[((long)w * 2 + s) * F + f] / (nm * nm);
+    const T Vf = Vs[((long)w * 2 + s) * F + f];
+    // FP32: the square of a norm beyond 10^+-15 leaves the range
+    T dn = sizeof(T) == 4 && !(nm > T(1e-15) && nm < T(1e15)) ? -dV * (Vf / nm) : -dXv * Vf / (nm * nm);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) dn += __shfl_xor_sync(0xffffffffu, dn, o);
     for (int k = 0; k < ns; ++k) {

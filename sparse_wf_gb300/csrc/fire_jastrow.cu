@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(256) k_att_sums(Nbr nb, Layout L, const T* __r
   }
 }
 
-// Readout input x = values / normalizer, flattened [2][16][16] -> 512 (jastrow.py:98).
+// Readout input x = values / normalizer, flattened [2][16][16] -> 512 (jastrow.py:98).  FP32: with a norm beyond 10^+-8
+// (attention logits of 20 and more) its square and cube, which the products below reach before they are divided, leave the
+// range; the quotients are then formed first.
 // Planes RX [W][512], RJ [W * 3n][512], RL [W][512].  One CTA (512 threads) per walker.
 template <typename T, bool FLM>
 __global__ void __launch_bounds__(512) k_readout_in(int n, const T* __restrict__ Ax, const T* __restrict__ Al,
@@ -263,6 +265,18 @@ __global__ void __launch_bounds__(512) k_readout_in(int n, const T* __restrict__
   const T* al = Al + ((size_t)w * 2 + s) * 272;
   T nj2 = T(0), vn = T(0);
   const int T3 = 3 * n;
+  if (sizeof(T) == 4 && !(N > T(1e-8) && N < T(1e8))) {
+    const T x = V * iN;
+    for (int tt = 0; tt < T3; ++tt) {
+      const T* a = AJ + (((size_t)w * T3 + tt) * 2 + s) * 272;
+      const T u = a[256 + r] * iN, v = a[rd] * iN;
+      nj2 += u * u;
+      vn += v * u;
+      RJ[((size_t)w * T3 + tt) * 512 + slot] = v - x * u;
+    }
+    RL[(size_t)w * 512 + slot] = al[rd] * iN - x * (al[256 + r] * iN) + T(2) * x * nj2 - T(2) * vn;
+    return;
+  }
   for (int tt = 0; tt < T3; ++tt) {
     const T* a = AJ + (((size_t)w * T3 + tt) * 2 + s) * 272;
     const T Nj = a[256 + r], Vj = a[rd];
