@@ -77,7 +77,9 @@ typedef enum {
                           hi x hi sums exact in one FP32 accumulator, the three other products in a second, four
                           MMAs per product; ~2^-20 of a row's largest value per element), K > 256 (the envelope rows) in split BF16 (three products per
                           FP32 product); value planes, orbital LU and inverse as in FIRE_PREC_FP32 */
-  FIRE_PREC_FP64 = 2   /* everything in FP64 (validation build of the same kernels) */
+  FIRE_PREC_FP64 = 2   /* everything in FP64 (validation build of the same kernels); dense layers as error-free
+                          slices on the tensor cores, whose error is bounded by 2^-58 K times the largest
+                          magnitudes of the row and the column and 2^-53 of the result */
 } fire_precision;
 
 typedef struct {
@@ -90,7 +92,8 @@ typedef struct {
   int32_t cap_pairs;     /* capacity: directed e-e pairs per walker (same + diff) */
   int32_t cap_nuc;       /* capacity: e-n neighbours per electron */
   int32_t precision;     /* fire_precision */
-  int32_t chunk_walkers; /* walkers per internal pass; 0 = choose from the workspace */
+  int32_t chunk_walkers; /* walkers per internal pass; 0 = choose from the workspace (the local energy takes fewer where
+                            the eliminations of the batch then take fewer rounds) */
   int32_t refine_cap;    /* FP32 / mixed fire_local_energy: at most this many ill-conditioned walkers per call are
                             evaluated again with FP64 orbital-matrix values (see fire_local_energy); 0 = none */
   float refine_ratio;    /* a walker is ill-conditioned when (|lap| + |grad|^2) / 2 > refine_ratio |E_loc|
@@ -242,7 +245,9 @@ typedef struct {
  * the values of the embedding, orbitals, envelopes and orbital matrices, their LU and inverse in FP64 (the
  * derivative planes on the FP32 CUDA cores), and their results replace the first ones.  status[5] reports how
  * many walkers were ill-conditioned; more than refine_cap sets FIRE_FLAG_REFINE_OVERFLOW (the others keep their
- * first results).  The workspace must then hold the refinement pass as well (fire_workspace_size does). */
+ * first results).  The workspace must then hold the refinement pass as well (fire_workspace_size does).  Unless
+ * stream is being captured, part of that pass runs on a stream that the call makes and releases; it starts after
+ * and joins stream, so that the results and the buffers follow stream as in every other call. */
 fire_status fire_local_energy(void* stream, const fire_problem* prob, const float* R, const float* Z,
                               const void* prepared, const void* r, void* logpsi, void* sign,
                               void* e_loc, double* e_stats, const fire_eloc_debug* debug,

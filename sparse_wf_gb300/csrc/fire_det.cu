@@ -139,7 +139,7 @@ constexpr int GJG_BW = 16, GJG_THREADS = 512;
 // A: element (i, o) of matrix (w, d) at A[((w * n + i) * NDET + d) * n + o]  (the orbital plane [G][D * n]);
 // A_lo (double-FP32 elimination only, may be null): the low parts of the same elements.
 // The block has 32 to 512 threads (launch_gjg): n steps with three barriers each leave a small matrix waiting, so small
-// matrices take small blocks and more of them share an SM.  The double-FP32 update packs two columns (SubDot2: 12 packed
+// matrices take small blocks and more of them share an SM.  The double-FP32 update packs two columns (PairDot: 12 packed
 // operations for two products; it is bound by their issue rate).  LU of 1024 matrices of 82: 1.53 ms with 512 threads each,
 // the logarithm of every pivot inside its step and scalar arithmetic.
 // Outputs: logdet[w * NDET + d], sign[...] (double); if INV the inverse, transposed and aligned for

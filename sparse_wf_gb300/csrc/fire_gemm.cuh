@@ -1,8 +1,9 @@
 // fire_gemm.cuh -- CUDA-core GEMM C = A[M,K] * B[K,N] with fused forward-Laplacian epilogues.
 //
 // k_gemm_f: FP32 (derivative planes of the FP32 path, plain value rows, gradients); k_gemm_d: FP64 (the refinement's values,
-// narrow layers; fire_sliced.cu has the FP64 build's wide ones); k_gemm_comp: the FP32 local energy's compensated value
-// rows; k_gemm_env_df: the refinement's envelope rows.  Every dense layer of the sparse forward Laplacian (sparse_fwd_lap.py:160-225) is applied to three "planes" of one node:
+// narrow layers and envelopes; fire_sliced.cu has the FP64 build's wide layers); k_gemm_comp: the FP32 local energy's
+// compensated value rows and every hi + lo envelope row; k_gemm_env_df: the refinement's envelope rows.  Every dense layer of
+// the sparse forward Laplacian (sparse_fwd_lap.py:160-225) is applied to three "planes" of one node:
 //   X plane  [nodes, K]        values            (bias added)
 //   J plane  [3 * positions, K] Jacobian rows    (sorted by center)
 //   L plane  [nodes, K]        Laplacians
@@ -126,8 +127,9 @@ __device__ __forceinline__ void cp_async_left() {  // at most N groups of this t
 // FP32 contraction on the CUDA cores: 128 x 128 (256 threads, 8 x 8 outputs each), 64 x 64 (64 threads, 8 x 8) or 32 x 32 (64
 // threads, 4 x 4) outputs per CTA, FGK k per stage, copied asynchronously FGS - 1 stages ahead.  Every output is one chain of fused
 // multiply-adds over ascending k, whatever the tile: all tiles and the scalar kernel before them give the same bits.  Bound by
-// the packed FMA rate (large tiles: 45 TFLOP/s) or, with few rows, by the chain of stages: a small tile then puts more SMs to
-// work.
+// the FMA pipes (128 and 64: 60 to 63 % busy, their latency between few warps the rest; 41 to 45 TFLOP/s), the 32 x 32 tile by
+// shared-memory loads (76 % of their rate, FMA pipes 57 %) or, with few rows, by the chain of stages: a small tile then puts
+// more SMs to work.
 constexpr int FGS = 4;
 template <int BM, bool BT = false>
 struct FgCfg {
@@ -346,8 +348,8 @@ inline cudaError_t launch_gemm_f(const GemmP<float>& p, cudaStream_t s) {
   return cudaPeekAtLastError();
 }
 
-// FP64 contraction on the CUDA cores (the refinement pass, the low-rank blocks, narrow layers): every output one chain of fused
-// multiply-adds over ascending k.  Bound by the FP64 pipe, which GB300 has at 1/64 of the FP32 rate: 128 x 128 outputs per CTA
+// FP64 contraction on the CUDA cores (the refinement pass, the low-rank blocks, narrow layers, envelopes): every output one chain
+// of fused multiply-adds over ascending k.  Bound by the FP64 pipe (97 % busy), which GB300 has at 1/64 of the FP32 rate: 128 x 128 outputs per CTA
 // at K = N = 256 kept an SM for 1.05 ms while the others idled.  16 x 16 outputs per CTA, 2 x 2 per thread: small enough that
 // any row count loads the SMs evenly, and two warps per CTA hide the chain.  At K = N = 256 with 160 / 600 / 2050 / 16400 rows
 // 48 / 110 / 271 / 1751 us (the pipe alone: 18 / 68 / 233 / 1861 at 1.9 GHz); 32 x 32 with 2 x 2 per thread 72 / 135 / 265 /
@@ -477,8 +479,9 @@ inline cudaError_t launch_gemm(const GemmP<T>& p, cudaStream_t s) {
 
 // ----------------------------------------------------------------------------- hi + lo value rows
 // FP32 and mixed paths: the value planes (one row per node) feed the orbital matrices, whose inverse amplifies
-// their rounding by the condition number in the derivatives of log det.  Their contractions (fire_sliced.cuh) give each
-// dot product as a hi + lo float pair, as if summed in twice the working precision; the orbital-matrix values and the
+// their rounding by the condition number in the derivatives of log det.  Their contractions (k_gemm_comp below; for the dense
+// layers of log|psi| alone k_gemm_sl, fire_sliced.cuh) give each dot product as a hi + lo float pair, as if summed in twice
+// the working precision; the orbital-matrix values and the
 // envelope values they are made of also leave as unevaluated pairs, so that the double-FP32 elimination sees them to
 // ~2^-48.
 //   COMP_PLAIN  C = a.b + bias (bias on rows with row % bias_period == 0)

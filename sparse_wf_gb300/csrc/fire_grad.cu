@@ -1509,7 +1509,7 @@ void mm(cudaStream_t s, long M, int N, int K, const T* A, long lda, const T* B, 
   if (M <= 0 || N <= 0) return;
   if constexpr (sizeof(T) == 4) {
     const bool al = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) == 0;
-    // few columns, rows enough to fill the SMs' warps twice (608 CTAs of 8 warps, 4 rows each); below that the 32 x 32 tiles
+    // few columns, rows enough to fill the SMs' warps twice (608 = 4 x 152 CTAs of 8 warps, 4 rows each); below that the 32 x 32 tiles
     // of k_gemm_f take 12 us at any row count
     if (BT && N <= 8 && K <= MMN_K && M >= 4096 && !bias && !acc && K % 4 == 0 && lda % 4 == 0 && al) {
       gk_mm_narrow<<<(unsigned)std::min<long>((M + 31) / 32, 608), 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);

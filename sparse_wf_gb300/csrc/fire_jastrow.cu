@@ -32,7 +32,6 @@ __device__ __forceinline__ void act3(T z, T& f, T& f1, T& f2) {
   }
 }
 
-// FLM: forward-Laplacian mode (X, J, L planes) or value mode (X only).
 // warp_sum of NC values (a power of two) at once: in every exchange a lane keeps half of the values it still holds, so that
 // NC + log2(32 / NC) - 1 shuffles do the work of 5 NC; the same pairs are added as in warp_sum.  Lane l returns value
 // l / (32 / NC).
@@ -54,6 +53,7 @@ __device__ __forceinline__ T warp_sums(T (&v)[NC], int lane) {
   return v[0];
 }
 
+// FLM: forward-Laplacian mode (X, J, L planes) or value mode (X only).
 template <typename T, int NC, int ACT, bool FLM>
 __global__ void __launch_bounds__(256) k_narrow(const T* __restrict__ X, const T* __restrict__ Jp,
                                                 const T* __restrict__ Lp, Nbr nb, Layout L, const T* __restrict__ Wn,

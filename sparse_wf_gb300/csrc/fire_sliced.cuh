@@ -85,6 +85,7 @@ inline size_t sl_a_bytes(long M, int K) {  // slices of M rows (whole 128-row ti
   return (size_t)sl_rows(M) * ((K + 15) / 16) * 32 * SlFmt<KIND>::NS;
 }
 // Row tiles of one pass over all segments: one per SM, as many whole tiles as that leaves to each of the `segs` segments.
+// (SL_SMS is GB300's count: the scratch is sized with it, so that another count only leaves a pass less even.)
 constexpr int SL_SMS = 152;
 inline long sl_pass_rows(long M, int segs) {
   return std::min<long>(sl_rows(M), 128 * std::max<long>(1, SL_SMS / segs));

@@ -697,10 +697,12 @@ __global__ void __launch_bounds__(TCP_THREADS, 1) k_gemm_tcs(GemmP<float> p, con
 // converters read a row tile twice, once ahead of time for the magnitudes (after a bulk prefetch into L2) and once, a
 // block ahead of the MMAs, to split.  The first version copied raw rows into the A ring, waited for all of the tile and
 // split in place: its four converter warps kept the chain of load, maximum, barrier and split serial.  What bounds it now:
-// the operands the MMAs read fill the shared memory's bandwidth (8 KB per 64 cycles), which the epilogue's staging shares;
-// without the epilogue 922500 x 256 x 256 takes 400 us (HBM alone: 278).  Before / after, with the plain epilogue 720 / 505
-// us, with the silu epilogue and its per-center sums 780 / 710, with the orbital one (N = 328) 1120 / 917.  Slower or no
-// gain: 16 epilogue and 4 converter warps (764, 944, 1097), weight stages of half the depth (510, 709, 936).
+// no unit alone.  The tensor pipe is 30 (silu sums) to 43 % (plain) busy, the shared-memory pipe of the converters and the
+// epilogue 63 to 39 %, on top of the operands that the MMAs read there (8 KB per 64 cycles); DRAM 34 % at most; the 18 warps
+// wait for loads in turn.  Without the epilogue 922500 x 256 x 256 takes 400 us, the MMAs alone 315 (HBM alone: 278).  Before /
+// after, with the plain epilogue 720 / 505 us, with the silu epilogue and its per-center sums 780 / 710, with the orbital one
+// (N = 328) 1120 / 917.  Slower or no gain: 16 epilogue and 4 converter warps (764, 944, 1097), weight stages of half the
+// depth (510, 709, 936).
 // Splitting: every row of A (and, at preparation, every column of the weights) is scaled and split on the grid of
 // its own largest magnitude (split_grid_f16x2, FP16 operands), so that the hi x hi products of a row and a column are
 // integers and their sum over K <= 256 is exact in FP32 whatever order and rounding the tensor core's accumulation
